@@ -76,6 +76,31 @@ def test_apply_stage(orc, n, pad, s):
         tb.apply_count_sketch(to_dense(A0, L.COL_MAJOR, NT.FP32_16), s, tier=tb.Tier.HALF, stage=True)
 
 
+@pytest.mark.parametrize("m,n,pad,s", [
+    (6007, 64, 0, 3),        # whole buckets of ~2000 rows, aligned narrow rows
+    (6007, 37, 0, 7),        # unaligned narrow rows
+    (1, 5, 3, 4),            # one row, empty buckets
+    (3001, 128, 0, 40),      # the widest FP32 narrow row; 16 chunks of 16-bit words
+    (3001, 129, 0, 40),      # unaligned, past it for FP32
+    (2049, 260, 4, 50),      # past it for 16-bit words
+    (1500, 1037, 0, 9),      # unaligned, three column panels
+    (60001, 8, 0, 50000)])   # more buckets than a CTA counts: the sorted path
+@pytest.mark.parametrize("numeric,tier", [(NT.FP32, tb.Tier.AUTO), (NT.FP32_16, tb.Tier.HALF),
+                                          (NT.FP32_16, tb.Tier.ACCURATE), (NT.FP32_BF16, tb.Tier.HALF)])
+def test_apply_row_shapes(orc, m, n, pad, s, numeric, tier):
+    """Row-major owner sums over every row shape, bit for bit the reference's
+    float path; sums of squares FP32 per bucket (<= ~2000 terms)."""
+    rng = np.random.default_rng(m + n)
+    A0 = (rng.standard_normal((m, n)) * np.logspace(-3, 3, n)).astype(np.float32)
+    A = to_dense(A0, L.ROW_MAJOR, numeric, pad=pad)
+    SA, fro2, colsq = tb.apply_count_sketch(A, s, tier=tier, with_colsq=True)
+    Ad = decoded(orc, A, tier).astype(np.float32)
+    assert np.array_equal(SA.view().cpu().numpy(), orc.countsketch_apply(Ad, s, row_major=True, acc="f32"))
+    sq = Ad.astype(np.float64) ** 2
+    np.testing.assert_allclose(colsq.cpu().numpy(), sq.sum(0), rtol=1e-5)
+    np.testing.assert_allclose(fro2.item(), sq.sum(), rtol=1e-5)
+
+
 def test_apply_reference_golden(orc):
     g = np.load(os.path.join(GOLD, "countsketch.npz"))
     A = to_dense(g["X"], L.COL_MAJOR)

@@ -797,7 +797,7 @@ tomos_status CsrPass::fro2(double* out, const double* d, cudaStream_t st) {
 template <Elem E>
 __global__ void cs_csr_kernel(const void* hi, const void* lo, const int32_t* row_ptrs,
                               const int32_t* col_idxs, int64_t n, int64_t s,
-                              const int32_t* offsets, const int32_t* perm, const int8_t* sign,
+                              const int32_t* offsets, const uint32_t* perm,
                               double* SA, int64_t ld_sa, double* fro_part) {
     extern __shared__ __align__(16) double racc[];
     __shared__ double smf[8];
@@ -815,10 +815,11 @@ __global__ void cs_csr_kernel(const void* hi, const void* lo, const int32_t* row
             int32_t rs = 0, re = 0;
             double sgl = 0.0;
             if (base + lane < o1) {
-                const int32_t r = perm[base + lane];
+                const uint32_t e = perm[base + lane];
+                const uint32_t r = e & ~kCsNeg;
                 rs = row_ptrs[r];
                 re = row_ptrs[r + 1];
-                sgl = (double)sign[r];
+                sgl = (e & kCsNeg) ? -1.0 : 1.0;
             }
             const int cnt = (o1 - base) < 32 ? (o1 - base) : 32;
             // the first 32 values of the next row, loaded ahead
@@ -1098,7 +1099,7 @@ tomos_status tomos_countsketch_apply_csr(const tomos_csr* A, int32_t tier, int64
                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,    \
                                                 (int)smem));                                    \
         cs_csr_kernel<EE><<<grid, nw * 32, smem, st>>>(A->values, lo, rp, ci, n, s, c.offsets,  \
-                                                       c.perm, c.sign, SA, ld_sa, c.fro_part); \
+                                                       c.perm, SA, ld_sa, c.fro_part);         \
     } while (0)
     switch (e) {
         case Elem::F32: TOMOS_CS_CSR(Elem::F32); break;

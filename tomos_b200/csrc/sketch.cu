@@ -7,15 +7,16 @@
 // bit-exact with the reference.  Unlike the reference (atomicAdd scatter,
 // order-dependent float sums), every bucket here is summed by one owner in
 // increasing row order, in FP64, so SA is deterministic:
-//   1. hash + bucket histogram       (integer atomics: order-free)
-//   2. exclusive scan of the counts  (one block)
-//   3. scatter row ids to buckets    (arbitrary order within a bucket)
-//   4. sort each bucket's row ids    (one warp per bucket)
-//   5. owner sums                    (row-major: a warp per bucket walks
-//                                     whole rows; column-major: a warp
-//                                     per (column, bucket) gathers down a
-//                                     contiguous column)
-// The sum of squares of the values read (||A||_F^2) falls out of step 5.
+//   1. per row segment: hash, and the segment's count of every bucket
+//   2. exclusive scans: over the segments of a bucket, then over buckets
+//   3. each segment places its rows in order: a stable counting sort, so a
+//      bucket lists its rows ascending (bit 31 of an entry: sign -1)
+//   4. owner sums        (row-major: threads own columns and walk the
+//                         bucket's rows; column-major: a warp per (column,
+//                         bucket) gathers down a contiguous column)
+// More buckets than a segment's shared counters hold (kCsMaxCounted) take a
+// global histogram, an unordered scatter and a sort of each bucket instead.
+// The sum of squares of the values read (||A||_F^2) falls out of step 4.
 #include <string>
 
 #include "common.cuh"
@@ -37,6 +38,103 @@ __global__ void cs_hash_kernel(int64_t m, int64_t s, uint64_t bseed, uint64_t ss
         bucket[i] = b;
         sign[i] = (splitmix64(gi ^ sseed) & 1ull) ? (int8_t)1 : (int8_t)-1;
         if (counts) atomicAdd(&counts[b], 1);
+    }
+}
+
+// Step 1: segment blockIdx.x hashes its rows (bucket[i], bit 31 set for
+// sign -1) and counts its buckets in shared memory into cnt[segment][bucket].
+__global__ void __launch_bounds__(256) cs_count_kernel(int64_t m, int64_t per, int32_t s, uint64_t bseed,
+                                                       uint64_t sseed, int64_t row0,
+                                                       uint32_t* __restrict__ bucket,
+                                                       int32_t* __restrict__ cnt) {
+    extern __shared__ int32_t hist[];
+    for (int j = threadIdx.x; j < s; j += blockDim.x) hist[j] = 0;
+    __syncthreads();
+    const int64_t r0 = (int64_t)blockIdx.x * per;
+    const int64_t r1 = r0 + per < m ? r0 + per : m;
+    for (int64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
+        const uint64_t gi = (uint64_t)(row0 + i);
+        const uint32_t b = (uint32_t)(splitmix64(gi ^ bseed) % (uint64_t)s);
+        bucket[i] = b | ((splitmix64(gi ^ sseed) & 1ull) ? 0u : kCsNeg);
+        atomicAdd(&hist[b], 1);
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < s; j += blockDim.x) cnt[(size_t)blockIdx.x * s + j] = hist[j];
+}
+
+// Step 2a: cnt[g][j] := rows of bucket j in the segments before g, tot[j] :=
+// all of them.  A CTA owns 32 buckets; its 32 warps split the segments.
+__global__ void __launch_bounds__(1024) cs_segment_scan_kernel(int32_t* __restrict__ cnt, int nseg, int32_t s,
+                                                               int32_t* __restrict__ tot) {
+    __shared__ int32_t part[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t j = (int64_t)blockIdx.x * 32 + lane;
+    const int per = (nseg + 31) / 32;
+    const int g0 = w * per < nseg ? w * per : nseg;
+    const int g1 = g0 + per < nseg ? g0 + per : nseg;
+    int32_t sum = 0;
+    if (j < s) {
+#pragma unroll 8
+        for (int g = g0; g < g1; ++g) sum += cnt[(size_t)g * s + j];
+    }
+    part[w][lane] = sum;
+    __syncthreads();
+    int32_t run = 0;
+    for (int h = 0; h < w; ++h) run += part[h][lane];
+    if (j >= s) return;
+    if (w == 31) tot[j] = run + sum;
+    int g = g0;
+    for (; g + 8 <= g1; g += 8) {
+        int32_t c[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) c[u] = cnt[(size_t)(g + u) * s + j];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            cnt[(size_t)(g + u) * s + j] = run;
+            run += c[u];
+        }
+    }
+    for (; g < g1; ++g) {
+        const int32_t c = cnt[(size_t)g * s + j];
+        cnt[(size_t)g * s + j] = run;
+        run += c;
+    }
+}
+
+// Step 3: segment blockIdx.x places its rows in increasing order.  Its
+// buckets' cursors sit in shared memory; one warp takes 32 rows a step, rows
+// of the same bucket ranked by lane (match_any), so the order is the rows'.
+__global__ void __launch_bounds__(256) cs_place_kernel(int64_t m, int64_t per, int32_t s,
+                                                       const uint32_t* __restrict__ bucket,
+                                                       const int32_t* __restrict__ cnt,
+                                                       const int32_t* __restrict__ offsets,
+                                                       uint32_t* __restrict__ perm) {
+    extern __shared__ int32_t cur[];
+    for (int j = threadIdx.x; j < s; j += blockDim.x) cur[j] = offsets[j] + cnt[(size_t)blockIdx.x * s + j];
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
+    const int64_t r0 = (int64_t)blockIdx.x * per;
+    const int64_t r1 = r0 + per < m ? r0 + per : m;
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t next = r0 + lane < r1 ? bucket[r0 + lane] : 0u;
+    for (int64_t i0 = r0; i0 < r1; i0 += 32) {
+        const uint32_t e = next;
+        const int64_t i = i0 + lane;
+        if (i + 32 < r1) next = bucket[i + 32];
+        const bool in = i < r1;
+        // lanes past the segment's end form a group of their own
+        const uint32_t b = in ? (e & ~kCsNeg) : 0xffffffffu;
+        const uint32_t same = __match_any_sync(0xffffffffu, b);
+        const int rank = __popc(same & below);
+        int32_t base = 0;
+        if (in) base = cur[b];
+        __syncwarp();
+        if (in) {
+            if (rank == 0) cur[b] = base + __popc(same);
+            perm[base + rank] = (uint32_t)i | (e & kCsNeg);
+        }
+        __syncwarp();
     }
 }
 
@@ -79,12 +177,12 @@ __global__ void cs_scan_kernel(const int32_t* __restrict__ counts, int64_t s,
 }
 
 __global__ void cs_scatter_kernel(int64_t m, const int32_t* __restrict__ bucket,
-                                  const int32_t* __restrict__ offsets, int32_t* __restrict__ cursor,
-                                  int32_t* __restrict__ perm) {
+                                  const int8_t* __restrict__ sign, const int32_t* __restrict__ offsets,
+                                  int32_t* __restrict__ cursor, uint32_t* __restrict__ perm) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int32_t b = bucket[i];
-        perm[offsets[b] + atomicAdd(&cursor[b], 1)] = (int32_t)i;
+        perm[offsets[b] + atomicAdd(&cursor[b], 1)] = (uint32_t)i | (sign[i] < 0 ? kCsNeg : 0u);
     }
 }
 
@@ -96,19 +194,19 @@ constexpr int kCsSortWarps = 4;
 
 __global__ void __launch_bounds__(kCsSortWarps * 32) cs_sort_kernel(int64_t s,
                                                                   const int32_t* __restrict__ offsets,
-                                                                  int32_t* __restrict__ perm) {
-    __shared__ int32_t buf[kCsSortWarps][kCsSortCap];
+                                                                  uint32_t* __restrict__ perm) {
+    __shared__ uint32_t buf[kCsSortWarps][kCsSortCap];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t b = (int64_t)blockIdx.x * kCsSortWarps + w;
     if (b >= s) return;
     const int32_t o0 = offsets[b], len = offsets[b + 1] - o0;
-    int32_t* seg = perm + o0;
+    uint32_t* seg = perm + o0;
     if (len > kCsSortCap) {
         for (int32_t pass = 0; pass < len; ++pass) {
             const int32_t start = pass & 1;
             for (int32_t k = start + 2 * lane; k + 1 < len; k += 64) {
-                int32_t x = seg[k], y = seg[k + 1];
-                if (x > y) {
+                const uint32_t x = seg[k], y = seg[k + 1];
+                if ((x & ~kCsNeg) > (y & ~kCsNeg)) {
                     seg[k] = y;
                     seg[k + 1] = x;
                 }
@@ -119,7 +217,7 @@ __global__ void __launch_bounds__(kCsSortWarps * 32) cs_sort_kernel(int64_t s,
     }
     int N = 1;
     while (N < len) N <<= 1;
-    int32_t* v = buf[w];
+    uint32_t* v = buf[w];
     for (int e = lane; e < N; e += 32) v[e] = e < len ? seg[e] : 0x7fffffff;
     __syncwarp();
     for (int k = 2; k <= N; k <<= 1) {
@@ -128,8 +226,8 @@ __global__ void __launch_bounds__(kCsSortWarps * 32) cs_sort_kernel(int64_t s,
             for (int i = lane; i < N; i += 32) {
                 const int p = i ^ j;
                 if (p > i) {
-                    const int32_t x = v[i], y = v[p];
-                    if ((x > y) == ((i & k) == 0)) {
+                    const uint32_t x = v[i], y = v[p];
+                    if (((x & ~kCsNeg) > (y & ~kCsNeg)) == ((i & k) == 0)) {
                         v[i] = y;
                         v[p] = x;
                     }
@@ -141,140 +239,177 @@ __global__ void __launch_bounds__(kCsSortWarps * 32) cs_sort_kernel(int64_t s,
     for (int e = lane; e < len; e += 32) seg[e] = v[e];
 }
 
-// Row-major owner sums: warp per bucket, lanes over columns of a panel of
-// 32 * KC columns (grid.y walks the panels).  Sums in FP32 with the rows
-// of a bucket in increasing order: bit for bit the reference's
-// countsketch_apply_impl<float> (countsketch_kernels.cpp:70-83).  The
-// column sums of squares are FP32 per bucket and FP64 across buckets.
-template <Elem E, int KC>
-__global__ void __launch_bounds__(256) cs_rows_kernel(const void* hi, const void* lo, int64_t n,
-                                                      int64_t ld, int64_t s,
-                                                      const int32_t* __restrict__ offsets,
-                                                      const int32_t* __restrict__ perm,
-                                                      const int8_t* __restrict__ sign,
-                                                      double* __restrict__ SA, int64_t ld_sa,
-                                                      double* __restrict__ fro_part,
-                                                      double* __restrict__ col_part) {
-    __shared__ double smf[8];
-    __shared__ float smc[8][32 * KC];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t b = (int64_t)blockIdx.x * 8 + w;
-    const int64_t c0 = (int64_t)blockIdx.y * 32 * KC;
-    float acc[KC], csq[KC];
-#pragma unroll
-    for (int k = 0; k < KC; ++k) acc[k] = csq[k] = 0.0f;
-    double f2 = 0.0;
-    if (b < s) {
-        const int32_t o0 = offsets[b], o1 = offsets[b + 1];
-        for (int32_t q = o0; q < o1; ++q) {
-            const int32_t r = perm[q];
-            const float sg = (float)sign[r];
-            const size_t base = (size_t)r * ld;
-#pragma unroll
-            for (int k = 0; k < KC; ++k) {
-                const int64_t j = c0 + k * 32 + lane;
-                if (j < n) {
-                    const float a = load_elem<E>(hi, lo, base + j);
-                    acc[k] = fmaf(sg, a, acc[k]);
-                    csq[k] = fmaf(a, a, csq[k]);
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < KC; ++k) {
-            const int64_t j = c0 + k * 32 + lane;
-            if (j < n) SA[(size_t)j * ld_sa + b] = (double)acc[k];
-            f2 += (double)csq[k];
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < KC; ++k) smc[w][k * 32 + lane] = csq[k];
-    f2 = warp_sum(f2);
-    if (lane == 0) smf[w] = f2;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) t += smf[k];
-        fro_part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
-    }
-    if (col_part) {
-        for (int e = threadIdx.x; e < 32 * KC; e += blockDim.x) {
-            const int64_t j = c0 + e;
-            if (j >= n) continue;
-            double t = 0.0;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) t += (double)smc[k][e];
-            col_part[(size_t)blockIdx.x * n + j] = t;
-        }
-    }
-}
-
-// colsq[j] = sum over nparts rows of part[r][j] (fixed order).
-__global__ void cs_col_reduce_kernel(const double* __restrict__ part, int64_t nparts, int64_t n,
-                                     double* __restrict__ colsq) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    double t = 0.0;
-    for (int64_t r = 0; r < nparts; ++r) t += part[(size_t)r * n + j];
-    colsq[j] = t;
-}
-
-// Row-major owner sums, gathered through shared memory by asynchronous
-// copies.
+// Row-major owner sums.  Sums are FP32 with the rows of a bucket in
+// increasing order, bit for bit the reference's countsketch_apply_impl<float>
+// (countsketch_kernels.cpp:70-83); every bucket writes its row of SA and its
+// FP32 column sums of squares (col_part, s x n), which cs_colsq_chunk_kernel
+// reduces in bucket order.
 //
-// One CTA per SM of kCsWarps warps; each warp takes (bucket, panel) work
-// items from a global counter (buckets hold ~m/s rows of uneven count, so
-// items are handed out dynamically) and walks the bucket's rows in
-// increasing order.  Lane l owns the 16-byte chunks l, l+32, ... (KCH of
-// them) of the panel: it copies them of kCsStages batches of RB rows ahead
-// into its slots of the warp's ring (cp.async, one commit group a batch)
-// and sums a batch once its own group has landed -- no lane reads another
-// lane's bytes, so no barrier is needed, and the rows being random, these
-// per-thread 16-byte copies issue far faster than one bulk copy per row.
-// Sums are FP32 in increasing row order (bit for bit the reference's
-// countsketch_apply_impl<float>, countsketch_kernels.cpp:70-83; the packed
-// FP32x2 FMAs round each element as fmaf does).  Each item writes its
-// bucket's row of SA and its FP32 column sums of squares to col_part
-// (s x n), which cs_colsq_chunk_kernel then reduces in bucket order, so the
-// results do not depend on which warp took which item.
-//
-// STAGE (FP32_16 HALF tier only): the fp32_16_half_only words of every
-// chunk read are also written to `plane` (row pitch ld_plane halves) -- the
-// fixed fp16 copy of the wh plane the LSQR HALF-tier iterations read -- so
-// a solve that follows the sketch needs no staging pass of its own.
-constexpr int kCsWarps = 12;
-constexpr int kCsStages = 4;
-constexpr int kCsStageBytes = 4096;  // per warp and stage
-constexpr int kCsPanelCols = 512;    // columns per work item
-constexpr int kCsList = 512;         // a bucket's row ids kept in shared memory
-
+// STAGE (FP32_16 HALF tier only): the fp32_16_half_only words of every chunk
+// read are also written to `plane` (row pitch ld_plane halves) -- the fixed
+// fp16 copy of the wh plane the LSQR HALF-tier iterations read -- so a solve
+// that follows the sketch needs no staging pass of its own.
 struct CsRowsArgs {
     const void* hi;
     const void* lo;
     int64_t n, ld, s;
-    int panels;
     const int32_t* offsets;
-    const int32_t* perm;
-    const int8_t* sign;
+    const uint32_t* perm;
     double* SA;
     int64_t ld_sa;
     float* col_part;  // s x n
     uint16_t* plane;
     int64_t ld_plane;
-    int* counter;     // zero at launch
 };
 
 template <Elem E>
-struct CsRowsShape {
+struct CsElem {
     static constexpr int VEC = ChunkElems<E>::value;
     static constexpr int ESZ = (E == Elem::F32) ? 4 : 2;
     static constexpr int PLANES = (E == Elem::A16 || E == Elem::AB16 || E == Elem::AB16R) ? 2 : 1;
-    static constexpr int KCH = kCsPanelCols / (32 * VEC);  // chunks per lane
-    static constexpr int PWB = kCsPanelCols * ESZ;         // panel bytes per row and plane
-    static constexpr int RB = kCsStageBytes / (PWB * PLANES);  // rows per batch
-    static_assert(RB >= 1, "a row's panel fits a stage");
 };
+
+// One 16-byte chunk as float pairs (STAGE: its fixed words to `stage`).
+template <Elem E, bool STAGE>
+__device__ __forceinline__ void cs_chunk_values(uint4& h, const uint4& l, uint16_t* stage,
+                                                float2 (&v)[CsElem<E>::VEC / 2]) {
+    if constexpr (E == Elem::H16) {
+        fix_half_chunk(h);
+        if constexpr (STAGE) *reinterpret_cast<uint4*>(stage) = h;
+        v[0] = h2f2(h.x);
+        v[1] = h2f2(h.y);
+        v[2] = h2f2(h.z);
+        v[3] = h2f2(h.w);
+    } else {
+        float f[CsElem<E>::VEC];
+        ChunkDecoder<E>::decode(h, l, f);
+#pragma unroll
+        for (int e = 0; e < CsElem<E>::VEC / 2; ++e) v[e] = make_float2(f[2 * e], f[2 * e + 1]);
+    }
+}
+
+// Rows 16-byte aligned: a CTA takes one bucket and blockDim.x chunks of its
+// rows, a thread one chunk.  Bound by HBM latency: a thread keeps kCsDepth
+// rows' loads in flight (16 bytes each), the row ids of the next batch
+// loaded before the current one is summed.  Chunks past column n are not
+// touched; the elements of the last chunk past n are summed and dropped.
+// 1e6 x 1000 FP32_16 with the staged plane (2 GB read, 2 GB written): 889 us
+// (4.5 TB/s) against 937 us for a shared-memory ring per warp.
+constexpr int kCsDepth = 8;
+constexpr int kCsThreads = 128;  // chunks (threads) a CTA at most
+
+template <Elem E, bool STAGE>
+__global__ void __launch_bounds__(kCsThreads) cs_rows_kernel(CsRowsArgs a) {
+    static_assert(!STAGE || E == Elem::H16, "staging writes FP32_16 wh planes");
+    constexpr int VEC = CsElem<E>::VEC, HV = VEC / 2, ESZ = CsElem<E>::ESZ, PLANES = CsElem<E>::PLANES;
+    constexpr int D = PLANES == 2 ? kCsDepth / 2 : kCsDepth;
+    const int64_t b = blockIdx.x;
+    const int64_t c = (int64_t)blockIdx.y * blockDim.x + threadIdx.x;
+    if (c * VEC >= a.n) return;
+    const int32_t o0 = a.offsets[b], len = a.offsets[b + 1] - o0;
+    const uint32_t* ids = a.perm + o0;
+    const uint8_t* hp = static_cast<const uint8_t*>(a.hi) + c * 16;
+    const uint8_t* lp = static_cast<const uint8_t*>(a.lo) + c * 16;
+    const size_t pitch = (size_t)a.ld * ESZ;
+    float2 acc[HV], csq[HV];
+#pragma unroll
+    for (int e = 0; e < HV; ++e) acc[e] = csq[e] = make_float2(0.0f, 0.0f);
+    uint32_t nid[D];
+#pragma unroll
+    for (int u = 0; u < D; ++u) nid[u] = u < len ? __ldg(ids + u) : 0u;
+    for (int32_t q = 0; q < len; q += D) {
+        uint32_t id[D];
+        uint4 h[D], l[PLANES == 2 ? D : 1];
+#pragma unroll
+        for (int u = 0; u < D; ++u) {
+            id[u] = nid[u];
+            if (q + u < len) {
+                const size_t off = (size_t)(id[u] & ~kCsNeg) * pitch;
+                h[u] = __ldcs(reinterpret_cast<const uint4*>(hp + off));
+                if constexpr (PLANES == 2) l[u] = __ldcs(reinterpret_cast<const uint4*>(lp + off));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < D; ++u) nid[u] = q + D + u < len ? __ldg(ids + q + D + u) : 0u;
+#pragma unroll
+        for (int u = 0; u < D; ++u) {
+            if (q + u < len) {
+                const float sg = (id[u] & kCsNeg) ? -1.0f : 1.0f;
+                const float2 sg2 = make_float2(sg, sg);
+                uint16_t* stage = nullptr;
+                if constexpr (STAGE) stage = a.plane + (size_t)(id[u] & ~kCsNeg) * a.ld_plane + c * VEC;
+                float2 v[HV];
+                cs_chunk_values<E, STAGE>(h[u], l[PLANES == 2 ? u : 0], stage, v);
+#pragma unroll
+                for (int e = 0; e < HV; ++e) {
+                    acc[e] = __ffma2_rn(v[e], sg2, acc[e]);
+                    csq[e] = __ffma2_rn(v[e], v[e], csq[e]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+        const int64_t j = c * VEC + e;
+        if (j >= a.n) continue;
+        a.SA[(size_t)j * a.ld_sa + b] = (double)((e & 1) ? acc[e / 2].y : acc[e / 2].x);
+        a.col_part[(size_t)b * a.n + j] = (e & 1) ? csq[e / 2].y : csq[e / 2].x;
+    }
+}
+
+// Rows at any alignment: as cs_rows_kernel, a thread owning kCsCols columns
+// blockDim.x apart and reading them one element at a time (coalesced).
+constexpr int kCsCols = 4;
+
+template <Elem E>
+__global__ void __launch_bounds__(kCsThreads) cs_rows_any_kernel(CsRowsArgs a) {
+    constexpr int D = CsElem<E>::PLANES == 2 ? kCsDepth / 2 : kCsDepth;
+    const int64_t b = blockIdx.x;
+    const int64_t j0 = (int64_t)blockIdx.y * blockDim.x * kCsCols + threadIdx.x;
+    if (j0 >= a.n) return;
+    const int32_t o0 = a.offsets[b], len = a.offsets[b + 1] - o0;
+    const uint32_t* ids = a.perm + o0;
+    float acc[kCsCols], csq[kCsCols];
+#pragma unroll
+    for (int k = 0; k < kCsCols; ++k) acc[k] = csq[k] = 0.0f;
+    uint32_t nid[D];
+#pragma unroll
+    for (int u = 0; u < D; ++u) nid[u] = u < len ? __ldg(ids + u) : 0u;
+    for (int32_t q = 0; q < len; q += D) {
+        uint32_t id[D];
+        float v[D][kCsCols];
+#pragma unroll
+        for (int u = 0; u < D; ++u) {
+            id[u] = nid[u];
+            const size_t base = (size_t)(id[u] & ~kCsNeg) * a.ld;
+#pragma unroll
+            for (int k = 0; k < kCsCols; ++k) {
+                const int64_t j = j0 + (int64_t)k * blockDim.x;
+                v[u][k] = (q + u < len && j < a.n) ? load_elem<E>(a.hi, a.lo, base + j) : 0.0f;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < D; ++u) nid[u] = q + D + u < len ? __ldg(ids + q + D + u) : 0u;
+#pragma unroll
+        for (int u = 0; u < D; ++u) {
+            if (q + u < len) {
+                const float sg = (id[u] & kCsNeg) ? -1.0f : 1.0f;
+#pragma unroll
+                for (int k = 0; k < kCsCols; ++k) {
+                    acc[k] = fmaf(sg, v[u][k], acc[k]);
+                    csq[k] = fmaf(v[u][k], v[u][k], csq[k]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kCsCols; ++k) {
+        const int64_t j = j0 + (int64_t)k * blockDim.x;
+        if (j >= a.n) continue;
+        a.SA[(size_t)j * a.ld_sa + b] = (double)acc[k];
+        a.col_part[(size_t)b * a.n + j] = csq[k];
+    }
+}
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
@@ -285,177 +420,114 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <Elem E, bool STAGE>
-__global__ void __launch_bounds__(kCsWarps * 32, 1) cs_rows_tma_kernel(CsRowsArgs a) {
-    using S = CsRowsShape<E>;
-    constexpr int VEC = S::VEC, HV = VEC / 2, KCH = S::KCH, RB = S::RB, PLANES = S::PLANES;
-    constexpr int ESZ = S::ESZ, PWB = S::PWB;
-    static_assert(!STAGE || E == Elem::H16, "staging writes FP32_16 wh planes");
-    extern __shared__ __align__(128) uint8_t smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint8_t* ring = smem + (size_t)warp * kCsStages * kCsStageBytes;
-    // the bucket's first kCsList row ids, bit 31 set for sign -1
-    uint32_t* list = reinterpret_cast<uint32_t*>(smem + (size_t)kCsWarps * kCsStages * kCsStageBytes) +
-                     (size_t)warp * kCsList;
-    const int64_t n = a.n, s = a.s;
-    const int64_t nch = (n + VEC - 1) / VEC;
-    const int64_t total = s * a.panels;
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(a.counter, 1);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= total) break;
-        const int64_t b = item % s;
-        const int64_t c0 = (int64_t)(item / s) * kCsPanelCols;
-        const int32_t o0 = a.offsets[b], len = a.offsets[b + 1] - o0;
-        const int nbat = (len + RB - 1) / RB;
-        // Row ids and signs of the bucket, gathered once (eight in flight
-        // a lane) instead of two dependent loads per row.
-        __syncwarp();  // the previous item's readers of the list are done
-        {
-            const int lim = len < kCsList ? len : kCsList;
-            for (int e0 = 0; e0 < lim; e0 += 8 * 32) {
-                int32_t rr[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int e = e0 + q * 32 + lane;
-                    rr[q] = e < lim ? a.perm[o0 + e] : 0;
+// Rows of at most kCsNarrowChunks chunks, of which there are few buckets
+// (s ~ 4 n) of many rows: a thread per chunk would leave the memory system
+// with a few KB in flight.  A CTA takes a whole bucket: all threads copy
+// batches of kCsNarrowRows rows into a three-stage ring, and thread j then
+// adds column j of the batch, row by row in order.  VECR: rows 16-byte
+// aligned, copied in chunks; otherwise element by element.  1e6 x 64 bf16
+// (256 buckets of ~3900 rows): 102 us, against 2.05 ms for a warp a bucket.
+constexpr int kCsNarrowChunks = 32;
+constexpr int kCsNarrowRows = 128;
+constexpr int kCsNarrowBytes = 16 * 1024;  // a stage at most
+constexpr int kCsNarrowStages = 3;
+
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+template <Elem E, bool STAGE, bool VECR>
+__global__ void __launch_bounds__(256) cs_rows_narrow_kernel(CsRowsArgs a, int rows) {
+    static_assert(!STAGE || (E == Elem::H16 && VECR), "staging writes FP32_16 wh planes");
+    constexpr int VEC = CsElem<E>::VEC, ESZ = CsElem<E>::ESZ, PLANES = CsElem<E>::PLANES;
+    constexpr int UNIT = VECR ? 16 : ESZ;  // bytes a copy moves
+    extern __shared__ __align__(16) uint8_t ring[];
+    __shared__ uint32_t sid[kCsNarrowStages][kCsNarrowRows];
+    const int t = threadIdx.x, T = blockDim.x;
+    const int nch = VECR ? (int)((a.n + VEC - 1) / VEC) : (int)a.n;  // copies a row and plane
+    const int rb = nch * UNIT;                     // bytes of a row and plane in the ring
+    const int plane_bytes = rows * rb;
+    const int64_t b = blockIdx.x;
+    const int32_t o0 = a.offsets[b], len = a.offsets[b + 1] - o0;
+    const int nbat = (len + rows - 1) / rows;
+    const size_t pitch = (size_t)a.ld * ESZ;
+    auto issue = [&](int q) {
+        if (q < nbat) {
+            uint8_t* st = ring + (size_t)(q % kCsNarrowStages) * plane_bytes * PLANES;
+            const int nr = len - q * rows < rows ? len - q * rows : rows;
+#pragma unroll 8
+            for (int e = t; e < nr * nch; e += T) {
+                const int u = e / nch, c = e - u * nch;
+                const uint32_t id = __ldg(a.perm + o0 + q * rows + u);
+                const size_t off = (size_t)(id & ~kCsNeg) * pitch + (size_t)c * UNIT;
+                const uint8_t* src = static_cast<const uint8_t*>(a.hi) + off;
+                const uint8_t* srl = static_cast<const uint8_t*>(a.lo) + off;
+                uint8_t* dst = st + u * rb + c * UNIT;
+                if constexpr (VECR) {
+                    cp_async16(dst, src);
+                    if constexpr (PLANES == 2) cp_async16(dst + plane_bytes, srl);
+                } else if constexpr (UNIT == 4) {
+                    cp_async4(dst, src);
+                } else {
+                    *reinterpret_cast<uint16_t*>(dst) = __ldg(reinterpret_cast<const uint16_t*>(src));
+                    if constexpr (PLANES == 2)
+                        *reinterpret_cast<uint16_t*>(dst + plane_bytes) = __ldg(reinterpret_cast<const uint16_t*>(srl));
                 }
-                int8_t sq[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) sq[q] = (e0 + q * 32 + lane) < lim ? a.sign[rr[q]] : 1;
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int e = e0 + q * 32 + lane;
-                    if (e < lim) list[e] = (uint32_t)rr[q] | (sq[q] < 0 ? 0x80000000u : 0u);
-                }
+                if (c == 0) sid[q % kCsNarrowStages][u] = id;
             }
-            __syncwarp();
         }
-        // row id and sign of the bucket's e-th row
-        auto row_of = [&](int e, int32_t& r, float& sg) {
-            if (e < kCsList) {
-                const uint32_t v = list[e];
-                r = (int32_t)(v & 0x7fffffffu);
-                sg = (v >> 31) ? -1.0f : 1.0f;
-            } else {
-                r = a.perm[o0 + e];
-                sg = (float)a.sign[r];
-            }
-        };
-        bool live[KCH];
-        int zero_from[KCH];  // elements of the chunk at or past column n
+        cp_async_commit();
+    };
+    float acc = 0.0f, csq = 0.0f;
 #pragma unroll
-        for (int k = 0; k < KCH; ++k) {
-            const int64_t c = c0 / VEC + k * 32 + lane;
-            live[k] = c < nch;
-            zero_from[k] = !live[k] ? 0 : ((c == nch - 1 && n % VEC != 0) ? (int)(n - c * VEC) : VEC);
+    for (int q = 0; q < kCsNarrowStages - 1; ++q) issue(q);
+    for (int q = 0; q < nbat; ++q) {
+        cp_async_wait<kCsNarrowStages - 2>();
+        __syncthreads();  // batch q landed; the stage of batch q - 1 is free
+        issue(q + kCsNarrowStages - 1);
+        const int sl = q % kCsNarrowStages;
+        uint8_t* st = ring + (size_t)sl * plane_bytes * PLANES;
+        const int nr = len - q * rows < rows ? len - q * rows : rows;
+        if constexpr (E == Elem::H16 && VECR) {
+            // the fixed fp16 words in place (and to the plane)
+            for (int e = t; e < nr * nch; e += T) {
+                const int u = e / nch, c = e - u * nch;
+                uint4* w = reinterpret_cast<uint4*>(st + u * rb + c * 16);
+                uint4 h = *w;
+                fix_half_chunk(h);
+                *w = h;
+                if constexpr (STAGE)
+                    *reinterpret_cast<uint4*>(a.plane + (size_t)(sid[sl][u] & ~kCsNeg) * a.ld_plane + c * VEC) = h;
+            }
+            __syncthreads();
         }
-        // this lane's chunks of batch t into ring stage t % kCsStages (one
-        // commit group, empty past the bucket's end)
-        auto issue = [&](int t) {
-            if (t < nbat) {
-                uint8_t* st = ring + (size_t)(t % kCsStages) * kCsStageBytes;
-                const int rows = (len - t * RB) < RB ? (len - t * RB) : RB;
-                for (int u = 0; u < rows; ++u) {
-                    int32_t r;
-                    float sg;
-                    row_of(t * RB + u, r, sg);
-                    const uint8_t* src = static_cast<const uint8_t*>(a.hi) + ((size_t)r * a.ld + c0) * ESZ;
-                    const uint8_t* srl = static_cast<const uint8_t*>(a.lo) + ((size_t)r * a.ld + c0) * ESZ;
-#pragma unroll
-                    for (int k = 0; k < KCH; ++k) {
-                        if (!live[k]) continue;
-                        const int coff = (k * 32 + lane) * 16;
-                        cp_async16(st + (size_t)(u * PLANES) * PWB + coff, src + coff);
-                        if (PLANES == 2) cp_async16(st + (size_t)(u * PLANES + 1) * PWB + coff, srl + coff);
-                    }
+        if (t < a.n) {
+            constexpr Elem V = E == Elem::H16 && VECR ? Elem::F16 : E;  // what the ring holds
+#pragma unroll 8
+            for (int u = 0; u < nr; ++u) {
+                const float sg = (sid[sl][u] & kCsNeg) ? -1.0f : 1.0f;
+                const uint8_t* hw = st + u * rb + t * ESZ;
+                float v;
+                if constexpr (V == Elem::F32) v = *reinterpret_cast<const float*>(hw);
+                else if constexpr (V == Elem::F16) v = half_bits_to_float(*reinterpret_cast<const uint16_t*>(hw));
+                else if constexpr (V == Elem::H16) v = half_bits_to_float(half_only_bits(*reinterpret_cast<const uint16_t*>(hw)));
+                else if constexpr (V == Elem::B16) v = u2f((uint32_t)*reinterpret_cast<const uint16_t*>(hw) << 16);
+                else {
+                    const uint32_t wh = *reinterpret_cast<const uint16_t*>(hw);
+                    const uint32_t wr = *reinterpret_cast<const uint16_t*>(hw + plane_bytes);
+                    v = V == Elem::A16 ? decode_fp32_16_exact_nb(wh, wr)
+                                       : decode_fp32_bf16_exact(wh, wr, V == Elem::AB16R);
                 }
-            }
-            cp_async_commit();
-        };
-#pragma unroll
-        for (int t = 0; t < kCsStages; ++t) issue(t);
-        float2 acc[KCH][HV], csq[KCH][HV];
-#pragma unroll
-        for (int k = 0; k < KCH; ++k)
-#pragma unroll
-            for (int e = 0; e < HV; ++e) acc[k][e] = csq[k][e] = make_float2(0.0f, 0.0f);
-        for (int t = 0; t < nbat; ++t) {
-            cp_async_wait<kCsStages - 1>();  // this lane's copies of batch t landed
-            const uint8_t* st = ring + (size_t)(t % kCsStages) * kCsStageBytes;
-            const int rows = (len - t * RB) < RB ? (len - t * RB) : RB;
-            for (int u = 0; u < rows; ++u) {
-                int32_t r;
-                float sgv;
-                row_of(t * RB + u, r, sgv);
-                const float2 sg2 = make_float2(sgv, sgv);
-                const uint8_t* hrow = st + (size_t)(u * PLANES) * PWB;
-#pragma unroll
-                for (int k = 0; k < KCH; ++k) {
-                    const int coff = (k * 32 + lane) * 16;
-                    uint4 h = make_uint4(0, 0, 0, 0), l = make_uint4(0, 0, 0, 0);
-                    if (live[k]) {
-                        h = *reinterpret_cast<const uint4*>(hrow + coff);
-                        if (PLANES == 2) l = *reinterpret_cast<const uint4*>(hrow + PWB + coff);
-                    }
-                    float2 v[HV];
-                    if constexpr (E == Elem::H16) {
-                        fix_half_chunk(h);
-                        if constexpr (STAGE) {
-                            if (live[k])
-                                *reinterpret_cast<uint4*>(a.plane + (size_t)r * a.ld_plane + c0 +
-                                                          (k * 32 + lane) * VEC) = h;
-                        }
-                        v[0] = h2f2(h.x);
-                        v[1] = h2f2(h.y);
-                        v[2] = h2f2(h.z);
-                        v[3] = h2f2(h.w);
-                    } else {
-                        float f[VEC];
-                        ChunkDecoder<E>::decode(h, l, f);
-#pragma unroll
-                        for (int e = 0; e < HV; ++e) v[e] = make_float2(f[2 * e], f[2 * e + 1]);
-                    }
-                    // chunks past the row's end and columns past n (the
-                    // last chunk's padding) add nothing (a zero word need
-                    // not decode to 0)
-                    if (zero_from[k] < VEC) {
-#pragma unroll
-                        for (int e = 0; e < HV; ++e) {
-                            if (2 * e >= zero_from[k]) v[e].x = 0.0f;
-                            if (2 * e + 1 >= zero_from[k]) v[e].y = 0.0f;
-                        }
-                    }
-#pragma unroll
-                    for (int e = 0; e < HV; ++e) {
-                        acc[k][e] = __ffma2_rn(v[e], sg2, acc[k][e]);
-                        csq[k][e] = __ffma2_rn(v[e], v[e], csq[k][e]);
-                    }
-                }
-            }
-            // this lane read its slots of stage t: refill them
-            issue(t + kCsStages);
-        }
-        cp_async_wait<0>();  // the trailing (empty) groups
-#pragma unroll
-        for (int k = 0; k < KCH; ++k) {
-            const int64_t cb = c0 + (int64_t)(k * 32 + lane) * VEC;
-#pragma unroll
-            for (int e = 0; e < VEC; ++e) {
-                if (!live[k] || cb + e >= n) continue;
-                const float va = (e & 1) ? acc[k][e / 2].y : acc[k][e / 2].x;
-                const float vq = (e & 1) ? csq[k][e / 2].y : csq[k][e / 2].x;
-                a.SA[(size_t)(cb + e) * a.ld_sa + b] = (double)va;
-                a.col_part[(size_t)b * n + cb + e] = vq;
+                acc = fmaf(sg, v, acc);
+                csq = fmaf(v, v, csq);
             }
         }
     }
-}
-
-template <Elem E>
-inline size_t cs_rows_tma_smem() {
-    return (size_t)kCsWarps * (kCsStages * kCsStageBytes + kCsList * sizeof(uint32_t));
+    cp_async_wait<0>();
+    if (t < a.n) {
+        a.SA[(size_t)t * a.ld_sa + b] = (double)acc;
+        a.col_part[(size_t)b * a.n + t] = csq;
+    }
 }
 
 // Column sums of squares from the per-bucket FP32 partials: chunk q of the
@@ -488,8 +560,7 @@ template <Elem E>
 __global__ void __launch_bounds__(256) cs_cols_kernel(const void* hi, const void* lo, int64_t n,
                                                       int64_t ld, int64_t s,
                                                       const int32_t* __restrict__ offsets,
-                                                      const int32_t* __restrict__ perm,
-                                                      const int8_t* __restrict__ sign,
+                                                      const uint32_t* __restrict__ perm,
                                                       double* __restrict__ SA, int64_t ld_sa,
                                                       double* __restrict__ fro_part,
                                                       double* __restrict__ colsq) {
@@ -502,9 +573,9 @@ __global__ void __launch_bounds__(256) cs_cols_kernel(const void* hi, const void
         const int32_t o0 = offsets[b], o1 = offsets[b + 1];
         double acc = 0.0;
         for (int32_t q = o0 + lane; q < o1; q += 32) {
-            const int32_t r = perm[q];
-            const double a = (double)load_elem<E>(hi, lo, cbase + r);
-            acc += (double)sign[r] * a;
+            const uint32_t r = perm[q];
+            const double a = (double)load_elem<E>(hi, lo, cbase + (r & ~kCsNeg));
+            acc += (r & kCsNeg) ? -a : a;
             f2 += a * a;
         }
         acc = warp_sum(acc);
@@ -550,10 +621,11 @@ CsScratch cs_layout(void* base, int64_t m, int64_t s, int64_t fro_parts, int64_t
     };
     c.bucket = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * (m > 0 ? m : 1)));
     c.sign = reinterpret_cast<int8_t*>(take(m > 0 ? m : 1));
+    c.cnt = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * (size_t)cs_segments(m, s) * s));
     c.counts = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * (s + 1)));
     c.offsets = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * (s + 1)));
     c.cursor = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * (s + 1)));
-    c.perm = reinterpret_cast<int32_t*>(take(sizeof(int32_t) * (m > 0 ? m : 1)));
+    c.perm = reinterpret_cast<uint32_t*>(take(sizeof(int32_t) * (m > 0 ? m : 1)));
     c.fro_part = reinterpret_cast<double*>(take(sizeof(double) * (fro_parts > 0 ? fro_parts : 1)));
     c.col_part = reinterpret_cast<double*>(take(sizeof(double) * (col_parts > 0 ? col_parts : 1)));
     c.bytes = off;
@@ -587,9 +659,46 @@ static bool cs_grid(int64_t m, int* g) {
     return true;
 }
 
-// Steps 1-4 (shared by the dense and CSR owner sums).
+// Row segments of the counting sort: enough single-warp placements to fill
+// the GPU (eight a SM), at least 256 rows each, and a count matrix (segments
+// x s) of at most 4 M words, which stays in L2.  0: s exceeds the shared
+// counters of a CTA.
+int64_t cs_segments(int64_t m, int64_t s) {
+    if (s > kCsMaxCounted || m <= 0) return 0;
+    int64_t g = (int64_t)sm_count() * 8;
+    if (g > (m + 255) / 256) g = (m + 255) / 256;
+    if (g > ((int64_t)4 << 20) / s) g = ((int64_t)4 << 20) / s;
+    return g < 1 ? 1 : g;
+}
+
+// Steps 1-3 (shared by the dense and CSR owner sums): offsets and perm.
+// The stable counting sort replaces a global histogram, an unordered scatter
+// and a sort of each bucket, whose cost grows with the square of a bucket's
+// length past kCsSortCap rows: 58 ms of it at 1e6 rows in 256 buckets, now
+// 32 us for all three kernels; 116 us -> 40 us at 1e6 rows in 4000 buckets.
 tomos_status cs_bucketize(int64_t m, int64_t s, uint64_t bseed, uint64_t sseed, const CsScratch& c,
                           cudaStream_t st, int64_t row0) {
+    const int64_t nseg = cs_segments(m, s);
+    if (nseg > 0) {
+        const int64_t per = (m + nseg - 1) / nseg;
+        const size_t smem = sizeof(int32_t) * (size_t)s;
+        if (smem > 48 * 1024) {
+            TOMOS_CUDA_TRY(cudaFuncSetAttribute(cs_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            TOMOS_CUDA_TRY(cudaFuncSetAttribute(cs_place_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        }
+        cs_count_kernel<<<(unsigned)nseg, 256, smem, st>>>(m, per, (int32_t)s, bseed, sseed, row0,
+                                                           reinterpret_cast<uint32_t*>(c.bucket), c.cnt);
+        TOMOS_LAUNCH_CHECK("cs_count_kernel");
+        cs_segment_scan_kernel<<<(unsigned)((s + 31) / 32), 1024, 0, st>>>(c.cnt, (int)nseg, (int32_t)s, c.counts);
+        TOMOS_LAUNCH_CHECK("cs_segment_scan_kernel");
+        cs_scan_kernel<<<1, 1024, 0, st>>>(c.counts, s, c.offsets);
+        TOMOS_LAUNCH_CHECK("cs_scan_kernel");
+        cs_place_kernel<<<(unsigned)nseg, 256, smem, st>>>(m, per, (int32_t)s,
+                                                           reinterpret_cast<const uint32_t*>(c.bucket), c.cnt,
+                                                           c.offsets, c.perm);
+        TOMOS_LAUNCH_CHECK("cs_place_kernel");
+        return TOMOS_OK;
+    }
     int g;
     cs_grid(m, &g);
     TOMOS_CUDA_TRY(cudaMemsetAsync(c.counts, 0, sizeof(int32_t) * (s + 1), st));
@@ -598,7 +707,7 @@ tomos_status cs_bucketize(int64_t m, int64_t s, uint64_t bseed, uint64_t sseed, 
     TOMOS_LAUNCH_CHECK("cs_hash_kernel");
     cs_scan_kernel<<<1, 1024, 0, st>>>(c.counts, s, c.offsets);
     TOMOS_LAUNCH_CHECK("cs_scan_kernel");
-    cs_scatter_kernel<<<g, 256, 0, st>>>(m, c.bucket, c.offsets, c.cursor, c.perm);
+    cs_scatter_kernel<<<g, 256, 0, st>>>(m, c.bucket, c.sign, c.offsets, c.cursor, c.perm);
     TOMOS_LAUNCH_CHECK("cs_scatter_kernel");
     cs_sort_kernel<<<(unsigned)((s + kCsSortWarps - 1) / kCsSortWarps), kCsSortWarps * 32, 0, st>>>(
         s, c.offsets, c.perm);
@@ -613,36 +722,53 @@ static bool rows_vec_ok(const tomos_dense* A, const void* lo, int esz) {
     return vec;
 }
 
-// The staged owner sums and the reductions behind them: SA, colsq and
-// fro2 (both optional).  Returns nonzero with the error set on failure.
+// The row-major owner sums and the reductions behind them: SA, colsq and
+// fro2 (both optional).
 template <Elem E, bool STAGE>
-static tomos_status launch_rows_tma(const tomos_dense* A, const void* lo, int64_t s, const CsScratch& c,
-                                    double* SA, int64_t ld_sa, double* colsq, double* fro2,
-                                    uint16_t* plane, int64_t ld_plane, cudaStream_t st) {
+static tomos_status launch_rows(const tomos_dense* A, const void* lo, int64_t s, const CsScratch& c,
+                                double* SA, int64_t ld_sa, double* colsq, double* fro2,
+                                uint16_t* plane, int64_t ld_plane, cudaStream_t st) {
+    constexpr int VEC = CsElem<E>::VEC, PLANES = CsElem<E>::PLANES;
     const int64_t n = A->cols;
-    const size_t smem = cs_rows_tma_smem<E>();
-    TOMOS_CUDA_TRY(cudaFuncSetAttribute(cs_rows_tma_kernel<E, STAGE>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // the work counter: the first int of cursor (free after the scatter)
-    TOMOS_CUDA_TRY(cudaMemsetAsync(c.cursor, 0, sizeof(int32_t), st));
     CsRowsArgs a;
     a.hi = A->values;
     a.lo = lo;
     a.n = n;
     a.ld = A->ld;
     a.s = s;
-    a.panels = (int)((n + kCsPanelCols - 1) / kCsPanelCols);
     a.offsets = c.offsets;
     a.perm = c.perm;
-    a.sign = c.sign;
     a.SA = SA;
     a.ld_sa = ld_sa;
     a.col_part = reinterpret_cast<float*>(c.col_part);
     a.plane = plane;
     a.ld_plane = ld_plane;
-    a.counter = c.cursor;
-    cs_rows_tma_kernel<E, STAGE><<<(unsigned)sm_count(), kCsWarps * 32, smem, st>>>(a);
-    TOMOS_LAUNCH_CHECK("cs_rows_tma_kernel");
+    const int64_t nch = (n + VEC - 1) / VEC;
+    const bool vec = rows_vec_ok(A, lo, CsElem<E>::ESZ);
+    if (nch <= kCsNarrowChunks) {
+        const int rb = (int)(vec ? nch * 16 : n * CsElem<E>::ESZ);
+        int rows = kCsNarrowBytes / (rb * PLANES);
+        if (rows > kCsNarrowRows) rows = kCsNarrowRows;
+        const size_t smem = (size_t)kCsNarrowStages * rows * rb * PLANES;
+        void (*kern)(CsRowsArgs, int) = cs_rows_narrow_kernel<E, STAGE, true>;
+        if constexpr (!STAGE)
+            if (!vec) kern = cs_rows_narrow_kernel<E, false, false>;
+        TOMOS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<(unsigned)s, n <= 128 ? 128 : 256, smem, st>>>(a, rows);
+        TOMOS_LAUNCH_CHECK("cs_rows_narrow_kernel");
+    } else {
+        // threads: the chunks (or columns / kCsCols) of a row in whole
+        // warps, split over CTAs of at most kCsThreads
+        const int64_t units = vec ? nch : (n + kCsCols - 1) / kCsCols;
+        const int64_t panels = (units + kCsThreads - 1) / kCsThreads;
+        const int64_t threads = ((units + panels - 1) / panels + 31) / 32 * 32;
+        const dim3 grid((unsigned)s, (unsigned)panels);
+        if (vec)
+            cs_rows_kernel<E, STAGE><<<grid, (unsigned)threads, 0, st>>>(a);
+        else
+            cs_rows_any_kernel<E><<<grid, (unsigned)threads, 0, st>>>(a);
+        TOMOS_LAUNCH_CHECK("cs_rows_kernel");
+    }
     // colsq (into the caller's buffer or the scratch after the partials),
     // then fro2 as their sum
     double* cs = colsq ? colsq : reinterpret_cast<double*>(a.col_part + s * n);
@@ -664,21 +790,10 @@ static tomos_status launch_rows_tma(const tomos_dense* A, const void* lo, int64_
 }
 
 template <Elem E>
-static unsigned launch_rows(const tomos_dense* A, const void* lo, int64_t s, const CsScratch& c,
-                            double* SA, int64_t ld_sa, bool want_cols, unsigned gx,
-                            cudaStream_t st) {
-    const unsigned panels = (unsigned)((A->cols + 255) / 256);
-    cs_rows_kernel<E, 8><<<dim3(gx, panels), 256, 0, st>>>(A->values, lo, A->cols, A->ld, s, c.offsets,
-                                                           c.perm, c.sign, SA, ld_sa, c.fro_part,
-                                                           want_cols ? c.col_part : nullptr);
-    return panels;
-}
-
-template <Elem E>
 static void launch_cols(const tomos_dense* A, const void* lo, int64_t s, const CsScratch& c,
                         double* SA, int64_t ld_sa, double* colsq, cudaStream_t st) {
     cs_cols_kernel<E><<<(unsigned)A->cols, 256, 0, st>>>(A->values, lo, A->cols, A->ld, s, c.offsets,
-                                                         c.perm, c.sign, SA, ld_sa, c.fro_part, colsq);
+                                                         c.perm, SA, ld_sa, c.fro_part, colsq);
 }
 
 }  // namespace tomos_b200
@@ -754,43 +869,24 @@ static tomos_status countsketch_apply(const tomos_dense* A, int32_t tier, int64_
     const void* lo = (e == Elem::A16 || e == Elem::AB16 || e == Elem::AB16R) ? dense_lo_plane(A)
                                                                              : nullptr;
     int64_t nparts;
-    if (A->layout == TOMOS_ROW_MAJOR && rows_vec_ok(A, lo, e == Elem::F32 ? 4 : 2)) {
-        // staged owner sums: colsq and fro2 come with them
-        tomos_status rs = TOMOS_OK;
-        switch (e) {
-            case Elem::F32: rs = launch_rows_tma<Elem::F32, false>(A, lo, s, c, SA, ld_sa, colsq, fro2, nullptr, 0, st); break;
-            case Elem::H16:
-                rs = plane ? launch_rows_tma<Elem::H16, true>(A, lo, s, c, SA, ld_sa, colsq, fro2, plane, ld_plane, st)
-                           : launch_rows_tma<Elem::H16, false>(A, lo, s, c, SA, ld_sa, colsq, fro2, nullptr, 0, st);
-                break;
-            case Elem::A16: rs = launch_rows_tma<Elem::A16, false>(A, lo, s, c, SA, ld_sa, colsq, fro2, nullptr, 0, st); break;
-            case Elem::F16: rs = launch_rows_tma<Elem::F16, false>(A, lo, s, c, SA, ld_sa, colsq, fro2, nullptr, 0, st); break;
-            case Elem::B16: rs = launch_rows_tma<Elem::B16, false>(A, lo, s, c, SA, ld_sa, colsq, fro2, nullptr, 0, st); break;
-            case Elem::AB16: rs = launch_rows_tma<Elem::AB16, false>(A, lo, s, c, SA, ld_sa, colsq, fro2, nullptr, 0, st); break;
-            case Elem::AB16R: rs = launch_rows_tma<Elem::AB16R, false>(A, lo, s, c, SA, ld_sa, colsq, fro2, nullptr, 0, st); break;
-            default: return fail(TOMOS_ERR_UNSUPPORTED, "countsketch_apply: element type");
-        }
-        return rs;
-    }
-    if (plane) return fail(TOMOS_ERR_UNSUPPORTED, "countsketch_apply_stage: rows of A not 16-byte aligned");
+    if (plane && !rows_vec_ok(A, lo, 2))
+        return fail(TOMOS_ERR_UNSUPPORTED, "countsketch_apply_stage: rows of A not 16-byte aligned");
     if (A->layout == TOMOS_ROW_MAJOR) {
-        const unsigned gx = (unsigned)((s + 7) / 8);
-        unsigned panels = 0;
+        // colsq and fro2 come with the owner sums
+#define TOMOS_CS_ROWS(EE) launch_rows<EE, false>(A, lo, s, c, SA, ld_sa, colsq, fro2, nullptr, 0, st)
         switch (e) {
-            case Elem::F32: panels = launch_rows<Elem::F32>(A, lo, s, c, SA, ld_sa, colsq, gx, st); break;
-            case Elem::H16: panels = launch_rows<Elem::H16>(A, lo, s, c, SA, ld_sa, colsq, gx, st); break;
-            case Elem::A16: panels = launch_rows<Elem::A16>(A, lo, s, c, SA, ld_sa, colsq, gx, st); break;
-            case Elem::F16: panels = launch_rows<Elem::F16>(A, lo, s, c, SA, ld_sa, colsq, gx, st); break;
-            case Elem::B16: panels = launch_rows<Elem::B16>(A, lo, s, c, SA, ld_sa, colsq, gx, st); break;
-            case Elem::AB16: panels = launch_rows<Elem::AB16>(A, lo, s, c, SA, ld_sa, colsq, gx, st); break;
-            case Elem::AB16R: panels = launch_rows<Elem::AB16R>(A, lo, s, c, SA, ld_sa, colsq, gx, st); break;
+            case Elem::F32: return TOMOS_CS_ROWS(Elem::F32);
+            case Elem::H16:
+                return plane ? launch_rows<Elem::H16, true>(A, lo, s, c, SA, ld_sa, colsq, fro2, plane, ld_plane, st)
+                             : TOMOS_CS_ROWS(Elem::H16);
+            case Elem::A16: return TOMOS_CS_ROWS(Elem::A16);
+            case Elem::F16: return TOMOS_CS_ROWS(Elem::F16);
+            case Elem::B16: return TOMOS_CS_ROWS(Elem::B16);
+            case Elem::AB16: return TOMOS_CS_ROWS(Elem::AB16);
+            case Elem::AB16R: return TOMOS_CS_ROWS(Elem::AB16R);
             default: return fail(TOMOS_ERR_UNSUPPORTED, "countsketch_apply: element type");
         }
-        nparts = (int64_t)gx * panels;
-        if (colsq) {
-            TOMOS_LAUNCH_CHECK("countsketch owner sums");
-            cs_col_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(c.col_part, gx, n, colsq);
-        }
+#undef TOMOS_CS_ROWS
     } else {
         switch (e) {
             case Elem::F32: launch_cols<Elem::F32>(A, lo, s, c, SA, ld_sa, colsq, st); break;

@@ -16,17 +16,21 @@ __host__ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 
 // Caller-scratch layout of one sketch application (256-byte aligned slices).
 struct CsScratch {
-    int32_t* bucket;    // m: bucket of row i
-    int8_t* sign;       // m: +1 / -1
+    int32_t* bucket;    // m: bucket of row i (counting sort: bit 31 for sign -1)
+    int8_t* sign;       // m: +1 / -1 (more than kCsMaxCounted buckets only)
+    int32_t* cnt;       // segments x s: the counting sort's counts, then cursors
     int32_t* counts;    // s + 1
     int32_t* offsets;   // s + 1: bucket b holds perm[offsets[b] .. offsets[b+1])
     int32_t* cursor;    // s + 1
-    int32_t* perm;      // m: row ids grouped by bucket, ascending within a bucket
+    uint32_t* perm;     // m: row ids grouped by bucket, ascending within a bucket; bit 31: sign -1
     double* fro_part;   // owner-sum partials of sum(A_ij^2)
     double* col_part;   // per-block partial column sums of squares
     size_t bytes;
 };
 
+constexpr uint32_t kCsNeg = 0x80000000u;      // perm entries of sign -1 (rows fit 31 bits)
+constexpr int64_t kCsMaxCounted = 48 * 1024;  // buckets whose counters fit a CTA's shared memory
+int64_t cs_segments(int64_t m, int64_t s);
 CsScratch cs_layout(void* base, int64_t m, int64_t s, int64_t fro_parts, int64_t col_parts);
 // Rows of col_part any caller may need (times the column count).
 int64_t cs_col_part_rows(int64_t m, int64_t s);

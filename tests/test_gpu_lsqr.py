@@ -151,6 +151,16 @@ def test_fused_pass_matches_oracle_lsqr(orc, numeric, n, ld, tier):
     assert np.linalg.norm(x - x_ref) / np.linalg.norm(x_ref) < 1e-4
 
 
+@pytest.mark.parametrize("tier", [tb.Tier.AUTO, tb.Tier.ACCURATE])
+@pytest.mark.parametrize("numeric", [NT.FP32, NT.FP32_16, NT.FP32_BF16])
+@pytest.mark.parametrize("n,ld", [(9, 9), (10, 16), (31, 31), (33, 40), (64, 64), (100, 100), (128, 128),
+                                  (129, 129), (256, 256), (258, 258), (511, 513), (777, 777), (1024, 1025)])
+def test_direct_pass_matches_oracle_lsqr(orc, numeric, n, ld, tier):
+    """The direct pass (narrow rows in 16-byte chunks; unaligned rows two or
+    one elements a load, one to 32 loads a lane): same checks."""
+    test_fused_pass_matches_oracle_lsqr(orc, numeric, n, ld, tier)
+
+
 def test_prestaged_plane_same_solve():
     """A solve handed the plane the staging sketch wrote runs the same passes
     as one that stages its own copy: bit-identical x and reports."""

@@ -392,7 +392,7 @@ tomos_status tomos_lsqr_adjoint_dense(const tomos_dense* A, const float* g, floa
     s = ensure_adj(ws);
     if (s) return s;
     const PassPlan pl = plan_dense_pass(ws, A, e, false);
-    if (!pl.fused) {
+    if (pass_needs_scratch(pl)) {
         s = ensure_scratch(ws, dense_pass_scratch(A));
         if (s) return s;
     }

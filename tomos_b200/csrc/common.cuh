@@ -155,6 +155,16 @@ __host__ __device__ __forceinline__ uint32_t half_only_bits(uint32_t h) {
     return sign | ((sig >> s) & 0x3FFu);
 }
 
+// half_only_bits by selects only: a branch on the control bit would make a
+// kernel wait for each load of an unrolled batch before the next.
+__host__ __device__ __forceinline__ uint32_t half_only_bits_nb(uint32_t h) {
+    const uint32_t sign = h & 0x8000u;
+    const uint32_t sig = 0x200u | ((h >> 1) & 0x1FFu);
+    const uint32_t sub = sign | ((sig >> ((h >> 10) & 0xFu)) & 0x3FFu);
+    const uint32_t ext = (h & 0x4000u) ? (sign | 0x7C00u) : sub;
+    return (h & 1u) ? ext : h;
+}
+
 // IEEE binary16 bits -> float (exact; normal, subnormal, Inf).
 __device__ __forceinline__ float half_bits_to_float(uint32_t hb) {
     return __half2float(__ushort_as_half((unsigned short)hb));
@@ -183,6 +193,10 @@ __host__ __device__ __forceinline__ float decode_fp32_bf16_exact(uint32_t h, uin
     return u2f((t << 16) | (r & 0xFFFEu));
 }
 
+// Asks for the line of p in L2: loads that follow some rounds later then wait
+// for L2, not for HBM, without a register held meanwhile.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // ------------------------------------------------------- warp reductions
 
 template <typename T>
@@ -205,7 +219,8 @@ enum class Elem : int {
                    // plane, control words already decoded)
 };
 
-// Scalar element decode at flat index idx (generic kernels).
+// Scalar element decode at flat index idx (generic kernels), branch-free so
+// that the loads of an unrolled batch stay in flight together.
 template <Elem E>
 __device__ __forceinline__ float load_elem(const void* p, const void* q, size_t idx);
 
@@ -216,7 +231,7 @@ __device__ __forceinline__ float load_elem<Elem::F32>(const void* p, const void*
 template <>
 __device__ __forceinline__ float load_elem<Elem::H16>(const void* p, const void*, size_t idx) {
     uint32_t h = __ldg(reinterpret_cast<const unsigned short*>(p) + idx);
-    return half_bits_to_float(half_only_bits(h));
+    return half_bits_to_float(half_only_bits_nb(h));
 }
 template <>
 __device__ __forceinline__ float load_elem<Elem::F16>(const void* p, const void*, size_t idx) {
@@ -226,7 +241,7 @@ template <>
 __device__ __forceinline__ float load_elem<Elem::A16>(const void* p, const void* q, size_t idx) {
     uint32_t h = __ldg(reinterpret_cast<const unsigned short*>(p) + idx);
     uint32_t r = __ldg(reinterpret_cast<const unsigned short*>(q) + idx);
-    return decode_fp32_16_exact(h, r);
+    return decode_fp32_16_exact_nb(h, r);
 }
 template <>
 __device__ __forceinline__ float load_elem<Elem::B16>(const void* p, const void*, size_t idx) {
@@ -244,6 +259,17 @@ __device__ __forceinline__ float load_elem<Elem::AB16R>(const void* p, const voi
     uint32_t h = __ldg(reinterpret_cast<const unsigned short*>(p) + idx);
     uint32_t r = __ldg(reinterpret_cast<const unsigned short*>(q) + idx);
     return decode_fp32_bf16_exact(h, r, true);
+}
+
+// The value of one element's words (FP32: its bits).
+template <Elem E>
+__device__ __forceinline__ float word_value(uint32_t h, uint32_t r) {
+    if constexpr (E == Elem::F32) return u2f(h);
+    else if constexpr (E == Elem::H16) return half_bits_to_float(half_only_bits_nb(h));
+    else if constexpr (E == Elem::F16) return half_bits_to_float(h);
+    else if constexpr (E == Elem::B16) return u2f(h << 16);
+    else if constexpr (E == Elem::A16) return decode_fp32_16_exact_nb(h, r);
+    else return decode_fp32_bf16_exact(h, r, E == Elem::AB16R);
 }
 
 // Resolves a tomos_dense + tier to the element tag it is read as.

@@ -14,8 +14,9 @@
 //                                         atomics; the reference uses
 //                                         atomicAdd, mv_cuda_kernels.cu:529)
 // HALF-tier and FP32 products accumulate in FP32, ACCURATE-tier in FP64.
-// The LSQR iteration uses the fused row-major pass in fused.cuh instead;
-// these kernels serve tomos_gemv and the shapes that pass does not cover.
+// The row passes (rowpass.cuh, rowpass_direct.cuh) take row-major LSQR
+// iterations and the products whose lines fit them; these kernels serve the
+// rest.
 #include <mutex>
 #include <string>
 
@@ -96,20 +97,61 @@ __global__ void __launch_bounds__(256) line_sum_partial_kernel(
     partial[(size_t)c * inner + i] = a0 + a1;
 }
 
+// A CTA owns 32 columns; its warps (up to 32) split the partials, each
+// thread with eight loads in flight, and sum what they hold in warp order.
+// Bound by the latency of one thread's share: a thread a column took 136 us
+// for 1173 partials of 777 columns.
 template <typename Acc>
-__global__ void line_sum_reduce_kernel(const Acc* __restrict__ partial, int64_t nchunks,
-                                       int64_t inner, double alpha, double beta,
-                                       const double* coef, const int* skip,
-                                       float* __restrict__ y) {
+__global__ void __launch_bounds__(1024) sum_parts_kernel(const Acc* __restrict__ part, int64_t nparts,
+                                                         int64_t stride, int64_t n, double alpha, double beta,
+                                                         const double* coef, const int* skip,
+                                                         float* __restrict__ y) {
     if (skip && *skip) return;
     resolve_coef(coef, alpha, beta);
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= inner) return;
-    double acc = 0.0;
-    for (int64_t c = 0; c < nchunks; ++c) acc += (double)partial[(size_t)c * inner + i];
-    double r = alpha * acc;
-    if (beta != 0.0) r += beta * (double)y[i];
-    y[i] = (float)r;
+    __shared__ double sm[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int64_t j = (int64_t)blockIdx.x * 32 + lane;
+    double s = 0.0;
+    if (j < n) {
+        int64_t c = w;
+        for (; c + 7 * nw < nparts; c += 8 * nw) {
+            Acc v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = part[(size_t)(c + u * nw) * stride + j];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += (double)v[u];
+        }
+        for (; c < nparts; c += nw) s += (double)part[(size_t)c * stride + j];
+    }
+    sm[w][lane] = s;
+    __syncthreads();
+    if (w != 0 || j >= n) return;
+    double t = 0.0;
+    for (int k = 0; k < nw; ++k) t += sm[k][lane];
+    double r = alpha * t;
+    if (beta != 0.0) r += beta * (double)y[j];
+    y[j] = (float)r;
+}
+
+template <typename Acc>
+static tomos_status sum_parts(const Acc* part, int64_t nparts, int64_t stride, int64_t n, double alpha,
+                              double beta, const double* coef, const int* skip, float* y, cudaStream_t st) {
+    int64_t warps = (nparts + 7) / 8;
+    if (warps > 32) warps = 32;
+    if (warps < 1) warps = 1;
+    sum_parts_kernel<Acc><<<(unsigned)((n + 31) / 32), (unsigned)warps * 32, 0, st>>>(part, nparts, stride, n, alpha,
+                                                                                     beta, coef, skip, y);
+    TOMOS_LAUNCH_CHECK("sum_parts_kernel");
+    return TOMOS_OK;
+}
+
+tomos_status launch_sum_parts(const float* part, int64_t nparts, int64_t stride, int64_t n, double alpha,
+                              double beta, const double* coef, const int* skip, float* y, cudaStream_t st) {
+    return sum_parts(part, nparts, stride, n, alpha, beta, coef, skip, y, st);
+}
+tomos_status launch_sum_parts(const double* part, int64_t nparts, int64_t stride, int64_t n, double alpha,
+                              double beta, const double* coef, const int* skip, float* y, cudaStream_t st) {
+    return sum_parts(part, nparts, stride, n, alpha, beta, coef, skip, y, st);
 }
 
 int64_t line_sum_chunks(int64_t outer) {
@@ -142,10 +184,7 @@ static tomos_status run_gemv(const GemvLaunch& L, cudaStream_t st) {
     line_sum_partial_kernel<E, ACC64><<<grid, 256, 0, st>>>(L.hi, L.lo, L.outer, L.inner, L.ld,
                                                             L.x, lpc, L.skip, partial);
     TOMOS_LAUNCH_CHECK("line_sum_partial_kernel");
-    line_sum_reduce_kernel<Acc><<<(unsigned)((L.inner + 255) / 256), 256, 0, st>>>(
-        partial, nchunks, L.inner, L.alpha, L.beta, L.coef, L.skip, L.y);
-    TOMOS_LAUNCH_CHECK("line_sum_reduce_kernel");
-    return TOMOS_OK;
+    return sum_parts(partial, nchunks, L.inner, L.inner, L.alpha, L.beta, L.coef, L.skip, L.y, st);
 }
 
 template <Elem E>
@@ -208,7 +247,7 @@ size_t gemv_scratch_bytes_max(const tomos_dense* A, int32_t trans) {
     std::string why;
     if (!gemv_shape(A, trans, &dot, &outer, &inner, &why) || dot) return 0;
     const size_t generic = (size_t)line_sum_chunks(outer) * (size_t)inner * 8;
-    const size_t rowpass = rowpass_gemv_scratch_bytes(inner);
+    const size_t rowpass = rowpass_gemv_scratch_bytes(outer, inner);
     return generic > rowpass ? generic : rowpass;
 }
 

@@ -35,10 +35,17 @@ size_t gemv_scratch_bytes_max(const tomos_dense* A, int32_t trans);
 
 tomos_status gemv_launch(const GemvLaunch& L, Elem e, bool acc64, cudaStream_t st);
 
+// y[j] = alpha * sum_c part[c * stride + j] + beta * y[j], j < n: the nparts
+// partials in a fixed order, in FP64 (coef and skip as in GemvLaunch).
+tomos_status launch_sum_parts(const float* part, int64_t nparts, int64_t stride, int64_t n, double alpha,
+                              double beta, const double* coef, const int* skip, float* y, cudaStream_t st);
+tomos_status launch_sum_parts(const double* part, int64_t nparts, int64_t stride, int64_t n, double alpha,
+                              double beta, const double* coef, const int* skip, float* y, cudaStream_t st);
+
 // The product through the row pass (rowpass_gemv.cu) when A's lines fit
 // it; *used false (nothing launched) otherwise.
 tomos_status rowpass_gemv(const GemvLaunch& L, Elem e, cudaStream_t st, bool* used);
-size_t rowpass_gemv_scratch_bytes(int64_t inner);
+size_t rowpass_gemv_scratch_bytes(int64_t outer, int64_t inner);
 
 tomos_status gemv_dispatch(int32_t trans, double alpha, const tomos_dense* A, int32_t tier,
                            const float* x, double beta, float* y, void* scratch,

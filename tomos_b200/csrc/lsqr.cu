@@ -33,6 +33,7 @@
 #include "gemv.cuh"
 #include "lsqr.cuh"
 #include "rowpass.cuh"
+#include "rowpass_direct.cuh"
 #include "rowpass_launch.cuh"
 #include "rowpass_mma.cuh"
 
@@ -570,8 +571,9 @@ __global__ void __launch_bounds__(128) stage_half_kernel(const uint16_t* __restr
     }
 }
 
-// Chooses the fused pass when A is row-major with 16-byte aligned rows
-// and n fits the consumer warps (12288 columns; 8192 or 6144 for ACC64); otherwise
+// A row-major A takes the direct pass when its rows are narrow or unaligned
+// (direct_shape), else the ring pass when its rows are 16-byte aligned and n
+// fits the consumer warps (12288 columns; 8192 or 6144 for ACC64); otherwise
 // the generic two-kernel path.
 PassPlan plan_dense_pass(tomos_workspace* ws, const tomos_dense* A, Elem e, bool acc64, bool runs) {
     PassPlan pl;
@@ -579,10 +581,25 @@ PassPlan plan_dense_pass(tomos_workspace* ws, const tomos_dense* A, Elem e, bool
     pl.acc64 = acc64 || elem_is_exact(e);
     // run-summed dots: the FP32 and two-plane FP64-summing passes
     pl.runs = runs && pl.acc64 && (e == Elem::F32 || elem_two_planes(e));
+    const void* plo = elem_is_exact(e) ? dense_lo_plane(A) : nullptr;
+    DirectShape ds;
+    if (A->layout == TOMOS_ROW_MAJOR) ds = direct_shape(e, A->cols, A->ld, A->values, plo);
+    if (ds.lpr > 0) {
+        pl.fused = true;
+        pl.direct = true;
+        pl.runs = false;  // FP64 products
+        pl.nch = ds.c;
+        pl.g = ds.lpr;
+        pl.grid = direct_grid(A->rows);
+        pl.gq = pl.acc64 ? 1 : pl.grid;  // FP64 partials are summed into one row
+        pl.gs = pl.grid;
+        pl.qstride = ws->qstride;
+        return pl;
+    }
     int nch = 0, g = 1;
     const bool ok = A->layout == TOMOS_ROW_MAJOR && A->cols > 0 &&
                     plan_row_lines(e, pl.acc64, pl.runs ? kRowBothRuns : kRowBoth, A->cols, A->ld, A->values,
-                                   elem_is_exact(e) ? dense_lo_plane(A) : nullptr, &nch, &g);
+                                   plo, &nch, &g);
     if (ok) {
         pl.fused = true;
         pl.nch = nch;
@@ -633,6 +650,22 @@ tomos_status enqueue_dense_pass(tomos_workspace* ws, const tomos_dense* A,
         P.sspart = ws->sspart;
         P.qstride = pl.qstride;
         P.skip = skip;
+        if (pl.direct) {
+            DirectParams T;
+            DirectShape ds;
+            ds.c = pl.nch;
+            ds.lpr = pl.g;
+            T.f = P;
+            T.qpart64 = static_cast<double*>(ws->scratch);
+            T.dot = T.axpy = T.write_u = 1;
+            T.aligned = direct_aligned(pl.e, A->ld, A->values, lo) ? 1 : 0;
+            tomos_status ls = launch_direct(pl.e, pl.acc64, T, ds, pl.grid, st);
+            if (ls) return ls;
+            ws->launches += 1;
+            if (!pl.acc64) return TOMOS_OK;
+            ws->launches += 1;
+            return launch_sum_parts(T.qpart64, pl.grid, pl.qstride, A->cols, 1.0, 0.0, nullptr, skip, ws->qpart, st);
+        }
         tomos_status ls = pl.tpw > 0 ? launch_fused_mma(pl.e, P, &ws->st->pipe_err, pl.tpw, pl.grid, st)
                                      : launch_fused(pl.e, pl.acc64, pl.runs, P, &ws->st->pipe_err, pl.nch, pl.g,
                                                     pl.grid, st);
@@ -748,7 +781,9 @@ struct DensePass : PassOps {
     tomos_dense staged{};
     DensePass(tomos_workspace* w, const tomos_dense* a, Elem ie, Elem ze)
         : ws(w), A(a), iter_e(ie), init_e(ze) {
-        stage = ie == Elem::H16 && plan_dense_pass(ws, A, ie, false).fused;
+        // rows the staging kernel can read: 16-byte aligned
+        const PassPlan pl = plan_dense_pass(ws, A, ie, false);
+        stage = ie == Elem::H16 && pl.fused && direct_aligned(ie, A->ld, A->values, nullptr);
         staged = *A;  // values set by prepare()
         staged.values_lo = nullptr;
         staged.ld = (A->cols + 7) / 8 * 8;
@@ -996,8 +1031,10 @@ tomos_status solve_driver(tomos_workspace* ws, PassOps& ops, const float* b, flo
                                  (uint64_t)pl_iter.g,
                                  (uint64_t)pl_iter.grid,
                                  (uint64_t)pl_iter.tpw,
+                                 (uint64_t)pl_iter.direct,
                                  reinterpret_cast<uint64_t>(x),
                                  reinterpret_cast<uint64_t>(dsc),
+                                 reinterpret_cast<uint64_t>(ws->scratch),
                                  (uint64_t)ws->has_precond,
                                  (uint64_t)n,
                                  (uint64_t)m,
@@ -1460,7 +1497,7 @@ tomos_status tomos_lsqr_solve_dense(const tomos_dense* A, const float* b, float*
         DensePass pa(ws, A, ie, ie), pr(ws, Rf, re, re);
         RefinePass ops(pa, pr);
         PassPlan a = ops.plan(true), b2 = ops.plan(false);
-        if (!a.fused || !b2.fused) {
+        if (pass_needs_scratch(a) || pass_needs_scratch(b2)) {
             const size_t sa = dense_pass_scratch(A), sr = dense_pass_scratch(Rf);
             s = ensure_scratch(ws, sa > sr ? sa : sr);
             if (s) return s;
@@ -1480,7 +1517,7 @@ tomos_status tomos_lsqr_solve_dense(const tomos_dense* A, const float* b, float*
         ops.given_ld = opts->staged_ld;
     }
     PassPlan a = ops.plan(true), b2 = ops.plan(false);
-    if (!a.fused || !b2.fused) {
+    if (pass_needs_scratch(a) || pass_needs_scratch(b2)) {
         s = ensure_scratch(ws, dense_pass_scratch(A));
         if (s) return s;
     }
@@ -1503,7 +1540,7 @@ tomos_status tomos_backward_error_dense(const tomos_dense* A, const float* b, co
     if (!resolve_elem(A, tier, &ze, &why)) return fail(TOMOS_ERR_UNSUPPORTED, why);
     DensePass ops(ws, A, ze, ze);
     PassPlan pl = ops.plan(true);
-    if (!pl.fused) {
+    if (pass_needs_scratch(pl)) {
         s = ensure_scratch(ws, dense_pass_scratch(A));
         if (s) return s;
     }

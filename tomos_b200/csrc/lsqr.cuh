@@ -51,6 +51,7 @@ struct PassPlan {
     int gs = 1;      // ||ut||^2 partials
     int64_t qstride = 0;
     int tpw = 0;     // > 0: the tensor-core pass, k-tiles per consumer warp
+    bool direct = false;  // the direct pass (nch chunks a lane, g lanes a row)
     int src = 0;     // 1: the pass reads the refine copy of A (RefinePass)
     bool runs = false;  // FP64-summing fused pass: dots as FP32 runs (kRowBothRuns)
 };
@@ -135,6 +136,9 @@ __device__ __forceinline__ double block_sum_array(const double* part, int64_t np
 // One pass over a dense A (the fused kernel when pl.fused, else the
 // generic two-kernel path): ut = cp A p + cu u_in into ws->u, the
 // partials of A^T ut into ws->qpart and of ||ut||^2 into ws->sspart.
+// Plans that need ws->scratch (dense_pass_scratch bytes): the generic path's
+// partials, and the FP64 partials of a direct pass.
+inline bool pass_needs_scratch(const PassPlan& pl) { return !pl.fused || (pl.direct && pl.acc64); }
 PassPlan plan_dense_pass(tomos_workspace* ws, const tomos_dense* A, Elem e, bool acc64, bool runs = false);
 
 // Options every solve entry accepts (stop rule, iteration counts).

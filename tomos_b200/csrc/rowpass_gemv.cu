@@ -9,10 +9,12 @@
 //   dot per line      kRowDot:  y_o = alpha (A_o . x) + beta y_o, one
 //                     warp (or G warps) per line, written in place;
 //   sum of lines      kRowAxpy: per-CTA partials of sum_o x_o A_o, then
-//                     rowpass_reduce_kernel sums the partials of every
-//                     column in CTA order (deterministic, no atomics; the
-//                     reference adds with atomicAdd, mv_cuda_kernels.cu:529)
-//                     into y = alpha sum + beta y.
+//                     sum_parts_kernel (gemv.cu) sums the partials of
+//                     every column in a fixed order (deterministic, no
+//                     atomics; the reference adds with atomicAdd,
+//                     mv_cuda_kernels.cu:529) into y = alpha sum + beta y.
+// Narrow lines, and lines that do not start on 16-byte boundaries, take the
+// direct pass (rowpass_direct.cuh) both ways instead.
 // FP32 and HALF-tier products accumulate in FP32.  The exact tiers form
 // FP32 products over short runs (a lane's part of a line, or 8 lines of a
 // column) and sum the runs in FP64.  Other shapes take the generic
@@ -22,25 +24,12 @@
 
 #include "common.cuh"
 #include "gemv.cuh"
+#include "rowpass_direct.cuh"
 #include "rowpass_launch.cuh"
 
 namespace tomos_b200 {
 
 namespace {
-
-// y[j] = alpha * sum_c part[c][j] + beta * y[j], the partials in CTA order.
-template <typename Acc>
-__global__ void __launch_bounds__(256) rowpass_reduce_kernel(const Acc* __restrict__ part, int nparts,
-                                                             int64_t stride, int64_t n, double alpha,
-                                                             double beta, float* __restrict__ y) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    double s = 0.0;
-    for (int c = 0; c < nparts; ++c) s += (double)part[(size_t)c * stride + j];
-    double r = alpha * s;
-    if (beta != 0.0) r += beta * (double)y[j];
-    y[j] = (float)r;
-}
 
 // The word a bounded pipeline wait of these launches records its expiry
 // in (one per device; nothing reads it back: an expired wait leaves the
@@ -83,15 +72,54 @@ tomos_status launch_mode(Elem e, bool acc64, const FusedParams& P, int* err, int
 
 }  // namespace
 
-size_t rowpass_gemv_scratch_bytes(int64_t inner) {
+size_t rowpass_gemv_scratch_bytes(int64_t outer, int64_t inner) {
     const int64_t qs = (inner + 31) / 32 * 32;
-    return (size_t)sm_count() * (size_t)qs * sizeof(double);
+    int64_t rows = sm_count();
+    if (inner <= kDirectMaxCols && direct_grid(outer) > rows) rows = direct_grid(outer);
+    return (size_t)rows * (size_t)qs * sizeof(double);
+}
+
+// The product through the direct pass (*used false: scratch too small).
+static tomos_status direct_gemv(const GemvLaunch& L, Elem e, const DirectShape& ds, cudaStream_t st, bool* used) {
+    const bool acc64 = elem_is_exact(e);
+    const int grid = direct_grid(L.outer);
+    const int64_t qs = (L.inner + 31) / 32 * 32;
+    if (!L.dot && (!L.scratch || L.scratch_bytes < (size_t)grid * qs * (acc64 ? 8 : 4))) return TOMOS_OK;
+    *used = true;
+    DirectParams T;
+    FusedParams& P = T.f;
+    P.hi = L.hi;
+    P.lo = L.lo;
+    P.m = L.outer;
+    P.n = L.inner;
+    P.ld = L.ld;
+    P.coef = nullptr;
+    P.sspart = nullptr;
+    P.skip = nullptr;
+    P.qstride = qs;
+    T.dot = L.dot ? 1 : 0;
+    T.axpy = L.dot ? 0 : 1;
+    T.write_u = T.dot;
+    T.aligned = direct_aligned(e, L.ld, L.hi, L.lo) ? 1 : 0;
+    P.p = L.dot ? L.x : nullptr;
+    P.u_in = L.dot ? L.y : L.x;
+    P.u_out = L.dot ? L.y : nullptr;
+    P.cp = L.dot ? L.alpha : 0.0;
+    P.cu = L.dot ? L.beta : 1.0;
+    P.qpart = static_cast<float*>(L.scratch);
+    T.qpart64 = static_cast<double*>(L.scratch);
+    tomos_status s = launch_direct(e, acc64, T, ds, grid, st);
+    if (s || L.dot) return s;
+    return acc64 ? launch_sum_parts(T.qpart64, grid, qs, L.inner, L.alpha, L.beta, nullptr, nullptr, L.y, st)
+                 : launch_sum_parts(P.qpart, grid, qs, L.inner, L.alpha, L.beta, nullptr, nullptr, L.y, st);
 }
 
 tomos_status rowpass_gemv(const GemvLaunch& L, Elem e, cudaStream_t st, bool* used) {
     *used = false;
     const bool acc64 = elem_is_exact(e);
     if (e == Elem::F64 || L.coef || L.skip) return TOMOS_OK;
+    const DirectShape ds = direct_shape(e, L.inner, L.ld, L.hi, L.lo);
+    if (ds.lpr > 0) return direct_gemv(L, e, ds, st, used);
     int nch = 0, g = 1;
     if (!plan_row_lines(e, acc64, L.dot ? kRowDot : kRowAxpy, L.inner, L.ld, L.hi, L.lo, &nch, &g)) return TOMOS_OK;
     const int grid = row_pass_grid(L.outer);
@@ -130,13 +158,8 @@ tomos_status rowpass_gemv(const GemvLaunch& L, Elem e, cudaStream_t st, bool* us
     double* q64 = acc64 ? static_cast<double*>(L.scratch) : nullptr;
     tomos_status s = launch_mode<kRowAxpy>(e, acc64, P, err, nch, g, grid, st, q64);
     if (s) return s;
-    const unsigned rb = (unsigned)((L.inner + 255) / 256);
-    if (acc64)
-        rowpass_reduce_kernel<double><<<rb, 256, 0, st>>>(q64, grid, qs, L.inner, L.alpha, L.beta, L.y);
-    else
-        rowpass_reduce_kernel<float><<<rb, 256, 0, st>>>(P.qpart, grid, qs, L.inner, L.alpha, L.beta, L.y);
-    TOMOS_LAUNCH_CHECK("rowpass_reduce_kernel");
-    return TOMOS_OK;
+    return acc64 ? launch_sum_parts(q64, grid, qs, L.inner, L.alpha, L.beta, nullptr, nullptr, L.y, st)
+                 : launch_sum_parts(P.qpart, grid, qs, L.inner, L.alpha, L.beta, nullptr, nullptr, L.y, st);
 }
 
 }  // namespace tomos_b200

@@ -50,6 +50,34 @@ def test_gemv_vs_fp64(orc, numeric, tier, rounded, layout, shape):
             assert np.all(np.abs(got - ref) <= tol + 1e-7 * np.abs(ref)), (trans, beta)
 
 
+@pytest.mark.parametrize("numeric,tier,rounded", CASES + [(NT.FP16, tb.Tier.AUTO, False)])
+@pytest.mark.parametrize("m,n,pad", [(5001, 9, 0), (3, 64, 0), (4999, 256, 0), (17, 258, 0), (2049, 65, 0),
+                                     (1501, 777, 0), (700, 1025, 0), (40003, 7, 1), (8200, 600, 4)])
+@pytest.mark.parametrize("layout", [L.ROW_MAJOR, L.COL_MAJOR])
+def test_gemv_line_shapes(orc, numeric, tier, rounded, m, n, pad, layout):
+    """Narrow and unaligned lines (the direct pass), few long lines (a CTA a
+    segment, chunks of eight lines), aligned or not, both ways."""
+    rng = np.random.default_rng(m + n)
+    A0 = (rng.standard_normal((m, n)) * np.where(rng.random((m, n)) < 0.05, 1e-6, 1.0)).astype(np.float32)
+    if numeric == NT.FP16:
+        A = tb.pack(to_dense(A0, layout, pad=pad), NT.FP16)
+        Ad = A.view().double().cpu().numpy()
+    else:
+        A = to_dense(A0, layout, numeric, pad=pad, rounded=rounded)
+        Ad = decoded(orc, A, tier)
+    for trans in (tb.NO_TRANSPOSE, tb.TRANSPOSE):
+        M = Ad if trans == tb.NO_TRANSPOSE else Ad.T
+        x = rng.standard_normal(M.shape[1]).astype(np.float32)
+        for beta in (0.0, -0.5):
+            y0 = rng.standard_normal(M.shape[0]).astype(np.float32) if beta else np.full(M.shape[0], np.nan, np.float32)
+            ref = 1.5 * (M @ x.astype(np.float64)) + (beta * y0.astype(np.float64) if beta else 0.0)
+            scale = 1.5 * (np.abs(M) @ np.abs(x.astype(np.float64))) + abs(beta) * np.abs(np.nan_to_num(y0))
+            got = run(A, trans, tier, x, 1.5, beta, y0)
+            # exact tiers: FP32 runs of at most 8 at worst, then one rounding
+            tol = (2e-6 if tier == tb.Tier.ACCURATE else 2e-5) * scale + 1e-30
+            assert np.all(np.abs(got - ref) <= tol + 1e-7 * np.abs(ref)), (trans, beta)
+
+
 def test_fp32_16_tiers_vs_reference_cpu(orc):
     """The reference's CPU tiers (fp32_16_kernels.cpp): our HALF tier is its
     'fast' tier (fp32_16_half_only decode, wide accumulation), ACCURATE its

@@ -5,7 +5,8 @@
 // A strided matrix is `outer` lines of `inner` contiguous elements.  An
 // op(A) product is then one of two shapes:
 //   line dots  (row-major NO_TRANSPOSE, col-major TRANSPOSE):
-//       y[o] = sum_i A[o, i] x[i]      -- one warp per line
+//       y[o] = sum_i A[o, i] x[i]      -- a warp per line, or a CTA per
+//                                         segment of a few long lines
 //   line sums  (row-major TRANSPOSE, col-major NO_TRANSPOSE):
 //       y[i] = sum_o A[o, i] x[o]      -- threads own i; blocks own a
 //                                         chunk of lines and write partials
@@ -21,6 +22,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "fused.cuh"
 #include "gemv.cuh"
 
 namespace tomos_b200 {
@@ -41,6 +43,23 @@ __device__ __forceinline__ void resolve_coef(const double* coef, double& alpha, 
     }
 }
 
+// V consecutive elements at flat index idx as floats: V = ChunkElems (one
+// 16-byte load a plane, idx 16-byte aligned) or 1.
+template <Elem E, int V>
+__device__ __forceinline__ void load_chunk(const void* hi, const void* lo, size_t idx, float* f) {
+    if constexpr (V == 1) {
+        f[0] = load_elem<E>(hi, lo, idx);
+    } else {
+        FusedParams P;
+        P.hi = hi;
+        P.lo = lo;
+        uint4 h, l;
+        ChunkDecoder<E>::load(P, idx, h, l);
+        ChunkDecoder<E>::decode(h, l, f);
+    }
+}
+
+// Line dots, a warp per line: y[o] = alpha A_o . x + beta y[o].
 template <Elem E, bool ACC64>
 __global__ void __launch_bounds__(256) line_dot_kernel(const void* __restrict__ hi,
                                                        const void* __restrict__ lo,
@@ -74,27 +93,117 @@ __global__ void __launch_bounds__(256) line_dot_kernel(const void* __restrict__ 
     }
 }
 
-template <Elem E, bool ACC64>
+// Line dots of few, long lines: a CTA per segment of a line, whose partial
+// (FP64 over the CTA's lanes) sum_parts_kernel adds in segment order.  A
+// warp a line left most SMs idle: 790 us for 300 lines of 100000 fp16 words.
+template <Elem E, bool ACC64, int V>
+__global__ void __launch_bounds__(256) line_dot_seg_kernel(const void* __restrict__ hi,
+                                                           const void* __restrict__ lo, int64_t inner,
+                                                           int64_t ld, const float* __restrict__ x,
+                                                           int64_t seg, int64_t outer, const int* skip,
+                                                           double* __restrict__ partial) {
+    if (skip && *skip) return;
+    using Acc = typename AccT<ACC64>::T;
+    __shared__ double sm[8];
+    const int64_t o = blockIdx.x, i0 = (int64_t)blockIdx.y * seg;  // seg: a multiple of 256 V
+    const int64_t i1 = i0 + seg < inner ? i0 + seg : inner;
+    const size_t base = (size_t)o * (size_t)ld;
+    Acc a[4] = {0, 0, 0, 0};
+    int64_t i = i0 + (int64_t)threadIdx.x * V;
+    const bool xvec = reinterpret_cast<uintptr_t>(x) % 16 == 0;  // k is a multiple of V
+    auto step = [&](int64_t k, Acc& acc, const float* f) {
+        float xv[V];
+        if (V % 4 == 0 && xvec) {
+#pragma unroll
+            for (int e = 0; e + 3 < V; e += 4) {
+                const float4 t = __ldg(reinterpret_cast<const float4*>(x + k + e));
+                xv[e] = t.x;
+                xv[e + 1] = t.y;
+                xv[e + 2] = t.z;
+                xv[e + 3] = t.w;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < V; ++e) xv[e] = __ldg(x + k + e);
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc += (Acc)f[e] * (Acc)xv[e];
+    };
+    for (; i + 3 * 256 * V + V <= i1; i += 4 * 256 * V) {
+        float f[4][V];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) load_chunk<E, V>(hi, lo, base + i + u * 256 * V, f[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) step(i + u * 256 * V, a[u], f[u]);
+    }
+    for (; i < i1; i += 256 * V) {
+        if (i + V <= i1) {
+            float f[V];
+            load_chunk<E, V>(hi, lo, base + i, f);
+            step(i, a[0], f);
+        } else {
+            for (int64_t k = i; k < i1; ++k) a[0] += (Acc)load_elem<E>(hi, lo, base + k) * (Acc)__ldg(x + k);
+        }
+    }
+    const double d = warp_sum((double)((a[0] + a[1]) + (a[2] + a[3])));
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = d;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += sm[w];
+        partial[(size_t)blockIdx.y * outer + o] = t;
+    }
+}
+
+// Line sums: a thread owns V consecutive elements of the lines of its
+// chunk, eight lines' loads in flight.
+template <Elem E, bool ACC64, int V>
 __global__ void __launch_bounds__(256) line_sum_partial_kernel(
     const void* __restrict__ hi, const void* __restrict__ lo, int64_t outer, int64_t inner,
     int64_t ld, const float* __restrict__ x, int64_t lines_per_chunk, const int* skip,
     typename AccT<ACC64>::T* __restrict__ partial) {
     if (skip && *skip) return;
     using Acc = typename AccT<ACC64>::T;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int U = V == 1 ? 8 : 4;
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
     const int64_t c = blockIdx.y;
     if (i >= inner) return;
-    int64_t o0 = c * lines_per_chunk;
+    const int64_t o0 = c * lines_per_chunk;
     int64_t o1 = o0 + lines_per_chunk;
     if (o1 > outer) o1 = outer;
-    Acc a0 = 0, a1 = 0;
-    int64_t o = o0;
-    for (; o + 1 < o1; o += 2) {
-        a0 += (Acc)load_elem<E>(hi, lo, (size_t)o * ld + i) * (Acc)__ldg(x + o);
-        a1 += (Acc)load_elem<E>(hi, lo, (size_t)(o + 1) * ld + i) * (Acc)__ldg(x + o + 1);
+    if (V > 1 && i + V > inner) {  // the last, partly filled chunk
+        for (int64_t k = i; k < inner; ++k) {
+            Acc a = 0;
+            for (int64_t o = o0; o < o1; ++o) a += (Acc)load_elem<E>(hi, lo, (size_t)o * ld + k) * (Acc)__ldg(x + o);
+            partial[(size_t)c * inner + k] = a;
+        }
+        return;
     }
-    if (o < o1) a0 += (Acc)load_elem<E>(hi, lo, (size_t)o * ld + i) * (Acc)__ldg(x + o);
-    partial[(size_t)c * inner + i] = a0 + a1;
+    Acc a[2][V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) a[0][e] = a[1][e] = 0;
+    int64_t o = o0;
+    for (; o + U <= o1; o += U) {
+        float f[U][V];
+#pragma unroll
+        for (int u = 0; u < U; ++u) load_chunk<E, V>(hi, lo, (size_t)(o + u) * ld + i, f[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const Acc xv = (Acc)__ldg(x + o + u);
+#pragma unroll
+            for (int e = 0; e < V; ++e) a[u & 1][e] += (Acc)f[u][e] * xv;
+        }
+    }
+    for (; o < o1; ++o) {
+        float f[V];
+        load_chunk<E, V>(hi, lo, (size_t)o * ld + i, f);
+        const Acc xv = (Acc)__ldg(x + o);
+#pragma unroll
+        for (int e = 0; e < V; ++e) a[0][e] += (Acc)f[e] * xv;
+    }
+#pragma unroll
+    for (int e = 0; e < V; ++e) partial[(size_t)c * inner + i + e] = a[0][e] + a[1][e];
 }
 
 // A CTA owns 32 columns; its warps (up to 32) split the partials, each
@@ -154,16 +263,37 @@ tomos_status launch_sum_parts(const double* part, int64_t nparts, int64_t stride
     return sum_parts(part, nparts, stride, n, alpha, beta, coef, skip, y, st);
 }
 
+// Chunks of the line sums' scratch: of 128 lines, at most 1184.
 int64_t line_sum_chunks(int64_t outer) {
     int64_t c = (outer + 127) / 128;
     if (c > 1184) c = 1184;
     return c < 1 ? 1 : c;
 }
 
-template <Elem E, bool ACC64>
-static tomos_status run_gemv(const GemvLaunch& L, cudaStream_t st) {
+// Segments of a line's dot: 1 while a warp per line fills the GPU (eight
+// warps an SM), else enough CTAs for four an SM, of at least 8192 elements.
+static int64_t line_dot_segments(int64_t outer, int64_t inner) {
+    if (outer >= (int64_t)sm_count() * 8) return 1;
+    int64_t g = ((int64_t)sm_count() * 4 + outer - 1) / (outer > 0 ? outer : 1);
+    if (g > (inner + 8191) / 8192) g = (inner + 8191) / 8192;
+    return g < 1 ? 1 : g;
+}
+
+template <Elem E, bool ACC64, int V>
+static tomos_status run_gemv_v(const GemvLaunch& L, cudaStream_t st) {
     using Acc = typename AccT<ACC64>::T;
     if (L.dot) {
+        const int64_t segs = line_dot_segments(L.outer, L.inner);
+        if (segs > 1 && L.scratch && L.scratch_bytes >= (size_t)segs * L.outer * sizeof(double)) {
+            const int64_t unit = 256 * V;
+            const int64_t seg = ((L.inner + segs - 1) / segs + unit - 1) / unit * unit;
+            const int64_t ns = (L.inner + seg - 1) / seg;
+            double* partial = static_cast<double*>(L.scratch);
+            line_dot_seg_kernel<E, ACC64, V><<<dim3((unsigned)L.outer, (unsigned)ns), 256, 0, st>>>(
+                L.hi, L.lo, L.inner, L.ld, L.x, seg, L.outer, L.skip, partial);
+            TOMOS_LAUNCH_CHECK("line_dot_seg_kernel");
+            return sum_parts(partial, ns, L.outer, L.outer, L.alpha, L.beta, L.coef, L.skip, L.y, st);
+        }
         int64_t blocks = (L.outer + 7) / 8;
         int64_t cap = (int64_t)sm_count() * 8;
         if (blocks > cap) blocks = cap;
@@ -173,18 +303,37 @@ static tomos_status run_gemv(const GemvLaunch& L, cudaStream_t st) {
         TOMOS_LAUNCH_CHECK("line_dot_kernel");
         return TOMOS_OK;
     }
+    const int64_t xb = (L.inner + 256 * V - 1) / (256 * V);
     int64_t nchunks = line_sum_chunks(L.outer);
     size_t need = (size_t)nchunks * (size_t)L.inner * sizeof(Acc);
     if (L.scratch_bytes < need || !L.scratch)
         return fail(TOMOS_ERR_INVALID,
                     "tomos_gemv: scratch too small (need " + std::to_string(need) + " bytes)");
-    int64_t lpc = (L.outer + nchunks - 1) / nchunks;
-    dim3 grid((unsigned)((L.inner + 255) / 256), (unsigned)nchunks);
+    // few, long lines (a column-major A x): chunks of at least eight lines
+    // until eight CTAs an SM, as far as the scratch holds their partials
+    int64_t more = ((int64_t)sm_count() * 8 + xb - 1) / xb;
+    if (more > (L.outer + 7) / 8) more = (L.outer + 7) / 8;
+    const int64_t fit = (int64_t)(L.scratch_bytes / ((size_t)L.inner * sizeof(Acc)));
+    if (more > fit) more = fit;
+    if (more > nchunks) nchunks = more;
+    const int64_t lpc = (L.outer + nchunks - 1) / nchunks;
+    nchunks = (L.outer + lpc - 1) / lpc;
+    dim3 grid((unsigned)xb, (unsigned)nchunks);
     Acc* partial = static_cast<Acc*>(L.scratch);
-    line_sum_partial_kernel<E, ACC64><<<grid, 256, 0, st>>>(L.hi, L.lo, L.outer, L.inner, L.ld,
-                                                            L.x, lpc, L.skip, partial);
+    line_sum_partial_kernel<E, ACC64, V><<<grid, 256, 0, st>>>(L.hi, L.lo, L.outer, L.inner, L.ld,
+                                                               L.x, lpc, L.skip, partial);
     TOMOS_LAUNCH_CHECK("line_sum_partial_kernel");
     return sum_parts(partial, nchunks, L.inner, L.inner, L.alpha, L.beta, L.coef, L.skip, L.y, st);
+}
+
+// 16-byte loads where every line starts on a 16-byte boundary.
+template <Elem E, bool ACC64>
+static tomos_status run_gemv(const GemvLaunch& L, cudaStream_t st) {
+    constexpr bool TWO = E == Elem::A16 || E == Elem::AB16 || E == Elem::AB16R;
+    const int esz = E == Elem::F32 ? 4 : 2;
+    const bool vec = (L.ld * esz) % 16 == 0 && reinterpret_cast<uintptr_t>(L.hi) % 16 == 0 &&
+                     (!TWO || reinterpret_cast<uintptr_t>(L.lo) % 16 == 0);
+    return vec ? run_gemv_v<E, ACC64, ChunkElems<E>::value>(L, st) : run_gemv_v<E, ACC64, 1>(L, st);
 }
 
 template <Elem E>
@@ -245,7 +394,11 @@ size_t gemv_scratch_bytes_max(const tomos_dense* A, int32_t trans) {
     bool dot;
     int64_t outer, inner;
     std::string why;
-    if (!gemv_shape(A, trans, &dot, &outer, &inner, &why) || dot) return 0;
+    if (!gemv_shape(A, trans, &dot, &outer, &inner, &why)) return 0;
+    if (dot) {
+        const int64_t segs = line_dot_segments(outer, inner);
+        return segs > 1 ? (size_t)segs * (size_t)outer * sizeof(double) : 0;
+    }
     const size_t generic = (size_t)line_sum_chunks(outer) * (size_t)inner * 8;
     const size_t rowpass = rowpass_gemv_scratch_bytes(outer, inner);
     return generic > rowpass ? generic : rowpass;

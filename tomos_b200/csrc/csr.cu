@@ -47,9 +47,8 @@ struct CsrPassParams {
     int write_u;            // 0: A p only feeds the transposed product
 };
 
-// One kernel, three uses: the fused LSQR pass (write_u, qpart, sspart),
-// the plain product (write_u only: y = cp A p + cu y) and the transposed
-// product (qpart only, with u_in as the input vector and cp = 0, cu = 1).
+// The fused LSQR pass (write_u, qpart, sspart) when the column-major copy
+// below does not fit, or for a refine copy.
 template <Elem E, bool ACC64>
 __global__ void __launch_bounds__(256) csr_pass_kernel(CsrPassParams P) {
     if (P.skip && *P.skip) return;
@@ -114,16 +113,97 @@ __global__ void __launch_bounds__(256) csr_pass_kernel(CsrPassParams P) {
     }
 }
 
-// y[j] = alpha * sum_c part[c][j] + beta * y[j] (fixed order).
-__global__ void csr_trans_reduce_kernel(const float* __restrict__ part, int g, int64_t stride,
-                                        int64_t n, double alpha, double beta, float* __restrict__ y) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    double s = 0.0;
-    for (int c = 0; c < g; ++c) s += (double)part[(size_t)c * stride + j];
-    double r = alpha * s;
-    if (beta != 0.0) r += beta * (double)y[j];
-    y[j] = (float)r;
+// The transposed product's partials, q_c = sum over CTA c's rows of
+// u_i A[i, :], accumulated as csr_pass_kernel does (a warp-private vector in
+// shared memory, the warp's rows in order).  Bound by the chain of loads a
+// row needs (extent, entries, accumulators): kTransRows rows' entries are
+// loaded while the rows before them are added, so a row costs its
+// shared-memory update (2e6 rows of 20 entries into 5000 columns: 1.78 ms
+// with a row at a time).
+constexpr int kTransRows = 16;
+
+template <Elem E>
+__global__ void __launch_bounds__(256) csr_trans_kernel(CsrPassParams P) {
+    extern __shared__ __align__(16) float qacc[];  // nw x n_pad
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int64_t npad = P.qstride;
+    const uint32_t n = (uint32_t)P.n;
+    float* acc = qacc + (size_t)w * npad;
+    for (int64_t j = lane; j < npad; j += 32) acc[j] = 0.0f;
+    __syncwarp();
+    const int64_t per = (P.m + gridDim.x - 1) / gridDim.x;
+    const int64_t r0 = (int64_t)blockIdx.x * per;
+    int64_t r1 = r0 + per;
+    if (r1 > P.m) r1 = P.m;
+    // row t of a batch starting at i0 is i0 + t nw; lane t holds its extent
+    // and u (an empty extent past the CTA's rows)
+    int32_t ks = 0, ke = 0;
+    float us = 0.0f;
+    auto rows = [&](int64_t i0) {
+        const int64_t i = i0 + (int64_t)lane * nw;
+        const bool in = lane < kTransRows && i < r1;
+        ks = in ? __ldg(P.row_ptrs + i) : 0;
+        ke = in ? __ldg(P.row_ptrs + i + 1) : 0;
+        us = in ? __ldg(P.u_in + i) : 0.0f;
+    };
+    // the entries in flight stay raw words: decoded where they are loaded,
+    // each would be waited for before the next
+    constexpr bool TWO = E == Elem::A16 || E == Elem::AB16 || E == Elem::AB16R;
+    int32_t c[kTransRows];
+    uint32_t h[kTransRows], l[TWO ? kTransRows : 1];
+    auto entries = [&]() {
+#pragma unroll
+        for (int t = 0; t < kTransRows; ++t) {
+            const int32_t k = __shfl_sync(0xffffffffu, ks, t) + lane;
+            const bool in = k < __shfl_sync(0xffffffffu, ke, t);
+            c[t] = -1;
+            h[t] = 0u;
+            if constexpr (TWO) l[t] = 0u;
+            if (in) {
+                c[t] = __ldg(P.col_idxs + k);
+                if constexpr (E == Elem::F32) h[t] = __ldg(static_cast<const uint32_t*>(P.hi) + k);
+                else h[t] = __ldg(static_cast<const uint16_t*>(P.hi) + k);
+                if constexpr (TWO) l[t] = __ldg(static_cast<const uint16_t*>(P.lo) + k);
+            }
+        }
+    };
+    const int64_t step = (int64_t)kTransRows * nw;
+    rows(r0 + w);
+    entries();
+    for (int64_t i0 = r0 + w; i0 < r1; i0 += step) {
+        const int32_t ks0 = ks, ke0 = ke;
+        const float us0 = us;
+        int32_t cc[kTransRows];
+        float vv[kTransRows];
+#pragma unroll
+        for (int t = 0; t < kTransRows; ++t) {
+            cc[t] = c[t];
+            vv[t] = word_value<E>(h[t], TWO ? l[t] : 0u);
+        }
+        rows(i0 + step);
+        entries();
+#pragma unroll
+        for (int t = 0; t < kTransRows; ++t) {
+            const float u = __shfl_sync(0xffffffffu, us0, t);
+            if ((uint32_t)cc[t] < n) acc[cc[t]] = fmaf(vv[t], u, acc[cc[t]]);
+            const int32_t k0 = __shfl_sync(0xffffffffu, ks0, t), k1 = __shfl_sync(0xffffffffu, ke0, t);
+            __syncwarp();
+            for (int32_t k = k0 + 32 + lane; k - lane < k1; k += 32) {  // a row longer than a warp
+                if (k < k1) {
+                    const int32_t cl = __ldg(P.col_idxs + k);
+                    if ((uint32_t)cl < n) acc[cl] = fmaf(load_elem<E>(P.hi, P.lo, k), u, acc[cl]);
+                }
+                __syncwarp();
+            }
+        }
+    }
+    __syncthreads();
+    float* out = P.qpart + (size_t)blockIdx.x * npad;
+    for (int64_t j = threadIdx.x; j < P.n; j += blockDim.x) {
+        float sum = 0.0f;
+        for (int k = 0; k < nw; ++k) sum += qacc[(size_t)k * npad + j];
+        out[j] = sum;
+    }
 }
 
 static int csr_warps_for(int64_t n) {
@@ -158,6 +238,30 @@ static tomos_status launch_csr(Elem e, bool acc64, const CsrPassParams& P, int g
         case Elem::A16: return launch_csr_t<Elem::A16, true>(P, grid, warps, st);
         case Elem::AB16: return launch_csr_t<Elem::AB16, true>(P, grid, warps, st);
         case Elem::AB16R: return launch_csr_t<Elem::AB16R, true>(P, grid, warps, st);
+        default: return fail(TOMOS_ERR_UNSUPPORTED, "csr: element type");
+    }
+}
+
+template <Elem E>
+static tomos_status launch_trans_t(const CsrPassParams& P, int grid, int warps, cudaStream_t st) {
+    const size_t smem = (size_t)warps * P.qstride * sizeof(float);
+    if (smem > 48 * 1024)
+        TOMOS_CUDA_TRY(cudaFuncSetAttribute(csr_trans_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)smem));
+    csr_trans_kernel<E><<<grid, warps * 32, smem, st>>>(P);
+    TOMOS_LAUNCH_CHECK("csr_trans_kernel");
+    return TOMOS_OK;
+}
+
+static tomos_status launch_trans(Elem e, const CsrPassParams& P, int grid, int warps, cudaStream_t st) {
+    switch (e) {
+        case Elem::F32: return launch_trans_t<Elem::F32>(P, grid, warps, st);
+        case Elem::H16: return launch_trans_t<Elem::H16>(P, grid, warps, st);
+        case Elem::F16: return launch_trans_t<Elem::F16>(P, grid, warps, st);
+        case Elem::B16: return launch_trans_t<Elem::B16>(P, grid, warps, st);
+        case Elem::A16: return launch_trans_t<Elem::A16>(P, grid, warps, st);
+        case Elem::AB16: return launch_trans_t<Elem::AB16>(P, grid, warps, st);
+        case Elem::AB16R: return launch_trans_t<Elem::AB16R>(P, grid, warps, st);
         default: return fail(TOMOS_ERR_UNSUPPORTED, "csr: element type");
     }
 }
@@ -398,17 +502,25 @@ __global__ void __launch_bounds__(kRowsThreads, 4) csr_rows_kernel(CsrPassParams
     const uint32_t n = (uint32_t)P.n;
     const int64_t step = (int64_t)gridDim.x * nw * 2 * rpw;
     double ss = 0.0;
-    for (int64_t base = ((int64_t)blockIdx.x * nw + w) * 2 * rpw; base < P.m; base += step) {
+    // the extents of a round's two rows, loaded a round ahead
+    int32_t na0 = 0, na1 = 0, nb0 = 0, nb1 = 0;
+    auto extents = [&](int64_t base) {
         const int64_t ia = base + grp, ib = base + rpw + grp;
-        int32_t ka0 = 0, ka1 = 0, kb0 = 0, kb1 = 0;
+        na0 = na1 = nb0 = nb1 = 0;
         if (dot && ia < P.m) {
-            ka0 = __ldg(P.row_ptrs + ia);
-            ka1 = __ldg(P.row_ptrs + ia + 1);
+            na0 = __ldg(P.row_ptrs + ia);
+            na1 = __ldg(P.row_ptrs + ia + 1);
         }
         if (dot && ib < P.m) {
-            kb0 = __ldg(P.row_ptrs + ib);
-            kb1 = __ldg(P.row_ptrs + ib + 1);
+            nb0 = __ldg(P.row_ptrs + ib);
+            nb1 = __ldg(P.row_ptrs + ib + 1);
         }
+    };
+    extents(((int64_t)blockIdx.x * nw + w) * 2 * rpw);
+    for (int64_t base = ((int64_t)blockIdx.x * nw + w) * 2 * rpw; base < P.m; base += step) {
+        const int64_t ia = base + grp, ib = base + rpw + grp;
+        const int32_t ka0 = na0, ka1 = na1, kb0 = nb0, kb1 = nb1;
+        extents(base + step);
         Dot da = 0, db = 0;
         {
             int32_t ca[4], cb[4];
@@ -755,11 +867,10 @@ __global__ void csr_fro2_kernel(const void* hi, const void* lo, const int32_t* c
 }
 
 __global__ void csr_sum_kernel(const double* part, int np, double* out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int k = 0; k < np; ++k) s += part[k];
-        *out = s;
-    }
+    double s = 0.0;
+    for (int k = threadIdx.x; k < np; k += 32) s += part[k];
+    s = warp_sum(s);
+    if (threadIdx.x == 0) *out = s;
 }
 
 tomos_status CsrPass::fro2(double* out, const double* d, cudaStream_t st) {
@@ -914,11 +1025,11 @@ __global__ void csr_col_reduce_kernel(const double* part, int64_t nparts, int64_
 }
 
 __global__ void cs_csr_fro_reduce(const double* part, int64_t np, double* out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int64_t k = 0; k < np; ++k) s += part[k];
-        *out = s;
-    }
+    __shared__ double sm[32];
+    double s = 0.0;
+    for (int64_t k = threadIdx.x; k < np; k += blockDim.x) s += part[k];
+    s = block_sum(s, sm);
+    if (threadIdx.x == 0) *out = s;
 }
 
 }  // namespace tomos_b200
@@ -980,10 +1091,8 @@ tomos_status tomos_csr_gemv(int32_t trans, double alpha, const tomos_csr* A, int
     if (!scratch || scratch_bytes < need)
         return fail(TOMOS_ERR_INVALID, "tomos_csr_gemv: scratch too small (need " + std::to_string(need) + " bytes)");
     if (A->rows == 0) {
-        csr_trans_reduce_kernel<<<(unsigned)((A->cols + 255) / 256), 256, 0, st>>>(
-            static_cast<float*>(scratch), 0, P.qstride, A->cols, alpha, beta, y);
-        TOMOS_LAUNCH_CHECK("csr_trans_reduce_kernel");
-        return TOMOS_OK;
+        return launch_sum_parts(static_cast<const float*>(scratch), 0, P.qstride, A->cols, alpha, beta, nullptr,
+                                nullptr, y, st);
     }
     P.p = nullptr;
     P.u_in = x;
@@ -992,12 +1101,9 @@ tomos_status tomos_csr_gemv(int32_t trans, double alpha, const tomos_csr* A, int
     P.cu_h = 1.0;
     P.qpart = static_cast<float*>(scratch);
     P.write_u = 0;
-    tomos_status s = launch_csr(e, elem_is_exact(e), P, grid, csr_warps_for(A->cols), st);
+    tomos_status s = launch_trans(e, P, grid, csr_warps_for(A->cols), st);
     if (s) return s;
-    csr_trans_reduce_kernel<<<(unsigned)((A->cols + 255) / 256), 256, 0, st>>>(
-        P.qpart, grid, P.qstride, A->cols, alpha, beta, y);
-    TOMOS_LAUNCH_CHECK("csr_trans_reduce_kernel");
-    return TOMOS_OK;
+    return launch_sum_parts(P.qpart, grid, P.qstride, A->cols, alpha, beta, nullptr, nullptr, y, st);
 }
 
 tomos_status tomos_lsqr_solve_csr(const tomos_csr* A, const float* b, float* x,
@@ -1114,7 +1220,7 @@ tomos_status tomos_countsketch_apply_csr(const tomos_csr* A, int32_t tier, int64
 #undef TOMOS_CS_CSR
     TOMOS_LAUNCH_CHECK("cs_csr_kernel");
     if (fro2) {
-        cs_csr_fro_reduce<<<1, 32, 0, st>>>(c.fro_part, grid, fro2);
+        cs_csr_fro_reduce<<<1, 1024, 0, st>>>(c.fro_part, grid, fro2);
         TOMOS_LAUNCH_CHECK("cs_csr_fro_reduce");
     }
     if (colsq) {

@@ -204,3 +204,20 @@ def test_mm_split_k(orc, numeric, tier, beta):
     # summation error grows with K)
     assert np.all(np.abs(b - ref) <= 1e-4 * S)
     assert np.abs(a - ref).max() <= np.abs(b - ref).max()
+
+
+@pytest.mark.parametrize("numeric", [NT.FP32_16, NT.FP32_BF16, NT.FP16])
+@pytest.mark.parametrize("la,lb", [(L.COL_MAJOR, L.COL_MAJOR), (L.ROW_MAJOR, L.ROW_MAJOR),
+                                   (L.ROW_MAJOR, L.COL_MAJOR)])
+@pytest.mark.parametrize("M,N,K,pad", [(1290, 1210, 300, 0), (1400, 2500, 257, 0), (1281, 1283, 1001, 3)])
+def test_mm_packed_operands(orc, numeric, la, lb, M, N, K, pad):
+    """Products with enough 128 x 128 (or 256) tiles for the packed 16-bit
+    kernel: ragged tiles and K stages, lines along K and across it, aligned
+    or not, beta, row-major C."""
+    rng = np.random.default_rng(M + N + K)
+    A0 = (rng.standard_normal((M, K)) * np.where(rng.random((M, K)) < 0.02, 1e-6, 1.0)).astype(np.float32)
+    A = to_dense(A0, la, numeric, pad=pad)
+    check(orc, A, A0, tb.Tier.HALF_OPERANDS, T.NO_TRANSPOSE, T.NO_TRANSPOSE, (K, N), (lb, L.COL_MAJOR), 0.0, rng,
+          bf16_ops=numeric == NT.FP32_BF16)
+    check(orc, A, A0, tb.Tier.HALF_OPERANDS, T.NO_TRANSPOSE, T.NO_TRANSPOSE, (K, N), (lb, L.ROW_MAJOR), -0.5, rng,
+          bf16_ops=numeric == NT.FP32_BF16)

@@ -38,6 +38,9 @@
 // applied in FP64 in the epilogue.  The error of an entry is a few units
 // of 2^-22 times sum_l |op(A)_il| |op(B)_lj| plus FP32 summation over K.
 //
+// Large kPure16 products take packed operands and a converter-free kernel
+// (gemm_packed_kernel below).
+//
 // Every mbarrier wait is bounded (mbarrier.cuh): a wait that expires
 // records an error word and the CTA stops work, drains its MMAs (bounded
 // again), frees its tensor memory and exits; such a launch's C is
@@ -929,6 +932,266 @@ __global__ void __launch_bounds__(kTmaThreads, 2) gemm_tma_kernel(GemmArgs g, co
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
 }
 
+// ------------------------------------------------- packed 16-bit products
+//
+// Large products on 16-bit operands.  In the pipelines above the converter
+// warps bound these (every CTA re-reads, rounds and re-tiles B for its 128
+// rows: 269 TF/s at 4096^3, tensor pipe ~14 % busy).  Here two small kernels
+// first write op(A)'s fp16 (bf16) values and op(B) rounded to that type as
+// K-major planes in the caller's scratch, and the product then runs without
+// converters: TMA copies of 128-byte-swizzled tiles straight into the MMA's
+// operands, 128 x BN output tiles, one persistent CTA an SM walking the
+// tiles with two accumulators in tensor memory, so that a tile's epilogue
+// overlaps the next tile's products.  Same operands, same FP32 accumulation
+// over K in one accumulator as the unpacked kernels.
+
+// Lines along K (the source's K stride is 1): eight values a thread.
+template <Elem E>
+__global__ void __launch_bounds__(256) pack16_lines_kernel(const void* src, int64_t line_stride, int64_t lines,
+                                                           int64_t K, int64_t Kp, uint16_t* dst) {
+    const int64_t per = Kp / 8;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < lines * per;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = t / per, l = (t - i * per) * 8;
+        const size_t base = (size_t)(i * line_stride + l);
+        uint32_t b[8];
+        if constexpr (E == Elem::H16 || E == Elem::F16 || E == Elem::B16) {
+            const uint16_t* p = static_cast<const uint16_t*>(src) + base;
+            if (l + 8 <= K && reinterpret_cast<uintptr_t>(p) % 16 == 0) {
+                *reinterpret_cast<uint4*>(dst + (size_t)i * Kp + l) =
+                    half_operands<E>(__ldg(reinterpret_cast<const uint4*>(p)));
+                continue;
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) b[e] = l + e < K ? bits16<E>(__ldg(p + e)) : 0u;
+        }
+        *reinterpret_cast<uint4*>(dst + (size_t)i * Kp + l) =
+            make_uint4(b[0] | (b[1] << 16), b[2] | (b[3] << 16), b[4] | (b[5] << 16), b[6] | (b[7] << 16));
+    }
+}
+
+template <bool BF>
+__global__ void __launch_bounds__(256) pack32_lines_kernel(const float* src, int64_t line_stride, int64_t lines,
+                                                           int64_t K, int64_t Kp, uint16_t* dst) {
+    const int64_t per = Kp / 8;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < lines * per;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = t / per, l = (t - i * per) * 8;
+        const float* p = src + (size_t)(i * line_stride + l);
+        float v[8];
+        if (l + 8 <= K && reinterpret_cast<uintptr_t>(p) % 16 == 0) {
+            const float4 f0 = __ldg(reinterpret_cast<const float4*>(p)), f1 = __ldg(reinterpret_cast<const float4*>(p) + 1);
+            v[0] = f0.x; v[1] = f0.y; v[2] = f0.z; v[3] = f0.w;
+            v[4] = f1.x; v[5] = f1.y; v[6] = f1.z; v[7] = f1.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = l + e < K ? __ldg(p + e) : 0.0f;
+        }
+        *reinterpret_cast<uint4*>(dst + (size_t)i * Kp + l) =
+            make_uint4(pack16x2<BF>(v[0], v[1]), pack16x2<BF>(v[2], v[3]), pack16x2<BF>(v[4], v[5]),
+                       pack16x2<BF>(v[6], v[7]));
+    }
+}
+
+// Lines strided along K (the source is contiguous across lines): 64 x 64
+// tiles through shared memory, read across lines and written along K.
+// E: F32 (op(B), rounded to fp16, or bf16 with BF) or a 16-bit type.
+template <Elem E, bool BF>
+__global__ void __launch_bounds__(256) pack_transpose_kernel(const void* src, int64_t k_stride, int64_t lines,
+                                                             int64_t K, int64_t Kp, uint16_t* dst) {
+    __shared__ uint16_t tile[64][72];  // [line][k]; 144-byte rows keep 16-byte reads aligned
+    const int64_t i0 = (int64_t)blockIdx.x * 64, l0 = (int64_t)blockIdx.y * 64;
+    const int c = threadIdx.x & 63, r0 = threadIdx.x >> 6;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const int k = r0 + 4 * j;
+        const int64_t i = i0 + c, l = l0 + k;
+        uint32_t b = 0;
+        if (i < lines && l < K) {
+            const size_t idx = (size_t)(l * k_stride + i);
+            if constexpr (E == Elem::F32) b = to16<BF>(__ldg(static_cast<const float*>(src) + idx));
+            else b = bits16<E>(__ldg(static_cast<const uint16_t*>(src) + idx));
+        }
+        tile[c][k] = (uint16_t)b;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int u = threadIdx.x + 256 * j, line = u >> 3, k = (u & 7) * 8;
+        if (i0 + line < lines && l0 + k < Kp)
+            *reinterpret_cast<uint4*>(dst + (size_t)(i0 + line) * Kp + l0 + k) =
+                *reinterpret_cast<const uint4*>(&tile[line][k]);
+    }
+}
+
+constexpr int kPackK = 64;         // K per stage (128 bytes)
+constexpr int kPackThreads = 256;  // warp 0: copies, warp 1: MMAs, warps 4-7: epilogue
+
+struct PackMaps {
+    CUtensorMap a, b;
+};
+
+struct PackArgs {
+    float* c;
+    int64_t c_si, c_sj;
+    int64_t M, N;
+    int nk;            // K stages a tile
+    int tm, tiles;     // tiles along M, all tiles
+    double alpha, beta;
+    int* err;
+};
+
+template <bool BF, int BN>
+struct PackTraits {
+    static constexpr uint32_t a_bytes = kGemmM * 128u, b_bytes = BN * 128u;
+    static constexpr uint32_t stage = a_bytes + b_bytes;
+    static constexpr int stages = BN == 256 ? 4 : 6;
+    static constexpr size_t smem = (size_t)stages * stage + 1024 + 256;
+};
+
+template <bool BF, int BN>
+__global__ void __launch_bounds__(kPackThreads, 1) gemm_packed_kernel(PackArgs g, const __grid_constant__ PackMaps maps) {
+    using T = PackTraits<BF, BN>;
+    constexpr int S = T::stages;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)S * T::stage);
+    uint64_t* empty = full + S;
+    uint64_t* tfull = empty + S;   // accumulator a holds a finished tile
+    uint64_t* tempty = tfull + 2;  // ... has been read
+    uint64_t* done = tempty + 2;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tslot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(&tfull[a], 1);
+            mbar_init(&tempty[a], 4);
+        }
+        mbar_init(done, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)),
+                     "r"(2u * BN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tslot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int issued = 0;
+            for (int tile = blockIdx.x; tile < g.tiles && !*abort_flag; tile += gridDim.x) {
+                const int m0 = (tile % g.tm) * kGemmM, n0 = (tile / g.tm) * BN;
+                for (int kt = 0; kt < g.nk; ++kt, ++issued) {
+                    const int s = issued % S;
+                    if (issued >= S && !mbar_wait(&empty[s], (uint32_t)((issued / S - 1) & 1))) {
+                        atomicExch(g.err, 5);
+                        *abort_flag = 1;
+                    }
+                    if (*abort_flag) break;
+                    const uint32_t st = smem_addr(smem + (size_t)s * T::stage);
+                    mbar_expect_tx(&full[s], T::stage);
+                    tma2d(st, &maps.a, kt * kPackK, m0, &full[s]);
+                    tma2d(st + T::a_bytes, &maps.b, kt * kPackK, n0, &full[s]);
+                }
+            }
+            // no copy may still be writing this CTA's memory when it exits
+            for (int k = issued > S ? issued - S : 0; k < issued; ++k)
+                if (!mbar_wait(&full[k % S], (uint32_t)((k / S) & 1))) atomicExch(g.err, 6);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            uint32_t idesc = (1u << 4);  // FP32 accumulator, K-major operands
+            const uint32_t fmt = BF ? 1u : 0u;
+            idesc |= fmt << 7;
+            idesc |= fmt << 10;
+            idesc |= ((uint32_t)BN >> 3) << 17;
+            idesc |= ((uint32_t)kGemmM >> 4) << 24;
+            int used = 0, nt = 0;
+            for (int tile = blockIdx.x; tile < g.tiles && !*abort_flag; tile += gridDim.x, ++nt) {
+                const int a = nt & 1;
+                if (nt >= 2 && !mbar_wait(&tempty[a], (uint32_t)((nt / 2 - 1) & 1))) {
+                    atomicExch(g.err, 7);
+                    *abort_flag = 1;
+                }
+                tc_fence_after();
+                uint32_t acc = 0;
+                for (int kt = 0; kt < g.nk; ++kt, ++used) {
+                    const int s = used % S;
+                    if (!*abort_flag && !mbar_wait(&full[s], (uint32_t)((used / S) & 1))) {
+                        atomicExch(g.err, 2);
+                        *abort_flag = 1;
+                    }
+                    if (*abort_flag) break;
+                    tc_fence_after();
+                    const uint32_t st = smem_addr(smem + (size_t)s * T::stage);
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks) {
+                        mma_issue(0, tmem + (uint32_t)(a * BN), sw128_desc(st, ks), sw128_desc(st + T::a_bytes, ks), idesc,
+                                  acc);
+                        acc = 1;
+                    }
+                    mma_commit(&empty[s]);
+                }
+                mma_commit(&tfull[a]);
+            }
+            mma_commit(done);
+            if (!mbar_wait(done, 0u)) atomicExch(g.err, 4);  // before the memory is freed
+        }
+    } else if (warp >= 4) {
+        const int q = warp & 3;
+        int nt = 0;
+        for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x, ++nt) {
+            const int a = nt & 1;
+            bool ok = !*abort_flag && mbar_wait(&tfull[a], (uint32_t)((nt / 2) & 1));
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok || *abort_flag) {
+                if (lane == 0) {
+                    atomicExch(g.err, 3);
+                    *abort_flag = 1;
+                }
+                break;
+            }
+            tc_fence_after();
+            const int64_t i = (int64_t)(tile % g.tm) * kGemmM + q * 32 + lane;
+            const int64_t n0 = (int64_t)(tile / g.tm) * BN;
+            for (int c = 0; c < BN; c += 8) {
+                uint32_t v[8];
+                tmem_ld8(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * BN + c), v);
+                if (i >= g.M) continue;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int64_t j = n0 + c + e;
+                    if (j >= g.N) break;
+                    float* cp = g.c + (size_t)(i * g.c_si + j * g.c_sj);
+                    double y = g.alpha * (double)u2f(v[e]);
+                    if (g.beta != 0.0) y += g.beta * (double)*cp;
+                    *cp = (float)y;
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty[a]);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * BN) : "memory");
+}
+
 // The word a bounded wait of these launches records its expiry in.
 __device__ int g_gemm_err;
 constexpr int kMaxDevices = 64;
@@ -1059,6 +1322,93 @@ tomos_status launch_gemm(GemmArgs& g, cudaStream_t st) {
     kern<<<grid, kGemmThreads, smem, st>>>(g);
     TOMOS_LAUNCH_CHECK("gemm_tc_kernel");
     return TOMOS_OK;
+}
+
+// Columns of a packed product's tiles, or 0 when the unpacked kernels are
+// used: fewer tiles than two thirds of the SMs (those kernels split K), a K
+// too short to repay the packing passes, or planes past 2 GiB of scratch.
+// 256 columns halve A's re-reads; 128 when their last wave wastes less.
+size_t packed_bytes(const GemmArgs& g);
+int packed_bn(const GemmArgs& g, int mode) {
+    if (mode != kPure16 || g.K < 256 || g.K > 65535 * 64 || packed_bytes(g) > ((size_t)2 << 30)) return 0;
+    const int64_t sms = sm_count(), tm = (g.M + kGemmM - 1) / kGemmM;
+    const int64_t t256 = tm * ((g.N + 255) / 256), t128 = tm * ((g.N + 127) / 128);
+    if (3 * t128 < 2 * sms) return 0;
+    const int64_t w256 = (t256 + sms - 1) / sms * 8, w128 = (t128 + sms - 1) / sms * 5;
+    return w256 <= w128 ? 256 : 128;
+}
+
+int64_t packed_ld(int64_t K) { return (K + 7) / 8 * 8; }
+size_t packed_plane(int64_t lines, int64_t K) { return ((size_t)lines * packed_ld(K) * 2 + 255) / 256 * 256; }
+size_t packed_bytes(const GemmArgs& g) { return packed_plane(g.M, g.K) + packed_plane(g.N, g.K); }
+
+template <Elem E, bool BF>
+tomos_status pack_operand(const void* src, bool k_contig, int64_t stride, int64_t lines, int64_t K, uint16_t* dst,
+                          cudaStream_t st) {
+    const int64_t Kp = packed_ld(K);
+    if (k_contig) {
+        int64_t blocks = (lines * (Kp / 8) + 255) / 256;
+        if (blocks > (int64_t)sm_count() * 16) blocks = (int64_t)sm_count() * 16;
+        if constexpr (E == Elem::F32)
+            pack32_lines_kernel<BF><<<(unsigned)blocks, 256, 0, st>>>(static_cast<const float*>(src), stride, lines, K,
+                                                                      Kp, dst);
+        else
+            pack16_lines_kernel<E><<<(unsigned)blocks, 256, 0, st>>>(src, stride, lines, K, Kp, dst);
+    } else {
+        pack_transpose_kernel<E, BF><<<dim3((unsigned)((lines + 63) / 64), (unsigned)((Kp + 63) / 64)), 256, 0, st>>>(
+            src, stride, lines, K, Kp, dst);
+    }
+    TOMOS_LAUNCH_CHECK("pack_operand");
+    return TOMOS_OK;
+}
+
+template <Elem E, int BN>
+tomos_status launch_packed(const GemmArgs& g, void* scratch, cudaStream_t st, bool* used) {
+    constexpr bool BF = E == Elem::B16;
+    using T = PackTraits<BF, BN>;
+    uint16_t* ap = static_cast<uint16_t*>(scratch);
+    uint16_t* bp = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(scratch) + packed_plane(g.M, g.K));
+    PackMaps maps;
+    const int64_t Kp = packed_ld(g.K);
+    if (!encode_2d(&maps.a, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, ap, g.K, g.M, Kp, kPackK, kGemmM,
+                   CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !encode_2d(&maps.b, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, bp, g.K, g.N, Kp, kPackK, BN, CU_TENSOR_MAP_SWIZZLE_128B))
+        return TOMOS_OK;
+    *used = true;
+    tomos_status s = pack_operand<E, BF>(g.a_hi, g.a_kc != 0, g.a_kc ? g.a_si : g.a_sl, g.M, g.K, ap, st);
+    if (s) return s;
+    s = pack_operand<Elem::F32, BF>(g.b, g.b_kc != 0, g.b_kc ? g.b_sj : g.b_sl, g.N, g.K, bp, st);
+    if (s) return s;
+    PackArgs a;
+    a.c = g.c;
+    a.c_si = g.c_si;
+    a.c_sj = g.c_sj;
+    a.M = g.M;
+    a.N = g.N;
+    a.nk = (int)((g.K + kPackK - 1) / kPackK);
+    a.tm = (int)((g.M + kGemmM - 1) / kGemmM);
+    a.tiles = a.tm * (int)((g.N + BN - 1) / BN);
+    a.alpha = g.alpha;
+    a.beta = g.beta;
+    a.err = g.err;
+    auto kern = gemm_packed_kernel<BF, BN>;
+    TOMOS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem));
+    const int grid = a.tiles < sm_count() ? a.tiles : sm_count();
+    kern<<<grid, kPackThreads, T::smem, st>>>(a, maps);
+    TOMOS_LAUNCH_CHECK("gemm_packed_kernel");
+    return TOMOS_OK;
+}
+
+tomos_status launch_packed_e(Elem e, int bn, const GemmArgs& g, void* scratch, cudaStream_t st, bool* used) {
+    switch (e) {
+        case Elem::H16: return bn == 256 ? launch_packed<Elem::H16, 256>(g, scratch, st, used)
+                                         : launch_packed<Elem::H16, 128>(g, scratch, st, used);
+        case Elem::F16: return bn == 256 ? launch_packed<Elem::F16, 256>(g, scratch, st, used)
+                                         : launch_packed<Elem::F16, 128>(g, scratch, st, used);
+        case Elem::B16: return bn == 256 ? launch_packed<Elem::B16, 256>(g, scratch, st, used)
+                                         : launch_packed<Elem::B16, 128>(g, scratch, st, used);
+        default: return TOMOS_OK;
+    }
 }
 
 template <int MODE>
@@ -1226,6 +1576,7 @@ size_t tomos_mm_scratch_bytes(int32_t trans_a, int32_t trans_b, const tomos_dens
     int mode;
     if (mm_prepare(trans_a, trans_b, 1.0, A, tier, B, 0.0, &C, &g, &e, &mode) != TOMOS_OK) return 0;
     if (g.M == 0 || g.N == 0 || g.K == 0) return 0;
+    if (packed_bn(g, mode)) return packed_bytes(g);
     int per;
     const int splits = split_count(g, mode, &per);
     return splits > 1 ? (size_t)splits * (size_t)g.M * (size_t)g.N * sizeof(float) : 0;
@@ -1250,6 +1601,14 @@ tomos_status tomos_mm_ex(int32_t trans_a, int32_t trans_b, double alpha, const t
                                                                                  beta);
         TOMOS_LAUNCH_CHECK("gemm_scale_c_kernel");
         return TOMOS_OK;
+    }
+    // large 16-bit products through packed operands, where the scratch holds
+    // them (16-byte aligned, as the copies need)
+    const int pbn = packed_bn(g, mode);
+    if (pbn && scratch && scratch_bytes >= packed_bytes(g) && reinterpret_cast<uintptr_t>(scratch) % 16 == 0) {
+        bool used = false;
+        s = launch_packed_e(e, pbn, g, scratch, st, &used);
+        if (used) return s;
     }
     int splits = split_count(g, mode, &g.kt_per);
     const size_t need = (size_t)splits * (size_t)g.M * (size_t)g.N * sizeof(float);

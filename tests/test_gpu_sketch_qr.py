@@ -235,6 +235,22 @@ def test_qr_panel_and_wide_paths(wide):
     assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-3000:]
 
 
+@pytest.mark.parametrize("k,n,cond", [(8400, 2100, 1.0), (2600, 2080, 1.0), (8400, 2100, 1e5)])
+def test_qr_past_the_plain_wide_columns(k, n, cond):
+    """Past 2048 columns a sketch of near-orthonormal columns takes the wide
+    path, the others (nearly square, or ill conditioned) the panel path;
+    LAPACK's R either way."""
+    rng = np.random.default_rng(k + n)
+    SA = rng.standard_normal((k, n)) * np.logspace(0, 2, n)
+    if cond > 1.0:
+        SA[:, 1900] = SA[:, 1800] + SA[:, 1900] / cond
+    Rinv, R = qr_on_gpu(SA)
+    Rl = np.linalg.qr(SA, mode="r")
+    np.testing.assert_allclose(R, Rl, rtol=1e-8, atol=1e-9 * np.abs(Rl).max())
+    Q = SA @ Rinv
+    np.testing.assert_allclose(Q.T @ Q, np.eye(n), atol=1e-8)
+
+
 def test_qr_rejects_wide_and_singular():
     with pytest.raises(tb.TomosError):
         qr_on_gpu(np.ones((3, 5)))

@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kQrThreads) qr_apply_kernel(double* A, int64_t
 //   panel passes (hr_q1, hr_v) on up to kQrPanelCtas CTAs, then the W
 //   partials and the apply tiles spread over every CTA.
 // The barrier is a counter and a generation word in global memory; waits
-// are bounded (kGridSpinLimit polls with a short sleep), and a CTA whose
+// are bounded (kGridSpinLimit polls, asleep between the later ones), and a CTA whose
 // wait expires sets an error word and leaves, so a broken barrier ends the
 // kernel with an error the host reports instead of hanging the GPU.
 
@@ -517,12 +517,14 @@ struct GridSync {
     int pad;
 };
 
-__device__ bool grid_sync(GridSync* gs, unsigned int& gen, int* sflag) {
+// Barrier over `count` CTAs (all of the grid unless given).
+__device__ bool grid_sync(GridSync* gs, unsigned int& gen, int* sflag, unsigned int count = 0) {
+    if (count == 0) count = gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned int g = gen;
-        if (atomicAdd(&gs->arrive, 1u) == gridDim.x - 1) {
+        if (atomicAdd(&gs->arrive, 1u) == count - 1) {
             atomicExch(&gs->arrive, 0u);
             __threadfence();
             atomicExch(&gs->gen, g + 1u);
@@ -533,7 +535,7 @@ __device__ bool grid_sync(GridSync* gs, unsigned int& gen, int* sflag) {
                     atomicExch(&gs->err, 1);
                     break;
                 }
-                __nanosleep(64);
+                if (k > 512) __nanosleep(64);  // most waits end within a microsecond
             }
         }
         __threadfence();
@@ -918,7 +920,8 @@ static tomos_status trtri_rt(const double* Rt, int64_t n, double* X, int64_t ldx
 
 // ------------------------------------------------------------ wide path
 //
-// For sketches of up to kQrWideMaxN columns, the factorisation is formed
+// For sketches of up to kQrWideMaxN columns (past kQrWidePlainN only well
+// conditioned ones), the factorisation is formed
 // from the whole sketch at once instead of 32-column panels (whose chains
 // leave most SMs waiting at grid barriers):
 //   G = SA^T SA                          (FP64 tensor-core GEMM)
@@ -930,19 +933,30 @@ static tomos_status trtri_rt(const double* Rt, int64_t n, double* X, int64_t ldx
 //   reconstruction of the panel path applied to all n columns, whose S is
 //   the sign LAPACK's dgeqr2 gives row j of R (R_h = S R, R_h^-1 = R^-1 S).
 // It is Cholesky QR once, so it is used only when kappa_F(U) =
-// ||U||_F ||U^-1||_F = sqrt(n) ||U^-1||_F is at most kQrWideMaxKappa (R then
-// agrees with the Householder R to about kappa * 1e-16) and every Cholesky
+// ||U||_F ||U^-1||_F = sqrt(n) ||U^-1||_F is at most kQrWideMaxKappa
+// (kQrWideRms n past kQrWidePlainN columns; R then agrees with the Householder R to about kappa * 1e-16) and every Cholesky
 // pivot is above kQrWideFloor; otherwise the panel path factors SA, which
 // the wide path leaves untouched until it has passed both checks.
 //
 // The two n x n factorisations run in one cooperative launch each
 // (fact_kernel): right-looking in 32-column blocks, one grid barrier a
-// block.  CTA 0 updates the next diagonal block first and factors it
-// (cta_chol / cta_lu_signed, and its inverses) while the other CTAs apply
-// the current block to the rest of the trailing matrix in 32 x 32 tiles.
+// block.  CTA 0 updates the next diagonal block and factors it (cta_chol_inv
+// / cta_lu_signed and its inverses) while the other CTAs form the block's
+// panels, meet, and apply them to the rest of the trailing matrix in 64 x 64
+// tiles.  Bound by CTA 0's chain of 32-column steps, not by the flops.
 
-constexpr int64_t kQrWideMaxN = 2048;
+constexpr int64_t kQrWideMaxN = 8192;
 constexpr double kQrWideMaxKappa = 1e6;
+// Past kQrWidePlainN columns the panel path's Householder steps are backward
+// stable where the Gram's Cholesky loses kappa_2 squared, so only a sketch
+// whose ||U^-1||_F is near that of orthonormal columns (sqrt(n); an RMS
+// inverse singular value of kQrWideRms at most, where a sketch of 4 n rows
+// has 1.15 and one of 2 n rows 1.41) keeps the wide path: there both round
+// alike.  The panel path's panels and blocks took 23 ms at
+// 12000 x 3000, most of it panel latency and updates at a fraction of the
+// FP64 tensor rate.
+constexpr int64_t kQrWidePlainN = 2048;
+constexpr double kQrWideRms = 1.5;
 constexpr double kQrWideFloor = 1e-10;
 
 struct WideScratch {
@@ -952,6 +966,7 @@ struct WideScratch {
     double* d;     // n: column norms of SA
     double* sgn;   // n: S
     double* Xd;    // 2 x 2 x 32 x 32: a diagonal block's inverse factors (by block parity)
+    double* pan;   // 2 x 32 x n: LU panels
     double* kap;   // ||U^-1||_F^2
     double* Tb;    // trtri level products
     double* P;     // GEMM split-K partials
@@ -977,6 +992,7 @@ static WideScratch wide_layout(void* base, int64_t n) {
     w.d = reinterpret_cast<double*>(take(sizeof(double) * nn));
     w.sgn = reinterpret_cast<double*>(take(sizeof(double) * nn));
     w.Xd = reinterpret_cast<double*>(take(sizeof(double) * 4 * kHB * kHB));
+    w.pan = reinterpret_cast<double*>(take(sizeof(double) * 2 * kHB * nn));
     w.kap = reinterpret_cast<double*>(take(sizeof(double) * 2));
     size_t tb = 1;
     for (int64_t b = 32; b < n; b *= 2) {
@@ -984,10 +1000,10 @@ static WideScratch wide_layout(void* base, int64_t n) {
         if (pairs * b * b > tb) tb = pairs * b * b;
     }
     w.Tb = reinterpret_cast<double*>(take(sizeof(double) * tb));
-    w.pcap = 4 * nn * nn;
+    w.pcap = (n > kQrWidePlainN ? 1 : 4) * nn * nn;  // large products fill the GPU unsplit
     w.P = reinterpret_cast<double*>(take(sizeof(double) * w.pcap));
     w.flag = reinterpret_cast<int*>(take(sizeof(int) * 4));
-    w.gs = reinterpret_cast<GridSync*>(take(sizeof(GridSync)));
+    w.gs = reinterpret_cast<GridSync*>(take(2 * sizeof(GridSync)));
     w.bytes = off;
     return w;
 }
@@ -1014,7 +1030,7 @@ __global__ void wide_equilibrate_kernel(double* G, int64_t n, const double* d) {
 }
 
 // ||X||_F^2 of the n x n column-major X: block b sums its contiguous
-// chunk into part[b], then one thread sums the parts in block order.
+// chunk into part[b], then one warp sums the parts in a fixed order.
 __global__ void wide_fro2_part_kernel(const double* X, int64_t total, double* part) {
     __shared__ double sm[32];
     const int64_t chunk = (total + gridDim.x - 1) / gridDim.x;
@@ -1034,11 +1050,10 @@ __global__ void wide_fro2_part_kernel(const double* X, int64_t total, double* pa
 }
 
 __global__ void wide_fro2_sum_kernel(const double* part, int np, double* out) {
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int b = 0; b < np; ++b) t += part[b];
-        *out = t;
-    }
+    double t = 0.0;
+    for (int b = threadIdx.x; b < np; b += 32) t += part[b];
+    t = warp_sum(t);
+    if (threadIdx.x == 0) *out = t;
 }
 
 // X <- D^-1 X (rows scaled: U^-1 -> R^-1).
@@ -1069,6 +1084,7 @@ struct FactArgs {
     int mode;       // 0: Cholesky of the upper half (U to Ur); 1: signed LU (signs to sgn)
     double* Ur;
     double* Xd;
+    double* pan;    // LU: 2 x 32 x n, the block column's L^T and U panels
     double* sgn;
     int64_t keep;   // LU: the column dlarfg leaves as the identity, or -1
     double floor;
@@ -1132,8 +1148,9 @@ __device__ __forceinline__ void warp_inv_unit_lower(const HMat& Q, HMat& Y) {
 // Factor the diagonal block of block column p (M's block already holds
 // every earlier update): Cholesky U_pp (to Ur) and X = U_pp^-1, or the
 // signed LU L\U of the block with X = U^-1, Y = L^-1; X (and Y) to
-// Xd[p & 1] as row-major 32 x 32.
-__device__ void fact_diag(const FactArgs& a, int64_t p, double* sm) {
+// Xd[p & 1] as row-major 32 x 32.  in_smem: the block is in B already
+// (fact_next_diag).
+__device__ void fact_diag(const FactArgs& a, int64_t p, double* sm, bool in_smem) {
     HMat& B = *reinterpret_cast<HMat*>(sm);
     HMat& R = *reinterpret_cast<HMat*>(sm + 1 * kHB * (kHB + 1));
     HMat& X = *reinterpret_cast<HMat*>(sm + 2 * kHB * (kHB + 1));
@@ -1144,16 +1161,16 @@ __device__ void fact_diag(const FactArgs& a, int64_t p, double* sm) {
     const int64_t n = a.n, jb = p * kHB;
     const int nb = (int)(n - jb < kHB ? n - jb : kHB);
     __syncthreads();
-    for (int e = t; e < kHB * kHB; e += blockDim.x) {
-        const int r = e & 31, c = e >> 5;
-        B[r][c] = (r < nb && c < nb) ? __ldcg(a.M + (size_t)(jb + c) * n + jb + r) : (r == c ? 1.0 : 0.0);
-    }
+    if (!in_smem)
+        for (int e = t; e < kHB * kHB; e += blockDim.x) {
+            const int r = e & 31, c = e >> 5;
+            B[r][c] = (r < nb && c < nb) ? __ldcg(a.M + (size_t)(jb + c) * n + jb + r) : (r == c ? 1.0 : 0.0);
+        }
     double* xd = a.Xd + (size_t)(p & 1) * 2 * kHB * kHB;
     __shared__ double dinv[kHB];
     if (a.mode == 0) {
-        const bool ok = cta_chol(B, R, a.floor, &okf);
+        const bool ok = cta_chol_inv(B, R, X, a.floor, &okf);
         if (!ok && t == 0) atomicExch(a.fail, 1);
-        warp_inv_upper(R, X, dinv);
         for (int e = t; e < kHB * kHB; e += blockDim.x) {
             const int r = e >> 5, c = e & 31;
             if (r < nb && c < nb) a.Ur[(size_t)(jb + r) * n + jb + c] = r <= c ? R[r][c] : 0.0;
@@ -1179,86 +1196,221 @@ __device__ void fact_diag(const FactArgs& a, int64_t p, double* sm) {
     __syncthreads();
 }
 
-// C = A^T B (TA) or A B over the CTA, 32 x 32 shared tiles.
+// d += A^T B (TA) or A B on 32 x 32 shared tiles, eight warps on the FP64
+// tensor cores: warp w holds rows 16 (w % 2) + g + {0, 8}, columns
+// 8 (w / 2) + 2 q + {0, 1} of the product (g = lane / 4, q = lane % 4).
 template <bool TA>
-__device__ __forceinline__ void fact_mm(const HMat& A, const HMat& B, HMat& C) {
-    const int t = threadIdx.x;
-    const int i = t & 31, j0 = (t >> 5) * 4;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int k = 0; k < kHB; ++k) {
-        const double x = TA ? A[k][i] : A[i][k];
+__device__ __forceinline__ void fact_mma(const HMat& A, const HMat& B, double (&d)[4]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const int m0 = 16 * (warp & 1) + g, n0 = 8 * (warp >> 1) + g;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) s[q] += x * B[k][j0 + q];
+    for (int k0 = 0; k0 < kHB; k0 += 8) {
+        double a[4], b[2];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int row = m0 + 8 * (u & 1), k = k0 + q + 4 * (u >> 1);
+            a[u] = TA ? A[k][row] : A[row][k];
+        }
+        b[0] = B[k0 + q][n0];
+        b[1] = B[k0 + q + 4][n0];
+        g_dmma1688(d, a, b);
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) C[i][j0 + q] = s[q];
 }
 
-// Trailing tile `tau` of block column p: Cholesky tiles (I <= J) in rows,
-// LU tiles (I, J) row by row; tile 0 is the next diagonal block.
-__device__ void fact_tile(const FactArgs& a, int64_t p, int64_t tau, double* sm) {
-    HMat& A1 = *reinterpret_cast<HMat*>(sm);
-    HMat& P1 = *reinterpret_cast<HMat*>(sm + 1 * kHB * (kHB + 1));
-    HMat& A2 = *reinterpret_cast<HMat*>(sm + 2 * kHB * (kHB + 1));
-    HMat& P2 = *reinterpret_cast<HMat*>(sm + 3 * kHB * (kHB + 1));
-    HMat& F1 = *reinterpret_cast<HMat*>(sm + 4 * kHB * (kHB + 1));
-    HMat& F2 = *reinterpret_cast<HMat*>(sm + 5 * kHB * (kHB + 1));
+// Row and column of element u of a fact_mma product.
+__device__ __forceinline__ void fact_pos(int u, int& r, int& c) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    r = 16 * (warp & 1) + (lane >> 2) + 8 * (u >> 1);
+    c = 8 * (warp >> 1) + 2 * (lane & 3) + (u & 1);
+}
+
+template <bool TA>
+__device__ __forceinline__ void fact_mm(const HMat& A, const HMat& B, HMat& C) {
+    double d[4] = {0.0, 0.0, 0.0, 0.0};
+    fact_mma<TA>(A, B, d);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        int r, c;
+        fact_pos(u, r, c);
+        C[r][c] = d[u];
+    }
+}
+
+// Panel tile tau of block column p, 32 wide, written with K (the block
+// column's 32 rows) outermost:
+//   Cholesky  U_pJ = X^T M_pJ                       (rows of Ur)
+//   LU        U_pJ = Y M_pJ (tau < nt), then L_Ip = M_Ip X (tau - nt),
+//             in pan: 32 x n of L^T, then 32 x n of U
+__device__ void fact_panel_tile(const FactArgs& a, int64_t p, int64_t nt, int64_t tau, double* sm) {
+    HMat& F = *reinterpret_cast<HMat*>(sm);
+    HMat& A = *reinterpret_cast<HMat*>(sm + 1 * kHB * (kHB + 1));
     const int t = threadIdx.x;
     const int64_t n = a.n, jb = p * kHB, t0 = jb + kHB;
-    const int64_t nt = (n - t0 + kHB - 1) / kHB;
-    int64_t I, J;
-    if (a.mode == 0) {
-        I = 0;
-        int64_t rest = tau;
-        while (rest >= nt - I) {
-            rest -= nt - I;
-            ++I;
-        }
-        J = I + rest;
-    } else {
-        I = tau / nt;
-        J = tau % nt;
-    }
-    const int64_t I0 = t0 + I * kHB, J0 = t0 + J * kHB;
-    const int wI = (int)(n - I0 < kHB ? n - I0 : kHB), wJ = (int)(n - J0 < kHB ? n - J0 : kHB);
-    const double* xd = a.Xd + (size_t)(p & 1) * 2 * kHB * kHB;
+    const bool lpan = tau >= nt;  // LU's L panel
+    const int64_t B0 = t0 + (lpan ? tau - nt : tau) * kHB;
+    const int w = (int)(n - B0 < kHB ? n - B0 : kHB);
+    const double* xd = a.Xd + (size_t)(p & 1) * 2 * kHB * kHB + (a.mode == 1 && !lpan ? kHB * kHB : 0);
     __syncthreads();
     for (int e = t; e < kHB * kHB; e += blockDim.x) {
         const int r = e & 31, c = e >> 5;
-        F1[r][c] = __ldcg(xd + r * kHB + c);
+        F[r][c] = __ldcg(xd + r * kHB + c);
+        if (lpan) A[r][c] = r < w ? __ldcg(a.M + (size_t)(jb + c) * n + B0 + r) : 0.0;
+        else A[r][c] = c < w ? __ldcg(a.M + (size_t)(B0 + c) * n + jb + r) : 0.0;
+    }
+    __syncthreads();
+    double d[4] = {0.0, 0.0, 0.0, 0.0};
+    if (a.mode == 0) fact_mma<true>(F, A, d);
+    else if (lpan) fact_mma<false>(A, F, d);
+    else fact_mma<false>(F, A, d);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        int r, c;
+        fact_pos(u, r, c);
         if (a.mode == 0) {
-            // row panel of G: A1 = G[jb.., I cols], A2 = G[jb.., J cols]
-            A1[r][c] = c < wI ? __ldcg(a.M + (size_t)(I0 + c) * n + jb + r) : 0.0;
-            A2[r][c] = c < wJ ? __ldcg(a.M + (size_t)(J0 + c) * n + jb + r) : 0.0;
-        } else {
-            F2[r][c] = __ldcg(xd + kHB * kHB + r * kHB + c);
-            // A1 = M[I rows, panel cols], A2 = M[panel rows, J cols]
-            A1[r][c] = r < wI ? __ldcg(a.M + (size_t)(jb + c) * n + I0 + r) : 0.0;
-            A2[r][c] = c < wJ ? __ldcg(a.M + (size_t)(J0 + c) * n + jb + r) : 0.0;
+            if (c < w) a.Ur[(size_t)(jb + r) * n + B0 + c] = d[u];
+        } else if (lpan) {
+            if (r < w) a.pan[(size_t)c * n + B0 + r] = d[u];
+        } else if (c < w) {
+            a.pan[(size_t)(kHB + r) * n + B0 + c] = d[u];
         }
+    }
+}
+
+// The panels of block column p as K-outermost rows (columns from t0 on).
+__device__ __forceinline__ const double* fact_left(const FactArgs& a, int64_t p) {
+    return a.mode == 0 ? a.Ur + (size_t)p * kHB * a.n : a.pan;
+}
+__device__ __forceinline__ const double* fact_right(const FactArgs& a, int64_t p) {
+    return a.mode == 0 ? a.Ur + (size_t)p * kHB * a.n : a.pan + (size_t)kHB * a.n;
+}
+
+// The next diagonal block less its update, into fact_diag's B.  CTA 0 forms
+// the two panel tiles it needs itself (the same products as
+// fact_panel_tile's), from the inverses fact_diag left in X and Y, so it
+// waits for no panel of another CTA.
+__device__ void fact_next_diag(const FactArgs& a, int64_t p, double* sm) {
+    HMat& B = *reinterpret_cast<HMat*>(sm);
+    HMat& L = *reinterpret_cast<HMat*>(sm + 1 * kHB * (kHB + 1));
+    HMat& X = *reinterpret_cast<HMat*>(sm + 2 * kHB * (kHB + 1));
+    HMat& Y = *reinterpret_cast<HMat*>(sm + 3 * kHB * (kHB + 1));
+    HMat& P = *reinterpret_cast<HMat*>(sm + 4 * kHB * (kHB + 1));
+    HMat& R = *reinterpret_cast<HMat*>(sm + 5 * kHB * (kHB + 1));
+    const int64_t n = a.n, jb = p * kHB, t0 = jb + kHB;
+    const int w = (int)(n - t0 < kHB ? n - t0 : kHB);
+    double cur[4], prod[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        int r, c;
+        fact_pos(u, r, c);
+        cur[u] = (r < w && c < w) ? __ldcg(a.M + (size_t)(t0 + c) * n + t0 + r) : (r == c ? 1.0 : 0.0);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < kHB * kHB; e += blockDim.x) {
+        const int r = e & 31, c = e >> 5;
+        P[r][c] = c < w ? __ldcg(a.M + (size_t)(t0 + c) * n + jb + r) : 0.0;  // M_p,p+1
+        if (a.mode == 1) B[r][c] = r < w ? __ldcg(a.M + (size_t)(jb + c) * n + t0 + r) : 0.0;  // M_p+1,p
     }
     __syncthreads();
     if (a.mode == 0) {
-        fact_mm<true>(F1, A1, P1);   // U_pI = X^T G_pI
-        if (I != J) fact_mm<true>(F1, A2, P2);  // U_pJ
-        __syncthreads();
-        const HMat& PJ = I != J ? P2 : P1;
-        fact_mm<true>(P1, PJ, A1);   // U_pI^T U_pJ
-        if (I == J)
-            for (int e = t; e < kHB * kHB; e += blockDim.x) {
-                const int r = e >> 5, c = e & 31;
-                if (c < wJ) a.Ur[(size_t)(jb + r) * n + J0 + c] = P1[r][c];
-            }
+        fact_mm<true>(X, P, R);   // U = X^T M
     } else {
-        fact_mm<false>(A1, F1, P1);  // L_Ip = M_Ip U_pp^-1
-        fact_mm<false>(F2, A2, P2);  // U_pJ = L_pp^-1 M_pJ
-        __syncthreads();
-        fact_mm<false>(P1, P2, A1);  // L_Ip U_pJ
+        fact_mm<false>(Y, P, R);  // U = Y M
+        fact_mm<false>(B, X, L);  // L = M X
     }
     __syncthreads();
-    for (int e = t; e < kHB * kHB; e += blockDim.x) {
-        const int r = e & 31, c = e >> 5;
-        if (r < wI && c < wJ) a.M[(size_t)(J0 + c) * n + I0 + r] -= A1[r][c];
+    if (a.mode == 0) fact_mma<true>(R, R, prod);
+    else fact_mma<false>(L, R, prod);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        int r, c;
+        fact_pos(u, r, c);
+        B[r][c] = cur[u] - prod[u];
+    }
+}
+
+// The trailing matrix less the panels' product, in 64 x 64 tiles (Cholesky:
+// those reaching the diagonal or above), all but the next diagonal block:
+// tiles first, first + step, ..  Eight warps of 16 x 32 entries on the FP64
+// tensor cores; the next tile's panels and entries are loaded while the
+// current tile is formed (a tile of 32 alone, its loads exposed and its
+// panels formed anew, left 12000 x 3000 at 6.4 ms of factorisation).
+constexpr int kFactTile = 64;
+constexpr int kFactPitch = kFactTile + 4;  // 16 lanes of a fragment read on 16 banks
+
+__device__ void fact_trailing(const FactArgs& a, int64_t p, int64_t first, int64_t step, double* sm) {
+    double (*Ls)[kFactPitch] = reinterpret_cast<double (*)[kFactPitch]>(sm);
+    double (*Rs)[kFactPitch] = reinterpret_cast<double (*)[kFactPitch]>(sm + kHB * kFactPitch);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = lane >> 2, q = lane & 3;
+    const int wm = 16 * (warp & 3), wn = 32 * (warp >> 2);
+    const int64_t n = a.n, t0 = (p + 1) * kHB;
+    const int64_t nt = (n - t0 + kFactTile - 1) / kFactTile;
+    const int64_t total = a.mode == 0 ? nt * (nt + 1) / 2 : nt * nt;
+    const double *pl = fact_left(a, p), *pr = fact_right(a, p);
+    double lv[8], rv[8], cv[16];
+    int64_t I0 = 0, J0 = 0;
+    auto fetch = [&](int64_t tau) {
+        int64_t I, J;
+        if (a.mode == 0) {
+            I = 0;
+            int64_t rest = tau;
+            while (rest >= nt - I) {
+                rest -= nt - I;
+                ++I;
+            }
+            J = I + rest;
+        } else {
+            I = tau / nt;
+            J = tau % nt;
+        }
+        I0 = t0 + I * kFactTile;
+        J0 = t0 + J * kFactTile;
+        const int i = t & 63, k0 = t >> 6;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = k0 + 4 * u;
+            lv[u] = I0 + i < n ? __ldcg(pl + (size_t)k * n + I0 + i) : 0.0;
+            rv[u] = J0 + i < n ? __ldcg(pr + (size_t)k * n + J0 + i) : 0.0;
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            const int64_t row = I0 + wm + g + 8 * ((e >> 1) & 1), col = J0 + wn + 8 * (e >> 2) + 2 * q + (e & 1);
+            cv[e] = (row < n && col < n) ? __ldcg(a.M + (size_t)col * n + row) : 0.0;
+        }
+    };
+    if (first < total) fetch(first);
+    for (int64_t tau = first; tau < total; tau += step) {
+        double acc[4][4];
+        const int64_t i0 = I0, j0 = J0;
+        __syncthreads();  // the previous tile's fragments are read
+        {
+            const int i = t & 63, k0 = t >> 6;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                Ls[k0 + 4 * u][i] = -lv[u];
+                Rs[k0 + 4 * u][i] = rv[u];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[e >> 2][e & 3] = cv[e];
+        if (tau + step < total) fetch(tau + step);
+        __syncthreads();
+#pragma unroll
+        for (int k0 = 0; k0 < kHB; k0 += 8) {
+            double av[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) av[u] = Ls[k0 + q + 4 * (u >> 1)][wm + g + 8 * (u & 1)];
+#pragma unroll
+            for (int nb = 0; nb < 4; ++nb) {
+                const double bv[2] = {Rs[k0 + q][wn + 8 * nb + g], Rs[k0 + q + 4][wn + 8 * nb + g]};
+                g_dmma1688(acc[nb], av, bv);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            const int64_t row = i0 + wm + g + 8 * ((e >> 1) & 1), col = j0 + wn + 8 * (e >> 2) + 2 * q + (e & 1);
+            const bool next = row < t0 + kHB && col < t0 + kHB;  // CTA 0's
+            if (row < n && col < n && !next) a.M[(size_t)col * n + row] = acc[e >> 2][e & 3];
+        }
     }
     __syncthreads();
 }
@@ -1270,19 +1422,32 @@ __global__ void __launch_bounds__(kQrThreads, 1) fact_kernel(FactArgs a) {
     const int64_t n = a.n;
     const int64_t np = (n + kHB - 1) / kHB;
     const int64_t G = gridDim.x;
-    if (blockIdx.x == 0) fact_diag(a, 0, fsm);
+    unsigned int pgen = 0;  // the panels' barrier, of all CTAs but 0
+    if (blockIdx.x == 0) fact_diag(a, 0, fsm, false);
     if (!grid_sync(a.gs, gen, &sflag)) return;
     for (int64_t p = 0; p + 1 < np; ++p) {
-        const int64_t t0 = (p + 1) * kHB;
-        const int64_t nt = (n - t0 + kHB - 1) / kHB;
-        const int64_t ntiles = a.mode == 0 ? nt * (nt + 1) / 2 : nt * nt;
-        if (blockIdx.x == 0) {
-            fact_tile(a, p, 0, fsm);
-            fact_diag(a, p + 1, fsm);
-            if (G == 1)
-                for (int64_t tau = 1; tau < ntiles; ++tau) fact_tile(a, p, tau, fsm);
+        const int64_t nt = (n - (p + 1) * kHB + kHB - 1) / kHB;
+        const int64_t panels = a.mode == 0 ? nt : 2 * nt;
+        if (blockIdx.x == 0 && G > 1) {
+            fact_next_diag(a, p, fsm);
+            fact_diag(a, p + 1, fsm, true);
         } else {
-            for (int64_t tau = blockIdx.x; tau < ntiles; tau += G - 1) fact_tile(a, p, tau, fsm);
+            const int64_t who = G > 1 ? blockIdx.x - 1 : 0, all = G > 1 ? G - 1 : 1;
+            for (int64_t tau = who; tau < panels; tau += all) fact_panel_tile(a, p, nt, tau, fsm);
+            if (!grid_sync(a.gs + 1, pgen, &sflag, (unsigned int)all)) return;
+            fact_trailing(a, p, who, all, fsm);
+            if (G == 1) {  // X and Y of fact_diag are overwritten: reload them
+                HMat& X = *reinterpret_cast<HMat*>(fsm + 2 * kHB * (kHB + 1));
+                HMat& Y = *reinterpret_cast<HMat*>(fsm + 3 * kHB * (kHB + 1));
+                const double* xd = a.Xd + (size_t)(p & 1) * 2 * kHB * kHB;
+                for (int e = threadIdx.x; e < kHB * kHB; e += blockDim.x) {
+                    X[e >> 5][e & 31] = xd[e];
+                    Y[e >> 5][e & 31] = xd[kHB * kHB + e];
+                }
+                __syncthreads();
+                fact_next_diag(a, p, fsm);
+                fact_diag(a, p + 1, fsm, true);
+            }
         }
         if (!grid_sync(a.gs, gen, &sflag)) return;
     }
@@ -1292,7 +1457,7 @@ __global__ void __launch_bounds__(kQrThreads, 1) fact_kernel(FactArgs a) {
 static tomos_status launch_fact(const FactArgs& fa, GridSync* gs, cudaStream_t st) {
     const size_t smem = sizeof(double) * kFactSmemMats * kHB * (kHB + 1);
     TOMOS_CUDA_TRY(cudaFuncSetAttribute(fact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    TOMOS_CUDA_TRY(cudaMemsetAsync(gs, 0, sizeof(GridSync), st));
+    TOMOS_CUDA_TRY(cudaMemsetAsync(gs, 0, 2 * sizeof(GridSync), st));
     FactArgs a = fa;
     void* args[] = {&a};
     cudaError_t e = cudaLaunchCooperativeKernel((const void*)fact_kernel, dim3((unsigned)sm_count()),
@@ -1326,6 +1491,7 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     fa.mode = 0;
     fa.Ur = w.Ur;
     fa.Xd = w.Xd;
+    fa.pan = w.pan;
     fa.sgn = w.sgn;
     fa.keep = -1;
     fa.floor = kQrWideFloor;
@@ -1345,14 +1511,15 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     }
     int flag = 0;
     double kap2 = 0.0;
-    GridSync gsh{};
+    GridSync gsh[2] = {};
     TOMOS_CUDA_TRY(cudaMemcpyAsync(&flag, w.flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     TOMOS_CUDA_TRY(cudaMemcpyAsync(&kap2, w.kap, sizeof(double), cudaMemcpyDeviceToHost, st));
-    TOMOS_CUDA_TRY(cudaMemcpyAsync(&gsh, w.gs, sizeof(gsh), cudaMemcpyDeviceToHost, st));
+    TOMOS_CUDA_TRY(cudaMemcpyAsync(gsh, w.gs, sizeof(gsh), cudaMemcpyDeviceToHost, st));
     TOMOS_CUDA_TRY(cudaStreamSynchronize(st));
-    if (gsh.err) return fail(TOMOS_ERR_CUDA, "sketch_qr: a bounded grid barrier wait expired");
+    if (gsh[0].err || gsh[1].err) return fail(TOMOS_ERR_CUDA, "sketch_qr: a bounded grid barrier wait expired");
     const double kappa = std::sqrt((double)n * kap2);
-    if (flag || !(kappa <= kQrWideMaxKappa)) return TOMOS_OK;  // the panel path takes over
+    const double kmax = n > kQrWidePlainN ? kQrWideRms * (double)n : kQrWideMaxKappa;
+    if (flag || !(kappa <= kmax)) return TOMOS_OK;  // the panel path takes over
     wide_row_scale_kernel<<<eb, 256, 0, st>>>(w.X, n, w.d);
     TOMOS_LAUNCH_CHECK("wide_row_scale_kernel");
     if (any_signs) {
@@ -1370,9 +1537,9 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     if (s) return s;
     wide_output_kernel<<<eb, 256, 0, st>>>(w.X, w.Ur, w.d, w.sgn, n, SA, ld, R);
     TOMOS_LAUNCH_CHECK("wide_output_kernel");
-    TOMOS_CUDA_TRY(cudaMemcpyAsync(&gsh, w.gs, sizeof(gsh), cudaMemcpyDeviceToHost, st));
+    TOMOS_CUDA_TRY(cudaMemcpyAsync(gsh, w.gs, sizeof(gsh), cudaMemcpyDeviceToHost, st));
     TOMOS_CUDA_TRY(cudaStreamSynchronize(st));
-    if (gsh.err) return fail(TOMOS_ERR_CUDA, "sketch_qr: a bounded grid barrier wait expired");
+    if (gsh[0].err || gsh[1].err) return fail(TOMOS_ERR_CUDA, "sketch_qr: a bounded grid barrier wait expired");
     *done = true;
     return TOMOS_OK;
 }

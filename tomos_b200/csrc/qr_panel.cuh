@@ -81,6 +81,45 @@ __device__ __noinline__ bool cta_chol(const HMat& G, HMat& R, double floor, int*
     return *okf != 0;
 }
 
+// cta_chol and X = R^{-1} in one sweep: the row operations that turn G into
+// R turn the identity into R^-T, so lane l carries column l of both and every
+// step's row of R reaches the lanes once for the two updates.
+__device__ __noinline__ bool cta_chol_inv(const HMat& G, HMat& R, HMat& X, double floor, int* okf) {
+    const int t = threadIdx.x;
+    __syncthreads();
+    if (t < 32) {
+        const int l = t;
+        double g[kHB], y[kHB];
+#pragma unroll
+        for (int i = 0; i < kHB; ++i) {
+            g[i] = G[i][l];
+            y[i] = i == l ? 1.0 : 0.0;
+        }
+        int ok = 1;
+#pragma unroll
+        for (int j = 0; j < kHB; ++j) {
+            const double d = __shfl_sync(0xffffffffu, g[j], j);
+            const bool good = d > floor && isfinite(d);
+            if (!good) ok = 0;
+            const double dd = good ? d : 1.0;
+            const double ri = rsqrt(dd);
+            const double rjl = l > j ? g[j] * ri : (l == j ? dd * ri : 0.0);
+            const double yj = y[j] * ri;
+            R[j][l] = rjl;
+            X[l][j] = yj;  // (R^-T)(j, l)
+#pragma unroll
+            for (int i = j + 1; i < kHB; ++i) {
+                const double rji = __shfl_sync(0xffffffffu, rjl, i);
+                g[i] -= rji * rjl;
+                y[i] -= rji * yj;
+            }
+        }
+        if (l == 0) *okf = ok;
+    }
+    __syncthreads();
+    return *okf != 0;
+}
+
 // X = R^{-1} for upper triangular R (X must not alias R; Tmp is scratch).
 // A level of block size b has kHB / (2b) pairs (I, J) of b x b blocks,
 // I = [2bp, 2bp + b), J = [2bp + b, 2bp + 2b): X_IJ = -X_II (R_IJ X_JJ).

@@ -37,6 +37,19 @@ __device__ __forceinline__ void g_cp_async8(void* dst, const void* src, bool val
                  "r"(valid ? 8 : 0)
                  : "memory");
 }
+__device__ __forceinline__ void g_cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+// Two neighbouring values of which the first n (0, 1, 2) exist, the others
+// zero; vec: both addresses are 16-byte aligned.
+__device__ __forceinline__ void g_copy_pair(double* dst, const double* src, const double* safe, int n, bool vec) {
+    if (vec && n == 2) {
+        g_cp_async16(dst, src);
+    } else {
+        g_cp_async8(dst, n > 0 ? src : safe, n > 0);
+        g_cp_async8(dst + 1, n > 1 ? src + 1 : safe, n > 1);
+    }
+}
 __device__ __forceinline__ void g_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void g_cp_async_wait() {
@@ -56,8 +69,9 @@ __device__ __forceinline__ void g_dmma1688(double* d, const double* a, const dou
 // D (M x N, column-major, ld ldd) = alpha * op(A) B + beta * D, B
 // column-major K x N.  KMAJOR: op(A) = A^T with A column-major K x M;
 // otherwise A is column-major M x K.  CTA tile 128 x 64, k-steps of 16
-// through kGstages shared-memory stages filled by 8-byte asynchronous
-// copies (zero-filled past the edges); 8 warps, each 32 x 32 = two by
+// through kGstages shared-memory stages filled by asynchronous copies of
+// pairs (16 bytes where the operand is aligned, zero-filled past the edges),
+// one barrier a stage; 8 warps, each 32 x 32 = two by
 // four m16n8k8 tiles.  Split-K: CTA z sums k in [z kc, (z + 1) kc); with
 // gridDim.z > 1 it writes its partial to P + z M N (ld M) for
 // qr_gemm_reduce_kernel.  sub: D -= op(A) B instead (alpha and beta
@@ -88,32 +102,30 @@ __global__ void __launch_bounds__(256, 2) qr_gemm_kernel(GemmArgs g) {
     const int64_t kb = (int64_t)blockIdx.z * g.kc;
     const int64_t ke = kb + g.kc < g.K ? kb + g.kc : g.K;
     const int nk = ke > kb ? (int)((ke - kb + kGbk - 1) / kGbk) : 0;
+    const bool avec = g.lda % 2 == 0 && reinterpret_cast<uintptr_t>(g.A) % 16 == 0;
+    const bool bvec = g.ldb % 2 == 0 && reinterpret_cast<uintptr_t>(g.B) % 16 == 0;
+    auto left = [](int64_t at, int64_t end) { return at + 1 < end ? 2 : (at < end ? 1 : 0); };
     auto issue = [&](int s, int64_t k0) {
         double* As = gsm + s * kGstage;
         double* Bs = As + kGa;
 #pragma unroll
-        for (int i = 0; i < kGbm * kGbk / 256; ++i) {
+        for (int i = 0; i < kGbm * kGbk / 512; ++i) {
             const int e = t + i * 256;
-            int m, kk;
-            if (KMAJOR) {
-                m = e >> 4;
-                kk = e & 15;
-            } else {
-                m = e & (kGbm - 1);
-                kk = e >> 7;
+            if (KMAJOR) {  // pairs along K
+                const int m = e >> 3, kk = (e & 7) * 2;
+                const int64_t gm = m0 + m, gk = k0 + kk;
+                g_copy_pair(As + m * (kGbk + kGpad) + kk, g.A + gk + gm * g.lda, g.A, gm < g.M ? left(gk, ke) : 0, avec);
+            } else {       // pairs along M
+                const int m = (e & (kGbm / 2 - 1)) * 2, kk = e >> 6;
+                const int64_t gm = m0 + m, gk = k0 + kk;
+                g_copy_pair(As + kk * (kGbm + kGpad) + m, g.A + gm + gk * g.lda, g.A, gk < ke ? left(gm, g.M) : 0, avec);
             }
-            const int64_t gm = m0 + m, gk = k0 + kk;
-            const bool ok = gm < g.M && gk < ke;
-            const double* src = KMAJOR ? g.A + gk + gm * g.lda : g.A + gm + gk * g.lda;
-            double* dst = KMAJOR ? As + m * (kGbk + kGpad) + kk : As + kk * (kGbm + kGpad) + m;
-            g_cp_async8(dst, ok ? src : g.A, ok);
         }
 #pragma unroll
-        for (int i = 0; i < kGbn * kGbk / 256; ++i) {
-            const int e = t + i * 256, nn = e >> 4, kk = e & 15;
+        for (int i = 0; i < kGbn * kGbk / 512; ++i) {
+            const int e = t + i * 256, nn = e >> 3, kk = (e & 7) * 2;
             const int64_t gn = n0 + nn, gk = k0 + kk;
-            const bool ok = gn < g.N && gk < ke;
-            g_cp_async8(Bs + nn * (kGbk + kGpad) + kk, ok ? g.B + gk + gn * g.ldb : g.B, ok);
+            g_copy_pair(Bs + nn * (kGbk + kGpad) + kk, g.B + gk + gn * g.ldb, g.B, gn < g.N ? left(gk, ke) : 0, bvec);
         }
         g_cp_async_commit();
     };
@@ -135,11 +147,11 @@ __global__ void __launch_bounds__(256, 2) qr_gemm_kernel(GemmArgs g) {
             }
     const double asg = g.sub ? -1.0 : 1.0;
     for (int i = 0; i < nk; ++i) {
+        g_cp_async_wait<kGstages - 2>();
+        __syncthreads();  // stage i landed, and stage i - 1 was read by all
         const int ni = i + kGstages - 1;
         if (ni < nk) issue(ni % kGstages, kb + (int64_t)ni * kGbk);
         else g_cp_async_commit();
-        g_cp_async_wait<kGstages - 1>();
-        __syncthreads();
         const double* As = gsm + (i % kGstages) * kGstage;
         const double* Bs = As + kGa;
 #pragma unroll
@@ -162,7 +174,6 @@ __global__ void __launch_bounds__(256, 2) qr_gemm_kernel(GemmArgs g) {
 #pragma unroll
                 for (int in = 0; in < 4; ++in) g_dmma1688(acc[im][in], a[im], b[in]);
         }
-        __syncthreads();  // the stage is refilled kGstages - 1 steps on
     }
     g_cp_async_wait<0>();
     const bool split = gridDim.z > 1;

@@ -23,8 +23,11 @@
 //   N2       z = M^T t, vh = z - beta v               (preconditioned only)
 //   N3       alpha = ||vh||, v = vh / alpha, p = M v, Givens, x and wt
 //   N4       state update, history, stopping rule, next cu = -alpha/beta
+// N1 to N4 are one launch for a preconditioned solve with n <=
+// kNsideClusterMaxN, four kernels otherwise.
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -177,6 +180,7 @@ struct NSide {
     int nb1;   // N1 blocks
     int nb3;   // N2/N3 blocks
     double* scal;
+    double* cpart;
     LsqrDev* st;
     const int* skip;
     const double* dscale;  // column scale D of the backward-error rule, or NULL
@@ -359,21 +363,15 @@ __global__ void __launch_bounds__(256) nside_update_kernel(NSide S) {
     }
 }
 
-// N4: one block -- state update and the stopping rule.  In the iteration
-// graph's while loop it also sets the loop's condition: 0 once the solver
-// stopped (a skipped body, the stopping rule, a breakdown or the restart's
-// max_iters iterations), so the loop runs at most max_iters + 1 bodies.
-__global__ void __launch_bounds__(256) nside_finish_kernel(NSide S) {
-    if (S.skip && *S.skip) {
-        if (S.use_cond && threadIdx.x == 0) cudaGraphSetConditional(S.cond, 0u);
-        return;
-    }
-    __shared__ double sm[32];
-    const double xn = sqrt(block_sum_array(S.xpart, S.nb3, sm));
-    const double qn = S.init ? sqrt(block_sum_array(S.qnpart, S.nb1, sm)) : 0.0;
-    if (threadIdx.x != 0) return;
+// The state update and the stopping rule (one thread); `in` is the state
+// before it (*S.st, or a copy), g the Givens step of (alpha, beta).  In the
+// iteration graph's while loop it also sets the loop's condition: 0 once the
+// solver stopped (a skipped body, the stopping rule, a breakdown or the
+// restart's max_iters iterations), so the loop runs at most max_iters + 1
+// bodies.
+__device__ __forceinline__ void finish_state(const NSide& S, const LsqrDev& in, const Givens& g, double beta,
+                                             double alpha, double xn, double qn) {
     LsqrDev* st = S.st;
-    const double beta = S.scal[0], alpha = S.scal[1];
     st->xnorm = xn;
     st->coef[0] = 1.0;
     st->coef[1] = beta > 0.0 ? -alpha / beta : 0.0;
@@ -385,42 +383,300 @@ __global__ void __launch_bounds__(256) nside_finish_kernel(NSide S) {
         st->beta_init = beta;
         st->arnorm = qn;
         st->iter_restart = 0;
-        st->relres = st->rhsnorm > 0.0 ? beta / st->rhsnorm : 0.0;
+        st->relres = in.rhsnorm > 0.0 ? beta / in.rhsnorm : 0.0;
         st->done = 0;
         st->breakdown = (alpha == 0.0 || beta == 0.0) ? 1 : 0;
         if (S.use_cond) cudaGraphSetConditional(S.cond, 0u);  // no loop runs init passes
         return;
     }
-    Givens g = givens(st->rho_bar, st->phi_bar, alpha, beta);
     st->alpha = alpha;
     st->beta = beta;
     st->rho_bar = g.rho_bar;
     st->phi_bar = g.phi_bar;
-    st->iter += 1;
-    st->iter_restart += 1;
-    const double relres = st->rhsnorm > 0.0 ? fabs(g.phi_bar) / st->rhsnorm : 0.0;
+    const int iter = in.iter + 1, iter_restart = in.iter_restart + 1;
+    st->iter = iter;
+    st->iter_restart = iter_restart;
+    const double relres = in.rhsnorm > 0.0 ? fabs(g.phi_bar) / in.rhsnorm : 0.0;
     st->relres = relres;
-    if (st->history && st->iter - 1 < st->history_cap) st->history[st->iter - 1] = relres;
+    if (in.history && iter - 1 < in.history_cap) in.history[iter - 1] = relres;
     int stop = 0;
-    if (st->rhsnorm == 0.0) stop = 1;
-    if (st->stop_rule == TOMOS_STOP_RELRES) {
-        if (relres < st->tol || relres < st->max_relres) {
+    if (in.rhsnorm == 0.0) stop = 1;
+    if (in.stop_rule == TOMOS_STOP_RELRES) {
+        if (relres < in.tol || relres < in.max_relres) {
             stop = 1;
             st->converged = 1;
         }
     } else {
-        const double den = st->anorm_fro * xn + st->bnorm;
+        const double den = in.anorm_fro * xn + in.bnorm;
         const double eta1 = den > 0.0 ? fabs(g.phi_bar) / den : 0.0;
-        if (eta1 <= st->inner_tol) stop = 1;
-        if (st->inner_rtol > 0.0 && fabs(g.phi_bar) <= st->inner_rtol * st->beta_init) stop = 1;
+        if (eta1 <= in.inner_tol) stop = 1;
+        if (in.inner_rtol > 0.0 && fabs(g.phi_bar) <= in.inner_rtol * in.beta_init) stop = 1;
     }
     if (alpha == 0.0 || beta == 0.0) {
         stop = 1;
         st->breakdown = 1;
     }
-    if (st->iter_restart >= st->max_iters) stop = 1;
+    if (iter_restart >= in.max_iters) stop = 1;
     if (stop) st->done = 1;
     if (S.use_cond) cudaGraphSetConditional(S.cond, stop ? 0u : 1u);
+}
+
+// N4: one block.
+__global__ void __launch_bounds__(256) nside_finish_kernel(NSide S) {
+    if (S.skip && *S.skip) {
+        if (S.use_cond && threadIdx.x == 0) cudaGraphSetConditional(S.cond, 0u);
+        return;
+    }
+    __shared__ double sm[32];
+    const double xn = sqrt(block_sum_array(S.xpart, S.nb3, sm));
+    const double qn = S.init ? sqrt(block_sum_array(S.qnpart, S.nb1, sm)) : 0.0;
+    if (threadIdx.x != 0) return;
+    const double beta = S.scal[0], alpha = S.scal[1];
+    finish_state(S, *S.st, givens(S.st->rho_bar, S.st->phi_bar, alpha, beta), beta, alpha, xn, qn);
+}
+
+// N1 to N4 in one launch, for a preconditioned solve of few columns: one CTA
+// up to kNsideOneMaxN columns, one cluster of 8 or 16 up to
+// kNsideClusterMaxN.  The four kernels are bound by latency, a launch, a
+// first load and a tail each (17 us an iteration at n = 64 beside a 33 us
+// pass); past that size the cluster's SMs read R^{-1} slower than the whole
+// GPU does (38 us against 34 us at n = 1000).  A warp keeps its columns of
+// R^{-1} in registers, loaded before the sums they wait for, then its rows
+// the same way; t and vh go through shared memory (of one CTA), or through
+// L2 between cluster barriers, which order the CTAs' global writes (data
+// another CTA wrote is read with __ldcg).  Each CTA leaves its partial sums
+// in cpart, summed by every CTA in the same order.
+constexpr int kNsideOneMaxN = 128;
+constexpr int kNsideClusterMaxN = 512;
+constexpr int kNsideThreads = 1024;
+
+template <bool ONE>
+__device__ __forceinline__ void nside_barrier() {
+    if constexpr (ONE) __syncthreads();
+    else asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// ONE: one CTA, a warp's columns w, w + 32, .. (four), of up to 128 entries;
+// otherwise a cluster, columns w ncta + rank, .. of up to 512 entries (one,
+// or two in a cluster of eight, loaded one after the other).
+template <bool ONE>
+__global__ void __launch_bounds__(kNsideThreads, 1) nside_fused_kernel(NSide S) {
+    constexpr int W = kNsideThreads / 32;
+    constexpr int MAXN = ONE ? kNsideOneMaxN : kNsideClusterMaxN;
+    constexpr int NL = MAXN / 32;               // entries of a column a lane holds
+    constexpr int CPW = ONE ? MAXN / W : 1;     // columns held at a time
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int rank = ONE ? 0 : (int)blockIdx.x, ncta = ONE ? 1 : (int)gridDim.x;
+    // the flag is written by CTA 0 after the last barrier only, so every CTA
+    // of the cluster takes the same way here
+    if (S.skip && *S.skip) {
+        if (S.use_cond && rank == 0 && threadIdx.x == 0) cudaGraphSetConditional(S.cond, 0u);
+        return;
+    }
+    __shared__ double sm[32];
+    __shared__ double smq[W][33];
+    __shared__ double tv[MAXN], vv[MAXN];
+    __shared__ LsqrDev st0;
+    const int n = (int)S.n;
+    const int first = w * ncta + rank, step = W * ncta;  // this warp's columns and rows
+    static_assert(sizeof(LsqrDev) % 4 == 0 && sizeof(LsqrDev) <= 4 * kNsideThreads, "state copied by words");
+    if (threadIdx.x < sizeof(LsqrDev) / 4)
+        reinterpret_cast<uint32_t*>(&st0)[threadIdx.x] = reinterpret_cast<const uint32_t*>(S.st)[threadIdx.x];
+    const bool full = S.scal[7] != 0.0;  // M is not upper triangular
+
+    double mv[CPW][NL];
+    // entries [k0, k1) of row (or column) j of a copy of M
+    auto fetch = [&](const double* __restrict__ M, int q, int j, int k0, int k1) {
+#pragma unroll
+        for (int u = 0; u < NL; ++u) {
+            const int k = lane + 32 * u;
+            mv[q][u] = (j < n && k >= k0 && k < k1) ? __ldg(M + (size_t)j * n + k) : 0.0;
+        }
+    };
+    auto dot = [&](int q, const double* b) {
+        double z0 = 0.0, z1 = 0.0;
+#pragma unroll
+        for (int u = 0; u < NL; u += 2) {  // entries past n hold zeros on both sides
+            z0 = fma(mv[q][u], b[lane + 32 * u], z0);
+            z1 = fma(mv[q][u + 1], b[lane + 32 * (u + 1)], z1);
+        }
+        return warp_sum(z0 + z1);
+    };
+#pragma unroll
+    for (int q = 0; q < CPW; ++q) {
+        const int j = first + q * step;
+        fetch(S.Rcm, q, j, 0, full ? n : j + 1);
+    }
+    for (int j = threadIdx.x; j < MAXN; j += kNsideThreads) tv[j] = vv[j] = 0.0;
+
+    // N1: beta, t = A^T ut / beta, ||D^-1 A^T ut||^2.  The warps of a CTA
+    // share its 32-column tiles, each taking every wpt-th partial.
+    const int tiles = (n + 31) / 32;
+    const int wpt = ONE ? (tiles <= 1 ? W : tiles <= 2 ? W / 2 : W / 4) : W;  // warps a tile
+    const int tile0 = ONE ? w / wpt : rank, wq = w % wpt;
+    double ssum = 0.0;
+    for (int k = threadIdx.x; k < S.gs; k += kNsideThreads) ssum += S.sspart[k];
+    double qn2 = 0.0, beta = 0.0, inv = 0.0;
+    for (int tile = tile0; tile - tile0 + (ONE ? 0 : rank) < (ONE ? 1 : tiles); tile += ncta) {
+        const int j = tile * 32 + lane;
+        double qv = 0.0;
+        if (S.qsum) {
+            qv = (wq == 0 && j < n) ? S.qsum[j] : 0.0;
+        } else if (j < n) {
+            int c = wq;
+            for (; c + 7 * wpt < S.gq; c += 8 * wpt) {
+                float f[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) f[u] = S.qpart[(size_t)(c + u * wpt) * S.qstride + j];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) qv += (double)f[u];
+            }
+            float f[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) f[u] = c + u * wpt < S.gq ? S.qpart[(size_t)(c + u * wpt) * S.qstride + j] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) qv += (double)f[u];
+        }
+        smq[w][lane] = qv;
+        if (tile == tile0) {
+            beta = sqrt(block_sum(ssum, sm));  // its barriers publish smq too
+            inv = beta > 0.0 ? 1.0 / beta : 0.0;
+        } else {
+            __syncthreads();
+        }
+        if (wq == 0 && j < n) {
+            double qs = 0.0;
+            for (int k = 0; k < wpt; ++k) qs += smq[w + k][lane];
+            if (ONE) tv[j] = qs * inv;
+            else S.t[j] = qs * inv;
+            const double qd = S.dscale ? qs / S.dscale[j] : qs;
+            qn2 += qd * qd;
+        }
+        __syncthreads();
+    }
+    if (!ONE && rank >= tiles) beta = sqrt(block_sum(ssum, sm));  // no tile of its own
+    qn2 = block_sum(qn2, sm);
+    if (!ONE) {
+        if (threadIdx.x == 0) S.cpart[rank] = qn2;
+        nside_barrier<ONE>();
+        for (int j = threadIdx.x; j < n; j += kNsideThreads) tv[j] = __ldcg(S.t + j);
+        __syncthreads();
+    }
+
+    // N2: vh = M^T t - beta v
+    double vh2 = 0.0;
+    for (int j0 = first; j0 < n; j0 += CPW * step) {
+        if (j0 != first) fetch(S.Rcm, 0, j0, 0, full ? n : j0 + 1);  // CPW == 1
+#pragma unroll
+        for (int q = 0; q < CPW; ++q) {
+            const int j = j0 + q * step;
+            const double z = dot(q, tv);
+            if (j >= n) continue;
+            const double vh = S.init ? z : z - beta * (double)S.v[j];
+            if (lane == 0) {
+                if (ONE) vv[j] = vh;
+                else S.vhat[j] = vh;
+            }
+            vh2 += vh * vh;
+        }
+    }
+    // the rows of M fly while the sums and barriers run
+#pragma unroll
+    for (int q = 0; q < CPW; ++q) {
+        const int i = first + q * step;
+        fetch(S.Rrm, q, i, full ? 0 : i, n);
+    }
+    double a2 = block_sum(lane == 0 ? vh2 : 0.0, sm);
+    if (!ONE) {
+        if (threadIdx.x == 0) S.cpart[16 + rank] = a2;
+        nside_barrier<ONE>();
+        a2 = 0.0;
+        for (int k = 0; k < ncta; ++k) a2 += __ldcg(S.cpart + 16 + k);
+        for (int j = threadIdx.x; j < n; j += kNsideThreads) vv[j] = __ldcg(S.vhat + j);
+        __syncthreads();
+    }
+
+    // N3: alpha, v, p = M v, x and wt
+    const double alpha = sqrt(a2);
+    const double inva = alpha > 0.0 ? 1.0 / alpha : 0.0;
+    const Givens g = givens(st0.rho_bar, st0.phi_bar, alpha, beta);
+    const double step_x = g.rho > 0.0 ? g.phi / g.rho : 0.0;
+    const double step_w = g.rho > 0.0 ? g.theta / g.rho : 0.0;
+    double xs = 0.0;
+    for (int i0 = first; i0 < n; i0 += CPW * step) {
+        if (i0 != first) fetch(S.Rrm, 0, i0, full ? 0 : i0, n);
+#pragma unroll
+        for (int q = 0; q < CPW; ++q) {
+            const int i = i0 + q * step;
+            const double pi = dot(q, vv) * inva;
+            if (i >= n || lane != 0) continue;
+            S.v[i] = (float)(vv[i] * inva);
+            double xi = (double)S.x[i];
+            if (S.init) {
+                S.wt[i] = (float)pi;
+            } else {
+                const double wi = (double)S.wt[i];
+                xi += step_x * wi;
+                S.x[i] = (float)xi;
+                S.wt[i] = (float)(pi - step_w * wi);
+            }
+            S.p[i] = (float)pi;
+            const double xf = (double)(float)xi * (S.dscale ? S.dscale[i] : 1.0);
+            xs += xf * xf;
+        }
+    }
+    xs = block_sum(xs, sm);
+    if (!ONE) {
+        if (threadIdx.x == 0) S.cpart[32 + rank] = xs;
+        nside_barrier<ONE>();
+    }
+
+    // N4
+    if (rank != 0 || threadIdx.x != 0) return;
+    if (!ONE) {
+        xs = qn2 = 0.0;
+        for (int k = 0; k < ncta; ++k) {
+            xs += __ldcg(S.cpart + 32 + k);
+            qn2 += __ldcg(S.cpart + k);
+        }
+    }
+    S.scal[0] = beta;
+    S.scal[1] = alpha;
+    finish_state(S, st0, g, beta, alpha, sqrt(xs), S.init ? sqrt(qn2) : 0.0);
+}
+
+// CTAs of the n-side cluster (0: the four kernels): sixteen where the GPU
+// can place such a cluster, else the portable eight.  Asked of the driver
+// once per process and device.
+static int nside_cluster_size() {
+    static std::mutex mu;
+    static int size[64];
+    static bool known[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    if (known[dev]) return size[dev];
+    size[dev] = 0;
+    cudaFuncSetAttribute(nside_fused_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int c : {16, 8}) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)c);
+        cfg.blockDim = dim3(kNsideThreads);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)c;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, nside_fused_kernel<false>, &cfg) == cudaSuccess && fit >= 1) {
+            size[dev] = c;
+            break;
+        }
+    }
+    cudaGetLastError();
+    known[dev] = true;
+    return size[dev];
 }
 
 // ------------------------------------------------------------ workspace
@@ -428,7 +684,7 @@ __global__ void __launch_bounds__(256) nside_finish_kernel(NSide S) {
 static void ws_free(tomos_workspace* ws) {
     void* ptrs[] = {ws->u,      ws->v,      ws->wt,     ws->p,    ws->qvec,   ws->t,
                     ws->vhat,   ws->qpart,  ws->sspart, ws->vpart, ws->xpart, ws->qnpart,
-                    ws->scal,   ws->coef_init, ws->bpart, ws->fro2, ws->st,   ws->Rcm,
+                    ws->scal,   ws->cpart,  ws->coef_init, ws->bpart, ws->fro2, ws->st,   ws->Rcm,
                     ws->Rrm,    ws->hist,   ws->scratch, ws->h16, ws->adj, ws->csc, ws->shard, ws->adjb,
                     ws->xg,     ws->dscale};
     for (void* q : ptrs)
@@ -741,6 +997,7 @@ static NSide make_nside(tomos_workspace* ws, const PassPlan& pl, float* x, bool 
     S.nb1 = ws->nb1;
     S.nb3 = ws->nb3;
     S.scal = ws->scal;
+    S.cpart = ws->cpart;
     S.st = ws->st;
     S.skip = skip;
     S.qsum = nullptr;
@@ -755,6 +1012,28 @@ static NSide make_nside(tomos_workspace* ws, const PassPlan& pl, float* x, bool 
 }
 
 static tomos_status enqueue_nside(tomos_workspace* ws, const NSide& S, cudaStream_t st) {
+    if (S.has_precond && S.n <= kNsideOneMaxN) {
+        nside_fused_kernel<true><<<1, kNsideThreads, 0, st>>>(S);
+        TOMOS_LAUNCH_CHECK("nside_fused_kernel");
+        ws->launches += 1;
+        return TOMOS_OK;
+    }
+    const int cl = S.has_precond && S.n <= kNsideClusterMaxN ? nside_cluster_size() : 0;
+    if (cl > 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)cl);
+        cfg.blockDim = dim3(kNsideThreads);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)cl;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        TOMOS_CUDA_TRY(cudaLaunchKernelEx(&cfg, nside_fused_kernel<false>, S));
+        ws->launches += 1;
+        return TOMOS_OK;
+    }
     nside_reduce_kernel<<<ws->nb1, 256, 0, st>>>(S);
     TOMOS_LAUNCH_CHECK("nside_reduce_kernel");
     if (S.has_precond) {
@@ -1375,6 +1654,7 @@ tomos_status tomos_workspace_create(int64_t m, int64_t n, int32_t value_type,
     A(alloc(&ws->xpart, (size_t)ws->nb3));
     A(alloc(&ws->qnpart, (size_t)ws->nb1));
     A(alloc(&ws->scal, 8));
+    A(alloc(&ws->cpart, 48));
     A(alloc(&ws->coef_init, 2));
     A(alloc(&ws->bpart, (size_t)ws->gs_max));
     A(alloc(&ws->fro2, 1));

@@ -186,6 +186,7 @@ struct tomos_workspace {
     double* xpart = nullptr;
     double* qnpart = nullptr;
     double* scal = nullptr;
+    double* cpart = nullptr;  // 3 x 16: the cluster n-side's per-CTA partials
     double* coef_init = nullptr;
     double* bpart = nullptr;
     double* fro2 = nullptr;

@@ -467,6 +467,19 @@ tomos_status tomos_lsqr_solve_dense(const tomos_dense* A, const float* b, float*
 tomos_status tomos_lsqr_solve_csr(const tomos_csr* A, const float* b, float* x,
                                   tomos_workspace* ws, const tomos_lsqr_opts* opts,
                                   tomos_lsqr_report* report, void* stream);
+/* min ||A x_k - b_k|| for the K columns of B (FP32, device, leading
+ * dimension ldb) into the columns of X, as K calls of tomos_lsqr_solve_dense
+ * would solve them, sharing every pass over A: an iteration reads A once for
+ * all columns.  Under the BACKWARD rule with ||A|| given (anorm_fro_dev or
+ * anorm_fro), a preconditioner attached, FP32 row-major A with 16-byte
+ * aligned rows, n <= 512 and 2 <= K <= 8; TOMOS_ERR_UNSUPPORTED otherwise
+ * (tomos_lsqr_batch_supported tells for the matrix).  Reports one per column.
+ * No reference counterpart (its lsqr_solve takes one right-hand side). */
+int32_t tomos_lsqr_batch_supported(const tomos_dense* A, int32_t K, const tomos_workspace* ws);
+tomos_status tomos_lsqr_solve_batch_dense(const tomos_dense* A, int32_t K, const float* B,
+                                          int64_t ldb, float* X, int64_t ldx, tomos_workspace* ws,
+                                          const tomos_lsqr_opts* opts, tomos_lsqr_report* reports,
+                                          void* stream);
 
 /* Normwise backward error of x (FP64, ACCURATE tier): fills report's
  * rnorm, arnorm, anorm_fro, xnorm, bnorm and backward_error.  col_scale

@@ -178,3 +178,44 @@ def test_adjoint_batch_packed_and_plain(orc, numeric):
     _, Lam_np, _, _, reps_np = gpu_grads(A0, B0, G0, precond=False, batch=True)
     assert all(r["converged"] for r in reps_np)
     assert rel(Lam_np[:, [0, 2]], Lr[:, [0, 2]]) < 1e-5
+
+
+@pytest.mark.parametrize("m,n,K,pad", [(5000, 100, 8, 0), (20011, 500, 5, 0), (777, 33, 2, 3), (3000, 511, 9, 1),
+                                       (40, 8, 3, 0)])
+def test_batched_solves_match_single(m, n, K, pad):
+    """lsqr_solve_batch (shared passes; K = 9 is a group of eight and a column
+    of its own): columns that stop at different times, one of them zero,
+    against lsqr_solve per column and the FP64 solution."""
+    rng = np.random.default_rng(m + n)
+    A0 = rng.standard_normal((m, n)).astype(np.float32)
+    X0 = rng.standard_normal((n, K))
+    B0 = (A0.astype(np.float64) @ X0 + 10.0 ** rng.uniform(-6, 0, K) * rng.standard_normal((m, K))).astype(np.float32)
+    B0[:, 1] = 0.0
+    A = to_dense(A0, L.ROW_MAJOR, pad=pad)
+    SA, _, colsq = tb.apply_count_sketch(A, 4 * n, with_colsq=True)
+    ws = tb.create_lsqr_workspace(None, (m, n), NT.FP32, NT.FP64)
+    Rinv = tb.generate_sketch_qr_precond(SA)
+    tb.add_precond(Rinv, ws)
+    d, an = tb.column_scale(colsq)
+    for tol in (1e-6, 1e-9):  # 1e-9: FP64 products in the certifying passes, never met
+        X, reps = tb.lsqr_solve_batch(A, cuda(B0), ws, tol, 30, 3, an, col_scale=d)
+        X = X.cpu().numpy()
+        ref = np.linalg.lstsq(A0.astype(np.float64), B0.astype(np.float64), rcond=None)[0]
+        for k in range(K):
+            x = torch.zeros(n, device="cuda")
+            rep = tb.lsqr_solve(None, A, cuda(B0[:, k]), x, ws, tol, 30, 0.0, restarts=3,
+                                stop_rule=tb.StopRule.BACKWARD, anorm_fro=an, col_scale=d)
+            x = x.cpu().numpy()
+            if k == 1:
+                assert not X[:, k].any() and reps[k]["converged"] == 1
+                continue
+            assert reps[k]["converged"] == rep["converged"], (k, reps[k], rep)
+            assert abs(reps[k]["iterations"] - rep["iterations"]) <= (1 if tol > 1e-7 else 90)
+            # a backward error of 1e-6 with ||A D^-1||_F = sqrt(n): A (x - x*)
+            # is below 1e-6 (sqrt(n) ||D x|| + ||b||), and the smallest
+            # singular value of A D^-1 (Gaussian) near 1 - sqrt(n / m)
+            bound = 1e-6 * (np.sqrt(n) + 2) / (1 - np.sqrt(n / m))
+            assert rel(X[:, k], ref[:, k]) < bound and rel(x, ref[:, k]) < bound, k
+    again, _ = tb.lsqr_solve_batch(A, cuda(B0), ws, 1e-6, 30, 3, an, col_scale=d)
+    first, _ = tb.lsqr_solve_batch(A, cuda(B0), ws, 1e-6, 30, 3, an, col_scale=d)
+    assert torch.equal(again, first)

@@ -708,6 +708,45 @@ def lsqr_solve(ctx, A, b, x, workspace, tol, max_iters, max_relres, iterations=N
     return out
 
 
+def lsqr_solve_batch(A, B, workspace, tol, max_iters, restarts, anorm_fro, col_scale=None, inner_rtol=0.0,
+                     stream=None):
+    """Solutions X (n x K) of min ||A x_k - b_k|| for the K columns of B (m x K
+    float32 CUDA tensor) under the BACKWARD rule, with the workspace's
+    preconditioner: columns in groups that share every pass over A
+    (tomos_lsqr_solve_batch_dense) where the matrix allows it, one by one
+    (lsqr_solve) otherwise.  anorm_fro: the device value of column_scale.
+    Returns (X, list of K reports)."""
+    m, n = A.size
+    K = B.shape[1]
+    Bc = B.t().contiguous().float()  # column-major m x K
+    Xc = torch.empty((K, n), dtype=torch.float32, device="cuda")
+    d = A.desc()
+    reports = []
+    for k0 in range(0, K, 8):
+        k = min(8, K - k0)
+        if isinstance(A, Dense) and C.lib().tomos_lsqr_batch_supported(ctypes.byref(d), k, workspace.handle):
+            opts = C.LsqrOpts()
+            opts.tol = float(tol)
+            opts.max_iters = int(max_iters)
+            opts.restarts = int(restarts)
+            opts.stop_rule = int(StopRule.BACKWARD)
+            opts.iter_tier = int(Tier.AUTO)
+            opts.inner_rtol = float(inner_rtol)
+            opts.anorm_fro_dev = anorm_fro.data_ptr()
+            opts.col_scale = col_scale.data_ptr() if col_scale is not None else None
+            reps = (C.LsqrReport * k)()
+            C.check(C.lib().tomos_lsqr_solve_batch_dense(ctypes.byref(d), k, _ptr(Bc[k0]), m, _ptr(Xc[k0]), n,
+                                                         workspace.handle, ctypes.byref(opts), reps, _stream(stream)),
+                    "lsqr_solve_batch")
+            reports += [r.as_dict() for r in reps]
+            continue
+        for j in range(k0, k0 + k):
+            reports.append(lsqr_solve(None, A, Bc[j], Xc[j], workspace, tol, max_iters, 0.0, restarts=restarts,
+                                      stop_rule=StopRule.BACKWARD, inner_rtol=inner_rtol, anorm_fro=anorm_fro,
+                                      col_scale=col_scale, stream=stream))
+    return Xc.t(), reports
+
+
 def backward_error(A, b, x, workspace, col_scale=None, stream=None):
     """Normwise backward error of x (FP64, accurate tier); with col_scale D
     (float64 CUDA tensor) the backward error of the column-scaled problem."""

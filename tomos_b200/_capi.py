@@ -96,6 +96,9 @@ SIGNATURES = {
     "tomos_mm_ex": (c_i32, [c_i32, c_i32, c_dbl, ctypes.POINTER(DenseDesc), c_i32,
                             ctypes.POINTER(DenseDesc), c_dbl, ctypes.POINTER(DenseDesc), c_vp,
                             ctypes.c_size_t, c_vp]),
+    "tomos_lsqr_batch_supported": (c_i32, [ctypes.POINTER(DenseDesc), c_i32, c_vp]),
+    "tomos_lsqr_solve_batch_dense": (c_i32, [ctypes.POINTER(DenseDesc), c_i32, c_vp, c_i64, c_vp, c_i64, c_vp,
+                                             ctypes.POINTER(LsqrOpts), ctypes.POINTER(LsqrReport), c_vp]),
     "tomos_lsqr_adjoint_batch_dense": (c_i32, [ctypes.POINTER(DenseDesc), c_i32, c_vp, c_i64, c_vp, c_i64,
                                                c_vp, ctypes.POINTER(LsqrOpts), c_vp, c_vp]),
     "tomos_mm_scratch_bytes": (ctypes.c_size_t, [c_i32, c_i32, ctypes.POINTER(DenseDesc), c_i32,

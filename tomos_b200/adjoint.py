@@ -1,7 +1,7 @@
 """Differentiable least squares over the C ABI.
 
-X = argmin ||A X - B|| column by column (sketch-preconditioned LSQR,
-tomos_lsqr_solve_dense), with gradients in A and B from the adjoint:
+X = argmin ||A X - B|| column by column (sketch-preconditioned LSQR, the
+columns sharing their passes over A: lsqr_solve_batch), with gradients in A and B from the adjoint:
 for a loss L with G = dL/dX,
     Lam   = (A^T A)^{-1} G        (tomos_lsqr_adjoint_batch_dense: all columns at
                                     once, reusing R^{-1})
@@ -11,9 +11,9 @@ the last two in one pass over A (tomos_lsqr_adjoint_grad_dense).
 """
 import torch
 
-from . import (Dense, Layout, NumericType, StopRule, add_precond, apply_count_sketch, column_scale,
+from . import (Dense, Layout, NumericType, add_precond, apply_count_sketch, column_scale,
                create_lsqr_workspace, generate_sketch_qr_precond, lsqr_adjoint_batch,
-               lsqr_adjoint_grad, lsqr_solve)
+               lsqr_adjoint_grad, lsqr_solve_batch)
 
 
 class LeastSquares(torch.autograd.Function):
@@ -34,12 +34,8 @@ class LeastSquares(torch.autograd.Function):
         dsc, anorm = column_scale(colsq)
         ws = create_lsqr_workspace(None, (m, n), NumericType.FP32, NumericType.FP64)
         add_precond(Rinv, ws)
-        X = torch.empty((n, B2.shape[1]), dtype=torch.float32, device=A.device)
-        for k in range(B2.shape[1]):
-            x = torch.zeros(n, dtype=torch.float32, device=A.device)
-            lsqr_solve(None, D, B2[:, k].contiguous(), x, ws, tol, max_iters, 0.0, restarts=4,
-                       stop_rule=StopRule.BACKWARD, anorm_fro=anorm, col_scale=dsc)
-            X[:, k] = x
+        X, _ = lsqr_solve_batch(D, B2, ws, tol, max_iters, 4, anorm, col_scale=dsc)
+        X = X.contiguous()
         ctx.save_for_backward(A, B2, X)
         ctx.state = (D, ws, Rinv, tol, max_iters, B.shape)
         return X if B.dim() == 2 else X[:, 0]

@@ -4,10 +4,11 @@
 // (adjoint.cu: CG on R^{-T} A^T A R^{-1} mu = R^{-T} g, lambda = R^{-1} mu),
 // one recurrence per right-hand side, but the products with A are shared:
 // every iteration forms, for all K directions P (n x K) at once,
-//   Q = A P      one tcgen05 product over A (tomos_mm_ex), and
-//   W = A^T Q    a second one, its long K (the m rows) split over CTAs,
-// so A is read twice an iteration for all K instead of once per right-hand
-// side.  The n-side kernels run every column k in blockIdx.y; a column
+//   Q = A P and W = A^T Q,
+// from one read of an FP32 row-major A (multi_rows_kernel, lsqr_batch.cu; K
+// <= 8, n <= 512), else as two products (tomos_mm_ex, the second one's long K
+// split over CTAs).  At 200000 x 500 and eight columns: two tensor-core
+// products took 400 us an iteration.  The n-side kernels run every column k in blockIdx.y; a column
 // whose recurrence has stopped returns at once.  Scalars and vectors are
 // FP64; the direction goes to the products as FP32.
 #include <cmath>
@@ -16,6 +17,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gemv.cuh"
 #include "lsqr.cuh"
 
 namespace tomos_b200 {
@@ -270,7 +272,11 @@ tomos_status tomos_lsqr_adjoint_batch_dense(const tomos_dense* A, int32_t K, con
     const size_t o_q32 = take(sizeof(float) * (size_t)(m > 0 ? m : 1) * K);
     const size_t o_col = take(sizeof(AdjCol) * K);
     const size_t o_part = take(sizeof(double) * (size_t)K * nbp * 3);
+    // FP32 row-major A: both products from one read of A (lsqr_batch.cu)
+    const bool multi = multi_pass_ok(A, K) && (tier == TOMOS_TIER_AUTO || tier == TOMOS_TIER_NATIVE);
     const size_t o_mm = take(mmb > 0 ? mmb : 1);
+    const size_t o_mp = take(multi ? sizeof(float) * (size_t)multi_pass_grid(m) * nk : 1);
+    const size_t o_coef = take(2 * sizeof(double));
     if (off > ws->adjb_bytes) {
         if (ws->adjb) cudaFree(ws->adjb);
         ws->adjb = nullptr;
@@ -301,6 +307,23 @@ tomos_status tomos_lsqr_adjoint_batch_dense(const tomos_dense* A, int32_t K, con
     a.rz_part = a.rr_part + (size_t)K * nbp;
     a.pw_part = a.rz_part + (size_t)K * nbp;
     void* mmscratch = base + o_mm;
+    MultiPass mp;
+    mp.A = static_cast<const float*>(A->values);
+    mp.m = m;
+    mp.n = n;
+    mp.ld = A->ld;
+    mp.K = K;
+    mp.p = a.p32;
+    mp.ps = n;
+    mp.u_in = nullptr;
+    mp.ui = 0;
+    mp.u_out = nullptr;
+    mp.uo = 0;
+    mp.coef = reinterpret_cast<const double*>(base + o_coef);  // ut = A p
+    mp.st = nullptr;
+    mp.qpart = reinterpret_cast<float*>(base + o_mp);
+    mp.qs = n;
+    mp.sspart = nullptr;
     a.G = G;
     a.ldg = ldg;
     a.tol = opts->tol > 0.0 ? opts->tol : 0.0;
@@ -317,6 +340,8 @@ tomos_status tomos_lsqr_adjoint_batch_dense(const tomos_dense* A, int32_t K, con
     const int64_t launches0 = ws->launches;
     s = refresh_precond(ws, st);
     if (s) return s;
+    const double one[2] = {1.0, 0.0};
+    TOMOS_CUDA_TRY(cudaMemcpyAsync(base + o_coef, one, sizeof(one), cudaMemcpyHostToDevice, st));
     a.Rcm = ws->has_precond ? ws->Rcm : nullptr;
     a.Rrm = ws->has_precond ? ws->Rrm : nullptr;
 
@@ -349,9 +374,16 @@ tomos_status tomos_lsqr_adjoint_batch_dense(const tomos_dense* A, int32_t K, con
         const int left = opts->max_iters - iters;
         const int kk = batch < left ? batch : left;
         for (int it = 0; it < kk; ++it) {
-            s = tomos_mm_ex(TOMOS_NO_TRANSPOSE, TOMOS_NO_TRANSPOSE, 1.0, A, tier, &P, 0.0, &Q, mmscratch, mmb, st);
-            if (s) return s;
-            s = tomos_mm_ex(TOMOS_TRANSPOSE, TOMOS_NO_TRANSPOSE, 1.0, A, tier, &Q, 0.0, &W, mmscratch, mmb, st);
+            if (multi) {
+                s = enqueue_multi_pass(mp, st);
+                if (s) return s;
+                s = launch_sum_parts(mp.qpart, multi_pass_grid(m), (int64_t)nk, (int64_t)nk, 1.0, 0.0, nullptr, nullptr,
+                                     a.w32, st);
+            } else {
+                s = tomos_mm_ex(TOMOS_NO_TRANSPOSE, TOMOS_NO_TRANSPOSE, 1.0, A, tier, &P, 0.0, &Q, mmscratch, mmb, st);
+                if (s) return s;
+                s = tomos_mm_ex(TOMOS_TRANSPOSE, TOMOS_NO_TRANSPOSE, 1.0, A, tier, &Q, 0.0, &W, mmscratch, mmb, st);
+            }
             if (s) return s;
             bk_w_kernel<<<gu, 256, 0, st>>>(a);
             TOMOS_LAUNCH_CHECK("bk_w_kernel");
@@ -385,7 +417,7 @@ tomos_status tomos_lsqr_adjoint_batch_dense(const tomos_dense* A, int32_t K, con
             R.converged = h[(size_t)k].converged;
             R.relres = h[(size_t)k].gg > 0.0 ? std::sqrt(h[(size_t)k].rr / h[(size_t)k].gg) : 0.0;
             R.elapsed_ms = ms;
-            R.half_passes = 2 * iters;  // shared: two products over A an iteration
+            R.half_passes = multi ? iters : 2 * iters;  // shared: one or two passes over A an iteration
             R.kernel_launches = (int32_t)(ws->launches - launches0);
         }
     }

@@ -157,39 +157,21 @@ __global__ void __launch_bounds__(256) column_scale_kernel(const double* __restr
 
 // ------------------------------------------------------------- n-side
 
-struct NSide {
-    int64_t n;
-    const float* qpart;
-    int64_t qstride;
-    int gq;
-    const double* sspart;
-    int gs;
-    double* t;
-    double* vhat;
-    float* v;
-    float* wt;
-    float* p;
-    float* x;
-    double* vpart;
-    double* xpart;
-    double* qnpart;
-    const double* Rcm;
-    const double* Rrm;
-    int has_precond;
-    int init;
-    int nb1;   // N1 blocks
-    int nb3;   // N2/N3 blocks
-    double* scal;
-    double* cpart;
-    LsqrDev* st;
-    const int* skip;
-    const double* dscale;  // column scale D of the backward-error rule, or NULL
-    const double* qsum;    // row-sharded solves: A^T ut summed over ranks (n), else NULL
-    // The iteration graph's while loop: N4 sets its condition (1: run the
-    // body again) on every path, so the loop ends once the solver stops.
-    cudaGraphConditionalHandle cond;
-    int use_cond;
-};
+// Sets the loop's condition at the end of a body: this solver's `again`, or,
+// for the last of a batch's columns to get here, whether any goes on.
+__device__ __forceinline__ void set_condition(const NSide& S, bool again) {
+    if (!S.ticket) {
+        cudaGraphSetConditional(S.cond, again ? 1u : 0u);
+        return;
+    }
+    __threadfence();  // this column's state before its ticket
+    if (atomicAdd(S.ticket, 1) != S.group - 1) return;
+    __threadfence();
+    *(volatile int*)S.ticket = 0;
+    bool any = false;
+    for (int k = 0; k < S.group; ++k) any = any || *(const volatile int*)&S.group_st[k].done == 0;
+    cudaGraphSetConditional(S.cond, any ? 1u : 0u);
+}
 
 // Givens step of LSQR (lsqr.cpp:633-679), FP64.
 struct Givens {
@@ -386,7 +368,7 @@ __device__ __forceinline__ void finish_state(const NSide& S, const LsqrDev& in, 
         st->relres = in.rhsnorm > 0.0 ? beta / in.rhsnorm : 0.0;
         st->done = 0;
         st->breakdown = (alpha == 0.0 || beta == 0.0) ? 1 : 0;
-        if (S.use_cond) cudaGraphSetConditional(S.cond, 0u);  // no loop runs init passes
+        if (S.use_cond) set_condition(S, false);  // no loop runs init passes
         return;
     }
     st->alpha = alpha;
@@ -418,7 +400,7 @@ __device__ __forceinline__ void finish_state(const NSide& S, const LsqrDev& in, 
     }
     if (iter_restart >= in.max_iters) stop = 1;
     if (stop) st->done = 1;
-    if (S.use_cond) cudaGraphSetConditional(S.cond, stop ? 0u : 1u);
+    if (S.use_cond) set_condition(S, !stop);
 }
 
 // N4: one block.
@@ -460,7 +442,7 @@ __device__ __forceinline__ void nside_barrier() {
 // otherwise a cluster, columns w ncta + rank, .. of up to 512 entries (one,
 // or two in a cluster of eight, loaded one after the other).
 template <bool ONE>
-__global__ void __launch_bounds__(kNsideThreads, 1) nside_fused_kernel(NSide S) {
+__device__ __forceinline__ void nside_fused(const NSide& S) {
     constexpr int W = kNsideThreads / 32;
     constexpr int MAXN = ONE ? kNsideOneMaxN : kNsideClusterMaxN;
     constexpr int NL = MAXN / 32;               // entries of a column a lane holds
@@ -470,7 +452,7 @@ __global__ void __launch_bounds__(kNsideThreads, 1) nside_fused_kernel(NSide S) 
     // the flag is written by CTA 0 after the last barrier only, so every CTA
     // of the cluster takes the same way here
     if (S.skip && *S.skip) {
-        if (S.use_cond && rank == 0 && threadIdx.x == 0) cudaGraphSetConditional(S.cond, 0u);
+        if (S.use_cond && rank == 0 && threadIdx.x == 0) set_condition(S, false);
         return;
     }
     __shared__ double sm[32];
@@ -645,6 +627,20 @@ __global__ void __launch_bounds__(kNsideThreads, 1) nside_fused_kernel(NSide S) 
     finish_state(S, st0, g, beta, alpha, sqrt(xs), S.init ? sqrt(qn2) : 0.0);
 }
 
+template <bool ONE>
+__global__ void __launch_bounds__(kNsideThreads, 1) nside_fused_kernel(NSide S) {
+    nside_fused<ONE>(S);
+}
+
+// The columns of a batched solve, one cluster (or CTA) each.
+struct NSideBatch {
+    NSide s[kBatchMax];
+};
+template <bool ONE>
+__global__ void __launch_bounds__(kNsideThreads, 1) nside_batch_kernel(const __grid_constant__ NSideBatch B) {
+    nside_fused<ONE>(B.s[blockIdx.y]);
+}
+
 // CTAs of the n-side cluster (0: the four kernels): sixteen where the GPU
 // can place such a cluster, else the portable eight.  Asked of the driver
 // once per process and device.
@@ -658,6 +654,7 @@ static int nside_cluster_size() {
     if (known[dev]) return size[dev];
     size[dev] = 0;
     cudaFuncSetAttribute(nside_fused_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(nside_batch_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     for (int c : {16, 8}) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)c);
@@ -686,11 +683,12 @@ static void ws_free(tomos_workspace* ws) {
                     ws->vhat,   ws->qpart,  ws->sspart, ws->vpart, ws->xpart, ws->qnpart,
                     ws->scal,   ws->cpart,  ws->coef_init, ws->bpart, ws->fro2, ws->st,   ws->Rcm,
                     ws->Rrm,    ws->hist,   ws->scratch, ws->h16, ws->adj, ws->csc, ws->shard, ws->adjb,
-                    ws->xg,     ws->dscale};
+                    ws->xg,     ws->dscale, ws->bat};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     if (ws->st_host) cudaFreeHost(ws->st_host);
     if (ws->graph) cudaGraphExecDestroy(ws->graph);
+    if (ws->bgraph) cudaGraphExecDestroy(ws->bgraph);
     if (ws->ev_start) cudaEventDestroy(ws->ev_start);
     if (ws->ev_stop) cudaEventDestroy(ws->ev_stop);
     if (ws->ev_fence) cudaEventDestroy(ws->ev_fence);
@@ -971,8 +969,8 @@ tomos_status enqueue_dense_pass(tomos_workspace* ws, const tomos_dense* A,
 
 // ------------------------------------------------------------ n-side glue
 
-static NSide make_nside(tomos_workspace* ws, const PassPlan& pl, float* x, bool init,
-                        const int* skip, const double* dscale = nullptr) {
+NSide make_nside(tomos_workspace* ws, const PassPlan& pl, float* x, bool init, const int* skip,
+                 const double* dscale) {
     NSide S;
     S.dscale = dscale;
     S.n = ws->n;
@@ -1003,6 +1001,9 @@ static NSide make_nside(tomos_workspace* ws, const PassPlan& pl, float* x, bool 
     S.qsum = nullptr;
     S.cond = 0;
     S.use_cond = 0;
+    S.ticket = nullptr;
+    S.group = 0;
+    S.group_st = nullptr;
     if (ws->comm) {  // the pass's partials were folded and summed across ranks
         S.qsum = ws->shard;
         S.sspart = ws->shard + ws->n;
@@ -1011,7 +1012,7 @@ static NSide make_nside(tomos_workspace* ws, const PassPlan& pl, float* x, bool 
     return S;
 }
 
-static tomos_status enqueue_nside(tomos_workspace* ws, const NSide& S, cudaStream_t st) {
+tomos_status enqueue_nside(tomos_workspace* ws, const NSide& S, cudaStream_t st) {
     if (S.has_precond && S.n <= kNsideOneMaxN) {
         nside_fused_kernel<true><<<1, kNsideThreads, 0, st>>>(S);
         TOMOS_LAUNCH_CHECK("nside_fused_kernel");
@@ -1045,6 +1046,32 @@ static tomos_status enqueue_nside(tomos_workspace* ws, const NSide& S, cudaStrea
     nside_finish_kernel<<<1, 256, 0, st>>>(S);
     TOMOS_LAUNCH_CHECK("nside_finish_kernel");
     ws->launches += S.has_precond ? 4 : 3;
+    return TOMOS_OK;
+}
+
+bool nside_batch_ok(int64_t n) { return n >= 1 && (n <= kNsideOneMaxN || (n <= kNsideClusterMaxN && nside_cluster_size() > 0)); }
+
+tomos_status enqueue_nside_batch(tomos_workspace* ws, const NSide* S, int K, cudaStream_t st) {
+    NSideBatch B;
+    for (int k = 0; k < kBatchMax; ++k) B.s[k] = S[k < K ? k : 0];
+    ws->launches += 1;
+    if (S[0].n <= kNsideOneMaxN) {
+        nside_batch_kernel<true><<<dim3(1, (unsigned)K), kNsideThreads, 0, st>>>(B);
+        TOMOS_LAUNCH_CHECK("nside_batch_kernel");
+        return TOMOS_OK;
+    }
+    const int cl = nside_cluster_size();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)cl, (unsigned)K);
+    cfg.blockDim = dim3(kNsideThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cl;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    TOMOS_CUDA_TRY(cudaLaunchKernelEx(&cfg, nside_batch_kernel<false>, B));
     return TOMOS_OK;
 }
 
@@ -1173,7 +1200,7 @@ static tomos_status sync_state(tomos_workspace* ws) {
     return TOMOS_OK;
 }
 
-static double eta_of(const LsqrDev& s) {
+double eta_of(const LsqrDev& s) {
     const double den1 = s.anorm_fro * s.xnorm + s.bnorm;
     const double e1 = den1 > 0.0 ? s.beta / den1 : 0.0;
     const double den2 = s.anorm_fro * s.beta;

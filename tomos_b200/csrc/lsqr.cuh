@@ -36,6 +36,47 @@ struct LsqrDev {
     int pad_;
 };
 
+// The n-side kernels' arguments: N1 to N4 of one column's iteration.
+struct NSide {
+    int64_t n;
+    const float* qpart;
+    int64_t qstride;
+    int gq;
+    const double* sspart;
+    int gs;
+    double* t;
+    double* vhat;
+    float* v;
+    float* wt;
+    float* p;
+    float* x;
+    double* vpart;
+    double* xpart;
+    double* qnpart;
+    const double* Rcm;
+    const double* Rrm;
+    int has_precond;
+    int init;
+    int nb1;   // N1 blocks
+    int nb3;   // N2/N3 blocks
+    double* scal;
+    double* cpart;
+    LsqrDev* st;
+    const int* skip;
+    const double* dscale;  // column scale D of the backward-error rule, or NULL
+    const double* qsum;    // row-sharded solves: A^T ut summed over ranks (n), else NULL
+    // The iteration graph's while loop: N4 sets its condition (1: run the
+    // body again) on every path, so the loop ends once the solver stops.
+    cudaGraphConditionalHandle cond;
+    int use_cond;
+    // Batched solves: the columns' states; the loop runs while one of them is
+    // not done, and the last of the group to finish a body (ticket, zero
+    // between bodies) sets the condition.
+    int* ticket;
+    int group;
+    const LsqrDev* group_st;
+};
+
 // How one pass over A is run.
 // The BACKWARD tolerance from which the accurate passes sum FP32 runs.
 constexpr double kRunsTolMin = 1e-6;
@@ -159,6 +200,37 @@ tomos_status refresh_precond(tomos_workspace* ws, cudaStream_t st);
 
 tomos_status solve_driver(tomos_workspace* ws, PassOps& ops, const float* b, float* x,
                           const tomos_lsqr_opts* o, tomos_lsqr_report* rep, void* user_stream);
+// The n-side of one column, and of the K columns of a batched solve (whose
+// arguments differ only in their vectors and state; nside_batch_ok(n)).
+constexpr int kBatchMax = 8;
+NSide make_nside(tomos_workspace* ws, const PassPlan& pl, float* x, bool init, const int* skip,
+                 const double* dscale = nullptr);
+tomos_status enqueue_nside(tomos_workspace* ws, const NSide& S, cudaStream_t st);
+bool nside_batch_ok(int64_t n);
+tomos_status enqueue_nside_batch(tomos_workspace* ws, const NSide* S, int K, cudaStream_t st);
+double eta_of(const LsqrDev& s);
+
+// A pass for K columns at once (lsqr_batch.cu): FP32 row-major A.
+struct MultiPass {
+    const float* A;
+    int64_t m, n, ld;
+    int K;
+    const float* p;      // column k at p + k ps
+    int64_t ps;
+    const float* u_in;   // u_in + k ui (NULL: cu is taken as 0)
+    int64_t ui;
+    float* u_out;        // u_out + k uo (NULL: not written)
+    int64_t uo;
+    const double* coef;  // [cp, cu] for every column, or NULL: st[k].coef (and st[k].done skips column k)
+    const LsqrDev* st;
+    float* qpart;        // [CTA][K][qs]
+    int64_t qs;
+    double* sspart;      // [K][CTA] (NULL: not formed)
+};
+bool multi_pass_ok(const tomos_dense* A, int64_t K);
+int multi_pass_grid(int64_t m);
+tomos_status enqueue_multi_pass(const MultiPass& P, cudaStream_t st);
+
 tomos_status workspace_check(tomos_workspace* ws, int64_t m, int64_t n);
 tomos_status ensure_scratch(tomos_workspace* ws, size_t bytes);
 
@@ -220,6 +292,13 @@ struct tomos_workspace {
     float* xg = nullptr;
     // the column scale of the backward-error rule (copied from the caller's)
     double* dscale = nullptr;
+    // batched solves (lsqr_batch.cu): the columns' vectors, states and
+    // partials, grown as needed, and their iteration graph
+    void* bat = nullptr;
+    size_t bat_bytes = 0;
+    cudaGraphExec_t bgraph = nullptr;
+    int64_t bgraph_kernels = 0;
+    std::vector<uint64_t> bgraph_key;
     tomos_comm* comm = nullptr;  // the running solve's communicator (or NULL)
 
     bool has_precond = false;

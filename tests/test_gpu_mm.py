@@ -221,3 +221,20 @@ def test_mm_packed_operands(orc, numeric, la, lb, M, N, K, pad):
           bf16_ops=numeric == NT.FP32_BF16)
     check(orc, A, A0, tb.Tier.HALF_OPERANDS, T.NO_TRANSPOSE, T.NO_TRANSPOSE, (K, N), (lb, L.ROW_MAJOR), -0.5, rng,
           bf16_ops=numeric == NT.FP32_BF16)
+
+
+@pytest.mark.parametrize("numeric,rounded", [(NT.FP32, False), (NT.FP32_16, False), (NT.FP32_BF16, False),
+                                             (NT.FP32_BF16, True)])
+@pytest.mark.parametrize("layout", [L.COL_MAJOR, L.ROW_MAJOR])
+@pytest.mark.parametrize("m,n,k,pad", [(1, 1, 1, 0), (300, 100, 16, 4), (513, 257, 9, 0), (4099, 1000, 16, 0),
+                                       (2000, 1030, 3, 2), (20011, 500, 8, 0)])
+def test_mm_few_columns(orc, numeric, rounded, layout, m, n, k, pad):
+    """At most 16 columns with an exact A (split in registers), A and A^T,
+    lines along K and across it, aligned or not, split runs of K."""
+    rng = np.random.default_rng(m + n + k)
+    A0 = (rng.standard_normal((m, n)) * np.where(rng.random((m, n)) < 0.02, 1e-6, 1.0)).astype(np.float32)
+    A = to_dense(A0, layout, numeric, pad=pad, rounded=rounded)
+    for ta, kk in ((T.NO_TRANSPOSE, n), (T.TRANSPOSE, m)):
+        for lb, beta in ((L.COL_MAJOR, 0.0), (L.ROW_MAJOR, -0.5)):
+            check(orc, A, A0, tb.Tier.ACCURATE if numeric != NT.FP32 else tb.Tier.AUTO, ta, T.NO_TRANSPOSE, (kk, k),
+                  (lb, lb), beta, rng)

@@ -32,7 +32,8 @@
 //             (half decode, wide accumulation, fp32_16_kernels.cpp:113-141).
 //   kTf32x3   A exact (FP32 storage, or packed read exactly) split as
 //             A_big + A_small, B likewise: A_big B_big + A_big B_small +
-//             A_small B_big, three kind::tf32 products -- FP32-level
+//             A_small B_big, three kind::tf32 products (of at most 16
+//             columns: gemm_skinny.cuh) -- FP32-level
 //             products for the accurate tier (fp32_16_kernels.cpp:57-85).
 // Every product accumulates in FP32 in tensor memory; alpha and beta are
 // applied in FP64 in the epilogue.  The error of an entry is a few units
@@ -57,6 +58,7 @@
 #include <cudaTypedefs.h>
 
 #include "common.cuh"
+#include "gemm_skinny.cuh"
 #include "mbarrier.cuh"
 
 namespace tomos_b200 {
@@ -1452,18 +1454,66 @@ namespace tomos_b200 {
 namespace {
 
 // C(i, j) = alpha sum_z part[z](i, j) + beta C(i, j), the splits summed in
-// FP64 in split order (deterministic).
-__global__ void gemm_split_reduce_kernel(const float* __restrict__ part, int splits, int64_t M, int64_t N,
-                                         double alpha, double beta, float* c, int64_t si, int64_t sj) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= M * N) return;
-    const int64_t i = t % M, j = t / M;
+// FP64 in a fixed order.  A CTA owns 32 entries; its warps split the splits,
+// a thread with eight loads in flight (~2000 splits of 16000 entries at
+// K = 1e6: a thread an entry would walk them one latency after another).
+__global__ void __launch_bounds__(1024) gemm_split_reduce_kernel(const float* __restrict__ part, int splits, int64_t M,
+                                                                 int64_t N, double alpha, double beta, float* c,
+                                                                 int64_t si, int64_t sj) {
+    __shared__ double sm[32][33];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int64_t total = M * N, t = (int64_t)blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int z = 0; z < splits; ++z) s += (double)part[(size_t)z * M * N + t];
-    float* p = c + (size_t)(i * si + j * sj);
-    double y = alpha * s;
+    if (t < total) {
+        int z = w;
+        for (; z + 7 * nw < splits; z += 8 * nw) {
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = part[(size_t)(z + u * nw) * total + t];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += (double)v[u];
+        }
+        for (; z < splits; z += nw) s += (double)part[(size_t)z * total + t];
+    }
+    sm[w][lane] = s;
+    __syncthreads();
+    if (w != 0 || t >= total) return;
+    double d = 0.0;
+    for (int k = 0; k < nw; ++k) d += sm[k][lane];
+    float* p = c + (size_t)((t % M) * si + (t / M) * sj);
+    double y = alpha * d;
     if (beta != 0.0) y += beta * (double)*p;
     *p = (float)y;
+}
+
+// Products of at most 16 columns with an exactly read A (gemm_skinny.cuh).
+tomos_status launch_skinny_e(Elem e, const GemmArgs& g, int64_t run, int64_t runs, cudaStream_t st) {
+    SkinnyArgs a;
+    a.hi = g.a_hi;
+    a.lo = g.a_lo;
+    a.stride = g.a_kc ? g.a_si : g.a_sl;
+    a.b = g.b;
+    a.b_sl = g.b_sl;
+    a.b_sj = g.b_sj;
+    a.c = g.c;
+    a.c_si = g.c_si;
+    a.c_sj = g.c_sj;
+    a.M = g.M;
+    a.N = g.N;
+    a.K = g.K;
+    a.run = run;
+    a.runs = (int)runs;
+    a.alpha = g.alpha;
+    a.beta = g.beta;
+    a.part = g.part;
+    const bool kc = g.a_kc != 0;
+    switch (e) {
+        case Elem::F32: return launch_skinny<Elem::F32>(a, kc, st);
+        case Elem::A16: return launch_skinny<Elem::A16>(a, kc, st);
+        case Elem::AB16: return launch_skinny<Elem::AB16>(a, kc, st);
+        case Elem::AB16R: return launch_skinny<Elem::AB16R>(a, kc, st);
+        default: return fail(TOMOS_ERR_UNSUPPORTED, "mm: element type");
+    }
 }
 
 // Validates a product and fills the launch arguments (all but the split).
@@ -1560,6 +1610,33 @@ int split_count(const GemmArgs& g, int mode, int* kt_per) {
     return (int)((nk_all + per - 1) / per);
 }
 
+// The runs of K of a product through gemm_skinny.cuh, at most max_runs (their
+// length in *run); 0: not served.  Lines along M: a run a warp of each 64
+// columns, one wave of warps over the chip, runs of at least 64 lines.
+int64_t skinny_runs(const GemmArgs& g, int mode, int64_t max_runs, int64_t* run) {
+    if (mode != kTf32x3 || g.N > kSkinnyMaxN) return 0;
+    if (max_runs < 1) max_runs = 1;
+    int64_t runs = 1, most = kSkinnyDotK;
+    if (g.a_kc) {
+        int per;
+        runs = split_count(g, mode, &per);
+        if (runs > 65535) runs = 65535;
+    } else {
+        most = kSkinnySumLines;
+        const int64_t groups = (g.M + 63) / 64;
+        runs = (int64_t)sm_count() * kSkinnySumWarps * kSkinnySumCtas / groups;
+        if (runs > g.K / 64) runs = g.K / 64;
+        const int64_t least = (g.K + most - 1) / most;  // whole waves past that, too
+        if (runs > 0 && runs < least) runs = (least + runs - 1) / runs * runs;
+        if (runs < least) runs = least;
+        if (groups * runs > (int64_t)1 << 30) return 0;
+    }
+    if (runs > max_runs) runs = max_runs;
+    if (runs < 1) runs = 1;
+    *run = ((g.K + runs - 1) / runs + 31) / 32 * 32;
+    return *run <= most ? (g.K + *run - 1) / *run : 0;
+}
+
 }  // namespace
 }  // namespace tomos_b200
 
@@ -1578,7 +1655,8 @@ size_t tomos_mm_scratch_bytes(int32_t trans_a, int32_t trans_b, const tomos_dens
     if (g.M == 0 || g.N == 0 || g.K == 0) return 0;
     if (packed_bn(g, mode)) return packed_bytes(g);
     int per;
-    const int splits = split_count(g, mode, &per);
+    int64_t run, splits = skinny_runs(g, mode, INT64_MAX, &run);
+    if (!splits) splits = split_count(g, mode, &per);
     return splits > 1 ? (size_t)splits * (size_t)g.M * (size_t)g.N * sizeof(float) : 0;
 }
 
@@ -1610,7 +1688,10 @@ tomos_status tomos_mm_ex(int32_t trans_a, int32_t trans_b, double alpha, const t
         s = launch_packed_e(e, pbn, g, scratch, st, &used);
         if (used) return s;
     }
-    int splits = split_count(g, mode, &g.kt_per);
+    const size_t slice = (size_t)g.M * (size_t)g.N * sizeof(float);
+    int64_t run = 0;
+    const int64_t runs = skinny_runs(g, mode, scratch ? (int64_t)(scratch_bytes / slice) : 1, &run);
+    int splits = runs ? (int)runs : split_count(g, mode, &g.kt_per);
     const size_t need = (size_t)splits * (size_t)g.M * (size_t)g.N * sizeof(float);
     if (splits > 1 && (!scratch || scratch_bytes < need)) {
         // no (or too little) scratch: one split
@@ -1622,6 +1703,10 @@ tomos_status tomos_mm_ex(int32_t trans_a, int32_t trans_b, double alpha, const t
         case kPure16: s = launch_mode<kPure16>(e, g, st); break;
         case kTf32x2: s = launch_mode<kTf32x2>(e, g, st); break;
         default:
+            if (runs) {
+                s = launch_skinny_e(e, g, run, runs, st);
+                break;
+            }
             switch (e) {
                 case Elem::F32: s = launch_gemm<Elem::F32, kTf32x3>(g, st); break;
                 case Elem::A16: s = launch_gemm<Elem::A16, kTf32x3>(g, st); break;
@@ -1631,8 +1716,9 @@ tomos_status tomos_mm_ex(int32_t trans_a, int32_t trans_b, double alpha, const t
             }
     }
     if (s || splits == 1) return s;
-    gemm_split_reduce_kernel<<<(unsigned)((g.M * g.N + 255) / 256), 256, 0, st>>>(g.part, splits, g.M, g.N, alpha,
-                                                                                  beta, g.c, g.c_si, g.c_sj);
+    const int warps = splits >= 256 ? 32 : (splits + 7) / 8;
+    gemm_split_reduce_kernel<<<(unsigned)((g.M * g.N + 31) / 32), 32 * warps, 0, st>>>(g.part, splits, g.M, g.N, alpha,
+                                                                                       beta, g.c, g.c_si, g.c_sj);
     TOMOS_LAUNCH_CHECK("gemm_split_reduce_kernel");
     return TOMOS_OK;
 }

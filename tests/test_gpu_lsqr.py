@@ -279,3 +279,41 @@ def test_repeated_solves_on_one_workspace():
     for x, it, c, e in out[1:]:
         assert c == 1 and it == it0 and e == e0
         assert np.array_equal(x, x0)
+
+
+@pytest.mark.parametrize("m,n", [(777, 33), (20011, 300)])
+def test_workspaces_made_and_closed_by_threads(m, n):
+    """Workspaces that come and go on several threads and streams, sharing the
+    memory earlier ones gave back: the same solutions as one at a time, and
+    no more than the pool's 64 MiB kept."""
+    import threading
+    rng = np.random.default_rng(m)
+    A0 = rng.standard_normal((m, n)).astype(np.float32)
+    A = to_dense(A0, L.ROW_MAJOR)
+    b = [cuda((A0 @ rng.standard_normal(n) + 1e-3 * rng.standard_normal(m)).astype(np.float32)) for _ in range(4)]
+    torch.cuda.synchronize()
+
+    def solve(i):
+        x, _, _ = tb.sketch_lsqr(A, b[i], 4 * n, max_iters=30)
+        torch.cuda.current_stream().synchronize()
+        return x.clone()
+
+    want = [solve(i) for i in range(4)]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(5):
+                if not torch.equal(solve(i), want[i]):
+                    bad.append(i)
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not bad
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    for q in (1, 7, 20):  # u of 4 to 80 MB
+        tb.create_lsqr_workspace(None, (q * 1000000, n), NT.FP32, NT.FP64).close()
+    assert free0 - torch.cuda.mem_get_info()[0] <= (64 << 20) + (4 << 20)

@@ -349,7 +349,7 @@ static tomos_status launch_grad_e(int kk, const tomos_dense* A, const float* B, 
 static tomos_status ensure_adj(tomos_workspace* ws) {
     if (ws->adj) return TOMOS_OK;
     const AdjBufs need = adj_layout(nullptr, ws->n);
-    if (cudaMalloc(&ws->adj, need.bytes) != cudaSuccess) {
+    if (pool_malloc(&ws->adj, need.bytes) != cudaSuccess) {
         ws->adj = nullptr;
         cudaGetLastError();
         return fail(TOMOS_ERR_ALLOC, "adjoint workspace allocation failed");

@@ -278,10 +278,10 @@ tomos_status tomos_lsqr_adjoint_batch_dense(const tomos_dense* A, int32_t K, con
     const size_t o_mp = take(multi ? sizeof(float) * (size_t)multi_pass_grid(m) * nk : 1);
     const size_t o_coef = take(2 * sizeof(double));
     if (off > ws->adjb_bytes) {
-        if (ws->adjb) cudaFree(ws->adjb);
+        release_memory(ws, ws->adjb);
         ws->adjb = nullptr;
         ws->adjb_bytes = 0;
-        if (cudaMalloc(&ws->adjb, off) != cudaSuccess) {
+        if (pool_malloc(&ws->adjb, off) != cudaSuccess) {
             cudaGetLastError();
             return fail(TOMOS_ERR_ALLOC, "lsqr_adjoint_batch: workspace allocation failed");
         }

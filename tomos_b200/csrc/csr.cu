@@ -769,10 +769,10 @@ struct CsrPass : PassOps {
         const bool with_lo = A->numeric != TOMOS_FP32 && (elem_is_exact(iter_e) || elem_is_exact(init_e));
         const CscCopy need = csc_layout(nullptr, A, with_lo);
         if (need.bytes > ws->csc_bytes) {
-            if (ws->csc) cudaFree(ws->csc);
+            release_memory(ws, ws->csc);
             ws->csc = nullptr;
             ws->csc_bytes = 0;
-            if (cudaMalloc(&ws->csc, need.bytes) != cudaSuccess) {
+            if (pool_malloc(&ws->csc, need.bytes) != cudaSuccess) {
                 cudaGetLastError();
                 return TOMOS_OK;  // not enough memory: the fused row pass
             }

@@ -29,6 +29,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -679,14 +680,10 @@ static int nside_cluster_size() {
 // ------------------------------------------------------------ workspace
 
 static void ws_free(tomos_workspace* ws) {
-    void* ptrs[] = {ws->u,      ws->v,      ws->wt,     ws->p,    ws->qvec,   ws->t,
-                    ws->vhat,   ws->qpart,  ws->sspart, ws->vpart, ws->xpart, ws->qnpart,
-                    ws->scal,   ws->cpart,  ws->coef_init, ws->bpart, ws->fro2, ws->st,   ws->Rcm,
-                    ws->Rrm,    ws->hist,   ws->scratch, ws->h16, ws->adj, ws->csc, ws->shard, ws->adjb,
-                    ws->xg,     ws->dscale, ws->bat};
+    void* ptrs[] = {ws->arena, ws->Rcm, ws->hist, ws->scratch, ws->h16, ws->adj, ws->csc, ws->adjb, ws->bat};
     for (void* q : ptrs)
-        if (q) cudaFree(q);
-    if (ws->st_host) cudaFreeHost(ws->st_host);
+        pool_free(q);
+    pool_free_host(ws->st_host);
     if (ws->graph) cudaGraphExecDestroy(ws->graph);
     if (ws->bgraph) cudaGraphExecDestroy(ws->bgraph);
     if (ws->ev_start) cudaEventDestroy(ws->ev_start);
@@ -699,15 +696,21 @@ static void ws_free(tomos_workspace* ws) {
 
 template <typename T>
 static cudaError_t alloc(T** p, size_t count) {
-    return cudaMalloc(reinterpret_cast<void**>(p), (count ? count : 1) * sizeof(T));
+    return pool_malloc(reinterpret_cast<void**>(p), (count ? count : 1) * sizeof(T));
+}
+
+void release_memory(tomos_workspace* ws, void* p) {
+    if (!p) return;
+    cudaStreamSynchronize(ws->stream);
+    pool_free(p);
 }
 
 tomos_status ensure_scratch(tomos_workspace* ws, size_t bytes) {
     if (bytes <= ws->scratch_bytes) return TOMOS_OK;
-    if (ws->scratch) cudaFree(ws->scratch);
+    release_memory(ws, ws->scratch);
     ws->scratch = nullptr;
     ws->scratch_bytes = 0;
-    cudaError_t e = cudaMalloc(&ws->scratch, bytes);
+    cudaError_t e = pool_malloc(&ws->scratch, bytes);
     if (e != cudaSuccess) return fail(TOMOS_ERR_ALLOC, "workspace scratch allocation failed");
     ws->scratch_bytes = bytes;
     return TOMOS_OK;
@@ -715,7 +718,7 @@ tomos_status ensure_scratch(tomos_workspace* ws, size_t bytes) {
 
 static tomos_status ensure_history(tomos_workspace* ws, int cap) {
     if (cap <= ws->hist_cap) return TOMOS_OK;
-    if (ws->hist) cudaFree(ws->hist);
+    release_memory(ws, ws->hist);
     ws->hist = nullptr;
     ws->hist_cap = 0;
     if (alloc(&ws->hist, (size_t)cap) != cudaSuccess)
@@ -1109,10 +1112,10 @@ struct DensePass : PassOps {
         const int64_t m = A->rows, n = A->cols, ldh = (n + 7) / 8 * 8;
         const size_t bytes = (size_t)m * ldh * sizeof(uint16_t);
         if (bytes > ws->h16_bytes) {
-            if (ws->h16) cudaFree(ws->h16);
+            release_memory(ws, ws->h16);
             ws->h16 = nullptr;
             ws->h16_bytes = 0;
-            if (cudaMalloc(&ws->h16, bytes) != cudaSuccess) {
+            if (pool_malloc(&ws->h16, bytes) != cudaSuccess) {
                 cudaGetLastError();
                 stage = false;  // not enough memory: iterate on A itself
                 return TOMOS_OK;
@@ -1663,33 +1666,48 @@ tomos_status tomos_workspace_create(int64_t m, int64_t n, int32_t value_type,
     if (ws->nb1 < 1) ws->nb1 = 1;
     if (ws->nb3 < 1) ws->nb3 = 1;
     ws->gs_max = sms * 2;
+    // One allocation holds every buffer a workspace starts with (25 of them
+    // cost 3 ms to make and 2 ms to free), from the pool (ws_pool.cu).
+    size_t total = 0;
+    auto layout = [&](char* base) {
+        size_t off = 0;
+        auto take = [&](auto** q, size_t count) {
+            using T = std::remove_pointer_t<std::remove_reference_t<decltype(*q)>>;
+            if (base) *q = reinterpret_cast<T*>(base + off);
+            off += ((count ? count : 1) * sizeof(T) + 255) / 256 * 256;
+        };
+        size_t qp = (size_t)ws->gmax * ws->qstride;
+        if (qp < (size_t)n) qp = n;
+        const size_t sp = (size_t)(ws->gmax > ws->gs_max ? ws->gmax : ws->gs_max);
+        take(&ws->u, (size_t)m);
+        take(&ws->v, (size_t)n);
+        take(&ws->wt, (size_t)n);
+        take(&ws->p, (size_t)n);
+        take(&ws->qvec, (size_t)n);
+        take(&ws->t, (size_t)n);
+        take(&ws->vhat, (size_t)n);
+        take(&ws->qpart, qp);
+        take(&ws->sspart, sp);
+        take(&ws->vpart, (size_t)(ws->nb1 > ws->nb3 ? ws->nb1 : ws->nb3));
+        take(&ws->xpart, (size_t)ws->nb3);
+        take(&ws->qnpart, (size_t)ws->nb1);
+        take(&ws->scal, (size_t)8);
+        take(&ws->cpart, (size_t)48);
+        take(&ws->coef_init, (size_t)2);
+        take(&ws->bpart, (size_t)ws->gs_max);
+        take(&ws->fro2, (size_t)1);
+        take(&ws->st, (size_t)1);
+        take(&ws->shard, (size_t)n + 1);
+        take(&ws->xg, (size_t)n);
+        take(&ws->dscale, (size_t)n);
+        total = off;
+    };
+    layout(nullptr);
     bool ok = true;
     auto A = [&](cudaError_t e) { ok = ok && e == cudaSuccess; };
-    A(alloc(&ws->u, (size_t)m));
-    A(alloc(&ws->v, (size_t)n));
-    A(alloc(&ws->wt, (size_t)n));
-    A(alloc(&ws->p, (size_t)n));
-    A(alloc(&ws->qvec, (size_t)n));
-    A(alloc(&ws->t, (size_t)n));
-    A(alloc(&ws->vhat, (size_t)n));
-    size_t qp = (size_t)ws->gmax * ws->qstride;
-    if (qp < (size_t)n) qp = n;
-    A(alloc(&ws->qpart, qp));
-    size_t sp = (size_t)(ws->gmax > ws->gs_max ? ws->gmax : ws->gs_max);
-    A(alloc(&ws->sspart, sp));
-    A(alloc(&ws->vpart, (size_t)(ws->nb1 > ws->nb3 ? ws->nb1 : ws->nb3)));
-    A(alloc(&ws->xpart, (size_t)ws->nb3));
-    A(alloc(&ws->qnpart, (size_t)ws->nb1));
-    A(alloc(&ws->scal, 8));
-    A(alloc(&ws->cpart, 48));
-    A(alloc(&ws->coef_init, 2));
-    A(alloc(&ws->bpart, (size_t)ws->gs_max));
-    A(alloc(&ws->fro2, 1));
-    A(alloc(&ws->st, 1));
-    A(alloc(&ws->shard, (size_t)n + 1));
-    A(alloc(&ws->xg, (size_t)n));
-    A(alloc(&ws->dscale, (size_t)n));
-    A(cudaMallocHost(reinterpret_cast<void**>(&ws->st_host), sizeof(LsqrDev)));
+    A(pool_malloc(&ws->arena, total));
+    if (ok) layout(static_cast<char*>(ws->arena));
+    A(pool_malloc_host(reinterpret_cast<void**>(&ws->st_host), sizeof(LsqrDev)));
     A(cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking));
     A(cudaEventCreate(&ws->ev_start));
     A(cudaEventCreate(&ws->ev_stop));
@@ -1739,9 +1757,12 @@ tomos_status tomos_workspace_add_precond(tomos_workspace* ws, const tomos_dense*
         return fail(TOMOS_ERR_INVALID, "add_precond: bad layout");
     if (Rinv->ld < ws->n) return fail(TOMOS_ERR_INVALID, "add_precond: bad leading dimension");
     if (!ws->Rcm) {
-        bool ok = alloc(&ws->Rcm, (size_t)ws->n * ws->n) == cudaSuccess &&
-                  alloc(&ws->Rrm, (size_t)ws->n * ws->n) == cudaSuccess;
-        if (!ok) return fail(TOMOS_ERR_ALLOC, "add_precond: allocation failed");
+        const size_t nn = ((size_t)ws->n * ws->n + 31) / 32 * 32;  // both copies in one allocation
+        if (alloc(&ws->Rcm, 2 * nn) != cudaSuccess) {
+            ws->Rcm = nullptr;
+            return fail(TOMOS_ERR_ALLOC, "add_precond: allocation failed");
+        }
+        ws->Rrm = ws->Rcm + nn;
     }
     ws->precond = *Rinv;
     ws->has_precond = true;

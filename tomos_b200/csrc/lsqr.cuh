@@ -177,6 +177,14 @@ __device__ __forceinline__ double block_sum_array(const double* part, int64_t np
 // One pass over a dense A (the fused kernel when pl.fused, else the
 // generic two-kernel path): ut = cp A p + cu u_in into ws->u, the
 // partials of A^T ut into ws->qpart and of ||ut||^2 into ws->sspart.
+// Device memory and small pinned blocks for workspaces, kept for later ones
+// when they are given back (ws_pool.cu); what used a block has finished by
+// then.
+cudaError_t pool_malloc(void** out, size_t bytes);
+void pool_free(void* p);
+cudaError_t pool_malloc_host(void** out, size_t bytes);  // at most 4 KB
+void pool_free_host(void* p);
+
 // Plans that need ws->scratch (dense_pass_scratch bytes): the generic path's
 // partials, and the FP64 partials of a direct pass.
 inline bool pass_needs_scratch(const PassPlan& pl) { return !pl.fused || (pl.direct && pl.acc64); }
@@ -233,6 +241,7 @@ tomos_status enqueue_multi_pass(const MultiPass& P, cudaStream_t st);
 
 tomos_status workspace_check(tomos_workspace* ws, int64_t m, int64_t n);
 tomos_status ensure_scratch(tomos_workspace* ws, size_t bytes);
+void release_memory(tomos_workspace* ws, void* p);  // pool_free once ws's stream is done
 
 }  // namespace tomos_b200
 
@@ -245,6 +254,7 @@ struct tomos_workspace {
     int nb1 = 0, nb3 = 0;  // n-side block counts
     int gs_max = 0;        // sum-of-squares partial blocks
 
+    void* arena = nullptr;  // the buffers below up to cpart, xg, shard and dscale
     float* u = nullptr;     // m: unnormalised u
     float* v = nullptr;     // n
     float* wt = nullptr;    // n: M w

@@ -339,10 +339,10 @@ tomos_status tomos_lsqr_solve_batch_dense(const tomos_dense* A, int32_t K, const
     const int64_t qs = ws->qstride;
     const BatchBufs need = batch_layout(nullptr, m, n, K, qs, grid, ws->gs_max);
     if (need.bytes > ws->bat_bytes) {
-        if (ws->bat) cudaFree(ws->bat);
+        release_memory(ws, ws->bat);
         ws->bat = nullptr;
         ws->bat_bytes = 0;
-        if (cudaMalloc(&ws->bat, need.bytes) != cudaSuccess) {
+        if (pool_malloc(&ws->bat, need.bytes) != cudaSuccess) {
             cudaGetLastError();
             return fail(TOMOS_ERR_ALLOC, "lsqr_solve_batch: workspace allocation failed");
         }

@@ -317,3 +317,21 @@ def test_workspaces_made_and_closed_by_threads(m, n):
     for q in (1, 7, 20):  # u of 4 to 80 MB
         tb.create_lsqr_workspace(None, (q * 1000000, n), NT.FP32, NT.FP64).close()
     assert free0 - torch.cuda.mem_get_info()[0] <= (64 << 20) + (4 << 20)
+
+
+@pytest.mark.parametrize("n", [1, 31, 128, 129, 512, 513, 777, 1030])
+def test_nside_at_its_sizes(n):
+    """The n-side of a preconditioned solve in one CTA, a cluster and separate
+    kernels, at the edges between them, against FP64."""
+    m = 8 * n + 64
+    rng = np.random.default_rng(n)
+    A0 = rng.standard_normal((m, n)).astype(np.float32)
+    b0 = (A0 @ rng.standard_normal(n) + 1e-4 * rng.standard_normal(m)).astype(np.float32)
+    x, rep, _ = tb.sketch_lsqr(to_dense(A0, L.ROW_MAJOR), cuda(b0), 4 * n, max_iters=60)
+    ref = np.linalg.lstsq(A0.astype(np.float64), b0.astype(np.float64), rcond=None)[0]
+    assert rep["converged"] == 1
+    # a backward error of 1e-6 with ||A D^-1||_F = sqrt(n): A (x - x*) is below
+    # 1e-6 (sqrt(n) ||D x|| + ||b||), ||b|| about ||D x||; the smallest singular
+    # value of A D^-1 (Gaussian) is near 1 - sqrt(n / m)
+    bound = 1e-6 * (np.sqrt(n) + 2) / (1 - np.sqrt(n / m))
+    assert np.linalg.norm(x.cpu().numpy() - ref) / np.linalg.norm(ref) < bound

@@ -24,7 +24,7 @@
 //   N3       alpha = ||vh||, v = vh / alpha, p = M v, Givens, x and wt
 //   N4       state update, history, stopping rule, next cu = -alpha/beta
 // N1 to N4 are one launch for a preconditioned solve with n <=
-// kNsideClusterMaxN, four kernels otherwise.
+// kNsideClusterMaxN, three kernels otherwise (N4 in N3's last block).
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -192,56 +192,67 @@ __device__ __forceinline__ Givens givens(double rho_bar, double phi_bar, double 
 }
 
 // sum over k = lane, lane + 32, .. < len of a[k] b[k] (the lane's share of a
-// warp's dot product over L2-resident vectors): eight independent FP64
-// chains, so a lane has sixteen loads in flight instead of two.
+// warp's dot product over L2-resident vectors): sixteen independent FP64
+// chains, so a column of up to 512 entries waits for L2 once (N2 at
+// n = 777: 9.6 us with eight, 4.1 us).
 __device__ __forceinline__ double strided_dot(const double* __restrict__ a, const double* __restrict__ b,
                                               int lane, int64_t len) {
-    double z[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    int64_t k = lane;
-    for (; k + 7 * 32 < len; k += 8 * 32) {
-        double av[8], bv[8];
+    constexpr int U = 16;
+    double z[U];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            av[u] = __ldg(a + k + 32 * u);
-            bv[u] = __ldg(b + k + 32 * u);
+    for (int u = 0; u < U; ++u) z[u] = 0.0;
+    for (int64_t k = lane; k < len; k += U * 32) {
+        double av[U], bv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = k + 32 * u < len;
+            av[u] = in ? __ldg(a + k + 32 * u) : 0.0;
+            bv[u] = in ? __ldg(b + k + 32 * u) : 0.0;
         }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) z[u] = fma(av[u], bv[u], z[u]);
+        for (int u = 0; u < U; ++u) z[u] = fma(av[u], bv[u], z[u]);
     }
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
-        if (k + 32 * u < len) z[u] = fma(__ldg(a + k + 32 * u), __ldg(b + k + 32 * u), z[u]);
-    return ((z[0] + z[1]) + (z[2] + z[3])) + ((z[4] + z[5]) + (z[6] + z[7]));
+    for (int h = U / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int u = 0; u < h; ++u) z[u] += z[u + h];
+    return z[0];
 }
 
 // N1: beta and t = A^T ut / beta (no preconditioner: vh = t - beta v).
-__global__ void __launch_bounds__(256) nside_reduce_kernel(NSide S) {
+// 32 columns a block, 32 warps sharing the partials of each: all of a warp's
+// loads (ten, at the two CTAs an SM of most passes) are in flight before the
+// sum of squares is formed: 6.2 us for 296 partials of 777 columns, 11 us by
+// eight warps with two in flight.
+constexpr int kReduceWarps = 32;
+__global__ void __launch_bounds__(32 * kReduceWarps) nside_reduce_kernel(NSide S) {
     if (S.skip && *S.skip) return;
     __shared__ double sm[32];
-    __shared__ double smq[8][33];
-    const double beta = sqrt(block_sum_array(S.sspart, S.gs, sm));
-    const double inv = beta > 0.0 ? 1.0 / beta : 0.0;
+    __shared__ double smq[kReduceWarps][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t j = (int64_t)blockIdx.x * 32 + lane;
-    double q = 0.0;
-    if (S.qsum)
-        q = (w == 0 && j < S.n) ? S.qsum[j] : 0.0;
-    else if (j < S.n) {
-        double q1 = 0.0;
-        int c = w;
-        for (; c + 8 < S.gq; c += 16) {
-            q += (double)S.qpart[(size_t)c * S.qstride + j];
-            q1 += (double)S.qpart[(size_t)(c + 8) * S.qstride + j];
-        }
-        if (c < S.gq) q += (double)S.qpart[(size_t)c * S.qstride + j];
-        q += q1;
+    constexpr int U = 10;
+    float f[U];
+    const bool parts = !S.qsum && j < S.n;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int c = w + u * kReduceWarps;
+        f[u] = parts && c < S.gq ? S.qpart[(size_t)c * S.qstride + j] : 0.0f;
     }
+    const double beta = sqrt(block_sum_array(S.sspart, S.gs, sm));
+    const double inv = beta > 0.0 ? 1.0 / beta : 0.0;
+    double q = 0.0;
+    if (S.qsum) q = (w == 0 && j < S.n) ? S.qsum[j] : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) q += (double)f[u];
+    if (parts)
+        for (int c = w + U * kReduceWarps; c < S.gq; c += kReduceWarps) q += (double)S.qpart[(size_t)c * S.qstride + j];
     smq[w][lane] = q;
     __syncthreads();
     if (w == 0) {
         double qs = 0.0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) qs += smq[k][lane];
+        for (int k = 0; k < kReduceWarps; ++k) qs += smq[k][lane];
         double vh2 = 0.0, qn = 0.0;
         if (j < S.n) {
             const double tj = qs * inv;
@@ -290,59 +301,6 @@ __global__ void __launch_bounds__(256) nside_precond_t_kernel(NSide S) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) s += smv[k];
         S.vpart[blockIdx.x] = s;
-    }
-}
-
-// N3: alpha, v, p = M v, and the x / wt update of the Givens step.
-__global__ void __launch_bounds__(256) nside_update_kernel(NSide S) {
-    if (S.skip && *S.skip) return;
-    __shared__ double sm[32];
-    __shared__ double smx[8];
-    const int nvp = S.has_precond ? S.nb3 : S.nb1;
-    const double alpha = sqrt(block_sum_array(S.vpart, nvp, sm));
-    const double inva = alpha > 0.0 ? 1.0 / alpha : 0.0;
-    const double beta = S.scal[0];
-    Givens g = givens(S.st->rho_bar, S.st->phi_bar, alpha, beta);
-    const double step_x = g.rho > 0.0 ? g.phi / g.rho : 0.0;
-    const double step_w = g.rho > 0.0 ? g.theta / g.rho : 0.0;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t i = (int64_t)blockIdx.x * 8 + w;
-    double xs = 0.0;
-    if (i < S.n) {
-        double pi;
-        if (S.has_precond) {
-            const double* __restrict__ row = S.Rrm + (size_t)i * S.n;
-            const double* __restrict__ vh = S.vhat;
-            // an upper triangular M: row i starts at column i
-            const int64_t j0 = S.scal[7] != 0.0 ? 0 : i;
-            pi = warp_sum(strided_dot(row + j0, vh + j0, lane, S.n - j0)) * inva;
-        } else {
-            pi = S.vhat[i] * inva;
-        }
-        if (lane == 0) {
-            S.v[i] = (float)(S.vhat[i] * inva);
-            double xi = (double)S.x[i];
-            if (S.init) {
-                S.wt[i] = (float)pi;
-            } else {
-                const double wi = (double)S.wt[i];
-                xi += step_x * wi;
-                S.x[i] = (float)xi;
-                S.wt[i] = (float)(pi - step_w * wi);
-            }
-            S.p[i] = (float)pi;
-            const double xf = (double)(float)xi * (S.dscale ? S.dscale[i] : 1.0);
-            xs = xf * xf;
-        }
-    }
-    if (lane == 0) smx[w] = xs;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) s += smx[k];
-        S.xpart[blockIdx.x] = s;
-        if (blockIdx.x == 0) S.scal[1] = alpha;
     }
 }
 
@@ -404,26 +362,85 @@ __device__ __forceinline__ void finish_state(const NSide& S, const LsqrDev& in, 
     if (S.use_cond) set_condition(S, !stop);
 }
 
-// N4: one block.
-__global__ void __launch_bounds__(256) nside_finish_kernel(NSide S) {
+// N3 and N4: alpha, v, p = M v, the x / wt update of the Givens step, and, by
+// the last block to get there, the state and the stopping rule (a launch of
+// its own took 5 us an iteration; N3 8.8 us then, 11.6 us with N4).  S.scal[6] counts the blocks and wraps to
+// zero.
+__global__ void __launch_bounds__(256) nside_update_kernel(NSide S) {
     if (S.skip && *S.skip) {
-        if (S.use_cond && threadIdx.x == 0) cudaGraphSetConditional(S.cond, 0u);
+        if (S.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(S.cond, 0u);
         return;
     }
     __shared__ double sm[32];
-    const double xn = sqrt(block_sum_array(S.xpart, S.nb3, sm));
-    const double qn = S.init ? sqrt(block_sum_array(S.qnpart, S.nb1, sm)) : 0.0;
-    if (threadIdx.x != 0) return;
-    const double beta = S.scal[0], alpha = S.scal[1];
-    finish_state(S, *S.st, givens(S.st->rho_bar, S.st->phi_bar, alpha, beta), beta, alpha, xn, qn);
+    __shared__ double smx[8];
+    __shared__ int last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t i = (int64_t)blockIdx.x * 8 + w;
+    double pi = 0.0;
+    if (i < S.n) {  // M vh needs no scalar
+        if (S.has_precond) {
+            // an upper triangular M: row i starts at column i
+            const int64_t j0 = S.scal[7] != 0.0 ? 0 : i;
+            pi = warp_sum(strided_dot(S.Rrm + (size_t)i * S.n + j0, S.vhat + j0, lane, S.n - j0));
+        } else {
+            pi = S.vhat[i];
+        }
+    }
+    const double alpha = sqrt(block_sum_array(S.vpart, S.has_precond ? S.nb3 : S.nb1, sm));
+    const double inva = alpha > 0.0 ? 1.0 / alpha : 0.0;
+    const double beta = S.scal[0];
+    const Givens g = givens(S.st->rho_bar, S.st->phi_bar, alpha, beta);
+    const double step_x = g.rho > 0.0 ? g.phi / g.rho : 0.0;
+    const double step_w = g.rho > 0.0 ? g.theta / g.rho : 0.0;
+    double xs = 0.0;
+    if (i < S.n) {
+        pi *= inva;
+        if (lane == 0) {
+            S.v[i] = (float)(S.vhat[i] * inva);
+            double xi = (double)S.x[i];
+            if (S.init) {
+                S.wt[i] = (float)pi;
+            } else {
+                const double wi = (double)S.wt[i];
+                xi += step_x * wi;
+                S.x[i] = (float)xi;
+                S.wt[i] = (float)(pi - step_w * wi);
+            }
+            S.p[i] = (float)pi;
+            const double xf = (double)(float)xi * (S.dscale ? S.dscale[i] : 1.0);
+            xs = xf * xf;
+        }
+    }
+    if (lane == 0) smx[w] = xs;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += smx[k];
+        S.xpart[blockIdx.x] = s;
+        __threadfence();
+        last = atomicInc(reinterpret_cast<unsigned*>(S.scal + 6), gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double x2 = 0.0, q2 = 0.0;
+    for (int b = threadIdx.x; b < S.nb3; b += blockDim.x) x2 += __ldcg(S.xpart + b);
+    const double xn = sqrt(block_sum(x2, sm));
+    if (S.init) {
+        for (int b = threadIdx.x; b < S.nb1; b += blockDim.x) q2 += S.qnpart[b];
+        q2 = sqrt(block_sum(q2, sm));
+    }
+    if (threadIdx.x == 0) finish_state(S, *S.st, g, beta, alpha, xn, q2);
 }
 
 // N1 to N4 in one launch, for a preconditioned solve of few columns: one CTA
 // up to kNsideOneMaxN columns, one cluster of 8 or 16 up to
-// kNsideClusterMaxN.  The four kernels are bound by latency, a launch, a
+// kNsideClusterMaxN.  Separate kernels are bound by latency, a launch, a
 // first load and a tail each (17 us an iteration at n = 64 beside a 33 us
 // pass); past that size the cluster's SMs read R^{-1} slower than the whole
-// GPU does (38 us against 34 us at n = 1000).  A warp keeps its columns of
+// GPU does (38 us against 34 us at n = 1000 when this was decided; the
+// separate kernels take 22 us at n = 777 since).  A warp keeps its columns of
 // R^{-1} in registers, loaded before the sums they wait for, then its rows
 // the same way; t and vh go through shared memory (of one CTA), or through
 // L2 between cluster barriers, which order the CTAs' global writes (data
@@ -642,7 +659,7 @@ __global__ void __launch_bounds__(kNsideThreads, 1) nside_batch_kernel(const __g
     nside_fused<ONE>(B.s[blockIdx.y]);
 }
 
-// CTAs of the n-side cluster (0: the four kernels): sixteen where the GPU
+// CTAs of the n-side cluster (0: separate kernels): sixteen where the GPU
 // can place such a cluster, else the portable eight.  Asked of the driver
 // once per process and device.
 static int nside_cluster_size() {
@@ -1038,7 +1055,7 @@ tomos_status enqueue_nside(tomos_workspace* ws, const NSide& S, cudaStream_t st)
         ws->launches += 1;
         return TOMOS_OK;
     }
-    nside_reduce_kernel<<<ws->nb1, 256, 0, st>>>(S);
+    nside_reduce_kernel<<<ws->nb1, 32 * kReduceWarps, 0, st>>>(S);
     TOMOS_LAUNCH_CHECK("nside_reduce_kernel");
     if (S.has_precond) {
         nside_precond_t_kernel<<<ws->nb3, 256, 0, st>>>(S);
@@ -1046,9 +1063,7 @@ tomos_status enqueue_nside(tomos_workspace* ws, const NSide& S, cudaStream_t st)
     }
     nside_update_kernel<<<ws->nb3, 256, 0, st>>>(S);
     TOMOS_LAUNCH_CHECK("nside_update_kernel");
-    nside_finish_kernel<<<1, 256, 0, st>>>(S);
-    TOMOS_LAUNCH_CHECK("nside_finish_kernel");
-    ws->launches += S.has_precond ? 4 : 3;
+    ws->launches += S.has_precond ? 3 : 2;
     return TOMOS_OK;
 }
 
@@ -1183,8 +1198,8 @@ struct DensePass : PassOps {
 // ------------------------------------------------------------ driver
 
 tomos_status refresh_precond(tomos_workspace* ws, cudaStream_t st) {
+    TOMOS_CUDA_TRY(cudaMemsetAsync(ws->scal + 6, 0, 2 * sizeof(double), st));  // N3's block count, the triangle flag
     if (!ws->has_precond) return TOMOS_OK;
-    TOMOS_CUDA_TRY(cudaMemsetAsync(ws->scal + 7, 0, sizeof(double), st));
     precond_copy_kernel<<<ws->gs_max, 256, 0, st>>>(ws->precond.values, ws->precond.numeric,
                                                    ws->precond.layout, ws->precond.ld, ws->n,
                                                    ws->Rcm, ws->Rrm, ws->scal + 7);
@@ -1885,7 +1900,7 @@ tomos_status tomos_backward_error_dense(const tomos_dense* A, const float* b, co
     ws->has_precond = false;
     NSide S = make_nside(ws, pl, nullptr, true, nullptr, col_scale);
     ws->has_precond = had;
-    nside_reduce_kernel<<<ws->nb1, 256, 0, st>>>(S);
+    nside_reduce_kernel<<<ws->nb1, 32 * kReduceWarps, 0, st>>>(S);
     TOMOS_LAUNCH_CHECK("nside_reduce_kernel");
     sum_to_scalar_kernel<<<1, 256, 0, st>>>(ws->qnpart, ws->nb1, ws->scal + 4);
     sumsq_partial_kernel<<<ws->gs_max, 256, 0, st>>>(b, A->rows, nullptr, ws->bpart);

@@ -286,10 +286,10 @@ def mm_numbers(tb, torch, Ap, m, n, sq=8192, rhs=16):
 def adjoint_numbers(tb, torch, m=200_000, n=500, K=8):
     """The adjoint workload (lambda_k = (A^T A)^{-1} g_k, K = 8 right-hand
     sides, A 200,000 x 500 FP32 ~ N(0,1), the sketch-QR preconditioner, CG
-    to 1e-7): all K at once (tomos_lsqr_adjoint_batch_dense: two tcgen05
-    products over A an iteration, shared) against K one-column solves (one
-    fused pass over A an iteration each).  Device time from the solver's
-    own events; achieved = the products' bytes (4 m n per product) / time."""
+    to 1e-7): all K at once (tomos_lsqr_adjoint_batch_dense: one shared
+    pass over A an iteration) against K one-column solves (one fused pass
+    over A an iteration each).  Device time from the solver's own events;
+    achieved = the shared passes' bytes (4 m n a pass) / time."""
     NT, L = tb.NumericType, tb.Layout
     g = torch.Generator(device="cuda")
     g.manual_seed(5)
@@ -312,8 +312,8 @@ def adjoint_numbers(tb, torch, m=200_000, n=500, K=8):
             "batched_ms": ms_b, "one_column_solves_ms": ms_s, "speedup": ms_s / ms_b,
             "iterations": [r["iterations"] for r in reps], "products_over_A": products,
             "achieved_gbs": gb, "frac_of_measured_hbm": gb / measured_peak()[0],
-            "note": "batched: Q = A P and W = A^T Q for all K directions by tomos_mm_ex "
-                    "(accurate TF32x3 tier, split-K for A^T Q)"}
+            "note": "batched: Q = A P and W = A^T Q for all K directions from one read of A "
+                    "an iteration; products_over_A counts the reads"}
 
 
 def count_launches(torch, fn):

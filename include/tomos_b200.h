@@ -194,9 +194,11 @@ tomos_status tomos_mm(int32_t trans_a, int32_t trans_b, double alpha, const tomo
 /* tomos_mm with caller scratch: a product with too few 128 x BN output tiles
  * to fill the GPU and a long K (e.g. A^T Q with A tall, the transposed
  * multi-right-hand-side product) splits K over CTAs, writes FP32 partial sums
- * to `scratch` and sums them in FP64 in a fixed order (deterministic).
- * tomos_mm_scratch_bytes gives the bytes (0: no split); with less scratch the
- * product runs unsplit, with the same result up to summation order. */
+ * to `scratch` and sums them in FP64 in a fixed order (deterministic); so does
+ * an exactly read A with at most 16 columns of op(B).  A large HALF_OPERANDS
+ * product keeps both operands there as 16-bit planes.  tomos_mm_scratch_bytes
+ * gives the bytes (0: none used); with less scratch the product runs in fewer
+ * runs or without planes, with the same result up to summation order. */
 size_t tomos_mm_scratch_bytes(int32_t trans_a, int32_t trans_b, const tomos_dense* A,
                               int32_t tier, const tomos_dense* B);
 tomos_status tomos_mm_ex(int32_t trans_a, int32_t trans_b, double alpha, const tomos_dense* A,
@@ -510,12 +512,12 @@ tomos_status tomos_lsqr_adjoint_dense(const tomos_dense* A, const float* g, floa
  * (n x K column-major FP32, leading dimension ldg) into Lambda (n x K, ld
  * ldl).  The same preconditioned CG as tomos_lsqr_adjoint_dense, one
  * recurrence per column, sharing the products with A: every iteration
- * forms Q = A P and W = A^T Q for all K directions with two tensor-core
- * products (tomos_mm_ex), so A is read twice an iteration for all K
- * columns instead of once per column.  Products at ~2^-22 relative
- * (three TF32 terms for FP32 or exactly read packed A).  reports (K
- * entries, may be NULL): each column's iterations, converged, relres;
- * half_passes counts the shared products.  The workspace grows a buffer
+ * forms Q = A P and W = A^T Q for all K directions, from one read of an FP32
+ * row-major A (2 <= K <= 8, n <= 512, 16-byte aligned rows; FP32 products),
+ * else as two products (tomos_mm_ex, ~2^-22 relative: three TF32 terms for
+ * FP32 or exactly read packed A).  reports (K entries, may be NULL): each
+ * column's iterations, converged, relres; half_passes counts the shared
+ * passes over A, one or two an iteration.  The workspace grows a buffer
  * for the K columns on first use.  Synchronous on stream. */
 tomos_status tomos_lsqr_adjoint_batch_dense(const tomos_dense* A, int32_t K, const float* G,
                                             int64_t ldg, float* Lambda, int64_t ldl,

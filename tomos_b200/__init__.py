@@ -84,6 +84,15 @@ def _stream(stream):
     return ctypes.c_void_p(stream.cuda_stream)
 
 
+def _scratch(nbytes, stream):
+    """Scratch of a call on `stream`, from that stream's own memory: a block of
+    another stream's could be reused before the call's kernels have run."""
+    if stream is None:
+        return torch.empty(nbytes or 1, dtype=torch.uint8, device="cuda")
+    with torch.cuda.stream(stream):
+        return torch.empty(nbytes or 1, dtype=torch.uint8, device="cuda")
+
+
 class Context:
     """include/core/context: only Device::CUDA is registered here."""
 
@@ -451,14 +460,14 @@ def mv_apply(dev, transpose, alpha, A, x, beta, y, compute_type=None, tier=None,
     if isinstance(A, Csr):
         d = A.desc()
         nb = C.lib().tomos_csr_gemv_scratch_bytes(ctypes.byref(d), int(transpose))
-        scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device="cuda")
+        scratch = _scratch(nb, stream)
         C.check(C.lib().tomos_csr_gemv(int(transpose), float(alpha), ctypes.byref(d), int(t),
                                        _ptr(xs), float(beta), _ptr(ys), _ptr(scratch), nb,
                                        _stream(stream)), "mv_apply")
         return 0
     d = A.desc()
     nb = C.lib().tomos_gemv_scratch_bytes(ctypes.byref(d), int(transpose))
-    scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device="cuda")
+    scratch = _scratch(nb, stream)
     C.check(C.lib().tomos_gemv(int(transpose), float(alpha), ctypes.byref(d), int(t), _ptr(xs),
                                float(beta), _ptr(ys), _ptr(scratch), nb, _stream(stream)),
             "mv_apply")
@@ -481,7 +490,10 @@ def mm_apply(dev, transA, transB, alpha, A, B, beta, Cm, use_workspace=False, ti
     da, db, dc = A.desc(), B.desc(), Cm.desc()
     nb = C.lib().tomos_mm_scratch_bytes(int(transA), int(transB), ctypes.byref(da), int(tier),
                                         ctypes.byref(db))
-    scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device="cuda") if nb else None
+    try:
+        scratch = _scratch(nb, stream) if nb else None
+    except torch.OutOfMemoryError:  # up to 2 GiB for packed operands: the product runs without
+        scratch, nb = None, 0
     C.check(C.lib().tomos_mm_ex(int(transA), int(transB), float(alpha), ctypes.byref(da), int(tier),
                                 ctypes.byref(db), float(beta), ctypes.byref(dc), _ptr(scratch), nb,
                                 _stream(stream)),
@@ -532,7 +544,7 @@ def apply_count_sketch(A, s, tier=Tier.AUTO, bucket_seed=CS_BUCKET_SEED, sign_se
     colsq = torch.empty(max(n, 1), dtype=torch.float64, device="cuda") if with_colsq else None
     m = A.size[0]
     nb = C.lib().tomos_countsketch_scratch_bytes(m, n, s)
-    scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device="cuda")
+    scratch = _scratch(nb, stream)
     d = A.desc()
     fn = C.lib().tomos_countsketch_apply_csr if isinstance(A, Csr) else C.lib().tomos_countsketch_apply
     C.check(fn(ctypes.byref(d), int(tier), s, bucket_seed, sign_seed, _ptr(SA.storage), s,
@@ -552,7 +564,7 @@ def _count_sketch_stage(A, s, bucket_seed, sign_seed, with_colsq, stream):
     fro2 = torch.empty(1, dtype=torch.float64, device="cuda")
     colsq = torch.empty(max(n, 1), dtype=torch.float64, device="cuda") if with_colsq else None
     nb = C.lib().tomos_countsketch_scratch_bytes(m, n, s)
-    scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device="cuda")
+    scratch = _scratch(nb, stream)
     d = A.desc()
     C.check(C.lib().tomos_countsketch_apply_stage(ctypes.byref(d), s, bucket_seed, sign_seed,
                                                   _ptr(SA.storage), s, _ptr(fro2), _ptr(colsq),
@@ -579,7 +591,7 @@ def generate_sketch_qr_precond(sketched, R_out=None, copy=True, any_signs=False,
                          "generate_sketch_qr_precond: sketched_mtx must have at least as many "
                          "rows as columns (k >= n).")
     nb = C.lib().tomos_sketch_qr_scratch_bytes(k, n)
-    scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device="cuda")
+    scratch = _scratch(nb, stream)
     C.check(C.lib().tomos_sketch_qr_precond_ex_f64(k, n, _ptr(sketched.storage), sketched.ld, _ptr(R_out),
                                                    C.TOMOS_QR_ANY_SIGNS if any_signs else 0, _ptr(scratch),
                                                    nb, _stream(stream)),
@@ -982,7 +994,7 @@ def apply_count_sketch_shard(A, s, row0, tier=Tier.AUTO, bucket_seed=CS_BUCKET_S
     fro2 = torch.empty(1, dtype=torch.float64, device="cuda")
     colsq = torch.empty(max(n, 1), dtype=torch.float64, device="cuda")
     nb = C.lib().tomos_countsketch_scratch_bytes(m, n, s)
-    scratch = torch.empty(max(nb, 1), dtype=torch.uint8, device="cuda")
+    scratch = _scratch(nb, stream)
     d = A.desc()
     C.check(C.lib().tomos_countsketch_apply_shard(
         ctypes.byref(d), int(tier), s, bucket_seed, sign_seed, int(row0), _ptr(SA.storage), s, _ptr(fro2),

@@ -84,13 +84,16 @@ def _stream(stream):
     return ctypes.c_void_p(stream.cuda_stream)
 
 
+_CUDA = torch.device("cuda")
+
+
 def _scratch(nbytes, stream):
     """Scratch of a call on `stream`, from that stream's own memory: a block of
     another stream's could be reused before the call's kernels have run."""
     if stream is None:
-        return torch.empty(nbytes or 1, dtype=torch.uint8, device="cuda")
+        return torch.empty(nbytes or 1, dtype=torch.uint8, device=_CUDA)
     with torch.cuda.stream(stream):
-        return torch.empty(nbytes or 1, dtype=torch.uint8, device="cuda")
+        return torch.empty(nbytes or 1, dtype=torch.uint8, device=_CUDA)
 
 
 class Context:

@@ -7,9 +7,9 @@
 //   Q = A P and W = A^T Q,
 // from one read of an FP32 row-major A (multi_rows_kernel, lsqr_batch.cu; K
 // <= 8, n <= 512), else as two products (tomos_mm_ex, the second one's long K
-// split over CTAs).  At 200000 x 500 and eight columns: two tensor-core
-// products took 400 us an iteration.  The n-side kernels run every column k in blockIdx.y; a column
-// whose recurrence has stopped returns at once.  Scalars and vectors are
+// split over CTAs).  At 200000 x 500 and eight columns: 170 us an iteration,
+// two tiled products took 400 us.  The n-side kernels run every column k in
+// blockIdx.y; a column whose recurrence has stopped returns at once.  Scalars and vectors are
 // FP64; the direction goes to the products as FP32.
 #include <cmath>
 #include <cstring>

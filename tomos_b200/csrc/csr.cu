@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(256) csr_pass_kernel(CsrPassParams P) {
 // shared memory, the warp's rows in order).  Bound by the chain of loads a
 // row needs (extent, entries, accumulators): kTransRows rows' entries are
 // loaded while the rows before them are added, so a row costs its
-// shared-memory update (2e6 rows of 20 entries into 5000 columns: 1.78 ms
-// with a row at a time).
+// shared-memory update (2e6 rows of 20 entries into 5000 columns: 0.50 ms;
+// 1.31 ms with a row at a time).
 constexpr int kTransRows = 16;
 
 template <Elem E>
@@ -901,8 +901,8 @@ tomos_status CsrPass::fro2(double* out, const double* d, cudaStream_t st) {
 // buckets' rows of SA together.  The rows' metadata (row id, sign, extent)
 // come 32 rows at a time, a row a lane, and sixteen rows' entries are loaded
 // before the first is added, so a row costs the shared-memory update rather
-// than a chain of dependent global loads (0.27 ms; one row ahead: 0.46 ms for 500000
-// rows of 20 in 12000 buckets of 3000 columns).  The CTA's nw
+// than a chain of dependent global loads (500000 rows of 20 in 12000 buckets
+// of 3000 columns: 0.27 ms; one row ahead: 0.46 ms).  The CTA's nw
 // buckets are consecutive rows of the column-major SA: for each column it
 // writes them as one run of nw doubles (SA is s x n, so writing a row of it
 // alone would touch one 8-byte word per 32-byte sector).

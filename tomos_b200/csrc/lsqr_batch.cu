@@ -32,8 +32,11 @@ namespace {
 //           accumulators, emptied into FP64 ones every kMultiFlush tiles
 //           (runs of at most 128 rows).
 // 32 FMAs an element and 4 bytes: 44 us of packed FP32 FMAs against 60 us of
-// HBM at 200000 x 500.  Sums in FP32 over a lane's columns and a run's rows,
-// FP64 beyond, products and ut as in the one-column pass.
+// HBM at 200000 x 500; a pass takes 170 us, bound by the phases' latencies.
+// (Sixteen warps of four columns a lane: 220 us.  Split-TF32 matrix
+// instructions: 150 us, and twice the iterations for want of precision.)
+// Sums in FP32 over a lane's columns and a run's rows, FP64 beyond, products
+// and ut as in the one-column pass.
 constexpr int kMultiThreads = 256;
 constexpr int kMultiRows = 32;
 constexpr int kMultiMaxN = 512;

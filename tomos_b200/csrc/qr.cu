@@ -691,9 +691,12 @@ __global__ void __launch_bounds__(32) qr_trtri_diag_kernel(const double* Rt, int
 // at n), X_IJ = -X_II R_IJ X_JJ, in two batched products
 //   mode 0:  T_p  = R_IJ X_JJ      (R from Rt, row-major)
 //   mode 1:  X_IJ = -X_II T_p
-// X_II and X_JJ come from the previous level.  32 x 32 output tiles (many
-// CTAs even at the widest level), k-steps of 32 through shared memory,
-// each warp two m8n8 FP64 tensor-core tiles.
+// X_II and X_JJ come from the previous level; both are upper triangular, so
+// the sums leave out k-steps that meet their zeros.  32 x 32 output tiles
+// (many CTAs even at the widest level), k-steps of 32 through shared memory,
+// each warp two m8n8 FP64 tensor-core tiles.  Bound by the latency of a
+// k-step, so the next one's values are in registers before this one's
+// products: all levels 118 us at n = 1000 (228 us with neither).
 __global__ void __launch_bounds__(256) trtri_level_kernel(const double* Rt, int64_t n, double* X,
                                                           int64_t ldx, double* Tb, int64_t b,
                                                           int mode) {
@@ -711,31 +714,36 @@ __global__ void __launch_bounds__(256) trtri_level_kernel(const double* Rt, int6
     const int lane = t & 31, warp = t >> 5, g = lane >> 2, q = lane & 3;
     const int mb = warp >> 1, nb0 = 2 * (warp & 1);
     double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-    for (int64_t k0 = 0; k0 < K; k0 += 32) {
-        __syncthreads();
-        for (int e = t; e < 32 * 32; e += 256) {
-            int i, kk;
-            double v = 0.0;
-            if (mode == 0) {  // R row-major: consecutive threads along k
-                i = e >> 5;
-                kk = e & 31;
-                if (row0 + i < M && k0 + kk < K) v = Rt[(size_t)(I0 + row0 + i) * n + J0 + k0 + kk];
-            } else {          // X column-major: consecutive threads along rows
-                i = e & 31;
-                kk = e >> 5;
-                if (row0 + i < M && k0 + kk < K) v = X[(size_t)(I0 + k0 + kk) * ldx + I0 + row0 + i];
-            }
-            As[kk][i] = v;
+    const int64_t kb = mode == 0 ? 0 : row0;
+    const int64_t ke = mode == 0 && col0 + 32 < K ? col0 + 32 : K;
+    const int lo = t & 31, hi = t >> 5;
+    double ra[4], rb[4];
+    auto load = [&](int64_t k0) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int h = hi + 8 * u;
+            // A: R row-major, consecutive threads along k; X column-major, along rows
+            const int64_t i = row0 + (mode == 0 ? h : lo), ka = k0 + (mode == 0 ? lo : h);
+            ra[u] = 0.0;
+            if (i < M && ka < K)
+                ra[u] = mode == 0 ? Rt[(size_t)(I0 + i) * n + J0 + ka] : X[(size_t)(I0 + ka) * ldx + I0 + i];
+            const int64_t j = col0 + h, kk = k0 + lo;
+            rb[u] = 0.0;
+            if (kk < K && j < N) rb[u] = mode == 0 ? X[(size_t)(J0 + j) * ldx + J0 + kk] : T[(size_t)j * b + kk];
         }
-        for (int e = t; e < 32 * 32; e += 256) {
-            const int kk = e & 31, j = e >> 5;
-            double v = 0.0;
-            if (k0 + kk < K && col0 + j < N)
-                v = mode == 0 ? X[(size_t)(J0 + col0 + j) * ldx + J0 + k0 + kk]
-                              : T[(size_t)(col0 + j) * b + k0 + kk];
-            Bs[kk][j] = v;
+    };
+    load(kb);
+    for (int64_t k0 = kb; k0 < ke; k0 += 32) {
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int h = hi + 8 * u;
+            if (mode == 0) As[lo][h] = ra[u];
+            else As[h][lo] = ra[u];
+            Bs[lo][h] = rb[u];
         }
         __syncthreads();
+        if (k0 + 32 < ke) load(k0 + 32);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
             const double a = As[4 * ks + q][8 * mb + g];

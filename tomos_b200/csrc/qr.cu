@@ -962,9 +962,11 @@ constexpr double kQrWideMaxKappa = 1e6;
 // stable where the Gram's Cholesky loses kappa_2 squared, so only a sketch
 // whose ||U^-1||_F is near that of orthonormal columns (sqrt(n); an RMS
 // inverse singular value of kQrWideRms at most, where a sketch of 4 n rows
-// has 1.15 and one of 2 n rows 1.41) keeps the wide path: there both round
-// alike.  The panel path's panels and blocks took 23 ms at 12000 x 3000, most
-// of it panel latency; the wide path takes 6.5 ms.
+// has 1.15 and one of 2 n rows 1.41) keeps the wide path: there both leave
+// Q^T Q - I at a few units of rounding an entry (1.9e-13 against 1.3e-13 in
+// the Frobenius norm at 12000 x 3000).  The panel path's panels and blocks
+// took 22 ms there, most of it panel latency; the wide path takes 12 ms with
+// LAPACK's signs and 6.5 ms with rows of any sign.
 constexpr int64_t kQrWidePlainN = 2048;
 constexpr double kQrWideRms = 1.5;
 constexpr double kQrWideFloor = 1e-10;
@@ -1026,6 +1028,29 @@ __global__ void wide_colnorm_kernel(const double* G, int64_t n, double* d, int* 
         if (!ok) atomicOr(flag, 1);
         d[i] = ok ? sqrt(gi) : 1.0;
     }
+}
+
+// The diagonal of G = SA^T SA anew, a block a column: squares all add up, so
+// the matrix product's one chain over k rows left each with an error of
+// ~sqrt(k) units, most of that of Q^T Q - I.  Short chains a thread, then a
+// tree: 1.9e-13 in the Frobenius norm at 12000 x 3000 (3.0e-13 without; the
+// panel path 1.3e-13), for 70 us.
+__global__ void __launch_bounds__(256) wide_diag_kernel(const double* SA, int64_t ld, int64_t k, int64_t n, double* G) {
+    __shared__ double sm[8];
+    const double* x = SA + (size_t)blockIdx.x * ld;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int64_t i = threadIdx.x;
+    for (; i + 3 * 256 < k; i += 4 * 256) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] += x[i + u * 256] * x[i + u * 256];
+    }
+    for (; i < k; i += 256) s[0] += x[i] * x[i];
+    const double w = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = w;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const double t = warp_sum(threadIdx.x < 8 ? sm[threadIdx.x] : 0.0);
+    if (threadIdx.x == 0) G[(size_t)blockIdx.x * n + blockIdx.x] = t;
 }
 
 // The upper half of D^-1 G D^-1 in place (d from wide_colnorm_kernel, so no
@@ -1491,6 +1516,10 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     tomos_status s = qr_gemm<true>(SA, ld, SA, ld, w.G, n, n, n, k, 1.0, 0.0, w.P, w.pcap, st, 0, true);
     if (s) return s;
     const unsigned eb = (unsigned)((n * n + 255) / 256 < 4096 ? (n * n + 255) / 256 : 4096);
+    if (n > kQrWidePlainN) {
+        wide_diag_kernel<<<(unsigned)n, 256, 0, st>>>(SA, ld, k, n, w.G);
+        TOMOS_LAUNCH_CHECK("wide_diag_kernel");
+    }
     wide_colnorm_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w.G, n, w.d, w.flag);
     TOMOS_LAUNCH_CHECK("wide_colnorm_kernel");
     wide_equilibrate_kernel<<<eb, 256, 0, st>>>(w.G, n, w.d);

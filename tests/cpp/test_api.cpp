@@ -103,6 +103,31 @@ int main() {
         CHECK(std::sqrt(err / nrm) < 1e-4, "packed rel err %g after %d iterations", std::sqrt(err / nrm), iters);
     }
 
+    // A row-major matrix and bucket count of odd sizes: the sketch of the same
+    // matrix stored by columns (FP32 sums of at most 100 entries below 1).
+    {
+        const std::size_t m = 100, n = 37, k = 7;
+        std::vector<float> row(m * n), col(m * n);
+        unsigned s = 777u;
+        for (std::size_t i = 0; i < m; ++i)
+            for (std::size_t j = 0; j < n; ++j) {
+                s = s * 1664525u + 1013904223u;
+                row[i * n + j] = col[i + m * j] = (float)((s >> 8) & 0xFFFF) / 32768.f - 1.f;
+            }
+        Dense R = Dense::create_strided(ctx, Layout::ROW_MAJOR, NumericType::FP32, {m, n});
+        cudaMemcpy(R.data(), row.data(), sizeof(float) * m * n, cudaMemcpyHostToDevice);
+        Dense Ccol = upload(ctx, col, m, n);
+        std::vector<double> h[2];
+        for (int q = 0; q < 2; ++q) {
+            Dense SA = Dense::create_strided(ctx, Layout::COL_MAJOR, NumericType::FP64, {k, n});
+            apply_count_sketch_hashed(q ? Ccol : R, SA);
+            h[q].resize(k * n);
+            cudaMemcpy(h[q].data(), SA.data(), sizeof(double) * k * n, cudaMemcpyDeviceToHost);
+        }
+        for (std::size_t e = 0; e < k * n; ++e)
+            CHECK(std::fabs(h[0][e] - h[1][e]) <= 100 * 100 * 6e-8, "sketch entry %zu: %g, %g", e, h[0][e], h[1][e]);
+    }
+
     // add_precond type mismatch throws std::invalid_argument
     // (test_workspace.cpp:17-79); FP16 storage has no kernel registered.
     {

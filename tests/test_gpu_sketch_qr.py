@@ -84,6 +84,7 @@ def test_apply_stage(orc, n, pad, s):
     (3001, 129, 0, 40),      # unaligned, past it for FP32
     (2049, 260, 4, 50),      # past it for 16-bit words
     (1500, 1037, 0, 9),      # unaligned, three column panels
+    (900, 301, 3, 5),        # odd sizes with rows on 16-byte boundaries
     (60001, 8, 0, 50000)])   # more buckets than a CTA counts: the sorted path
 @pytest.mark.parametrize("numeric,tier", [(NT.FP32, tb.Tier.AUTO), (NT.FP32_16, tb.Tier.HALF),
                                           (NT.FP32_16, tb.Tier.ACCURATE), (NT.FP32_BF16, tb.Tier.HALF)])
@@ -99,6 +100,10 @@ def test_apply_row_shapes(orc, m, n, pad, s, numeric, tier):
     sq = Ad.astype(np.float64) ** 2
     np.testing.assert_allclose(colsq.cpu().numpy(), sq.sum(0), rtol=1e-5)
     np.testing.assert_allclose(fro2.item(), sq.sum(), rtol=1e-5)
+    # without the caller's column sums they go to the scratch, behind s n FP32
+    # words (an odd count of them for odd sizes)
+    SA2, fro2b = tb.apply_count_sketch(A, s, tier=tier)
+    assert torch.equal(SA2.view(), SA.view()) and fro2b.item() == fro2.item()
 
 
 def test_apply_reference_golden(orc):

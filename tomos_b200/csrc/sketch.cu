@@ -633,7 +633,8 @@ CsScratch cs_layout(void* base, int64_t m, int64_t s, int64_t fro_parts, int64_t
 }
 
 int64_t cs_col_part_rows(int64_t m, int64_t s) {
-    // row-major: s x n FP32 per-bucket partials, then n FP64 column sums
+    // row-major: s x n FP32 per-bucket partials, then n FP64 column sums, from
+    // entry (s n + 1) / 2 <= n (s + 1) / 2 on
     const int64_t rows = (s + 1) / 2 + 1;
     int64_t csr = (int64_t)sm_count() * 2;             // CSR row-chunk blocks
     const int64_t cm = (m + 63) / 64;
@@ -769,9 +770,10 @@ static tomos_status launch_rows(const tomos_dense* A, const void* lo, int64_t s,
             cs_rows_any_kernel<E><<<grid, (unsigned)threads, 0, st>>>(a);
         TOMOS_LAUNCH_CHECK("cs_rows_kernel");
     }
-    // colsq (into the caller's buffer or the scratch after the partials),
-    // then fro2 as their sum
-    double* cs = colsq ? colsq : reinterpret_cast<double*>(a.col_part + s * n);
+    // colsq (into the caller's buffer, or the scratch after the s n FP32
+    // partials: an odd count is rounded up, doubles start on 8 bytes), then
+    // fro2 as their sum
+    double* cs = colsq ? colsq : c.col_part + (s * n + 1) / 2;
     int64_t chunks = (s + 63) / 64;
     const int64_t cap = cs_fro_parts(A->rows, s) / (n > 0 ? n : 1);
     if (chunks > cap) chunks = cap > 0 ? cap : 1;

@@ -319,6 +319,34 @@ def test_workspaces_made_and_closed_by_threads(m, n):
     assert free0 - torch.cuda.mem_get_info()[0] <= (64 << 20) + (4 << 20)
 
 
+def test_workspace_made_behind_queued_default_stream_work():
+    """A workspace made while the default stream is busy does nothing on that
+    stream: solves on another stream see no write of it, whenever the queued
+    work ends."""
+    rng = np.random.default_rng(3)
+    m, n = 4000, 60
+    A0 = rng.standard_normal((m, n)).astype(np.float32)
+    A, b = to_dense(A0, L.ROW_MAJOR), cuda((A0 @ rng.standard_normal(n)).astype(np.float32))
+    want, rep0, _ = tb.sketch_lsqr(A, b, 4 * n, max_iters=30)
+    want = want.clone()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        torch.cuda._sleep(100_000_000)  # ~50 ms of the default stream
+        idle = torch.cuda.Event()
+        idle.record()
+        with torch.cuda.stream(side):
+            tb.create_lsqr_workspace(None, (m, n), NT.FP32, NT.FP64).close()  # its memory goes to the next
+            while True:
+                ended = idle.query()
+                x, rep, _ = tb.sketch_lsqr(A, b, 4 * n, max_iters=30)
+                assert rep["iterations"] == rep0["iterations"] and rep["converged"] == 1
+                assert torch.equal(x, want)
+                if ended:
+                    break
+        torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("n", [1, 31, 128, 129, 512, 513, 777, 1030])
 def test_nside_at_its_sizes(n):
     """The n-side of a preconditioned solve in one CTA, a cluster and separate

@@ -1729,13 +1729,17 @@ tomos_status tomos_workspace_create(int64_t m, int64_t n, int32_t value_type,
     A(cudaEventCreate(&ws->ev_pa));
     A(cudaEventCreate(&ws->ev_pb));
     A(cudaEventCreateWithFlags(&ws->ev_fence, cudaEventDisableTiming));
+    // on the workspace's stream, as every use of its memory: the default
+    // stream's work would run at any time beside a solve, or after the block
+    // has gone to another workspace
+    if (ok) A(cudaMemsetAsync(ws->st, 0, sizeof(LsqrDev), ws->stream));
     if (!ok) {
+        if (ws->stream) cudaStreamSynchronize(ws->stream);
         ws_free(ws);
         delete ws;
         return fail(TOMOS_ERR_ALLOC, "tomos_workspace_create: device allocation failed");
     }
     std::memset(ws->st_host, 0, sizeof(LsqrDev));
-    cudaMemset(ws->st, 0, sizeof(LsqrDev));
     *out = ws;
     return TOMOS_OK;
 }

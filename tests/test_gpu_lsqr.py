@@ -320,31 +320,38 @@ def test_workspaces_made_and_closed_by_threads(m, n):
 
 
 def test_workspace_made_behind_queued_default_stream_work():
-    """A workspace made while the default stream is busy does nothing on that
-    stream: solves on another stream see no write of it, whenever the queued
-    work ends."""
+    """A workspace made while the default stream is busy leaves nothing on
+    that stream: neither its own solve nor one on the memory that a closed
+    workspace gave back sees a write of it when the queued work ends, which is
+    after the first cycle (its history is read behind that work)."""
     rng = np.random.default_rng(3)
     m, n = 4000, 60
     A0 = rng.standard_normal((m, n)).astype(np.float32)
     A, b = to_dense(A0, L.ROW_MAJOR), cuda((A0 @ rng.standard_normal(n)).astype(np.float32))
-    want, rep0, _ = tb.sketch_lsqr(A, b, 4 * n, max_iters=30)
-    want = want.clone()
-    torch.cuda.synchronize()
+    SA, _, colsq = tb.apply_count_sketch(A, 4 * n, with_colsq=True)
+    Rinv = tb.generate_sketch_qr_precond(SA)
+    d, an = tb.column_scale(colsq)
+
+    def solve(stream):
+        ws = tb.create_lsqr_workspace(None, (m, n), NT.FP32, NT.FP64)
+        tb.add_precond(Rinv, ws)
+        x = torch.empty(n, device="cuda")
+        rep = tb.lsqr_solve(None, A, b, x, ws, 1e-6, 4, 0.0, restarts=8, stop_rule=tb.StopRule.BACKWARD,
+                            anorm_fro=an, col_scale=d, stream=stream)
+        return ws, x, rep
+
+    _, want, rep0 = solve(None)
+    assert rep0["converged"] == 1 and rep0["restarts_used"] > 2
     side = torch.cuda.Stream()
-    for _ in range(3):
-        torch.cuda._sleep(100_000_000)  # ~50 ms of the default stream
-        idle = torch.cuda.Event()
-        idle.record()
-        with torch.cuda.stream(side):
-            tb.create_lsqr_workspace(None, (m, n), NT.FP32, NT.FP64).close()  # its memory goes to the next
-            while True:
-                ended = idle.query()
-                x, rep, _ = tb.sketch_lsqr(A, b, 4 * n, max_iters=30)
-                assert rep["iterations"] == rep0["iterations"] and rep["converged"] == 1
-                assert torch.equal(x, want)
-                if ended:
-                    break
+    for rows in (None, m + 300):
         torch.cuda.synchronize()
+        torch.cuda._sleep(100_000_000)  # ~50 ms of the default stream
+        if rows is not None:  # its memory goes to the solve's workspace, laid out otherwise
+            tb.create_lsqr_workspace(None, (rows, n), NT.FP32, NT.FP64).close()
+        ws, x, rep = solve(side)
+        torch.cuda.synchronize()
+        assert rep["iterations"] == rep0["iterations"] and rep["converged"] == 1
+        assert torch.equal(x, want)
 
 
 @pytest.mark.parametrize("n", [1, 31, 128, 129, 512, 513, 777, 1030])

@@ -219,3 +219,59 @@ def test_batched_solves_match_single(m, n, K, pad):
     again, _ = tb.lsqr_solve_batch(A, cuda(B0), ws, 1e-6, 30, 3, an, col_scale=d)
     first, _ = tb.lsqr_solve_batch(A, cuda(B0), ws, 1e-6, 30, 3, an, col_scale=d)
     assert torch.equal(again, first)
+
+
+def test_calls_on_another_stream_order_their_own_copies():
+    """With stream= given, what a call copies, fills or allocates itself is
+    ordered on that stream, whatever the current stream still has to run: the
+    results of the same calls on the current stream."""
+    rng = np.random.default_rng(12)
+    m, n, K = 20011, 40, 5
+    A0 = rng.standard_normal((m, n)).astype(np.float32)
+    A = to_dense(A0, L.ROW_MAJOR)
+    B = cuda(rng.standard_normal((m, K)).astype(np.float32))
+    G = cuda(rng.standard_normal((n, K)).astype(np.float32))
+    R0 = tb.generate_sketch_qr_precond(tb.apply_count_sketch(A, 4 * n)[0])
+    torch.cuda.synchronize()
+    kept = []
+
+    def calls(stream):
+        SA, fro2, colsq = tb.apply_count_sketch(A, 4 * n, with_colsq=True, stream=stream)
+        d, an = tb.column_scale(colsq, stream=stream)
+        ws = tb.create_lsqr_workspace(None, (m, n), NT.FP32, NT.FP64)
+        tb.add_precond(R0, ws)
+        X, _ = tb.lsqr_solve_batch(A, B, ws, 1e-6, 30, 3, an, col_scale=d, stream=stream)
+        Lam, _ = tb.lsqr_adjoint_batch(A, G, ws, stream=stream)
+        gA, gB = tb.lsqr_adjoint_grad(A, B, X, Lam, stream=stream)
+        P = tb.pack(A, NT.FP32_16, stream=stream)
+        kept.append(ws)  # closing it waits for the device
+        return [SA, fro2, colsq, X, Lam, gA, gB, P.storage]
+
+    want = calls(None)
+    want[0] = want[0].storage
+    want = [t.clone() for t in want]
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+
+    class Handle:  # any object that carries a stream's handle
+        cuda_stream = side.cuda_stream
+
+    calls(side)  # its memory is there from now on
+    torch.cuda.synchronize()
+    for stream in (side, Handle()):
+        # freed blocks of the current stream, with a write of them queued
+        # behind 50 ms of other work
+        junk = [torch.empty_like(t) for t in want]
+        torch.cuda._sleep(100_000_000)
+        for t in junk:
+            t.fill_(1)
+        del t, junk
+        got = calls(stream)
+        side.synchronize()
+        assert not torch.cuda.current_stream().query()  # all of it ran beside the queued work
+        # a cooperative launch, which waits for the queued work
+        Rinv = tb.generate_sketch_qr_precond(got[0], stream=stream)
+        torch.cuda.synchronize()
+        assert torch.equal(Rinv.storage, R0.storage)
+        for g, w in zip(got[1:], want[1:]):
+            assert torch.equal(g, w)

@@ -8,6 +8,7 @@ apply_count_sketch, generate_sketch_qr_precond.  Device memory comes from
 torch (CUDA tensors); every product runs in the sm_100a kernels of
 libtomos_b200.so.  There is no CPU path: a CPU Context raises.
 """
+import contextlib
 import ctypes
 import enum
 import os
@@ -87,13 +88,40 @@ def _stream(stream):
 _CUDA = torch.device("cuda")
 
 
+def _on(stream):
+    """torch's current stream for what a call on `stream` allocates, fills or
+    copies: memory of another stream's could be written by that stream's work,
+    or reused, before the call's kernels have run."""
+    if stream is None:
+        return contextlib.nullcontext()
+    if not isinstance(stream, torch.cuda.Stream):
+        stream = torch.cuda.ExternalStream(stream.cuda_stream)
+    return torch.cuda.stream(stream)
+
+
 def _scratch(nbytes, stream):
-    """Scratch of a call on `stream`, from that stream's own memory: a block of
-    another stream's could be reused before the call's kernels have run."""
+    """Scratch of a call on `stream`."""
     if stream is None:
         return torch.empty(nbytes or 1, dtype=torch.uint8, device=_CUDA)
-    with torch.cuda.stream(stream):
+    with _on(stream):
         return torch.empty(nbytes or 1, dtype=torch.uint8, device=_CUDA)
+
+
+def _result(t, stream):
+    """Marks a result that a call allocated on `stream`: the caller's stream
+    uses it too, so its memory waits for both before it is reused."""
+    if stream is not None:
+        t.record_stream(torch.cuda.current_stream())
+    return t
+
+
+def _empty(shape, dtype, stream):
+    """A result of a call on `stream`, written in full by it."""
+    if stream is None:
+        return torch.empty(shape, dtype=dtype, device=_CUDA)
+    with _on(stream):
+        t = torch.empty(shape, dtype=dtype, device=_CUDA)
+    return _result(t, stream)
 
 
 class Context:
@@ -153,11 +181,11 @@ class Dense:
         return cls(st, layout, size, ld, buf, rounded)
 
     @classmethod
-    def _empty_f64(cls, layout, size):
-        """An FP64 Dense whose values the caller's kernel writes in full (no
-        zero fill)."""
+    def _empty_f64(cls, layout, size, stream):
+        """An FP64 Dense whose values the caller's kernel (on `stream`) writes
+        in full (no zero fill)."""
         outer, inner = cls._outer_inner(layout, size)
-        buf = torch.empty(max(inner * outer, 1), dtype=torch.float64, device="cuda")
+        buf = _empty(max(inner * outer, 1), torch.float64, stream)
         return cls(NumericType.FP64, layout, size, inner, buf)
 
     @classmethod
@@ -417,7 +445,9 @@ def pack_fp16(A_fp32, P, stream=None):
 def pack(A_fp32, store_type, rounded=False, stream=None):
     """Convenience: a packed (or native FP16) copy of an FP32 Dense with the
     same layout."""
-    P = Dense.create_strided(None, A_fp32.layout, store_type, A_fp32.size, A_fp32.ld, rounded)
+    with _on(stream):
+        P = Dense.create_strided(None, A_fp32.layout, store_type, A_fp32.size, A_fp32.ld, rounded)
+    _result(P.storage, stream)
     if NumericType(store_type) == NumericType.FP16:
         return pack_fp16(A_fp32, P, stream=stream)
     if NumericType(store_type) == NumericType.FP32_16:
@@ -524,8 +554,8 @@ def mm_apply_fp32_16_ext(dev, transA, transB, alpha, A, B, beta, Cm, stream=None
 
 def countsketch_hash(m, s, bucket_seed=CS_BUCKET_SEED, sign_seed=CS_SIGN_SEED, stream=None):
     """Per-row bucket and sign of the hash CountSketch (device tensors)."""
-    bucket = torch.empty(max(m, 1), dtype=torch.int32, device="cuda")
-    sign = torch.empty(max(m, 1), dtype=torch.int8, device="cuda")
+    bucket = _empty(max(m, 1), torch.int32, stream)
+    sign = _empty(max(m, 1), torch.int8, stream)
     C.check(C.lib().tomos_countsketch_hash(m, s, bucket_seed, sign_seed, _ptr(bucket), _ptr(sign),
                                            _stream(stream)), "countsketch_hash")
     return bucket[:m], sign[:m]
@@ -542,9 +572,9 @@ def apply_count_sketch(A, s, tier=Tier.AUTO, bucket_seed=CS_BUCKET_SEED, sign_se
         return _count_sketch_stage(A, s, bucket_seed, sign_seed, with_colsq, stream)
     n = A.size[1]
     # every output is written in full by the sketch
-    SA = Dense._empty_f64(Layout.COL_MAJOR, (s, n))
-    fro2 = torch.empty(1, dtype=torch.float64, device="cuda")
-    colsq = torch.empty(max(n, 1), dtype=torch.float64, device="cuda") if with_colsq else None
+    SA = Dense._empty_f64(Layout.COL_MAJOR, (s, n), stream)
+    fro2 = _empty(1, torch.float64, stream)
+    colsq = _empty(max(n, 1), torch.float64, stream) if with_colsq else None
     m = A.size[0]
     nb = C.lib().tomos_countsketch_scratch_bytes(m, n, s)
     scratch = _scratch(nb, stream)
@@ -562,10 +592,10 @@ def _count_sketch_stage(A, s, bucket_seed, sign_seed, with_colsq, stream):
         raise TomosError(C.TOMOS_ERR_INVALID, "apply_count_sketch: stage needs a row-major FP32_16 A")
     m, n = A.size
     ldp = (n + 7) // 8 * 8
-    plane = torch.empty((max(m, 1), ldp), dtype=torch.int16, device="cuda")
-    SA = Dense._empty_f64(Layout.COL_MAJOR, (s, n))
-    fro2 = torch.empty(1, dtype=torch.float64, device="cuda")
-    colsq = torch.empty(max(n, 1), dtype=torch.float64, device="cuda") if with_colsq else None
+    plane = _empty((max(m, 1), ldp), torch.int16, stream)
+    SA = Dense._empty_f64(Layout.COL_MAJOR, (s, n), stream)
+    fro2 = _empty(1, torch.float64, stream)
+    colsq = _empty(max(n, 1), torch.float64, stream) if with_colsq else None
     nb = C.lib().tomos_countsketch_scratch_bytes(m, n, s)
     scratch = _scratch(nb, stream)
     d = A.desc()
@@ -601,8 +631,10 @@ def generate_sketch_qr_precond(sketched, R_out=None, copy=True, any_signs=False,
             "generate_sketch_qr_precond")
     if not copy:
         return Dense(NumericType.FP64, Layout.COL_MAJOR, (n, n), sketched.ld, sketched.storage)
-    Rinv = Dense.create_strided(None, Layout.COL_MAJOR, NumericType.FP64, (n, n))
-    Rinv.view()[...] = sketched.view()[:n, :n]
+    with _on(stream):
+        Rinv = Dense.create_strided(None, Layout.COL_MAJOR, NumericType.FP64, (n, n))
+        Rinv.view()[...] = sketched.view()[:n, :n]
+    _result(Rinv.storage, stream)
     return Rinv
 
 
@@ -733,8 +765,9 @@ def lsqr_solve_batch(A, B, workspace, tol, max_iters, restarts, anorm_fro, col_s
     Returns (X, list of K reports)."""
     m, n = A.size
     K = B.shape[1]
-    Bc = B.t().contiguous().float()  # column-major m x K
-    Xc = torch.empty((K, n), dtype=torch.float32, device="cuda")
+    with _on(stream):
+        Bc = B.t().contiguous().float()  # column-major m x K
+    Xc = _empty((K, n), torch.float32, stream)
     d = A.desc()
     reports = []
     for k0 in range(0, K, 8):
@@ -783,7 +816,7 @@ def lsqr_adjoint(A, g, workspace, tol=1e-7, max_iters=500, tier=None, stream=Non
     opts.max_iters = int(max_iters)
     opts.restarts = 1
     opts.iter_tier = int(Tier.AUTO if tier is None else Tier(tier))
-    lam = torch.empty(A.size[1], dtype=torch.float32, device="cuda")
+    lam = _empty(A.size[1], torch.float32, stream)
     rep = C.LsqrReport()
     d = A.desc()
     C.check(C.lib().tomos_lsqr_adjoint_dense(ctypes.byref(d), _ptr(_vec(g)), _ptr(lam),
@@ -805,8 +838,9 @@ def lsqr_adjoint_batch(A, G, workspace, tol=1e-7, max_iters=500, tier=None, stre
     opts.max_iters = int(max_iters)
     opts.restarts = 1
     opts.iter_tier = int(Tier.AUTO if tier is None else Tier(tier))
-    Gc = G.t().contiguous().float()  # column-major n x K
-    Lc = torch.empty((K, n), dtype=torch.float32, device="cuda")
+    with _on(stream):
+        Gc = G.t().contiguous().float()  # column-major n x K
+    Lc = _empty((K, n), torch.float32, stream)
     reps = (C.LsqrReport * max(K, 1))()
     d = A.desc()
     C.check(C.lib().tomos_lsqr_adjoint_batch_dense(ctypes.byref(d), K, _ptr(Gc), n, _ptr(Lc), n,
@@ -822,11 +856,12 @@ def lsqr_adjoint_grad(A, B, X, Lam, want_grad_a=True, stream=None):
     Lam: (n, K) float32 CUDA tensors.  Returns (gradA or None, gradB)."""
     m, n = A.size
     K = B.shape[1]
-    Bc = B.t().contiguous()  # column-major (m x K)
-    Xc = X.t().contiguous()
-    Lc = Lam.t().contiguous()
-    gB = torch.empty((K, m), dtype=torch.float32, device="cuda")
-    gA = torch.empty((m, n), dtype=torch.float32, device="cuda") if want_grad_a else None
+    with _on(stream):
+        Bc = B.t().contiguous()  # column-major (m x K)
+        Xc = X.t().contiguous()
+        Lc = Lam.t().contiguous()
+    gB = _empty((K, m), torch.float32, stream)
+    gA = _empty((m, n), torch.float32, stream) if want_grad_a else None
     d = A.desc()
     C.check(C.lib().tomos_lsqr_adjoint_grad_dense(ctypes.byref(d), K, _ptr(Bc), m, _ptr(Xc), n,
                                                   _ptr(Lc), n, _ptr(gB), m, _ptr(gA), n,
@@ -841,8 +876,8 @@ def column_scale(colsq, stream=None):
     returns (d, anorm) with anorm a one-element float64 CUDA tensor, which
     lsqr_solve takes as anorm_fro without a host round trip."""
     n = colsq.numel()
-    d = torch.empty(max(n, 1), dtype=torch.float64, device="cuda")
-    an = torch.empty(1, dtype=torch.float64, device="cuda")
+    d = _empty(max(n, 1), torch.float64, stream)
+    an = _empty(1, torch.float64, stream)
     C.check(C.lib().tomos_column_scale(_ptr(colsq), n, _ptr(d), _ptr(an), _stream(stream)),
             "column_scale")
     return d[:n], an
@@ -903,7 +938,7 @@ def sketch_lsqr(A, b, s, tol=1e-6, max_iters=200, restarts=8, inner_rtol=None, w
         ws = create_lsqr_workspace(None, (m, n), NumericType.FP32, NumericType.FP64)
     add_precond(Rinv, ws)
     if x is None:
-        x = torch.empty(n, dtype=torch.float32, device="cuda")  # the solve zeroes x
+        x = _empty(n, torch.float32, stream)  # the solve zeroes x
     if inner_rtol is None:
         inner_rtol = 2e-3 if packed else 0.0
     rep = lsqr_solve(None, A, b, x, ws, tol, max_iters, 0.0, restarts=restarts,
@@ -992,10 +1027,10 @@ def apply_count_sketch_shard(A, s, row0, tier=Tier.AUTO, bucket_seed=CS_BUCKET_S
     plane = None
     if stage:
         ldp = (n + 7) // 8 * 8
-        plane = torch.empty((max(m, 1), ldp), dtype=torch.int16, device="cuda")
-    SA = Dense._empty_f64(Layout.COL_MAJOR, (s, n))
-    fro2 = torch.empty(1, dtype=torch.float64, device="cuda")
-    colsq = torch.empty(max(n, 1), dtype=torch.float64, device="cuda")
+        plane = _empty((max(m, 1), ldp), torch.int16, stream)
+    SA = Dense._empty_f64(Layout.COL_MAJOR, (s, n), stream)
+    fro2 = _empty(1, torch.float64, stream)
+    colsq = _empty(max(n, 1), torch.float64, stream)
     nb = C.lib().tomos_countsketch_scratch_bytes(m, n, s)
     scratch = _scratch(nb, stream)
     d = A.desc()

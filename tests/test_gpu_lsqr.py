@@ -319,6 +319,46 @@ def test_workspaces_made_and_closed_by_threads(m, n):
     assert free0 - torch.cuda.mem_get_info()[0] <= (64 << 20) + (4 << 20)
 
 
+def test_second_matrix_on_one_workspace():
+    """Solves of two matrices of one size on a workspace: the second iterates
+    over its own values and row offsets, also where addresses and leading
+    dimensions (dense), or only the row offsets (CSR), tell the two apart."""
+    rng = np.random.default_rng(8)
+    m, n = 1024, 250
+    buf = torch.zeros(6 << 20, dtype=torch.float32, device="cuda")
+    base = (-buf.data_ptr() // 4) % (2 << 20)  # 8 MiB boundary
+    ws = tb.create_lsqr_workspace(None, (m, n), NT.FP32, NT.FP32)
+
+    def solve(A, b):
+        x = torch.zeros(n, device="cuda")
+        rep = tb.lsqr_solve(None, A, cuda(b), x, ws, 1e-6, 200, 0.0)
+        assert rep["converged"] == 1
+        return x.cpu().numpy()
+
+    for off, ld in ((0, 1024), (1 << 20, 1028)):  # 4 MiB apart
+        A0 = rng.standard_normal((m, n)).astype(np.float32)
+        A = tb.Dense(NT.FP32, L.ROW_MAJOR, (m, n), ld, buf[base + off:base + off + m * ld])
+        A.view()[...] = cuda(A0)
+        xt = rng.standard_normal(n)
+        x = solve(A, (A0.astype(np.float64) @ xt).astype(np.float32))
+        # relative residual 1e-6 over the condition number of a 1024 x 250 Gaussian, ~3
+        assert np.linalg.norm(x - xt) < 1e-5 * np.linalg.norm(xt)
+    # CSR: the same entries dealt to rows of 6, then to rows of 7 and 5 in turn
+    # (columns 37 apart: distinct within a row)
+    cols = np.arange(6 * m, dtype=np.int32) * 37 % n
+    vals = rng.standard_normal(6 * m).astype(np.float32)
+    rows6 = np.arange(0, 6 * m + 1, 6, dtype=np.int32)
+    ptrs = [cuda(r, torch.int32) for r in (rows6, rows6 + np.arange(m + 1, dtype=np.int32) % 2)]
+    c, v = cuda(cols, torch.int32), cuda(vals)
+    for rp in ptrs:
+        S = np.zeros((m, n))
+        S[np.repeat(np.arange(m), np.diff(rp.cpu().numpy())), cols] = vals
+        xt = rng.standard_normal(n)
+        x = solve(tb.Csr(NT.FP32, (m, n), rp, c, v), (S @ xt).astype(np.float32))
+        # relative residual 1e-6 times the condition number
+        assert np.linalg.norm(x - xt) < 2e-6 * np.linalg.cond(S) * np.linalg.norm(xt)
+
+
 def test_workspace_made_behind_queued_default_stream_work():
     """A workspace made while the default stream is busy leaves nothing on
     that stream: neither its own solve nor one on the memory that a closed

@@ -837,9 +837,10 @@ struct CsrPass : PassOps {
         return launch_csr(pl.e, pl.acc64, P, pl.grid, pl.nch, st);
     }
     tomos_status fro2(double* out, const double* d, cudaStream_t st) override;
-    uint64_t key() override {
-        return reinterpret_cast<uint64_t>(A->values) ^ (reinterpret_cast<uint64_t>(A->col_idxs) << 1) ^
-               (reinterpret_cast<uint64_t>(cc.rows) << 3) ^ (uint64_t)csc;
+    void key(std::vector<uint64_t>* k) override {
+        const CscCopy c = csc ? cc : CscCopy{};
+        const void* ptrs[] = {A->values, csr_lo(A), A->row_ptrs, A->col_idxs, c.col_ptr, c.rows, c.hi, c.lo};
+        for (const void* p : ptrs) k->push_back(reinterpret_cast<uint64_t>(p));
     }
     int64_t rows() override { return A->rows; }
     int64_t cols() override { return A->cols; }

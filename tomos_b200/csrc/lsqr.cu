@@ -1186,10 +1186,13 @@ struct DensePass : PassOps {
         TOMOS_LAUNCH_CHECK("sum_to_scalar_kernel");
         return TOMOS_OK;
     }
-    uint64_t key() override {
-        return reinterpret_cast<uint64_t>(A->values) ^ ((uint64_t)A->layout << 60) ^
-               ((uint64_t)A->ld << 20) ^
-               (stage ? reinterpret_cast<uint64_t>(staged.values) * 31 ^ ((uint64_t)staged.ld << 40) : 0);
+    void key(std::vector<uint64_t>* k) override {
+        for (const tomos_dense* D : {A, static_cast<const tomos_dense*>(stage ? &staged : nullptr)}) {
+            k->push_back(D ? reinterpret_cast<uint64_t>(D->values) : 0);
+            k->push_back(D && elem_is_exact(iter_e) ? reinterpret_cast<uint64_t>(dense_lo_plane(D)) : 0);
+            k->push_back(D ? (uint64_t)D->layout : 0);
+            k->push_back(D ? (uint64_t)D->ld : 0);
+        }
     }
     int64_t rows() override { return A->rows; }
     int64_t cols() override { return A->cols; }
@@ -1348,8 +1351,7 @@ tomos_status solve_driver(tomos_workspace* ws, PassOps& ops, const float* b, flo
     PassPlan pl_iter = ops.plan(false);
 
     // Capture (or reuse) the graph of one iteration.
-    std::vector<uint64_t> key = {ops.key(),
-                                 (uint64_t)pl_iter.fused,
+    std::vector<uint64_t> key = {(uint64_t)pl_iter.fused,
                                  (uint64_t)pl_iter.e,
                                  (uint64_t)pl_iter.nch,
                                  (uint64_t)pl_iter.g,
@@ -1363,6 +1365,7 @@ tomos_status solve_driver(tomos_workspace* ws, PassOps& ops, const float* b, flo
                                  (uint64_t)n,
                                  (uint64_t)m,
                                  reinterpret_cast<uint64_t>(o->comm)};
+    ops.key(&key);
     if (!ws->graph || ws->graph_key != key) {
         if (ws->graph) cudaGraphExecDestroy(ws->graph);
         ws->graph = nullptr;

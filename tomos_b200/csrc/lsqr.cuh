@@ -109,7 +109,9 @@ struct PassOps {
                                  const double* coef, const int* skip, cudaStream_t st) = 0;
     // sum of squares of A's elements divided by d[column] (d may be NULL)
     virtual tomos_status fro2(double* out_dev, const double* d, cudaStream_t st) = 0;
-    virtual uint64_t key() = 0;
+    // What an iteration's launches take from this pass besides its plan: every
+    // pointer and size, an entry each (folded together, two matrices could agree).
+    virtual void key(std::vector<uint64_t>* k) = 0;
     virtual int64_t rows() = 0;
     virtual int64_t cols() = 0;
     // Work done once per solve before the first pass (e.g. staging).
@@ -139,7 +141,10 @@ struct RefinePass : PassOps {
         return pl.src ? re.enqueue(pl, p, u_in, coef, skip, st) : it.enqueue(pl, p, u_in, coef, skip, st);
     }
     tomos_status fro2(double* out, const double* d, cudaStream_t st) override { return re.fro2(out, d, st); }
-    uint64_t key() override { return it.key() ^ (re.key() * 0x9E3779B97F4A7C15ull); }
+    void key(std::vector<uint64_t>* k) override {
+        it.key(k);
+        re.key(k);
+    }
     int64_t rows() override { return it.rows(); }
     int64_t cols() override { return it.cols(); }
     tomos_status prepare(cudaStream_t st) override {

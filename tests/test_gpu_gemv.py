@@ -1,6 +1,7 @@
 """tomos_gemv (every storage type, tier, layout, transpose, beta) against
 an FP64 product of the values the tier reads (oracle decode), and against
 the reference's own CPU FP32_16 tiers."""
+import ctypes
 import os
 
 import numpy as np
@@ -8,6 +9,7 @@ import pytest
 import torch
 
 import tomos_b200 as tb
+from tomos_b200 import _capi as C
 from gpu_util import to_dense, decoded, cuda
 
 GOLD = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden")
@@ -76,6 +78,28 @@ def test_gemv_line_shapes(orc, numeric, tier, rounded, m, n, pad, layout):
             # exact tiers: FP32 runs of at most 8 at worst, then one rounding
             tol = (2e-6 if tier == tb.Tier.ACCURATE else 2e-5) * scale + 1e-30
             assert np.all(np.abs(got - ref) <= tol + 1e-7 * np.abs(ref)), (trans, beta)
+
+
+@pytest.mark.parametrize("offset", [0, 4])
+def test_few_long_dots_scratch_alignment(offset):
+    """Dots of few, long lines with a scratch on 8 bytes (FP64 partials of a
+    line's segments) and on 4 bytes only (a warp a line)."""
+    rng = np.random.default_rng(5)
+    m, n = 40000, 3
+    A0 = rng.standard_normal((m, n)).astype(np.float32)
+    A, x = to_dense(A0, L.COL_MAJOR), rng.standard_normal(m).astype(np.float32)
+    lib, d = C.lib(), A.desc()
+    nb = lib.tomos_gemv_scratch_bytes(ctypes.byref(d), int(tb.TRANSPOSE))
+    assert nb > 0
+    scratch = torch.empty(nb + 8, dtype=torch.uint8, device="cuda")
+    xt, y = torch.from_numpy(x).cuda(), torch.empty(n, device="cuda")
+    C.check(lib.tomos_gemv(int(tb.TRANSPOSE), 1.0, ctypes.byref(d), int(tb.Tier.AUTO), xt.data_ptr(), 0.0,
+                           y.data_ptr(), scratch.data_ptr() + offset, nb, None), "gemv")
+    torch.cuda.synchronize()
+    ref = A0.astype(np.float64).T @ x
+    # FP32 products and sums of at most m / 32 terms a lane
+    tol = (m / 32 + 40) * 6e-8 * (np.abs(A0).astype(np.float64).T @ np.abs(x))
+    assert np.all(np.abs(y.cpu().numpy() - ref) <= tol)
 
 
 def test_fp32_16_tiers_vs_reference_cpu(orc):

@@ -285,7 +285,9 @@ static tomos_status run_gemv_v(const GemvLaunch& L, cudaStream_t st) {
     using Acc = typename AccT<ACC64>::T;
     if (L.dot) {
         const int64_t segs = line_dot_segments(L.outer, L.inner);
-        if (segs > 1 && L.scratch && L.scratch_bytes >= (size_t)segs * L.outer * sizeof(double)) {
+        // (a scratch that cannot hold doubles: a warp a line, which needs none)
+        if (segs > 1 && L.scratch && reinterpret_cast<uintptr_t>(L.scratch) % sizeof(double) == 0 &&
+            L.scratch_bytes >= (size_t)segs * L.outer * sizeof(double)) {
             const int64_t unit = 256 * V;
             const int64_t seg = ((L.inner + segs - 1) / segs + unit - 1) / unit * unit;
             const int64_t ns = (L.inner + seg - 1) / seg;

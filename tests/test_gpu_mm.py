@@ -238,3 +238,54 @@ def test_mm_few_columns(orc, numeric, rounded, layout, m, n, k, pad):
         for lb, beta in ((L.COL_MAJOR, 0.0), (L.ROW_MAJOR, -0.5)):
             check(orc, A, A0, tb.Tier.ACCURATE if numeric != NT.FP32 else tb.Tier.AUTO, ta, T.NO_TRANSPOSE, (kk, k),
                   (lb, lb), beta, rng)
+
+
+@pytest.mark.parametrize("numeric", [NT.FP32, NT.FP32_16, NT.FP32_BF16])
+@pytest.mark.parametrize("m,n,k,trans", [(20000, 9, 16, False), (20000, 16, 16, False), (20000, 33, 8, False),
+                                         (20000, 64, 9, False), (20000, 1500, 16, False), (48, 300, 16, True),
+                                         (64, 300, 3, True), (1000000, 24, 16, True), (1000000, 24, 8, True)])
+def test_mm_few_columns_no_less_exact_than_tiles(numeric, m, n, k, trans):
+    """At most 16 columns against FP64: no further from it than the tiled
+    kernels, which compute the same columns as part of 17.  A^T times columns
+    of A itself has sums of one sign on its diagonal."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + n + k)
+    A0 = torch.randn(m, n, generator=g, device="cuda")
+    A = tb.Dense.from_tensor(A0, L.ROW_MAJOR)
+    A = A if numeric == NT.FP32 else tb.pack(A, numeric)
+    K = m if trans else n
+    B = A0[:, :k] if trans else torch.randn(K, k, generator=g, device="cuda")
+    B17 = torch.cat([B, torch.randn(K, 17 - k, generator=g, device="cuda")], 1)
+    tier = tb.Tier.AUTO if numeric == NT.FP32 else tb.Tier.ACCURATE
+    Ad = A0.double()
+    if numeric == NT.FP32_BF16:  # truncated low words: the value itself is read
+        back = tb.Dense.create_strided(None, L.ROW_MAJOR, NT.FP32, (m, n))
+        tb.combine_fp32_bf16(A, back)
+        Ad = back.view().double()
+    ref = (Ad.t() if trans else Ad) @ B.double()
+
+    def errors(cols):
+        C = tb.Dense.create_strided(None, L.COL_MAJOR, NT.FP32, (n if trans else m, cols.shape[1]))
+        tb.mm_apply(tb.Device.CUDA, T.TRANSPOSE if trans else T.NO_TRANSPOSE, T.NO_TRANSPOSE, 1.0, A,
+                    tb.Dense.from_tensor(cols, L.COL_MAJOR), 0.0, C, tier=tier)
+        e = C.view()[:, :k].double() - ref
+        diag = torch.arange(min(n, k), device="cuda")
+        return torch.linalg.norm(e).item(), torch.linalg.norm(e[diag, diag]).item()
+
+    few, tiled = errors(B), errors(B17)
+    assert few[0] <= tiled[0] and (not trans or few[1] <= tiled[1]), (few, tiled)
+
+
+@pytest.mark.parametrize("bits", [0x7FFFFFFF, 0x7FC00000, 0x7F800001, 0xFFFFFFFF])
+def test_mm_few_columns_nan(bits):
+    """A NaN of any payload in A reaches its row (or column) of C, whole."""
+    A0 = torch.ones(40, 37, device="cuda")
+    A0.view(torch.int32)[3, 5] = bits - (1 << 32) if bits >> 31 else bits
+    for trans, row in ((False, 3), (True, 5)):
+        B = torch.ones(40 if trans else 37, 9, device="cuda")
+        C = tb.Dense.create_strided(None, L.COL_MAJOR, NT.FP32, (37 if trans else 40, 9))
+        tb.mm_apply(tb.Device.CUDA, T.TRANSPOSE if trans else T.NO_TRANSPOSE, T.NO_TRANSPOSE, 1.0,
+                    tb.Dense(NT.FP32, L.ROW_MAJOR, (40, 37), 37, A0.reshape(-1)),
+                    tb.Dense.from_tensor(B, L.COL_MAJOR), 0.0, C)
+        bad = torch.isnan(C.view())
+        assert bad[row].all() and bad.sum().item() == 9

@@ -20,12 +20,17 @@
 // What is left an element is its decode and its split.  No barrier and no
 // shared-memory write in either loop; the next chunk is in
 // flight in a warp's registers, later ones are asked into L2.
-// 1e6 x 1000 x 16 FP32_16: 1.05 ms along K, 1.34 ms along M (3.8 and 3.0 TB/s;
+// 1e6 x 1000 x 16 FP32_16: 1.05 ms along K, 1.40 ms along M (3.8 and 2.9 TB/s;
 // bound by the decode, the split and the products' issue together); 200000 x
-// 500 x 8 FP32, both: 390 us to 181 us; unaligned 300000 x 257 x 16 FP32:
-// 1.30 ms to 0.27 ms.
-// Accuracy: a hardware sum of 32 products (its adds round toward zero) is
-// added to an FP32 total; runs of K are summed in FP64 by the caller.
+// 500 x 8 FP32, both: 390 us to 217 us; unaligned 300000 x 257 x 16 FP32:
+// 1.30 ms to 0.25 ms.
+// Accuracy: the hardware's adds round toward zero, so a hardware sum is short:
+// along K the products of 32 K, those with a small half apart, added to an
+// FP32 total (48 adds at most); along M 48 lines, added to an FP64 total (a
+// run of 16384 lines, as of the diagonal of A^T A, all of one sign).  Runs
+// are summed in FP64 by the caller.  Relative to FP64: 1.7e-7 along K, 4e-7
+// along M at 1e6 x 1000 (the tiled kernels 7e-6 and 4.6e-6); 1.0e-7 at K = 9
+// and 16 (2.0e-7).
 #pragma once
 
 #include "common.cuh"
@@ -56,9 +61,13 @@ constexpr int kSkinnySumCtas = 3;      // an SM
 constexpr int kSkinnySumLines = 16384; // lines of a run of skinny_sum_kernel, at most
 constexpr int kSkinnyAhead = 8;        // chunks asked into L2 ahead
 
+// x as two TF32 values, both rounded to nearest: 24 bits (truncated halves
+// keep 22 and lean toward zero).  The first one's rounding is two integer
+// instructions, cheaper than the conversion; a NaN whose carry leaves the
+// exponent still has a NaN remainder.
 __device__ __forceinline__ void skinny_split(float x, uint32_t& big, uint32_t& small) {
-    big = __float_as_uint(x) & 0xFFFFE000u;
-    small = __float_as_uint(x - __uint_as_float(big)) & 0xFFFFE000u;
+    big = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(small) : "f"(x - __uint_as_float(big)));
 }
 
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -200,7 +209,7 @@ __global__ void __launch_bounds__(32 * kSkinnyDotWarps, 1) skinny_dot_kernel(Ski
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             load(w[u ^ 1]);
-            float d[NT][4] = {};
+            float d[NT][4] = {}, ds[NT][4] = {};  // ds: the products with a small half
             const float4* bp = bs + (size_t)c * (4 * NT * 32) + lane;
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
@@ -213,15 +222,15 @@ __global__ void __launch_bounds__(32 * kSkinnyDotWarps, 1) skinny_dot_kernel(Ski
 #pragma unroll
                 for (int j = 0; j < NT; ++j) {
                     const float4 b = bp[(s * NT + j) * 32];
-                    mma_tf32(d[j], bg, __float_as_uint(b.z), __float_as_uint(b.w));
-                    mma_tf32(d[j], sm, __float_as_uint(b.x), __float_as_uint(b.y));
+                    mma_tf32(ds[j], bg, __float_as_uint(b.z), __float_as_uint(b.w));
+                    mma_tf32(ds[j], sm, __float_as_uint(b.x), __float_as_uint(b.y));
                     mma_tf32(d[j], bg, __float_as_uint(b.x), __float_as_uint(b.y));
                 }
             }
 #pragma unroll
             for (int j = 0; j < NT; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) tot[j][e] += d[j][e];
+                for (int e = 0; e < 4; ++e) tot[j][e] += d[j][e] + ds[j][e];
             if (++c == nc) {
                 if (tile < tiles) {
 #pragma unroll
@@ -250,7 +259,16 @@ __global__ void __launch_bounds__(32 * kSkinnySumWarps, kSkinnySumCtas) skinny_s
     if (run >= g.runs) return;
     const int64_t k0 = run * g.run;
     const int64_t k1 = k0 + g.run < g.K ? k0 + g.run : g.K;
-    float tot[4][NT][4] = {};
+    // the FP64 totals: 16 fit the registers, 32 would be spilled
+    constexpr bool SM = NT > 1;
+    __shared__ double tsum[SM ? kSkinnySumWarps : 1][SM ? 16 * NT : 1][32];
+    double treg[SM ? 1 : 16];
+    auto tot = [&](int p, int j, int e) -> double& {
+        if constexpr (SM) return tsum[threadIdx.x >> 5][(p * NT + j) * 4 + e][lane];
+        else return treg[p * 4 + e];
+    };
+#pragma unroll
+    for (int i = 0; i < 16 * NT; ++i) tot(i / (4 * NT), i / 4 % NT, i % 4) = 0.0;
     Words w[2][2];
     float b[2][NT][2];
     const int64_t pitch = g.stride * Words::ESZ, left = g.M - e0;
@@ -304,7 +322,7 @@ __global__ void __launch_bounds__(32 * kSkinnySumWarps, kSkinnySumCtas) skinny_s
                 }
             }
         }
-        if (++held < 3 && k + 16 < k1) continue;  // 48 products in one hardware sum
+        if (++held < 3 && k + 16 < k1) continue;  // 48 lines in one hardware sum
         held = 0;
 #pragma unroll
         for (int p = 0; p < 4; ++p)
@@ -312,7 +330,7 @@ __global__ void __launch_bounds__(32 * kSkinnySumWarps, kSkinnySumCtas) skinny_s
             for (int j = 0; j < NT; ++j)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    tot[p][j][e] += d[p][j][e];
+                    tot(p, j, e) += (double)d[p][j][e];
                     d[p][j][e] = 0.0f;
                 }
     }
@@ -322,7 +340,8 @@ __global__ void __launch_bounds__(32 * kSkinnySumWarps, kSkinnySumCtas) skinny_s
         for (int j = 0; j < NT; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                skinny_store(g, run, e0 + Words::elem(q8, 2 * p + (e >> 1)), 8 * j + 2 * t + (e & 1), tot[p][j][e]);
+                skinny_store(g, run, e0 + Words::elem(q8, 2 * p + (e >> 1)), 8 * j + 2 * t + (e & 1),
+                             (float)tot(p, j, e));
 }
 
 template <Elem E, int NT, bool VECL>

@@ -256,6 +256,51 @@ def test_qr_past_the_plain_wide_columns(k, n, cond):
     np.testing.assert_allclose(Q.T @ Q, np.eye(n), atol=1e-8)
 
 
+def _exact_gram(X):
+    """(hi, lo, s): the Gram of X diag(s) (s powers of two, columns below 1) as
+    FP64 products of 19-bit slices, each exact over up to 2^14 rows."""
+    s = torch.ldexp(torch.ones_like(X[0]), -(torch.floor(torch.log2(X.abs().amax(0))) + 1).int())
+    Y, S = X * s, []
+    for i in range(1, 4):
+        S.append(torch.round(Y * 2.0 ** (19 * i)) / 2.0 ** (19 * i))
+        Y = Y - S[-1]
+    hi = torch.zeros(X.shape[1], X.shape[1], dtype=torch.float64, device="cuda")
+    lo = hi.clone()
+    for i, j in ((0, 0), (0, 1), (1, 0), (1, 1), (0, 2), (2, 0), (1, 2), (2, 1)):
+        p = S[i].t() @ S[j]
+        t = hi + p
+        b = t - hi
+        lo += (hi - (t - b)) + (p - b)
+        hi = t
+    return hi, lo, s
+
+
+@pytest.mark.parametrize("k,n", [(800, 200), (2000, 500), (4000, 1000), (8400, 2100), (4300, 2100), (2600, 2080)])
+def test_qr_error_is_householders(k, n):
+    """R against the exact Gram of the sketch: ||R^-T (SA^T SA - R^T R) R^-1||_F
+    stays at what blocked Householder steps leave (0.25 to 0.45 units of
+    rounding an entry), on the path each size and conditioning takes."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k + n)
+    SA = torch.randn(k, n, dtype=torch.float64, device="cuda", generator=g)
+    D = tb.Dense.create_strided(None, L.COL_MAJOR, NT.FP64, (k, n))
+    D.view()[...] = SA
+    R = torch.empty(n, n, dtype=torch.float64, device="cuda")
+    tb.generate_sketch_qr_precond(D, R_out=R)
+    R = R.t()  # written column-major
+    gh, gl, s = _exact_gram(SA)
+    rh, rl, rs = _exact_gram(R)
+    f = s / rs  # both Grams in units of s
+    diff = (gh - rh * f[:, None] * f) + (gl - rl * f[:, None] * f)
+    Ri = torch.linalg.inv(R * s)
+    err = torch.linalg.norm(Ri.t() @ diff @ Ri).item()
+    # the entries of a random E, and the n diagonal ones, whose sums are near 1;
+    # the inverse of a nearly square sketch amplifies both
+    rms = torch.linalg.norm(Ri * torch.linalg.norm(R * s, dim=0)[:, None]).item() / np.sqrt(n)
+    bound = (0.28 * n + 1.5 * np.sqrt(n)) * 2.0 ** -53 * max(1.0, (rms / 1.16) ** 2)
+    assert err <= bound, (err, bound)
+
+
 def test_qr_rejects_wide_and_singular():
     with pytest.raises(tb.TomosError):
         qr_on_gpu(np.ones((3, 5)))

@@ -784,7 +784,8 @@ __global__ void qr_mirror_lower_kernel(double* D, int64_t ldd, int64_t n) {
 template <bool KMAJOR>
 static tomos_status qr_gemm(const double* A, int64_t lda, const double* B, int64_t ldb, double* D,
                             int64_t ldd, int64_t M, int64_t N, int64_t K, double alpha, double beta,
-                            double* P, size_t pcap, cudaStream_t st, int sub = 0, bool upper = false) {
+                            double* P, size_t pcap, cudaStream_t st, int sub = 0, bool upper = false,
+                            int run = 0) {
     if (M <= 0 || N <= 0) return TOMOS_OK;
     const int64_t tm = (M + kGbm - 1) / kGbm, tn = (N + kGbn - 1) / kGbn;
     int64_t active = tm * tn;
@@ -795,7 +796,7 @@ static tomos_status qr_gemm(const double* A, int64_t lda, const double* B, int64
                 if (i * kGbm <= j * kGbn + kGbn - 1) ++active;
     }
     int64_t splits = 1;
-    if (P) {
+    if (P && run == 0) {
         const int64_t slots = 2 * (int64_t)sm_count(), tiles = active;
         int64_t kmax = K / (16 * kGbk);
         if (kmax > kGmaxSplits) kmax = kGmaxSplits;
@@ -832,6 +833,7 @@ static tomos_status qr_gemm(const double* A, int64_t lda, const double* B, int64
     g.beta = beta;
     g.sub = sub;
     g.upper = upper ? 1 : 0;
+    g.run = run;
     TOMOS_CUDA_TRY(cudaFuncSetAttribute(qr_gemm_kernel<KMAJOR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)kGemmSmem));
     qr_gemm_kernel<KMAJOR><<<dim3((unsigned)tm, (unsigned)tn, (unsigned)splits), 256, kGemmSmem, st>>>(g);
@@ -962,13 +964,17 @@ constexpr double kQrWideMaxKappa = 1e6;
 // stable where the Gram's Cholesky loses kappa_2 squared, so only a sketch
 // whose ||U^-1||_F is near that of orthonormal columns (sqrt(n); an RMS
 // inverse singular value of kQrWideRms at most, where a sketch of 4 n rows
-// has 1.15 and one of 2 n rows 1.41) keeps the wide path: there both leave
-// Q^T Q - I at a few units of rounding an entry (1.9e-13 against 1.3e-13 in
-// the Frobenius norm at 12000 x 3000).  The panel path's panels and blocks
-// took 22 ms there, most of it panel latency; the wide path takes 12 ms with
-// LAPACK's signs and 6.5 ms with rows of any sign.
+// has 1.15 and one of 2 n rows 1.41) keeps the wide path.  Its Gram is summed
+// there in runs of kQrWideRun rows (one chain over all rows was most of its
+// error), its diagonal in wide_diag_kernel's short chains.  With
+// E = R^-T (SA^T SA - R^T R) R^-1 from the exact Gram, ||E||_F is 3.8e-14 at
+// 12000 x 3000 (panel path 9.8e-14; 1.7e-13 in one chain), 3.1e-14 at 8400 x
+// 2100 (7.1e-14) and 5.5e-14 at 4300 x 2100 (1.04e-13).  The panel path's
+// panels and blocks took 24 ms at 12000 x 3000, most of it panel latency; the
+// wide path takes 12.5 ms with LAPACK's signs and 7.2 ms with rows of any sign.
 constexpr int64_t kQrWidePlainN = 2048;
 constexpr double kQrWideRms = 1.5;
+constexpr int kQrWideRun = 512;
 constexpr double kQrWideFloor = 1e-10;
 
 struct WideScratch {
@@ -1031,10 +1037,9 @@ __global__ void wide_colnorm_kernel(const double* G, int64_t n, double* d, int* 
 }
 
 // The diagonal of G = SA^T SA anew, a block a column: squares all add up, so
-// the matrix product's one chain over k rows left each with an error of
-// ~sqrt(k) units, most of that of Q^T Q - I.  Short chains a thread, then a
-// tree: 1.9e-13 in the Frobenius norm at 12000 x 3000 (3.0e-13 without; the
-// panel path 1.3e-13), for 70 us.
+// even a chain of kQrWideRun rows leaves an error of several units.  Short
+// chains a thread, then a tree: the largest entry of E 1.6e-15 at 12000 x 3000
+// (1.9e-15 without; the panel path 1.4e-15), for 70 us.
 __global__ void __launch_bounds__(256) wide_diag_kernel(const double* SA, int64_t ld, int64_t k, int64_t n, double* G) {
     __shared__ double sm[8];
     const double* x = SA + (size_t)blockIdx.x * ld;
@@ -1368,7 +1373,10 @@ __device__ void fact_next_diag(const FactArgs& a, int64_t p, double* sm) {
 // tiles first, first + step, ..  Eight warps of 16 x 32 entries on the FP64
 // tensor cores; the next tile's panels and entries are loaded while the
 // current tile is formed (a tile of 32 alone, its loads exposed and its
-// panels formed anew, left 12000 x 3000 at 6.4 ms of factorisation).
+// panels formed anew, left 12000 x 3000 at 6.4 ms of factorisation).  A tile's
+// product is summed from zero and subtracted once: summed onto the entry, each
+// of its 32 terms is rounded at the entry's size, which on the diagonal (near
+// 1) was most of R's error: ||E||_F 2.9e-14 at 4000 x 1000, 4.5e-14 that way.
 constexpr int kFactTile = 64;
 constexpr int kFactPitch = kFactTile + 4;  // 16 lanes of a fragment read on 16 banks
 
@@ -1414,19 +1422,22 @@ __device__ void fact_trailing(const FactArgs& a, int64_t p, int64_t first, int64
     };
     if (first < total) fetch(first);
     for (int64_t tau = first; tau < total; tau += step) {
-        double acc[4][4];
+        double acc[4][4], old[16];
         const int64_t i0 = I0, j0 = J0;
         __syncthreads();  // the previous tile's fragments are read
         {
             const int i = t & 63, k0 = t >> 6;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                Ls[k0 + 4 * u][i] = -lv[u];
+                Ls[k0 + 4 * u][i] = lv[u];
                 Rs[k0 + 4 * u][i] = rv[u];
             }
         }
 #pragma unroll
-        for (int e = 0; e < 16; ++e) acc[e >> 2][e & 3] = cv[e];
+        for (int e = 0; e < 16; ++e) {
+            old[e] = cv[e];
+            acc[e >> 2][e & 3] = 0.0;
+        }
         if (tau + step < total) fetch(tau + step);
         __syncthreads();
 #pragma unroll
@@ -1444,7 +1455,7 @@ __device__ void fact_trailing(const FactArgs& a, int64_t p, int64_t first, int64
         for (int e = 0; e < 16; ++e) {
             const int64_t row = i0 + wm + g + 8 * ((e >> 1) & 1), col = j0 + wn + 8 * (e >> 2) + 2 * q + (e & 1);
             const bool next = row < t0 + kHB && col < t0 + kHB;  // CTA 0's
-            if (row < n && col < n && !next) a.M[(size_t)col * n + row] = acc[e >> 2][e & 3];
+            if (row < n && col < n && !next) a.M[(size_t)col * n + row] = old[e] - acc[e >> 2][e & 3];
         }
     }
     __syncthreads();
@@ -1513,7 +1524,8 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     *done = false;
     TOMOS_CUDA_TRY(cudaMemsetAsync(w.flag, 0, sizeof(int) * 4, st));
     // the Gram S^T S: its upper triangle, mirrored
-    tomos_status s = qr_gemm<true>(SA, ld, SA, ld, w.G, n, n, n, k, 1.0, 0.0, w.P, w.pcap, st, 0, true);
+    tomos_status s = qr_gemm<true>(SA, ld, SA, ld, w.G, n, n, n, k, 1.0, 0.0, w.P, w.pcap, st, 0, true,
+                                 n > kQrWidePlainN ? kQrWideRun / kGbk : 0);
     if (s) return s;
     const unsigned eb = (unsigned)((n * n + 255) / 256 < 4096 ? (n * n + 255) / 256 : 4096);
     if (n > kQrWidePlainN) {

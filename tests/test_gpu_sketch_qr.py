@@ -256,6 +256,38 @@ def test_qr_past_the_plain_wide_columns(k, n, cond):
     np.testing.assert_allclose(Q.T @ Q, np.eye(n), atol=1e-8)
 
 
+@pytest.mark.timeout(300)
+def test_which_path_serves_past_the_plain_wide_columns():
+    """TOMOS_QR_WIDE=3 turns the wide path's refusal into an error: of the
+    8400 x 2100 sketches it serves the one of independent columns and refuses
+    those with a common part in all columns (RMS 1.55, its diagonal's part
+    1.44: after the inverse) or a column almost repeated (at its pivot, early
+    or late)."""
+    import subprocess
+    import sys
+    code = (
+        "import numpy as np, sys\n"
+        "sys.path.insert(0, %r)\n"
+        "import tomos_b200 as tb\n"
+        "from test_gpu_sketch_qr import qr_on_gpu\n"
+        "for k, n, col in ((8400, 2100, 0), (8400, 2100, -1), (8400, 2100, 1900), (8400, 2100, 20), (8400, 2100, 2099)):\n"
+        "    rng = np.random.default_rng(k + n)\n"
+        "    SA = rng.standard_normal((k, n)) * np.logspace(0, 2, n)\n"
+        "    if col < 0:\n"
+        "        SA += np.sqrt(0.8) * rng.standard_normal((k, 1)) * np.logspace(0, 2, n)\n"
+        "    elif col:\n"
+        "        SA[:, col] = SA[:, 10] + SA[:, col] / 1e5\n"
+        "    try:\n"
+        "        qr_on_gpu(SA)\n"
+        "        print('wide', end=' ')\n"
+        "    except tb.TomosError as e:\n"
+        "        assert 'wide path refused' in str(e), e\n"
+        "        print('panel', end=' ')\n" % os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                       env=dict(os.environ, TOMOS_QR_WIDE="3"), timeout=280)
+    assert r.stdout.split() == ["wide", "panel", "panel", "panel", "panel"], (r.stdout, r.stderr[-3000:])
+
+
 def _exact_gram(X):
     """(hi, lo, s): the Gram of X diag(s) (s powers of two, columns below 1) as
     FP64 products of 19-bit slices, each exact over up to 2^14 rows."""

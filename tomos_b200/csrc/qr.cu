@@ -964,7 +964,11 @@ constexpr double kQrWideMaxKappa = 1e6;
 // stable where the Gram's Cholesky loses kappa_2 squared, so only a sketch
 // whose ||U^-1||_F is near that of orthonormal columns (sqrt(n); an RMS
 // inverse singular value of kQrWideRms at most, where a sketch of 4 n rows
-// has 1.15 and one of 2 n rows 1.41) keeps the wide path.  Its Gram is summed
+// has 1.15 and one of 2 n rows 1.41; below 1.8 n rows none is tried) keeps the
+// wide path.  A refused sketch pays the Gram and the Cholesky up to the block
+// column where the sum of 1 / u_jj^2 passes the bound, before the panel path:
+// 13.7 to 14.6 ms at 8400 x 2100, 12.6 ms without (14.9 ms with the inverse);
+// 27.3 to 28.9 ms at 12000 x 3000 (24.1 ms).  The wide path's Gram is summed
 // there in runs of kQrWideRun rows (one chain over all rows was most of its
 // error), its diagonal in wide_diag_kernel's short chains.  With
 // E = R^-T (SA^T SA - R^T R) R^-1 from the exact Gram, ||E||_F is 3.8e-14 at
@@ -985,11 +989,11 @@ struct WideScratch {
     double* sgn;   // n: S
     double* Xd;    // 2 x 2 x 32 x 32: a diagonal block's inverse factors (by block parity)
     double* pan;   // 2 x 32 x n: LU panels
-    double* kap;   // ||U^-1||_F^2
+    double* kap;   // [0] ||U^-1||_F^2, [1] its diagonal's part
     double* Tb;    // trtri level products
     double* P;     // GEMM split-K partials
     size_t pcap;
-    int* flag;     // [0] a Cholesky pivot failed or d_j == 0
+    int* flag;     // [0] the Cholesky ended early or d_j == 0, [1] 1 + the block column it ended at
     GridSync* gs;
     size_t bytes;
 };
@@ -1128,7 +1132,9 @@ struct FactArgs {
     double* sgn;
     int64_t keep;   // LU: the column dlarfg leaves as the identity, or -1
     double floor;
-    int* fail;
+    int* fail;      // [0] set when a pivot or the sum below ends the Cholesky, [1] 1 + that block column
+    double* inv2;   // Cholesky: sum of 1 / u_jj^2 so far (at most ||U^-1||_F^2)
+    double inv2_max;
     GridSync* gs;
 };
 
@@ -1210,7 +1216,17 @@ __device__ void fact_diag(const FactArgs& a, int64_t p, double* sm, bool in_smem
     __shared__ double dinv[kHB];
     if (a.mode == 0) {
         const bool ok = cta_chol_inv(B, R, X, a.floor, &okf);
-        if (!ok && t == 0) atomicExch(a.fail, 1);
+        if (t < 32) {
+            const double s = warp_sum(t < nb ? X[t][t] * X[t][t] : 0.0);
+            if (t == 0) {
+                const double sum = p == 0 ? s : *a.inv2 + s;
+                *a.inv2 = sum;
+                if (!ok || !(sum <= a.inv2_max)) {  // refused: every CTA leaves at block column p
+                    atomicExch(a.fail, 1);
+                    if (a.fail[1] == 0) atomicExch(a.fail + 1, (int)p + 1);
+                }
+            }
+        }
         for (int e = t; e < kHB * kHB; e += blockDim.x) {
             const int r = e >> 5, c = e & 31;
             if (r < nb && c < nb) a.Ur[(size_t)(jb + r) * n + jb + c] = r <= c ? R[r][c] : 0.0;
@@ -1472,6 +1488,11 @@ __global__ void __launch_bounds__(kQrThreads, 1) fact_kernel(FactArgs a) {
     if (blockIdx.x == 0) fact_diag(a, 0, fsm, false);
     if (!grid_sync(a.gs, gen, &sflag)) return;
     for (int64_t p = 0; p + 1 < np; ++p) {
+        if (a.mode == 0) {
+            // CTA 0 writes p + 2 at the earliest while others read it here
+            const int stop = __ldcg(a.fail + 1);
+            if (stop != 0 && stop - 1 <= p) return;
+        }
         const int64_t nt = (n - (p + 1) * kHB + kHB - 1) / kHB;
         const int64_t panels = a.mode == 0 ? nt : 2 * nt;
         if (blockIdx.x == 0 && G > 1) {
@@ -1547,9 +1568,22 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     fa.keep = -1;
     fa.floor = kQrWideFloor;
     fa.fail = w.flag;
+    fa.inv2 = w.kap + 1;
+    const double kmax = n > kQrWidePlainN ? kQrWideRms * (double)n : kQrWideMaxKappa;
+    fa.inv2_max = kmax * kmax / (double)n;  // ||U^-1||_F^2 where kappa_F(U) = kmax
     fa.gs = w.gs;
     s = launch_fact(fa, w.gs, st);
     if (s) return s;
+    int flag = 0;
+    GridSync gsh[2] = {};
+    if (n > kQrWidePlainN) {
+        // a large inverse is not begun for a sketch that is refused already
+        TOMOS_CUDA_TRY(cudaMemcpyAsync(&flag, w.flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        TOMOS_CUDA_TRY(cudaMemcpyAsync(gsh, w.gs, sizeof(gsh), cudaMemcpyDeviceToHost, st));
+        TOMOS_CUDA_TRY(cudaStreamSynchronize(st));
+        if (gsh[0].err || gsh[1].err) return fail(TOMOS_ERR_CUDA, "sketch_qr: a bounded grid barrier wait expired");
+        if (flag) return TOMOS_OK;
+    }
     s = trtri_rt(w.Ur, n, w.X, n, w.Tb, w.P, w.pcap, st);
     if (s) return s;
     {
@@ -1560,16 +1594,13 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
         wide_fro2_sum_kernel<<<1, 32, 0, st>>>(w.P, np, w.kap);
         TOMOS_LAUNCH_CHECK("wide_fro2_sum_kernel");
     }
-    int flag = 0;
     double kap2 = 0.0;
-    GridSync gsh[2] = {};
     TOMOS_CUDA_TRY(cudaMemcpyAsync(&flag, w.flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     TOMOS_CUDA_TRY(cudaMemcpyAsync(&kap2, w.kap, sizeof(double), cudaMemcpyDeviceToHost, st));
     TOMOS_CUDA_TRY(cudaMemcpyAsync(gsh, w.gs, sizeof(gsh), cudaMemcpyDeviceToHost, st));
     TOMOS_CUDA_TRY(cudaStreamSynchronize(st));
     if (gsh[0].err || gsh[1].err) return fail(TOMOS_ERR_CUDA, "sketch_qr: a bounded grid barrier wait expired");
     const double kappa = std::sqrt((double)n * kap2);
-    const double kmax = n > kQrWidePlainN ? kQrWideRms * (double)n : kQrWideMaxKappa;
     if (flag || !(kappa <= kmax)) return TOMOS_OK;  // the panel path takes over
     wide_row_scale_kernel<<<eb, 256, 0, st>>>(w.X, n, w.d);
     TOMOS_LAUNCH_CHECK("wide_row_scale_kernel");
@@ -1595,7 +1626,8 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     return TOMOS_OK;
 }
 
-// Whether the wide path is tried: n from 64 to kQrWideMaxN columns.
+// Whether the wide path is tried: n from 64 to kQrWideMaxN columns, of a
+// sketch of at least 1.8 n rows past kQrWidePlainN.
 // TOMOS_QR_WIDE=0 turns it off, =1 tries it at every size up to the max,
 // =3 requires it there (a sketch it refuses is then an error; for tests).
 static int qr_wide_mode() {
@@ -1607,9 +1639,10 @@ static int qr_wide_mode() {
     return mode;
 }
 
-static bool qr_wide_used(int64_t n) {
+static bool qr_wide_used(int64_t k, int64_t n) {
     const int mode = qr_wide_mode();
     if (mode == 0 || n > kQrWideMaxN) return false;
+    if (n > kQrWidePlainN && 5 * k < 9 * n) return false;  // see kQrWideRms
     return mode == 1 || mode == 3 ? n >= 1 : n >= 64;
 }
 
@@ -1622,7 +1655,7 @@ extern "C" {
 size_t tomos_sketch_qr_scratch_bytes(int64_t k, int64_t n) {
     if (k < 0 || n < 0) return 0;
     const size_t panel = qr_layout(nullptr, k, n).bytes;
-    return qr_wide_used(n) ? panel + wide_layout(nullptr, n).bytes : panel;
+    return qr_wide_used(k, n) ? panel + wide_layout(nullptr, n).bytes : panel;
 }
 
 tomos_status tomos_sketch_qr_precond_ex_f64(int64_t k, int64_t n, double* SA, int64_t ld, double* R,
@@ -1640,7 +1673,7 @@ tomos_status tomos_sketch_qr_precond_ex_f64(int64_t k, int64_t n, double* SA, in
                     "sketch_qr: scratch too small (need " + std::to_string(need.bytes) + " bytes)");
     QrScratch q = qr_layout(scratch, k, n);
     cudaStream_t st = as_stream(stream);
-    if (qr_wide_used(n) && scratch_bytes >= need.bytes + wide_layout(nullptr, n).bytes) {
+    if (qr_wide_used(k, n) && scratch_bytes >= need.bytes + wide_layout(nullptr, n).bytes) {
         bool done = false;
         tomos_status ws = qr_wide(k, n, SA, ld, R, wide_layout(static_cast<char*>(scratch) + need.bytes, n),
                                   st, &done, (flags & TOMOS_QR_ANY_SIGNS) != 0);

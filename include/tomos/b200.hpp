@@ -395,8 +395,12 @@ inline void generate_sketch_qr_precond(Dense& sketched_mtx) {
         throw std::runtime_error("generate_sketch_qr_precond: FP64 column-major only");
     std::size_t nb = tomos_sketch_qr_scratch_bytes(d.rows, d.cols);
     void* scratch = nullptr;
-    if (cudaMalloc(&scratch, nb ? nb : 4) != cudaSuccess)
-        throw std::runtime_error("generate_sketch_qr_precond: scratch allocation");
+    if (cudaMalloc(&scratch, nb ? nb : 4) != cudaSuccess) {
+        cudaGetLastError();
+        nb = tomos_sketch_qr_min_scratch_bytes(d.rows, d.cols);
+        if (cudaMalloc(&scratch, nb ? nb : 4) != cudaSuccess)
+            throw std::runtime_error("generate_sketch_qr_precond: scratch allocation");
+    }
     tomos_status s = tomos_sketch_qr_precond_f64(d.rows, d.cols, static_cast<double*>(d.values),
                                                  d.ld, nullptr, scratch, nb, nullptr);
     cudaStreamSynchronize(nullptr);

@@ -291,8 +291,11 @@ tomos_status tomos_countsketch_apply_shard(const tomos_dense* A, int32_t tier, i
  * R^{-1} (upper triangular, zeros below), exactly the contract of
  * generate_sketch_qr_precond (src/core/precond/sketch_qr.hpp:19,
  * sketch_qr.cpp:38-64: geqrf + trtri).  R (device, may be NULL, n x n
- * column-major, ld n) receives R itself. */
+ * column-major, ld n) receives R itself.  tomos_sketch_qr_scratch_bytes is
+ * what the fastest path for k x n uses; from tomos_sketch_qr_min_scratch_bytes
+ * on, a smaller scratch takes the panel path. */
 size_t tomos_sketch_qr_scratch_bytes(int64_t k, int64_t n);
+size_t tomos_sketch_qr_min_scratch_bytes(int64_t k, int64_t n);
 tomos_status tomos_sketch_qr_precond_f64(int64_t k, int64_t n, double* SA, int64_t ld,
                                          double* R, void* scratch,
                                          size_t scratch_bytes, void* stream);

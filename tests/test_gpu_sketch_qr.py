@@ -288,6 +288,27 @@ def test_which_path_serves_past_the_plain_wide_columns():
     assert r.stdout.split() == ["wide", "panel", "panel", "panel", "panel"], (r.stdout, r.stderr[-3000:])
 
 
+@pytest.mark.parametrize("k,n", [(1200, 300), (6000, 3000)])
+def test_qr_with_little_memory(monkeypatch, k, n):
+    """Where the wide path's scratch cannot be had, the panel path's serves."""
+    rng = np.random.default_rng(n)
+    SA = rng.standard_normal((k, n))
+    asked = []
+    scratch = tb._scratch
+
+    def short(nbytes, stream):
+        asked.append(nbytes)
+        if len(asked) == 1:
+            raise torch.OutOfMemoryError("short of memory")
+        return scratch(nbytes, stream)
+
+    monkeypatch.setattr(tb, "_scratch", short)
+    _, R = qr_on_gpu(SA)
+    assert len(asked) == 2 and asked[1] < asked[0]
+    Rl = np.linalg.qr(SA, mode="r")
+    np.testing.assert_allclose(R, Rl, rtol=1e-8, atol=1e-9 * np.abs(Rl).max())
+
+
 def _exact_gram(X):
     """(hi, lo, s): the Gram of X diag(s) (s powers of two, columns below 1) as
     FP64 products of 19-bit slices, each exact over up to 2^14 rows."""

@@ -624,7 +624,14 @@ def generate_sketch_qr_precond(sketched, R_out=None, copy=True, any_signs=False,
                          "generate_sketch_qr_precond: sketched_mtx must have at least as many "
                          "rows as columns (k >= n).")
     nb = C.lib().tomos_sketch_qr_scratch_bytes(k, n)
-    scratch = _scratch(nb, stream)
+    try:
+        scratch = _scratch(nb, stream)
+    except torch.OutOfMemoryError:  # a few n x n planes: the panel path needs less
+        least = C.lib().tomos_sketch_qr_min_scratch_bytes(k, n)
+        if least >= nb:
+            raise
+        nb = least
+        scratch = _scratch(nb, stream)
     C.check(C.lib().tomos_sketch_qr_precond_ex_f64(k, n, _ptr(sketched.storage), sketched.ld, _ptr(R_out),
                                                    C.TOMOS_QR_ANY_SIGNS if any_signs else 0, _ptr(scratch),
                                                    nb, _stream(stream)),

@@ -120,6 +120,7 @@ SIGNATURES = {
     "tomos_countsketch_apply_csr": (c_i32, [ctypes.POINTER(CsrDesc), c_i32, c_i64, c_u64, c_u64,
                                             c_vp, c_i64, c_vp, c_vp, c_vp, c_sz, c_vp]),
     "tomos_sketch_qr_scratch_bytes": (c_sz, [c_i64, c_i64]),
+    "tomos_sketch_qr_min_scratch_bytes": (c_sz, [c_i64, c_i64]),
     "tomos_sketch_qr_precond_f64": (c_i32, [c_i64, c_i64, c_vp, c_i64, c_vp, c_vp, c_sz, c_vp]),
     "tomos_sketch_qr_precond_ex_f64": (c_i32, [c_i64, c_i64, c_vp, c_i64, c_vp, c_i32, c_vp, c_sz, c_vp]),
     "tomos_column_scale": (c_i32, [c_vp, c_i64, c_vp, c_vp, c_vp]),

@@ -1652,10 +1652,16 @@ using namespace tomos_b200;
 
 extern "C" {
 
-size_t tomos_sketch_qr_scratch_bytes(int64_t k, int64_t n) {
+size_t tomos_sketch_qr_min_scratch_bytes(int64_t k, int64_t n) {
     if (k < 0 || n < 0) return 0;
-    const size_t panel = qr_layout(nullptr, k, n).bytes;
-    return qr_wide_used(k, n) ? panel + wide_layout(nullptr, n).bytes : panel;
+    return qr_layout(nullptr, k, n).bytes;
+}
+
+size_t tomos_sketch_qr_scratch_bytes(int64_t k, int64_t n) {
+    const size_t panel = tomos_sketch_qr_min_scratch_bytes(k, n);
+    if (k < 0 || n < 0 || !qr_wide_used(k, n)) return panel;
+    const size_t wide = wide_layout(nullptr, n).bytes;  // one path after the other uses the scratch
+    return wide > panel ? wide : panel;
 }
 
 tomos_status tomos_sketch_qr_precond_ex_f64(int64_t k, int64_t n, double* SA, int64_t ld, double* R,
@@ -1673,10 +1679,10 @@ tomos_status tomos_sketch_qr_precond_ex_f64(int64_t k, int64_t n, double* SA, in
                     "sketch_qr: scratch too small (need " + std::to_string(need.bytes) + " bytes)");
     QrScratch q = qr_layout(scratch, k, n);
     cudaStream_t st = as_stream(stream);
-    if (qr_wide_used(k, n) && scratch_bytes >= need.bytes + wide_layout(nullptr, n).bytes) {
+    if (qr_wide_used(k, n) && scratch_bytes >= wide_layout(nullptr, n).bytes) {
         bool done = false;
-        tomos_status ws = qr_wide(k, n, SA, ld, R, wide_layout(static_cast<char*>(scratch) + need.bytes, n),
-                                  st, &done, (flags & TOMOS_QR_ANY_SIGNS) != 0);
+        tomos_status ws = qr_wide(k, n, SA, ld, R, wide_layout(scratch, n), st, &done,
+                                  (flags & TOMOS_QR_ANY_SIGNS) != 0);
         if (ws) return ws;
         if (done) return TOMOS_OK;
         if (qr_wide_mode() == 3)

@@ -289,3 +289,15 @@ def test_mm_few_columns_nan(bits):
                     tb.Dense.from_tensor(B, L.COL_MAJOR), 0.0, C)
         bad = torch.isnan(C.view())
         assert bad[row].all() and bad.sum().item() == 9
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 200, 1024), (512, 512, 4096), (1000, 1000, 900), (200, 40, 4096),
+                                   (40, 33, 50000)])
+def test_mm_split_sums(orc, M, N, K):
+    """Split products whose partials are few (a thread an entry; more than
+    eight of them with many entries) and many (warps an entry)."""
+    rng = np.random.default_rng(M + K)
+    A0 = rng.standard_normal((M, K)).astype(np.float32)
+    A = to_dense(A0, L.ROW_MAJOR)
+    for lc, beta in ((L.COL_MAJOR, 0.0), (L.ROW_MAJOR, -0.5)):
+        check(orc, A, A0, tb.Tier.AUTO, T.NO_TRANSPOSE, T.NO_TRANSPOSE, (K, N), (L.COL_MAJOR, lc), beta, rng)

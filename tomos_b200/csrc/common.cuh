@@ -219,6 +219,30 @@ enum class Elem : int {
                    // plane, control words already decoded)
 };
 
+// How partial sums are added up: a thread an entry where there are few of
+// them, or entries enough to fill the GPU; several warps an entry otherwise.
+// One warp for 32 entries of a few partials is a CTA of almost no work: 1e6
+// entries of one partial took 20 us that way, 6 us with a thread an entry.
+__host__ __device__ inline bool few_parts(int64_t nparts, int64_t entries) {
+    return nparts <= 8 || (nparts <= 32 && entries >= 32768);
+}
+
+// sum over c < nparts of part[c stride], in order, eight loads in flight.
+template <typename Acc>
+__device__ __forceinline__ double sum_few(const Acc* __restrict__ part, int64_t nparts, int64_t stride) {
+    double s = 0.0;
+    int64_t c = 0;
+    for (; c + 8 <= nparts; c += 8) {
+        Acc v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = part[(size_t)(c + u) * stride];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += (double)v[u];
+    }
+    for (; c < nparts; ++c) s += (double)part[(size_t)c * stride];
+    return s;
+}
+
 // Scalar element decode at flat index idx (generic kernels), branch-free so
 // that the loads of an unrolled batch stay in flight together.
 template <Elem E>

@@ -1487,6 +1487,18 @@ __global__ void __launch_bounds__(1024) gemm_split_reduce_kernel(const float* __
     *p = (float)y;
 }
 
+// Few splits: a thread an entry.
+__global__ void __launch_bounds__(256) gemm_few_splits_kernel(const float* __restrict__ part, int splits, int64_t M,
+                                                              int64_t N, double alpha, double beta, float* c,
+                                                              int64_t si, int64_t sj) {
+    const int64_t total = M * N, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    float* p = c + (size_t)((t % M) * si + (t / M) * sj);
+    double y = alpha * sum_few(part + t, splits, total);
+    if (beta != 0.0) y += beta * (double)*p;
+    *p = (float)y;
+}
+
 // Products of at most 16 columns with an exactly read A (gemm_skinny.cuh).
 tomos_status launch_skinny_e(Elem e, const GemmArgs& g, int64_t run, int64_t runs, cudaStream_t st) {
     SkinnyArgs a;
@@ -1717,6 +1729,12 @@ tomos_status tomos_mm_ex(int32_t trans_a, int32_t trans_b, double alpha, const t
             }
     }
     if (s || splits == 1) return s;
+    if (few_parts(splits, g.M * g.N)) {
+        gemm_few_splits_kernel<<<(unsigned)((g.M * g.N + 255) / 256), 256, 0, st>>>(g.part, splits, g.M, g.N, alpha,
+                                                                                    beta, g.c, g.c_si, g.c_sj);
+        TOMOS_LAUNCH_CHECK("gemm_few_splits_kernel");
+        return TOMOS_OK;
+    }
     const int warps = splits >= 256 ? 32 : (splits + 7) / 8;
     gemm_split_reduce_kernel<<<(unsigned)((g.M * g.N + 31) / 32), 32 * warps, 0, st>>>(g.part, splits, g.M, g.N, alpha,
                                                                                        beta, g.c, g.c_si, g.c_sj);

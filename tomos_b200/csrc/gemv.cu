@@ -243,12 +243,32 @@ __global__ void __launch_bounds__(1024) sum_parts_kernel(const Acc* __restrict__
     y[j] = (float)r;
 }
 
+// Few partials: a thread a column.
+template <typename Acc>
+__global__ void __launch_bounds__(256) sum_few_parts_kernel(const Acc* __restrict__ part, int64_t nparts,
+                                                            int64_t stride, int64_t n, double alpha, double beta,
+                                                            const double* coef, const int* skip,
+                                                            float* __restrict__ y) {
+    if (skip && *skip) return;
+    resolve_coef(coef, alpha, beta);
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    double r = alpha * sum_few(part + j, nparts, stride);
+    if (beta != 0.0) r += beta * (double)y[j];
+    y[j] = (float)r;
+}
+
 template <typename Acc>
 static tomos_status sum_parts(const Acc* part, int64_t nparts, int64_t stride, int64_t n, double alpha,
                               double beta, const double* coef, const int* skip, float* y, cudaStream_t st) {
+    if (few_parts(nparts, n)) {
+        sum_few_parts_kernel<Acc><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, nparts, stride, n, alpha, beta,
+                                                                               coef, skip, y);
+        TOMOS_LAUNCH_CHECK("sum_few_parts_kernel");
+        return TOMOS_OK;
+    }
     int64_t warps = (nparts + 7) / 8;
     if (warps > 32) warps = 32;
-    if (warps < 1) warps = 1;
     sum_parts_kernel<Acc><<<(unsigned)((n + 31) / 32), (unsigned)warps * 32, 0, st>>>(part, nparts, stride, n, alpha,
                                                                                      beta, coef, skip, y);
     TOMOS_LAUNCH_CHECK("sum_parts_kernel");
@@ -329,13 +349,18 @@ static tomos_status run_gemv_v(const GemvLaunch& L, cudaStream_t st) {
     return sum_parts(partial, nchunks, L.inner, L.inner, L.alpha, L.beta, L.coef, L.skip, L.y, st);
 }
 
-// 16-byte loads where every line starts on a 16-byte boundary.
+// 16-byte loads where every line starts on a 16-byte boundary; sums of few
+// lines (kVecSumLines) take an element a thread, which leaves more threads than
+// a chunk each: 1e6 x 16 bf16, exact, 26 us in chunks, 18 us.
+constexpr int64_t kVecSumLines = 128;
+
 template <Elem E, bool ACC64>
 static tomos_status run_gemv(const GemvLaunch& L, cudaStream_t st) {
     constexpr bool TWO = E == Elem::A16 || E == Elem::AB16 || E == Elem::AB16R;
     const int esz = E == Elem::F32 ? 4 : 2;
     const bool vec = (L.ld * esz) % 16 == 0 && reinterpret_cast<uintptr_t>(L.hi) % 16 == 0 &&
-                     (!TWO || reinterpret_cast<uintptr_t>(L.lo) % 16 == 0);
+                     (!TWO || reinterpret_cast<uintptr_t>(L.lo) % 16 == 0) &&
+                     (L.dot || L.outer >= kVecSumLines);
     return vec ? run_gemv_v<E, ACC64, ChunkElems<E>::value>(L, st) : run_gemv_v<E, ACC64, 1>(L, st);
 }
 

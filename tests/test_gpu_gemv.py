@@ -55,7 +55,8 @@ def test_gemv_vs_fp64(orc, numeric, tier, rounded, layout, shape):
 @pytest.mark.parametrize("numeric,tier,rounded", CASES + [(NT.FP16, tb.Tier.AUTO, False)])
 @pytest.mark.parametrize("m,n,pad", [(5001, 9, 0), (3, 64, 0), (4999, 256, 0), (17, 258, 0), (2049, 65, 0),
                                      (1501, 777, 0), (700, 1025, 0), (40003, 7, 1), (8200, 600, 4),
-                                     (33000, 100, 0), (2000, 127, 0), (2000, 128, 0)])
+                                     (33000, 100, 0), (2000, 127, 0), (2000, 128, 0), (24001, 65, 0),
+                                     (10001, 64, 0), (40011, 513, 0), (23, 999, 0), (25, 999, 0)])
 @pytest.mark.parametrize("layout", [L.ROW_MAJOR, L.COL_MAJOR])
 def test_gemv_line_shapes(orc, numeric, tier, rounded, m, n, pad, layout):
     """Narrow and unaligned lines (the direct pass), few long lines (a CTA a

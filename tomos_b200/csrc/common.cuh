@@ -296,6 +296,28 @@ __device__ __forceinline__ float word_value(uint32_t h, uint32_t r) {
     else return decode_fp32_bf16_exact(h, r, E == Elem::AB16R);
 }
 
+// The elements at flat indices idx + u step.  HALF-tier control words are
+// rare: all words are loaded first, then one branch decodes them for all U.
+template <Elem E, int U>
+__device__ __forceinline__ void load_elems(const void* p, const void* q, size_t idx, size_t step, float (&v)[U]) {
+    if constexpr (E == Elem::H16) {
+        uint32_t h[U], any = 0u;
+#pragma unroll
+        for (int u = 0; u < U; ++u) h[u] = __ldg(static_cast<const uint16_t*>(p) + idx + u * step);
+#pragma unroll
+        for (int u = 0; u < U; ++u) any |= h[u];
+        if (any & 1u) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) h[u] = half_only_bits_nb(h[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = half_bits_to_float(h[u]);
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = load_elem<E>(p, q, idx + u * step);
+    }
+}
+
 // Resolves a tomos_dense + tier to the element tag it is read as.
 // Returns false (with a message) if the combination has no kernel, the
 // reference's "no kernel registered" contract.

@@ -43,19 +43,24 @@ __device__ __forceinline__ void resolve_coef(const double* coef, double& alpha, 
     }
 }
 
-// V consecutive elements at flat index idx as floats: V = ChunkElems (one
-// 16-byte load a plane, idx 16-byte aligned) or 1.
-template <Elem E, int V>
-__device__ __forceinline__ void load_chunk(const void* hi, const void* lo, size_t idx, float* f) {
+// V consecutive elements at each of the flat indices idx + u step as floats:
+// V = ChunkElems (one 16-byte load a plane, aligned) or 1.
+template <Elem E, int V, int U>
+__device__ __forceinline__ void load_chunks(const void* hi, const void* lo, size_t idx, size_t step, float (&f)[U][V]) {
     if constexpr (V == 1) {
-        f[0] = load_elem<E>(hi, lo, idx);
+        float v[U];
+        load_elems<E, U>(hi, lo, idx, step, v);
+#pragma unroll
+        for (int u = 0; u < U; ++u) f[u][0] = v[u];
     } else {
         FusedParams P;
         P.hi = hi;
         P.lo = lo;
-        uint4 h, l;
-        ChunkDecoder<E>::load(P, idx, h, l);
-        ChunkDecoder<E>::decode(h, l, f);
+        uint4 h[U], l[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) ChunkDecoder<E>::load(P, idx + u * step, h[u], l[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) ChunkDecoder<E>::decode(h[u], l[u], f[u]);
     }
 }
 
@@ -78,10 +83,19 @@ __global__ void __launch_bounds__(256) line_dot_kernel(const void* __restrict__ 
         Acc a0 = 0, a1 = 0, a2 = 0, a3 = 0;
         int64_t i = lane;
         for (; i + 96 < inner; i += 128) {
-            a0 += (Acc)load_elem<E>(hi, lo, base + i) * (Acc)__ldg(x + i);
-            a1 += (Acc)load_elem<E>(hi, lo, base + i + 32) * (Acc)__ldg(x + i + 32);
-            a2 += (Acc)load_elem<E>(hi, lo, base + i + 64) * (Acc)__ldg(x + i + 64);
-            a3 += (Acc)load_elem<E>(hi, lo, base + i + 96) * (Acc)__ldg(x + i + 96);
+            if constexpr (E == Elem::H16) {
+                float v[4];
+                load_elems<E, 4>(hi, lo, base + i, 32, v);
+                a0 += (Acc)v[0] * (Acc)__ldg(x + i);
+                a1 += (Acc)v[1] * (Acc)__ldg(x + i + 32);
+                a2 += (Acc)v[2] * (Acc)__ldg(x + i + 64);
+                a3 += (Acc)v[3] * (Acc)__ldg(x + i + 96);
+            } else {
+                a0 += (Acc)load_elem<E>(hi, lo, base + i) * (Acc)__ldg(x + i);
+                a1 += (Acc)load_elem<E>(hi, lo, base + i + 32) * (Acc)__ldg(x + i + 32);
+                a2 += (Acc)load_elem<E>(hi, lo, base + i + 64) * (Acc)__ldg(x + i + 64);
+                a3 += (Acc)load_elem<E>(hi, lo, base + i + 96) * (Acc)__ldg(x + i + 96);
+            }
         }
         for (; i < inner; i += 32) a0 += (Acc)load_elem<E>(hi, lo, base + i) * (Acc)__ldg(x + i);
         Acc acc = warp_sum((a0 + a1) + (a2 + a3));
@@ -132,16 +146,15 @@ __global__ void __launch_bounds__(256) line_dot_seg_kernel(const void* __restric
     };
     for (; i + 3 * 256 * V + V <= i1; i += 4 * 256 * V) {
         float f[4][V];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) load_chunk<E, V>(hi, lo, base + i + u * 256 * V, f[u]);
+        load_chunks<E, V, 4>(hi, lo, base + i, 256 * V, f);
 #pragma unroll
         for (int u = 0; u < 4; ++u) step(i + u * 256 * V, a[u], f[u]);
     }
     for (; i < i1; i += 256 * V) {
         if (i + V <= i1) {
-            float f[V];
-            load_chunk<E, V>(hi, lo, base + i, f);
-            step(i, a[0], f);
+            float f[1][V];
+            load_chunks<E, V, 1>(hi, lo, base + i, 0, f);
+            step(i, a[0], f[0]);
         } else {
             for (int64_t k = i; k < i1; ++k) a[0] += (Acc)load_elem<E>(hi, lo, base + k) * (Acc)__ldg(x + k);
         }
@@ -187,8 +200,7 @@ __global__ void __launch_bounds__(256) line_sum_partial_kernel(
     int64_t o = o0;
     for (; o + U <= o1; o += U) {
         float f[U][V];
-#pragma unroll
-        for (int u = 0; u < U; ++u) load_chunk<E, V>(hi, lo, (size_t)(o + u) * ld + i, f[u]);
+        load_chunks<E, V, U>(hi, lo, (size_t)o * ld + i, (size_t)ld, f);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const Acc xv = (Acc)__ldg(x + o + u);
@@ -197,11 +209,11 @@ __global__ void __launch_bounds__(256) line_sum_partial_kernel(
         }
     }
     for (; o < o1; ++o) {
-        float f[V];
-        load_chunk<E, V>(hi, lo, (size_t)o * ld + i, f);
+        float f[1][V];
+        load_chunks<E, V, 1>(hi, lo, (size_t)o * ld + i, 0, f);
         const Acc xv = (Acc)__ldg(x + o);
 #pragma unroll
-        for (int e = 0; e < V; ++e) a[0][e] += (Acc)f[e] * xv;
+        for (int e = 0; e < V; ++e) a[0][e] += (Acc)f[0][e] * xv;
     }
 #pragma unroll
     for (int e = 0; e < V; ++e) partial[(size_t)c * inner + i + e] = a[0][e] + a[1][e];

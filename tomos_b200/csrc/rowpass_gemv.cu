@@ -14,7 +14,7 @@
 //                     atomics; the reference adds with atomicAdd,
 //                     mv_cuda_kernels.cu:529) into y = alpha sum + beta y.
 // Narrow lines, and lines that do not start on 16-byte boundaries, take the
-// direct pass (rowpass_direct.cuh) both ways instead.
+// direct pass (rowpass_direct.cuh) instead, where it is the better one.
 // FP32 and HALF-tier products accumulate in FP32.  The exact tiers form
 // FP32 products over short runs (a lane's part of a line, or 8 lines of a
 // column) and sum the runs in FP64.  Other shapes take the generic
@@ -79,10 +79,31 @@ size_t rowpass_gemv_scratch_bytes(int64_t outer, int64_t inner) {
     return (size_t)rows * (size_t)qs * sizeof(double);
 }
 
+// Whether the direct pass forms a product of lines it covers.  Sums of very
+// few lines, and the dots of few, are shorter in the generic kernels (gemv.cu;
+// a warp a line for dots), which start faster (times warm in L2):
+//   sums   8 lines of 1000 FP32 3.5 us (direct 5.3), 64 lines 7.0 us (5.1);
+//   dots   3000 lines of 64 aligned FP32 2.1 us (3.6), 10000 3.5 us (3.8);
+//          unaligned: 3000 lines of 65 FP32 2.2 us (4.2), 30000 6.4 us (5.5);
+//          777 at 30000 19.2 us (18.7); exact FP32_16 of 500 at 30000 31 us
+//          (33), at 100000 152 us (105);
+// and so are the dots of 16-bit lines whose chunks leave the 32 lanes' slots
+// half empty: 100000 lines of 257 exact FP32_16 77 us (101), FP16 21 us (23).
+static bool direct_better(const GemvLaunch& L, Elem e, const DirectShape& ds) {
+    if (!L.dot) return L.outer >= 24;
+    if (direct_aligned(e, L.ld, L.hi, L.lo) || (e == Elem::H16 && L.inner > 256)) return L.outer >= 10000;
+    if (L.outer < (ds.c > 1 || (elem_is_exact(e) && ds.lpr > 8) ? 40000 : 24000)) return false;
+    const int64_t nch = (L.inner + 14) / 8;
+    return e == Elem::F32 || e == Elem::H16 || ds.lpr < 32 || 10 * nch >= 7 * 32 * ds.c;
+}
+
 // The product through the direct pass (*used false: scratch too small).
 static tomos_status direct_gemv(const GemvLaunch& L, Elem e, const DirectShape& ds, cudaStream_t st, bool* used) {
     const bool acc64 = elem_is_exact(e);
-    const int grid = direct_grid(L.outer);
+    // sums of narrow lines: 64 lines a CTA at least, which leaves fewer partials
+    // (300 lines of 20 FP32: 4.8 us, with 16 lines a CTA 5.9 us)
+    int grid = direct_grid(L.outer);
+    if (!L.dot && ds.lpr < 32 && grid > (L.outer + 63) / 64) grid = (int)((L.outer + 63) / 64);
     const int64_t qs = (L.inner + 31) / 32 * 32;
     if (!L.dot && (!L.scratch || L.scratch_bytes < (size_t)grid * qs * (acc64 ? 8 : 4))) return TOMOS_OK;
     *used = true;
@@ -119,7 +140,7 @@ tomos_status rowpass_gemv(const GemvLaunch& L, Elem e, cudaStream_t st, bool* us
     const bool acc64 = elem_is_exact(e);
     if (e == Elem::F64 || L.coef || L.skip) return TOMOS_OK;
     const DirectShape ds = direct_shape(e, L.inner, L.ld, L.hi, L.lo);
-    if (ds.lpr > 0) return direct_gemv(L, e, ds, st, used);
+    if (ds.lpr > 0) return direct_better(L, e, ds) ? direct_gemv(L, e, ds, st, used) : TOMOS_OK;
     int nch = 0, g = 1;
     if (!plan_row_lines(e, acc64, L.dot ? kRowDot : kRowAxpy, L.inner, L.ld, L.hi, L.lo, &nch, &g)) return TOMOS_OK;
     const int grid = row_pass_grid(L.outer);

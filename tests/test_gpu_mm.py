@@ -209,7 +209,8 @@ def test_mm_split_k(orc, numeric, tier, beta):
 @pytest.mark.parametrize("numeric", [NT.FP32_16, NT.FP32_BF16, NT.FP16])
 @pytest.mark.parametrize("la,lb", [(L.COL_MAJOR, L.COL_MAJOR), (L.ROW_MAJOR, L.ROW_MAJOR),
                                    (L.ROW_MAJOR, L.COL_MAJOR)])
-@pytest.mark.parametrize("M,N,K,pad", [(1290, 1210, 300, 0), (1400, 2500, 257, 0), (1281, 1283, 1001, 3)])
+@pytest.mark.parametrize("M,N,K,pad", [(1290, 1210, 300, 0), (1400, 2500, 257, 0), (1281, 1283, 1001, 3),
+                                       (13000, 128, 264, 0), (13000, 129, 264, 0), (13001, 5, 257, 0)])
 def test_mm_packed_operands(orc, numeric, la, lb, M, N, K, pad):
     """Products with enough 128 x 128 (or 256) tiles for the packed 16-bit
     kernel: ragged tiles and K stages, lines along K and across it, aligned

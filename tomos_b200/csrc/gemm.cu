@@ -1005,17 +1005,23 @@ __global__ void __launch_bounds__(256) pack_transpose_kernel(const void* src, in
     __shared__ uint16_t tile[64][72];  // [line][k]; 144-byte rows keep 16-byte reads aligned
     const int64_t i0 = (int64_t)blockIdx.x * 64, l0 = (int64_t)blockIdx.y * 64;
     const int c = threadIdx.x & 63, r0 = threadIdx.x >> 6;
+    uint32_t w[16];  // all 16 words are loaded before the first is converted
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-        const int k = r0 + 4 * j;
-        const int64_t i = i0 + c, l = l0 + k;
-        uint32_t b = 0;
+        const int64_t i = i0 + c, l = l0 + r0 + 4 * j;
+        const size_t idx = (size_t)(l * k_stride + i);
+        w[j] = 0u;
         if (i < lines && l < K) {
-            const size_t idx = (size_t)(l * k_stride + i);
-            if constexpr (E == Elem::F32) b = to16<BF>(__ldg(static_cast<const float*>(src) + idx));
-            else b = bits16<E>(__ldg(static_cast<const uint16_t*>(src) + idx));
+            if constexpr (E == Elem::F32) w[j] = __ldg(static_cast<const uint32_t*>(src) + idx);
+            else w[j] = __ldg(static_cast<const uint16_t*>(src) + idx);
         }
-        tile[c][k] = (uint16_t)b;
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        uint32_t b = w[j];
+        if constexpr (E == Elem::F32) b = to16<BF>(u2f(b));
+        else if constexpr (E == Elem::H16) b = half_only_bits_nb(b);
+        tile[c][r0 + 4 * j] = (uint16_t)b;
     }
     __syncthreads();
 #pragma unroll
@@ -1329,11 +1335,17 @@ tomos_status launch_gemm(GemmArgs& g, cudaStream_t st) {
 
 // Columns of a packed product's tiles, or 0 when the unpacked kernels are
 // used: fewer tiles than two thirds of the SMs (those kernels split K), a K
-// too short to repay the packing passes, or planes past 2 GiB of scratch.
+// too short to repay the packing passes, planes past 2 GiB of scratch, or one
+// column of tiles (N <= 128), for which the unpacked kernels read A once and
+// the packing three times over: 100000 x 1000 FP16 by 128 columns 121 to 134 us
+// unpacked, 126 to 162 us packed; by 200, 215 to 238 us and 157 to 193 us.
+// Lines that no vector load fits are packed at any N: 100000 x 300 FP16 by 2
+// columns 85 us unpacked, 47 us packed.
 // 256 columns halve A's re-reads; 128 when their last wave wastes less.
 size_t packed_bytes(const GemmArgs& g);
 int packed_bn(const GemmArgs& g, int mode) {
     if (mode != kPure16 || g.K < 256 || g.K > 65535 * 64 || packed_bytes(g) > ((size_t)2 << 30)) return 0;
+    if (g.N <= 128 && g.a_vec) return 0;
     const int64_t sms = sm_count(), tm = (g.M + kGemmM - 1) / kGemmM;
     const int64_t t256 = tm * ((g.N + 255) / 256), t128 = tm * ((g.N + 127) / 128);
     if (3 * t128 < 2 * sms) return 0;

@@ -296,11 +296,21 @@ __device__ __forceinline__ float word_value(uint32_t h, uint32_t r) {
     else return decode_fp32_bf16_exact(h, r, E == Elem::AB16R);
 }
 
-// The elements at flat indices idx + u step.  HALF-tier control words are
-// rare: all words are loaded first, then one branch decodes them for all U.
+// decode_fp32_16_exact of a word without the control bit.
+__device__ __forceinline__ float decode_fp32_16_plain(uint32_t hh, uint32_t rr) {
+    const uint32_t mag = ((((hh >> 10) & 0x1Fu) + 112u) << 23) + ((hh & 0x3FEu) << 13) + (rr >> 2) - ((rr & 1u) << 14);
+    return u2f(((hh & 0x8000u) << 16) | mag);
+}
+
+// The elements at flat indices idx + u step.  FP32_16 control words are rare:
+// all words are loaded first, then one branch decodes them for all U.
 template <Elem E, int U>
 __device__ __forceinline__ void load_elems(const void* p, const void* q, size_t idx, size_t step, float (&v)[U]) {
-    if constexpr (E == Elem::H16) {
+    if constexpr (U == 1 && E == Elem::H16) {
+        v[0] = half_bits_to_float(half_only_bits(__ldg(static_cast<const uint16_t*>(p) + idx)));
+    } else if constexpr (U == 1 && E == Elem::A16) {
+        v[0] = decode_fp32_16_exact(__ldg(static_cast<const uint16_t*>(p) + idx), __ldg(static_cast<const uint16_t*>(q) + idx));
+    } else if constexpr (E == Elem::H16) {
         uint32_t h[U], any = 0u;
 #pragma unroll
         for (int u = 0; u < U; ++u) h[u] = __ldg(static_cast<const uint16_t*>(p) + idx + u * step);
@@ -312,6 +322,22 @@ __device__ __forceinline__ void load_elems(const void* p, const void* q, size_t 
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) v[u] = half_bits_to_float(h[u]);
+    } else if constexpr (E == Elem::A16) {
+        uint32_t h[U], l[U], any = 0u;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            h[u] = __ldg(static_cast<const uint16_t*>(p) + idx + u * step);
+            l[u] = __ldg(static_cast<const uint16_t*>(q) + idx + u * step);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) any |= h[u];
+        if (any & 1u) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = decode_fp32_16_exact_nb(h[u], l[u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = decode_fp32_16_plain(h[u], l[u]);
+        }
     } else {
 #pragma unroll
         for (int u = 0; u < U; ++u) v[u] = load_elem<E>(p, q, idx + u * step);

@@ -188,8 +188,9 @@ __global__ void __launch_bounds__(256) csr_trans_kernel(CsrPassParams P) {
             if ((uint32_t)cc[t] < n) acc[cc[t]] = fmaf(vv[t], u, acc[cc[t]]);
             const int32_t k0 = __shfl_sync(0xffffffffu, ks0, t), k1 = __shfl_sync(0xffffffffu, ke0, t);
             __syncwarp();
-            for (int32_t k = k0 + 32 + lane; k - lane < k1; k += 32) {  // a row longer than a warp
-                if (k < k1) {
+            if (k0 + 32 < k1) {  // a row longer than a warp (its columns are distinct)
+#pragma unroll 4
+                for (int32_t k = k0 + 32 + lane; k < k1; k += 32) {
                     const int32_t cl = __ldg(P.col_idxs + k);
                     if ((uint32_t)cl < n) acc[cl] = fmaf(load_elem<E>(P.hi, P.lo, k), u, acc[cl]);
                 }
@@ -1039,8 +1040,8 @@ __global__ void csr_colsq_kernel(const void* hi, const void* lo, const int32_t* 
             }
             const int32_t k0 = __shfl_sync(0xffffffffu, ks, q), k1 = __shfl_sync(0xffffffffu, ke, q);
             __syncwarp();
-            for (int32_t k = k0 + 32 + lane; k - lane < k1; k += 32) {  // a row longer than a warp
-                if (k < k1) {
+            if (k0 + 32 < k1) {  // a row longer than a warp (its columns are distinct)
+                for (int32_t k = k0 + 32 + lane; k < k1; k += 32) {
                     const double a = load_elem<E>(hi, lo, k);
                     acc[col_idxs[k]] += a * a;
                 }

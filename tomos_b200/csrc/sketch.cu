@@ -358,7 +358,9 @@ __global__ void __launch_bounds__(kCsThreads) cs_rows_kernel(CsRowsArgs a) {
 }
 
 // Rows at any alignment: as cs_rows_kernel, a thread owning kCsCols columns
-// blockDim.x apart and reading them one element at a time (coalesced).
+// blockDim.x apart and reading them one element at a time (coalesced).  A
+// batch's words are loaded before the first is decoded, which would wait for
+// each: 50000 x 1001 FP16 into 1064 buckets 159 us decoded at the load.
 constexpr int kCsCols = 4;
 
 template <Elem E>
@@ -376,8 +378,8 @@ __global__ void __launch_bounds__(kCsThreads) cs_rows_any_kernel(CsRowsArgs a) {
 #pragma unroll
     for (int u = 0; u < D; ++u) nid[u] = u < len ? __ldg(ids + u) : 0u;
     for (int32_t q = 0; q < len; q += D) {
-        uint32_t id[D];
-        float v[D][kCsCols];
+        constexpr bool TWO = CsElem<E>::PLANES == 2;
+        uint32_t id[D], h[D][kCsCols], l[TWO ? D : 1][kCsCols];
 #pragma unroll
         for (int u = 0; u < D; ++u) {
             id[u] = nid[u];
@@ -385,7 +387,11 @@ __global__ void __launch_bounds__(kCsThreads) cs_rows_any_kernel(CsRowsArgs a) {
 #pragma unroll
             for (int k = 0; k < kCsCols; ++k) {
                 const int64_t j = j0 + (int64_t)k * blockDim.x;
-                v[u][k] = (q + u < len && j < a.n) ? load_elem<E>(a.hi, a.lo, base + j) : 0.0f;
+                // an element that is not summed or stored: the first of A
+                const size_t at = q + u < len && j < a.n ? base + j : 0;
+                if constexpr (E == Elem::F32) h[u][k] = __ldg(static_cast<const uint32_t*>(a.hi) + at);
+                else h[u][k] = __ldg(static_cast<const uint16_t*>(a.hi) + at);
+                if constexpr (TWO) l[u][k] = __ldg(static_cast<const uint16_t*>(a.lo) + at);
             }
         }
 #pragma unroll
@@ -396,8 +402,9 @@ __global__ void __launch_bounds__(kCsThreads) cs_rows_any_kernel(CsRowsArgs a) {
                 const float sg = (id[u] & kCsNeg) ? -1.0f : 1.0f;
 #pragma unroll
                 for (int k = 0; k < kCsCols; ++k) {
-                    acc[k] = fmaf(sg, v[u][k], acc[k]);
-                    csq[k] = fmaf(v[u][k], v[u][k], csq[k]);
+                    const float v = word_value<E>(h[u][k], TWO ? l[TWO ? u : 0][k] : 0u);
+                    acc[k] = fmaf(sg, v, acc[k]);
+                    csq[k] = fmaf(v, v, csq[k]);
                 }
             }
         }
@@ -572,10 +579,30 @@ __global__ void __launch_bounds__(256) cs_cols_kernel(const void* hi, const void
     for (int64_t b = w; b < s; b += 8) {
         const int32_t o0 = offsets[b], o1 = offsets[b + 1];
         double acc = 0.0;
-        for (int32_t q = o0 + lane; q < o1; q += 32) {
+        int32_t q = o0 + lane;
+        if (o1 - o0 > 32) {  // four of a long bucket's rows in flight
+            for (; q + 96 < o1; q += 128) {
+                uint32_t r[4];
+                float v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) r[u] = perm[q + 32 * u];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = load_elem<E>(hi, lo, cbase + (r[u] & ~kCsNeg));
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const double a = (double)u2f(__float_as_uint(v[u]) ^ (r[u] & kCsNeg));
+                    acc += a;
+                    f2 += a * a;
+                }
+            }
+        }
+#pragma unroll 1
+        for (; q < o1; q += 32) {
             const uint32_t r = perm[q];
-            const double a = (double)load_elem<E>(hi, lo, cbase + (r & ~kCsNeg));
-            acc += (r & kCsNeg) ? -a : a;
+            float v[1];
+            load_elems<E, 1>(hi, lo, cbase + (r & ~kCsNeg), 0, v);
+            const double a = (double)u2f(__float_as_uint(v[0]) ^ (r & kCsNeg));  // the row's sign on the value
+            acc += a;
             f2 += a * a;
         }
         acc = warp_sum(acc);

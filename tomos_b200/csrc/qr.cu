@@ -777,7 +777,7 @@ __global__ void qr_mirror_lower_kernel(double* D, int64_t ldd, int64_t n) {
 // buffer P of pcap doubles, K is split over CTAs (partials summed in
 // order) by the count that wastes the least of the last wave of resident
 // CTAs (two per SM), each split keeping at least 16 k-stages and all
-// partials fitting P.  sub: D -= op(A) B.  upper (a symmetric product,
+// partials fitting P; want > 0 sets the count.  sub: D -= op(A) B.  upper (a symmetric product,
 // op(A) = B^T, square D): only the tiles that reach the diagonal or above
 // are formed, and the lower triangle is then copied from the upper
 // (qr_mirror_lower_kernel), exactly symmetric.
@@ -785,7 +785,7 @@ template <bool KMAJOR>
 static tomos_status qr_gemm(const double* A, int64_t lda, const double* B, int64_t ldb, double* D,
                             int64_t ldd, int64_t M, int64_t N, int64_t K, double alpha, double beta,
                             double* P, size_t pcap, cudaStream_t st, int sub = 0, bool upper = false,
-                            int run = 0) {
+                            int64_t want = 0) {
     if (M <= 0 || N <= 0) return TOMOS_OK;
     const int64_t tm = (M + kGbm - 1) / kGbm, tn = (N + kGbn - 1) / kGbn;
     int64_t active = tm * tn;
@@ -796,7 +796,9 @@ static tomos_status qr_gemm(const double* A, int64_t lda, const double* B, int64
                 if (i * kGbm <= j * kGbn + kGbn - 1) ++active;
     }
     int64_t splits = 1;
-    if (P && run == 0) {
+    if (want > 0) {
+        splits = want;
+    } else if (P) {
         const int64_t slots = 2 * (int64_t)sm_count(), tiles = active;
         int64_t kmax = K / (16 * kGbk);
         if (kmax > kGmaxSplits) kmax = kGmaxSplits;
@@ -833,7 +835,6 @@ static tomos_status qr_gemm(const double* A, int64_t lda, const double* B, int64
     g.beta = beta;
     g.sub = sub;
     g.upper = upper ? 1 : 0;
-    g.run = run;
     TOMOS_CUDA_TRY(cudaFuncSetAttribute(qr_gemm_kernel<KMAJOR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)kGemmSmem));
     qr_gemm_kernel<KMAJOR><<<dim3((unsigned)tm, (unsigned)tn, (unsigned)splits), 256, kGemmSmem, st>>>(g);
@@ -967,18 +968,18 @@ constexpr double kQrWideMaxKappa = 1e6;
 // has 1.15 and one of 2 n rows 1.41; below 1.8 n rows none is tried) keeps the
 // wide path.  A refused sketch pays the Gram and the Cholesky up to the block
 // column where the sum of 1 / u_jj^2 passes the bound, before the panel path:
-// 13.7 to 14.6 ms at 8400 x 2100, 12.6 ms without (14.9 ms with the inverse);
-// 27.3 to 28.9 ms at 12000 x 3000 (24.1 ms).  The wide path's Gram is summed
-// there in runs of kQrWideRun rows (one chain over all rows was most of its
-// error), its diagonal in wide_diag_kernel's short chains.  With
-// E = R^-T (SA^T SA - R^T R) R^-1 from the exact Gram, ||E||_F is 3.8e-14 at
-// 12000 x 3000 (panel path 9.8e-14; 1.7e-13 in one chain), 3.1e-14 at 8400 x
-// 2100 (7.1e-14) and 5.5e-14 at 4300 x 2100 (1.04e-13).  The panel path's
+// 13.6 to 14.4 ms at 8400 x 2100, 12.6 ms without (14.9 ms with the inverse);
+// 26.7 to 28.2 ms at 12000 x 3000 (24.1 ms).  The wide path's Gram is summed
+// there over kQrWideSplits parts of the rows (one chain over all of them was
+// most of its error), its diagonal in wide_diag_kernel's short chains.  With
+// E = R^-T (SA^T SA - R^T R) R^-1 from the exact Gram, ||E||_F is 7.1e-14 at
+// 12000 x 3000 (panel path 9.8e-14; 1.7e-13 in one chain), 5.1e-14 at 8400 x
+// 2100 (7.1e-14) and 7.5e-14 at 4300 x 2100 (1.04e-13).  The panel path's
 // panels and blocks took 24 ms at 12000 x 3000, most of it panel latency; the
-// wide path takes 12.5 ms with LAPACK's signs and 7.2 ms with rows of any sign.
+// wide path takes 12.4 ms with LAPACK's signs and 6.9 ms with rows of any sign.
 constexpr int64_t kQrWidePlainN = 2048;
 constexpr double kQrWideRms = 1.5;
-constexpr int kQrWideRun = 512;
+constexpr int kQrWideSplits = 4;  // of the Gram's rows past kQrWidePlainN, in G, Ur, X and P
 constexpr double kQrWideFloor = 1e-10;
 
 struct WideScratch {
@@ -989,7 +990,7 @@ struct WideScratch {
     double* sgn;   // n: S
     double* Xd;    // 2 x 2 x 32 x 32: a diagonal block's inverse factors (by block parity)
     double* pan;   // 2 x 32 x n: LU panels
-    double* kap;   // [0] ||U^-1||_F^2, [1] its diagonal's part
+    double* kap;   // ||U^-1||_F^2
     double* Tb;    // trtri level products
     double* P;     // GEMM split-K partials
     size_t pcap;
@@ -1008,9 +1009,13 @@ static WideScratch wide_layout(void* base, int64_t n) {
         return r;
     };
     const size_t nn = n > 0 ? (size_t)n : 1;
-    w.G = reinterpret_cast<double*>(take(sizeof(double) * nn * nn));
-    w.Ur = reinterpret_cast<double*>(take(sizeof(double) * nn * nn));
-    w.X = reinterpret_cast<double*>(take(sizeof(double) * nn * nn));
+    // G, Ur, X and P one behind the other: the Gram's partials use all four
+    const size_t planes = n > kQrWidePlainN ? kQrWideSplits : 3 + 4;
+    w.G = reinterpret_cast<double*>(take(sizeof(double) * planes * nn * nn));
+    w.Ur = w.G + nn * nn;
+    w.X = w.Ur + nn * nn;
+    w.P = w.X + nn * nn;
+    w.pcap = (planes - 3) * nn * nn;
     w.d = reinterpret_cast<double*>(take(sizeof(double) * nn));
     w.sgn = reinterpret_cast<double*>(take(sizeof(double) * nn));
     w.Xd = reinterpret_cast<double*>(take(sizeof(double) * 4 * kHB * kHB));
@@ -1022,8 +1027,6 @@ static WideScratch wide_layout(void* base, int64_t n) {
         if (pairs * b * b > tb) tb = pairs * b * b;
     }
     w.Tb = reinterpret_cast<double*>(take(sizeof(double) * tb));
-    w.pcap = (n > kQrWidePlainN ? 1 : 4) * nn * nn;  // large products fill the GPU unsplit
-    w.P = reinterpret_cast<double*>(take(sizeof(double) * w.pcap));
     w.flag = reinterpret_cast<int*>(take(sizeof(int) * 4));
     w.gs = reinterpret_cast<GridSync*>(take(2 * sizeof(GridSync)));
     w.bytes = off;
@@ -1041,7 +1044,7 @@ __global__ void wide_colnorm_kernel(const double* G, int64_t n, double* d, int* 
 }
 
 // The diagonal of G = SA^T SA anew, a block a column: squares all add up, so
-// even a chain of kQrWideRun rows leaves an error of several units.  Short
+// even a chain of a few thousand leaves an error of several units.  Short
 // chains a thread, then a tree: the largest entry of E 1.6e-15 at 12000 x 3000
 // (1.9e-15 without; the panel path 1.4e-15), for 70 us.
 __global__ void __launch_bounds__(256) wide_diag_kernel(const double* SA, int64_t ld, int64_t k, int64_t n, double* G) {
@@ -1133,8 +1136,7 @@ struct FactArgs {
     int64_t keep;   // LU: the column dlarfg leaves as the identity, or -1
     double floor;
     int* fail;      // [0] set when a pivot or the sum below ends the Cholesky, [1] 1 + that block column
-    double* inv2;   // Cholesky: sum of 1 / u_jj^2 so far (at most ||U^-1||_F^2)
-    double inv2_max;
+    double inv2_max;  // Cholesky: bound on the sum of 1 / u_jj^2
     GridSync* gs;
 };
 
@@ -1214,13 +1216,14 @@ __device__ void fact_diag(const FactArgs& a, int64_t p, double* sm, bool in_smem
         }
     double* xd = a.Xd + (size_t)(p & 1) * 2 * kHB * kHB;
     __shared__ double dinv[kHB];
+    __shared__ double inv2;  // sum of 1 / u_jj^2 so far (at most ||U^-1||_F^2)
     if (a.mode == 0) {
         const bool ok = cta_chol_inv(B, R, X, a.floor, &okf);
         if (t < 32) {
             const double s = warp_sum(t < nb ? X[t][t] * X[t][t] : 0.0);
             if (t == 0) {
-                const double sum = p == 0 ? s : *a.inv2 + s;
-                *a.inv2 = sum;
+                const double sum = p == 0 ? s : inv2 + s;
+                inv2 = sum;
                 if (!ok || !(sum <= a.inv2_max)) {  // refused: every CTA leaves at block column p
                     atomicExch(a.fail, 1);
                     if (a.fail[1] == 0) atomicExch(a.fail + 1, (int)p + 1);
@@ -1488,7 +1491,7 @@ __global__ void __launch_bounds__(kQrThreads, 1) fact_kernel(FactArgs a) {
     if (blockIdx.x == 0) fact_diag(a, 0, fsm, false);
     if (!grid_sync(a.gs, gen, &sflag)) return;
     for (int64_t p = 0; p + 1 < np; ++p) {
-        if (a.mode == 0) {
+        if (a.mode == 0 && p % 8 == 7) {  // (a load every CTA waits for)
             // CTA 0 writes p + 2 at the earliest while others read it here
             const int stop = __ldcg(a.fail + 1);
             if (stop != 0 && stop - 1 <= p) return;
@@ -1545,8 +1548,9 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     *done = false;
     TOMOS_CUDA_TRY(cudaMemsetAsync(w.flag, 0, sizeof(int) * 4, st));
     // the Gram S^T S: its upper triangle, mirrored
-    tomos_status s = qr_gemm<true>(SA, ld, SA, ld, w.G, n, n, n, k, 1.0, 0.0, w.P, w.pcap, st, 0, true,
-                                 n > kQrWidePlainN ? kQrWideRun / kGbk : 0);
+    const bool plain = n <= kQrWidePlainN;
+    tomos_status s = qr_gemm<true>(SA, ld, SA, ld, w.G, n, n, n, k, 1.0, 0.0, plain ? w.P : w.G, w.pcap, st, 0, true,
+                                   plain ? 0 : kQrWideSplits);
     if (s) return s;
     const unsigned eb = (unsigned)((n * n + 255) / 256 < 4096 ? (n * n + 255) / 256 : 4096);
     if (n > kQrWidePlainN) {
@@ -1568,7 +1572,6 @@ static tomos_status qr_wide(int64_t k, int64_t n, double* SA, int64_t ld, double
     fa.keep = -1;
     fa.floor = kQrWideFloor;
     fa.fail = w.flag;
-    fa.inv2 = w.kap + 1;
     const double kmax = n > kQrWidePlainN ? kQrWideRms * (double)n : kQrWideMaxKappa;
     fa.inv2_max = kmax * kmax / (double)n;  // ||U^-1||_F^2 where kappa_F(U) = kmax
     fa.gs = w.gs;

@@ -90,7 +90,6 @@ struct GemmArgs {
     double alpha, beta;
     int sub;
     int upper;  // skip the tiles wholly below the diagonal (a symmetric product's other half)
-    int run;    // > 0: D = op(A) B in runs of this many k-steps, each summed from zero and added to D
 };
 
 template <bool KMAJOR>
@@ -176,26 +175,8 @@ __global__ void __launch_bounds__(256, 2) qr_gemm_kernel(GemmArgs g) {
 #pragma unroll
                 for (int in = 0; in < 4; ++in) g_dmma1688(acc[im][in], a[im], b[in]);
         }
-        if (g.run > 0 && ((i + 1) % g.run == 0 || i + 1 == nk)) {
-            const bool first = i < g.run;
-#pragma unroll
-            for (int im = 0; im < 2; ++im)
-#pragma unroll
-                for (int in = 0; in < 4; ++in)
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int64_t row = m0 + wm + im * 16 + gq + 8 * (u >> 1);
-                        const int64_t col = n0 + wn + in * 8 + 2 * qq + (u & 1);
-                        if (row < g.M && col < g.N) {
-                            double* d = g.D + row + col * g.ldd;
-                            *d = first ? acc[im][in][u] : *d + acc[im][in][u];
-                        }
-                        acc[im][in][u] = 0.0;
-                    }
-        }
     }
     g_cp_async_wait<0>();
-    if (g.run > 0) return;
     const bool split = gridDim.z > 1;
 #pragma unroll
     for (int im = 0; im < 2; ++im)
@@ -218,9 +199,10 @@ __global__ void __launch_bounds__(256, 2) qr_gemm_kernel(GemmArgs g) {
             }
 }
 
-// D = alpha * sum_z P[z] + beta * D, the splits summed in order.
-__global__ void qr_gemm_reduce_kernel(const double* __restrict__ P, int splits, int64_t M, int64_t N,
-                                      double alpha, double beta, double* __restrict__ D, int64_t ldd) {
+// D = alpha * sum_z P[z] + beta * D, the splits summed in order.  D may be
+// P[0] (ldd = M): a thread reads an entry's partials before it writes the entry.
+__global__ void qr_gemm_reduce_kernel(const double* P, int splits, int64_t M, int64_t N,
+                                      double alpha, double beta, double* D, int64_t ldd) {
     const int64_t total = M * N;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (int64_t)gridDim.x * blockDim.x) {

@@ -170,12 +170,14 @@ fused_direct_kernel(DirectParams T) {
     float uin[K];
     auto load = [&](int b) {  // the rows of the iteration whose first row is r0 + b
         const int64_t first = (r0 + b) * P.ld - shift;
-        int64_t last = r0 + b + (GR - 1) * rg + (U - 1) * ru;
-        if (last >= P.m) last = P.m - 1;  // rows past the CTA's are not read
+        int64_t last = r0 + b + (int64_t)(GR - 1) * rg + (int64_t)(U - 1) * ru;
+        // narrow rows, many a batch: those past A are not read, and aligned
+        // ones never reach past it
+        if (C == 1 && last >= P.m) last = P.m - 1;
         last = last * P.ld - shift + (int64_t)nch * VEC;
         // one branch for the whole batch: inside it the loads are predicated
         // only, so all of them issue before the first is waited for
-        if (T.aligned || (first >= 0 && last <= lim)) {
+        if ((C == 1 && T.aligned) || (first >= 0 && last <= lim)) {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int i = b + grp * rg + u * ru;
@@ -199,17 +201,20 @@ fused_direct_kernel(DirectParams T) {
 #pragma unroll
                 for (int c = 0; c < C; ++c) {
                     const int ch = c * LPR + sub;
+                    const bool in = i < rows && ch < nch;
                     const int64_t at = idx + (int64_t)ch * VEC;
-                    h[u][c] = make_uint4(0u, 0u, 0u, 0u);
-                    if constexpr (D::TWO) l[u][c] = make_uint4(0u, 0u, 0u, 0u);
-                    if (i >= rows || ch >= nch) continue;
-                    if (at >= 0 && at + VEC <= lim) {
+                    if (C == 1 && in && at >= 0 && at + VEC <= lim) {
                         h[u][c] = D::chunk(P.hi, at);
                         if constexpr (D::TWO) l[u][c] = D::chunk(P.lo, at);
-                    } else {
-                        h[u][c] = D::slow(P.hi, at, 0, lim);
-                        if constexpr (D::TWO) l[u][c] = D::slow(P.lo, at, 0, lim);
+                        continue;
                     }
+                    if (C == 1 && !in) {
+                        h[u][c] = make_uint4(0u, 0u, 0u, 0u);
+                        if constexpr (D::TWO) l[u][c] = make_uint4(0u, 0u, 0u, 0u);
+                        continue;
+                    }
+                    h[u][c] = D::slow(P.hi, at, 0, in ? lim : 0);
+                    if constexpr (D::TWO) l[u][c] = D::slow(P.lo, at, 0, in ? lim : 0);
                 }
             }
         }

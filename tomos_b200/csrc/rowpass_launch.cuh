@@ -86,7 +86,7 @@ inline bool plan_row_lines(Elem e, bool acc64, int mode, int64_t inner, int64_t 
     if (elem_two_planes(e) && reinterpret_cast<uintptr_t>(lo) % 16 != 0) return false;
     int nch = 0, g = 1;
     const int nmax = fused_nch_max(e, acc64, mode);
-    for (int c : {1, 2, 4, 8}) {
+    for (int c : {2, 4, 8}) {  // one chunk a lane: the direct pass's (direct_shape)
         if (c > nmax) break;
         if ((int64_t)32 * c * vec >= inner) {
             nch = c;
@@ -121,7 +121,7 @@ inline int row_pass_grid(int64_t outer) {
     return grid < 1 ? 1 : (int)grid;
 }
 
-// (nch, g) pairs with an instantiation: one warp per row with 1..NCHMAX
+// (nch, g) pairs with an instantiation: one warp per row with 2..NCHMAX
 // chunks per lane, or G warps per row (fused_g_list) at NCHMAX.
 template <Elem E, bool ACC64, int MODE>
 inline tomos_status launch_fused_e(const FusedParams& P, int* err, int nch, int g, int grid,
@@ -129,7 +129,6 @@ inline tomos_status launch_fused_e(const FusedParams& P, int* err, int nch, int 
     constexpr int NMAX = RowNchMax<E, ACC64, MODE>::value;
     if (g == 1) {
         switch (nch) {
-            case 1: return launch_fused_t<E, 1, 1, ACC64, MODE>(P, err, grid, st, qpart64);
             case 2: return launch_fused_t<E, 2, 1, ACC64, MODE>(P, err, grid, st, qpart64);
             case 4:
                 if constexpr (NMAX >= 4) return launch_fused_t<E, 4, 1, ACC64, MODE>(P, err, grid, st, qpart64);

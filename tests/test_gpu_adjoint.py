@@ -210,7 +210,10 @@ def test_batched_solves_match_single(m, n, K, pad):
                 assert not X[:, k].any() and reps[k]["converged"] == 1
                 continue
             assert reps[k]["converged"] == rep["converged"], (k, reps[k], rep)
-            assert abs(reps[k]["iterations"] - rep["iterations"]) <= (1 if tol > 1e-7 else 90)
+            if tol > 1e-7:
+                assert abs(reps[k]["iterations"] - rep["iterations"]) <= 1
+            else:  # every cycle runs its course: the residual's error is that of an FP32 x
+                assert reps[k]["backward_error"] <= 2 * rep["backward_error"]
             # a backward error of 1e-6 with ||A D^-1||_F = sqrt(n): A (x - x*)
             # is below 1e-6 (sqrt(n) ||D x|| + ||b||), and the smallest
             # singular value of A D^-1 (Gaussian) near 1 - sqrt(n / m)

@@ -412,3 +412,11 @@ def test_nside_at_its_sizes(n):
     # value of A D^-1 (Gaussian) is near 1 - sqrt(n / m)
     bound = 1e-6 * (np.sqrt(n) + 2) / (1 - np.sqrt(n / m))
     assert np.linalg.norm(x.cpu().numpy() - ref) / np.linalg.norm(ref) < bound
+    # with a residual, cycles of 25 iterations that each run their course (the
+    # preconditioned error halves a step): x to a few units of its FP32 rounding
+    # and of the FP32 vectors that the last cycle's small step is made of
+    b1 = (b0 + 1e-2 * np.sqrt(n) * rng.standard_normal(m)).astype(np.float32)
+    x, rep, _ = tb.sketch_lsqr(to_dense(A0, L.ROW_MAJOR), cuda(b1), 4 * n, max_iters=25)
+    ref = np.linalg.lstsq(A0.astype(np.float64), b1.astype(np.float64), rcond=None)[0]
+    err = np.linalg.norm(x.cpu().numpy() - ref) / np.linalg.norm(ref)
+    assert err < 1e-6

@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(32) csc_scatter_kernel(const int32_t* __restri
     }
 }
 
-// ut_i = cp (A p)_i + cu u_i for every row (u_out, when write_u) and
+// ut_i = cp (A p)_i + cu u_i for every row (u_out) and
 // ||ut||^2 per CTA (sspart, when set).  2^lg lanes per row; a warp holds
 // two rounds of 32 >> lg rows.  Each lane sums its entries in order, then
 // the group sums by a fixed butterfly.

@@ -35,8 +35,9 @@ namespace {
 // HBM at 200000 x 500; a pass takes 170 us, bound by the phases' latencies.
 // (Sixteen warps of four columns a lane: 220 us.  Split-TF32 matrix
 // instructions: 150 us, and twice the iterations for want of precision.)
-// Sums in FP32 over a lane's columns and a run's rows, FP64 beyond, products
-// and ut as in the one-column pass.
+// A dot's sums are FP32 over a lane's columns and the warp's lanes, a column's
+// FP32 over a run's rows; FP64 beyond, products and ut as in the one-column
+// pass.
 constexpr int kMultiThreads = 256;
 constexpr int kMultiRows = 32;
 constexpr int kMultiMaxN = 512;

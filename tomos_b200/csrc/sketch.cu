@@ -6,7 +6,8 @@
 // row splitmix64(i ^ bucket_seed) mod s of SA.  Integer hashing is
 // bit-exact with the reference.  Unlike the reference (atomicAdd scatter,
 // order-dependent float sums), every bucket here is summed by one owner in
-// increasing row order, in FP64, so SA is deterministic:
+// a fixed order, so SA is deterministic: row-major matrices in FP32, as the
+// reference's sums, column-major and CSR ones in FP64.
 //   1. per row segment: hash, and the segment's count of every bucket
 //   2. exclusive scans: over the segments of a bucket, then over buckets
 //   3. each segment places its rows in order: a stable counting sort, so a

@@ -5,12 +5,14 @@
 // cudaFree, 1.1 to 2.8 ms for 4 KB of pinned memory and 0.4 ms to free it,
 // 4 to 8 ms of a 200000 x 500 call of 20.  So blocks that workspaces give
 // back are kept for later ones: at most kKeepBytes of device memory and
-// kKeepHost pinned blocks a process, released when an allocation fails.
+// kKeepHost pinned blocks a process; the device memory is released when an
+// allocation fails.
 //
-// A workspace's memory is used on its own stream only, which its owner waits
-// for before a block comes back (release_memory, lsqr.cuh), so the next one
-// to be given it finds it idle; not by a wait for the device, which another
-// thread's stream capture forbids.  One lock guards the lists; no block is in
+// A workspace's memory is used on its own stream, and by the blocking copy of
+// a solve's residual history, which is over when it returns.  Its owner waits
+// for that stream before a block comes back (release_memory, lsqr.cuh), so
+// the next one to be given it finds it idle; not by a wait for the device,
+// which another thread's stream capture forbids.  One lock guards the lists; no block is in
 // two hands.
 #include <mutex>
 #include <unordered_map>
